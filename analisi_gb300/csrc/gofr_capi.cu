@@ -645,6 +645,27 @@ Bound error_bound_cells_tric(const TrajDev &t, const CellwGeom &g)
     return b;
 }
 
+// Component bound of the warp-streamed kernel for the pairs its bin map can
+// place (computed |dx_k| <= R, R = rmax + 2 dr): as error_bound_cells and
+// error_bound_cells_tric, but the neighbour moved to its image lies within R
+// of the first atom (|b| <= A + R, so its rounding is d4 = u (A + R)), and the
+// rounding of the difference itself, u |dx_k|, is counted by radial_margin.
+Bound radial_bound_cells(const TrajDev &t, const CellwGeom &g, double R)
+{
+    Bound b{};
+    const double u = std::ldexp(1.0, -24), v = std::ldexp(1.0, -53);
+    const CellSlop cs = cell_slop(t);
+    for (int k = 0; k < 3; ++k) {
+        const double d3 = (u + 2.0 * v) * cs.Mw[k];
+        const double A = cs.Mw[k] * (1.0 + 2.0 * u) + d3;
+        const double d4 = u * (A + R) * (1.0 + 2.0 * u);
+        b.e[k] = (g.eT[k] + 2.0 * cs.ew[k] + 2.0 * d3 + d4 + cs.eref[k]) *
+                 (1.0 + std::ldexp(1.0, -20));
+    }
+    b.enorm = std::sqrt(b.e[0] * b.e[0] + b.e[1] * b.e[1] + b.e[2] * b.e[2]);
+    return b;
+}
+
 inline double Efun(const Bound &b, double s)
 {
     if (s < 0) s = 0;
@@ -671,6 +692,63 @@ void certify(const Bound &b, const double *th, unsigned nbin, Windows &w)
     w.hi_f = f_up(th[nbin] + Efun(b, th[nbin]));
     w.lo_f = th[0] <= 0.0 ? -INFINITY : f_down(th[0] - Efun(b, th[0]));
     w.E_rmax = Efun(b, th[nbin]);
+}
+
+// Constants of the kernels that bin a pair where they find it (RadialMap) for
+// the component bound b, the frames' own bound b1 (the atoms' pairs with
+// themselves) and the exact thresholds th.
+//
+// The kernel's q' = fma(fl(d2 inv_dr), rs, q_off), rs = rsqrt.approx.ftz(d2), d2 the
+// FP32 sum, stands for Q - 1/2, Q = (sqrt(d2_ref) - rmin) / dr.  With u = 2^-24 and
+// for r up to R = rmax + 2 dr (a pair further out is further from every bin than
+// its error):
+//   |sqrt(d2) - sqrt(d2_ref)| <= |e| + R u (1 + 1.5)   component errors e_k + u |x_k|; the
+//       three roundings of the sum (3 u of d2)
+//   |q' - (Q - 1/2)| <= that / dr + R / dr u (2.15 + 1 + 1)   rsqrt's relative 2^-22.9; inv_dr
+//       and the product rounded; + u |q_off| + u (R / dr + 1)   q_off's and the FMA's rounding
+// and the reference's bin changes at th[b], which lies off the real edge by the
+// rounding of its FP32 quotient: `quirk`, measured over every bin.  A pair whose
+// q' is further than the sum (with R u / dr and 0.1 % of slack) from a bin edge is
+// in the bin it seems to be in.
+double radial_margin(const Bound &b, const BinMap &bm, const double *th, unsigned b0)
+{
+    const double u = std::ldexp(1.0, -24);
+    const double R = bm.rmax + 2.0 * bm.dr, q_off = std::fabs(bm.rmin / bm.dr + 0.5);
+    const double d0 = (b.enorm + 2.5 * u * R) / bm.dr + 5.15 * u * R / bm.dr + u * q_off +
+                      u * (R / bm.dr + 1.0);
+    double quirk = 0.0;
+    for (unsigned k = b0; k <= bm.nbin; ++k)
+        quirk = std::max(quirk, std::fabs((std::sqrt(th[k]) - bm.rmin) / bm.dr - (double)k));
+    return (d0 + quirk) * 1.001 + 1e-9;
+}
+
+RadialMap radial_map(const TrajDev &t, const Bound &b, const Bound &b1, const gofr_params &p,
+                     const std::vector<double> &th)
+{
+    RadialMap m{};
+    const BinMap bm(p.rmin, p.rmax, p.nbin);
+    m.inv_dr = (float)(1.0 / bm.dr);
+    m.q_off = (float)(-bm.rmin / bm.dr - 0.5);
+    m.mode = p.rmin > 0.0 ? 1 : (p.rmin < 0.0 ? 2 : 0);
+    // rmin < 0: the reference counts from |rmin| on, inside bin `edge`, whose
+    // pairs and those of the bin before it are never certain
+    double edge = 0.0;
+    if (m.mode == 2) edge = std::floor((std::sqrt(th[0]) - bm.rmin) / bm.dr);
+    const unsigned b0 = m.mode == 2 ? (unsigned)std::min(edge + 1.0, (double)p.nbin) : 0u;
+    const double md = radial_margin(b, bm, th.data(), b0),
+                 md1 = radial_margin(b1, bm, th.data(), b0);
+    // a margin of a quarter of a bin or more: every pair in the window is
+    // recomputed, the window widened by the margin
+    m.lim = md < 0.25 ? f_down(0.5 - md) : -1.0f;
+    m.lim_self = md1 < 0.25 ? f_down(0.5 - md1) : -1.0f;
+    const double wide = md < 0.25 ? 0.0 : std::min(std::ceil(md), 1048576.0);
+    const double magic = 12582912.0;
+    m.t_end = (float)(magic + p.nbin);
+    m.t_hi = (float)(magic + p.nbin + wide);
+    m.t_lo = (float)(magic + (m.mode == 2 ? edge - 1.0 : (m.mode == 1 ? -1.0 : 0.0)) - wide);
+    m.t_ok = (float)(magic + edge + 1.0);
+    m.self_max = f_down(0.25 * std::min(t.bs.Lmin[0], std::min(t.bs.Lmin[1], t.bs.Lmin[2])));
+    return m;
 }
 
 struct RunShape {
@@ -873,7 +951,7 @@ struct Plan {
     double cell_fraction = 1.0;  // neighbourhood cells / all cells
     double cell_time = 1e300;    // modelled time / the all-pairs kernel's
     bool cellw = false;          // the warp-streamed form of the cell-list kernel
-    int wblk[3] = {1, 1, 1}, nw[3] = {1, 1, 1}, parts = 1;  // its warp blocks
+    int wblk[3] = {1, 1, 1}, nw[3] = {1, 1, 1};  // its warp blocks
     int cta_warps = 8, hcopy = 1;  // its CTA size and histogram privatisation depth
     CellwGeom geom;                // its neighbourhood tables and image vectors
     bool wrapcheck = false;
@@ -882,6 +960,15 @@ struct Plan {
     Bound b{};
     std::vector<double> th;
 };
+
+// The bin map of the plan's kernel (FP32 kinds).
+RadialMap plan_radial_map(const TrajDev &t, const gofr_params &p, const Plan &pl)
+{
+    const BinMap bm(p.rmin, p.rmax, p.nbin);
+    const Bound b1 = error_bound(t);
+    return radial_map(t, pl.cellw ? radial_bound_cells(t, pl.geom, bm.rmax + 2.0 * bm.dr) : b1, b1,
+                      p, pl.th);
+}
 
 // One cell-list configuration: cells of edge >= rmax (1 + 1e-6) / reach, so
 // two atoms at minimum-image distance <= rmax are at most `reach` cells apart
@@ -1090,11 +1177,7 @@ std::vector<CellwCand> cellw_candidates(const TrajDev &t, const gofr_params &p)
                     const double blocks = (double)((nc[0] + wx - 1) / wx) *
                                           ((nc[1] + wy - 1) / wy) * ((nc[2] + wz - 1) / wz);
                     const double chr = cellw_chunk_records();
-                    // a row wrapping the box is two pieces
-                    const double pieces_per_row = 1.0 + (double)(wx + g.nx_span) / nc[0];
-                    const double per_chunk =
-                        std::min(chr, cellw_chunk_pieces() * row_atoms / pieces_per_row);
-                    const double chunks = std::ceil(nbhd / per_chunk) + 0.5;
+                    const double chunks = std::ceil(nbhd / chr) + 0.5;
                     const double batches =
                         std::ceil(std::max(atoms + 2.0 * std::sqrt(atoms), 1.0) /
                                   cellw_batch_atoms());
@@ -1162,11 +1245,6 @@ bool make_cellw_plan(const TrajDev &t, const gofr_params &p, Plan &pl, const Cel
         q.wblk[k] = c.w[k];
         q.nw[k] = (c.nc[k] + c.w[k] - 1) / c.w[k];
     }
-    // parts of the warp blocks per (lag, origin): items of fewer than 2^31
-    // all-pairs-equivalent pairs (the kernel checks the evaluated ones)
-    const double n2 = (double)t.N * (double)t.N;
-    q.parts = (int)std::max(1.0, std::ceil(n2 / 2147483648.0));
-    q.parts = std::min(q.parts, q.nw[0] * q.nw[1] * q.nw[2]);
     // one CTA of 16 warps per SM where its shared memory fits (measured faster
     // on the 16k-atom workload, within 2 % of two CTAs of 8 on the 131k-atom
     // one), else two CTAs of 8; one histogram copy
@@ -1257,6 +1335,29 @@ int make_plan(gofr_ctx *ctx, const TrajDev &t, const gofr_params &p, Plan &pl,
     return GOFR_OK;
 }
 
+// The plan for frames in one box with coordinates within [coord_min, coord_max]
+// (host state only: the planner touches no device), t and pl empty on entry.
+int host_plan(const double *box, int box_kind, const double *coord_min, const double *coord_max,
+              size_t natoms, unsigned ntypes, const gofr_params &p, TrajDev &t, Plan &pl)
+{
+    if (box_kind != GOFR_BOX_ORTHO && box_kind != GOFR_BOX_TRICLINIC) return GOFR_ERR_ARG;
+    if (natoms == 0 || ntypes == 0 || ntypes > 255) return GOFR_ERR_ARG;
+    t.T = 1;
+    t.N = natoms;
+    t.ntypes = ntypes;
+    t.tric = box_kind == GOFR_BOX_TRICLINIC;
+    std::vector<Box32> b32(1);
+    if (!read_boxes(t, box, 1, t.tric ? 9 : 6, b32).empty()) return GOFR_ERR_ARG;
+    for (int k = 0; k < 3; ++k) {
+        if (!(coord_min[k] <= coord_max[k]) || !std::isfinite(coord_min[k]) ||
+            !std::isfinite(coord_max[k]))
+            return GOFR_ERR_ARG;
+        set_extent(t, k, coord_min[k], coord_max[k]);
+    }
+    gofr_ctx ctx;
+    return make_plan(&ctx, t, p, pl);
+}
+
 int check_device_error(gofr_ctx *ctx)
 {
     unsigned e = 0;
@@ -1281,6 +1382,15 @@ void set_cellw_geometry(CellwLaunch &C, const CellwGeom &g)
     for (int k = 0; k < 15; ++k) { C.nx_lo[k] = g.nx_lo[k]; C.nx_hi[k] = g.nx_hi[k]; }
     C.ny_span = g.ny_span;
     for (int k = 0; k < CELLW_NSHIFT; ++k) C.shift[k] = g.shift[k];
+}
+
+// Warp blocks of a CTA's chunk at most: chunks of fewer than 2^31 all-pairs-
+// equivalent pairs (or a block a warp), so that no u32 shared bin overflows
+// between two flushes (the kernel checks the pairs it evaluated).
+long long cellw_most(size_t N, const int nw[3])
+{
+    const double n2 = (double)N * (double)N, nwb = (double)nw[0] * nw[1] * nw[2];
+    return (long long)std::max(16.0, std::min(std::floor(2147483648.0 / n2 * nwb), 1e15));
 }
 
 // Builds (once per grid and frames) the cell-sorted copy of t's frames.  On
@@ -1414,6 +1524,7 @@ int enqueue_run(gofr_ctx *ctx, const TrajDev &t, const gofr_params &p, const Run
         L.rmin_f = (float)p.rmin;
         L.inv_dr_f = (float)(1.0 / bm.dr);
         L.wlim = (float)(0.5 - pl.b.eta);
+        L.rm = plan_radial_map(t, p, pl);
     }
     if (pl.cells && pl.cellw && !ghist) {
         int brc = ensure_cells(ctx, t, pl);
@@ -1423,14 +1534,9 @@ int enqueue_run(gofr_ctx *ctx, const TrajDev &t, const gofr_params &p, const Run
         C.pair.a0 = 0;
         C.pair.a1 = (int)t.N;
         C.pair.counts = counts;
-        const int nwb = pl.nw[0] * pl.nw[1] * pl.nw[2];
-        // items: (lag, origin, part); at least 8 per SM, so few (lag, origin)
-        // pairs still fill the GPU
-        const long long lo = (long long)L.n_lags * L.n_orig;
-        long long parts = std::max<long long>(pl.parts, (8LL * ctx->num_sms + lo - 1) / lo);
-        parts = std::min<long long>(parts, nwb);
-        C.parts = (int)std::max<long long>(parts, 1);
-        C.pair.n_items = lo * C.parts;
+        C.pair.n_items = (long long)L.n_lags * L.n_orig;
+        C.most = cellw_most(t.N, pl.nw);
+        C.queue = reinterpret_cast<unsigned *>(ctx->d_stats + ST_QUEUE);
         C.start = t.d_cstart;
         C.wpos = t.d_wpos;
         for (int k = 0; k < 3; ++k) { C.nc[k] = pl.nc[k]; C.w[k] = pl.wblk[k]; C.nw[k] = pl.nw[k]; }
@@ -2035,12 +2141,10 @@ int build_batch(gofr_ctx *ctx)
         if (rc) return rc;
         CellwLaunch C{};
         C.pair = B.launches[k];
-        C.pair.win = B.d_win + win_off[k];  // the windows of the block plan: same bound
-        const long long lo = (long long)rs.n_lags * rs.n_orig;
-        const int nwb = q.nw[0] * q.nw[1] * q.nw[2];
-        long long parts = std::max<long long>(q.parts, (8LL * ctx->num_sms + lo - 1) / lo);
-        C.parts = (int)std::max<long long>(std::min<long long>(parts, nwb), 1);
-        C.pair.n_items = lo * C.parts;
+        C.pair.rm = plan_radial_map(t, p, q);
+        C.pair.n_items = (long long)rs.n_lags * rs.n_orig;
+        C.most = cellw_most(t.N, q.nw);
+        C.queue = reinterpret_cast<unsigned *>(ctx->d_stats + ST_QUEUE);
         C.start = t.d_cstart;
         C.wpos = t.d_wpos;
         for (int a = 0; a < 3; ++a) { C.nc[a] = q.nc[a]; C.w[a] = q.wblk[a]; C.nw[a] = q.nw[a]; }
@@ -2731,25 +2835,10 @@ int gofr_plan_query(const double *box, int box_kind, const double *coord_min,
                     const gofr_params *p, int *out)
 {
     if (!box || !coord_min || !coord_max || !p || !out) return GOFR_ERR_ARG;
-    if (box_kind != GOFR_BOX_ORTHO && box_kind != GOFR_BOX_TRICLINIC) return GOFR_ERR_ARG;
-    if (natoms == 0 || ntypes == 0 || ntypes > 255) return GOFR_ERR_ARG;
-    TrajDev t;
-    t.T = 1;
-    t.N = natoms;
-    t.ntypes = ntypes;
-    t.tric = box_kind == GOFR_BOX_TRICLINIC;
-    std::vector<Box32> b32(1);
-    if (!read_boxes(t, box, 1, t.tric ? 9 : 6, b32).empty()) return GOFR_ERR_ARG;
-    for (int k = 0; k < 3; ++k) {
-        if (!(coord_min[k] <= coord_max[k]) || !std::isfinite(coord_min[k]) ||
-            !std::isfinite(coord_max[k]))
-            return GOFR_ERR_ARG;
-        set_extent(t, k, coord_min[k], coord_max[k]);
-    }
-    gofr_ctx ctx;  // host state only: the planner touches no device
-    Plan pl;
-    const int rc = make_plan(&ctx, t, *p, pl);
     for (int k = 0; k < 10; ++k) out[k] = 0;
+    TrajDev t;
+    Plan pl;
+    const int rc = host_plan(box, box_kind, coord_min, coord_max, natoms, ntypes, *p, t, pl);
     if (rc) return rc;
     out[0] = pl.kind == 1 ? GOFR_KERNEL_F64
                           : (pl.cellw ? GOFR_KERNEL_CELL_WARP
@@ -2763,6 +2852,22 @@ int gofr_plan_query(const double *box, int box_kind, const double *coord_min,
         out[8] = pl.cellw ? pl.cta_warps : 0;
     }
     out[9] = pl.wrapcheck ? 1 : 0;
+    return GOFR_OK;
+}
+
+int gofr_radial_query(const double *box, int box_kind, const double *coord_min,
+                      const double *coord_max, size_t natoms, unsigned ntypes,
+                      const gofr_params *p, double *out)
+{
+    if (!box || !coord_min || !coord_max || !p || !out) return GOFR_ERR_ARG;
+    TrajDev t;
+    Plan pl;
+    const int rc = host_plan(box, box_kind, coord_min, coord_max, natoms, ntypes, *p, t, pl);
+    if (rc) return rc;
+    if (pl.kind != 0 || pl.empty) return GOFR_ERR_UNSUPPORTED;
+    const RadialMap m = plan_radial_map(t, *p, pl);
+    const float f[8] = {m.inv_dr, m.q_off, m.lim, m.lim_self, m.t_lo, m.t_hi, m.t_ok, m.self_max};
+    for (int k = 0; k < 8; ++k) out[k] = f[k];
     return GOFR_OK;
 }
 

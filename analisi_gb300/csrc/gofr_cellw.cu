@@ -10,28 +10,27 @@
 // shrink from the neighbourhood of a CTA-sized block to the neighbourhood of
 // a warp-sized one.
 //
-// Lanes hold neighbours, not first atoms: a chunk buffer holds 128 records
-// of the neighbourhood (rows packed back to back, several per chunk when
-// they are short), each lane keeps four of them in registers, and the warp
-// walks the block's first atoms one at a time, each broadcast
-// from shared memory, so no lane idles for want of a first atom whatever the
-// block's atom count (only the last chunk of a neighbourhood is partly
-// padding).
+// Lanes hold neighbours, not first atoms: the records of the neighbourhood,
+// rows back to back, are taken 128 at a time, four per lane in registers, and
+// the warp walks the block's first atoms one at a time, each broadcast from
+// shared memory, so no lane idles for want of a first atom whatever the
+// block's atom count (only the last chunk of a neighbourhood is partly empty).
 //
 // Layout per frame (built once per upload and grid): records
 // {x, y, z, type << 24 | atom id} (float4, the coordinates wrapped into the
 // box in FP64 and rounded to FP32 about the box centre, exactly as the block
 // kernel's), sorted by cell, x fastest; cell start offsets.  A row of cells
-// of a neighbourhood is one contiguous run of 16-byte records, so a warp
-// stages it into shared memory with one 1-D bulk copy (TMA, cp.async.bulk)
-// per piece (a row's run of records, or the part of it that fits), up to
-// MAXP pieces and CH records per chunk, two chunk buffers per warp,
-// completion tracked by one mbarrier per buffer.  Cells reached across the
-// box boundary are the periodic image of the cell: after the copy lands,
-// each lane moves its records to their piece's image (x += fl32 of the
-// lattice vector, one FP32 rounding per axis; orthorhombic: s fl32(L), the
-// block kernel's arithmetic), so the pair arithmetic and its certified error
-// bound (gofr_capi.cu, error_bound_cells) are the block kernel's.
+// of a neighbourhood is one or two contiguous runs of 16-byte records; a warp
+// lists the runs that hold records with their prefix sums, and a lane finds
+// the run of its record by counting run starts among the 32 records of its
+// group (one OR-reduction of start bits), then loads it from L2: coalesced
+// 512-byte loads straight into registers.  (Staging through shared memory by
+// bulk copies cost the copies' issue, an mbarrier wait and a pass over the
+// records per chunk, and needed the buffers for a candidate queue that is
+// gone.)  Cells reached across the box boundary are the periodic image of the
+// cell: each record is moved to its run's image (x += fl32 of the lattice
+// vector, one FP32 rounding per axis; orthorhombic: s fl32(L), the block
+// kernel's arithmetic).
 //
 // Triclinic boxes (upper-triangular cell vectors a, b, c) use the same
 // kernel.  The reference's minimum image (z, then y, then x) leaves every
@@ -46,19 +45,27 @@
 // more cell where the shift is not whole), together with the FP32 lattice
 // vector of each image.
 //
-// Warps never wait for one another inside a work item (lag, origin, part of
-// the warp blocks): they pull warp blocks from a shared counter, stream
-// their own neighbourhoods and add their candidates to the CTA's shared
-// histogram; the CTA synchronises only at the end of the item, to add the
-// histogram to the counts.  Candidates (FP32 d2 <= hi_f) are compacted into
-// a dense per-warp queue as they are found (one ballot per first atom and
-// record slot: each candidate lane writes at the warp's count plus the
-// candidates of the lanes below it); an entry names the first atom and the
-// record of the current chunk buffer, 16 bits.  The queue is binned 32
-// entries at a time, every lane busy: when it is nearly full and at the end
-// of each chunk (before the buffer is refilled), d2 recomputed with the
-// pair loop's arithmetic (the same value), then the block kernel's
-// certified window test and predicated shared-memory reductions.
+// Every evaluated pair goes straight into the CTA's shared histogram
+// (bin_pair2, gofr_device.cuh), and the pairs near a bin edge (the radial
+// margin of gofr_capi.cu; 0.13 % of them at 16k atoms) are noted in a bit per
+// first atom and record, then taken out of their cell and recomputed in FP64,
+// 32 at a time.
+//
+// Work is a list of (lag, origin, warp block) units, dealt to the CTAs in
+// chunks of decreasing size from one counter; the warps of a CTA take the
+// chunk's units one by one and never wait for one another inside a chunk.
+// The histogram is added to the counts when the lag changes.  (Items of one
+// (lag, origin) dealt round-robin, a barrier and a flush after each, left 10 % of
+// the 16k-atom job idle in the last round and 18 % of the 131k-atom one.)
+//
+// Bound by instruction issue: 73 instructions per 128 pairs (46 of them the
+// pairs' own), 77 % of the issue slots used, the shared-memory pipe 57 %
+// busy, the FP32 pipe 59 %, no DRAM traffic to speak of.  16384 atoms, 25
+// origins x 100 lags (17 % of N^2 evaluated, 26 % of those within rmax): 66.0
+// ms, where the form that queued its candidates and binned the queue took
+// 178.9; 131072 atoms, 5 x 10: 8.6 ms against 21.7; 32768 atoms, triclinic,
+// 10 x 20: 20.8 ms against 59.8.  64 registers, 32 warps per SM: with 128
+// registers and 16 warps 74.9 ms.
 #include <cstdint>
 #include <cuda_runtime.h>
 
@@ -68,223 +75,243 @@
 namespace gofr {
 namespace cellw {
 
-constexpr int CH = 128;        // neighbour records per chunk buffer: 4 per lane
-constexpr int MAXP = 8;        // pieces (bulk copies) per chunk
+constexpr int CH = 128;        // neighbour records per chunk: 4 per lane
 constexpr int FA = 64;         // first atoms per batch
-constexpr int CQ = 1024;       // candidate queue entries of a warp
-constexpr int CQ_ROOM = 4 * 32; // entries one first atom can add (4 records x 32 lanes)
-constexpr int QW = 32;         // FP64 recheck queue of a warp
 constexpr int MAXROWS = CELLW_MAX_ROWS;  // neighbourhood rows of a warp block
+constexpr int MAXSEG = 2 * MAXROWS;      // sorted ranges of them (two when a row wraps the box)
+constexpr int QW = 64;         // FP64 recheck queue of a warp
 static_assert(CH == 4 * 32, "four records per lane");
-static_assert(CQ / 32 <= 32, "one bit per binning round in a 32-bit recheck mask");
-static_assert(CH <= 256 && FA <= 256, "a queue entry names a first atom and a record in 8 bits each");
+static_assert(QW >= 64, "a round adds at most 32 entries to a queue drained at 32");
+
+constexpr unsigned SLOT_MASK = 0x1ffffffu;  // a sorted slot below its image's index
 
 // floor(a / n) for n > 0
 __device__ __forceinline__ int floordiv(int a, int n) { return a >= 0 ? a / n : -((n - 1 - a) / n); }
 
-constexpr unsigned SEG_BEGIN = 0x1ffffffu;  // a segment's begin; its image index above bit 25
-
-// Orders this thread's generic-proxy shared-memory accesses before later
-// async-proxy (bulk copy) writes to the same buffer.
-__device__ __forceinline__ void fence_proxy_async_smem()
-{
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-}
-
 // Shared memory of one warp.
 struct WarpArea {
-    float4 buf[2][CH];           // chunk buffers (bulk-copy destinations, 16-byte aligned)
-    float4 fi[FA];               // first atoms of the batch {x, y, z, type << 24 | id}
-    unsigned short cq[CQ];       // candidate queue: first atom << 8 | record of the current chunk
-    uint4 q[QW];                 // FP64 recheck queue {ia, ja, channel, 0}
-    int2 seg[2 * MAXROWS];       // sorted ranges of the neighbourhood rows (two halves each):
-                                 // {begin | image << 25, end}
-    int4 pc[2][MAXP];            // pieces of each buffer {first record, source record, count, image}
-    uint64_t bar[2];             // one mbarrier per chunk buffer
-    int n[2];                    // records in each buffer
-    int np[2];                   // pieces in each buffer
-    int qn;                      // entries in q
-    int pad[3];
+    ulonglong2 fa[FA][2];        // first atoms {x x | y y}, {z z | w, run end << 8 | type}: coordinates
+                                 // duplicated for f32x2, w = type << 24 | id, and the end of the run
+                                 // of first atoms of the same type
+    uint2 near[QW];              // pairs near a bin edge: {first atom, image << 25 | sorted slot}
+    uint2 q[QW];                 // FP64 recheck queue: w of both atoms
+    int2 src[MAXSEG];            // {sorted slot of the segment's first record - its flat index, image}
+    int pre[MAXSEG + 33];        // flat index of each segment's first record (INT_MAX past the last)
 };
 
-// Chunk walker state (the same values in every lane of a warp).
-struct Walk {
-    int row, half, off;          // current segment (row, half) and offset into it
-};
+// Units [u0, u1) of chunk c of a launch of G CTAs over U units: every round of G
+// chunks takes half of what is left (a CTA meets few chunk ends, and the last
+// chunks are small enough for the CTAs to finish together), no chunk more
+// than `most` units or fewer than `least`.
+__device__ __forceinline__ void chunk_range(long long c, long long G, long long U, long long most,
+                                            long long least, long long &u0, long long &u1)
+{
+    long long r = c / G, s = 0;
+    // rounds of full chunks, while half of the rest is more than G of them
+    const long long capped = U > 2 * G * most ? (U - 2 * G * most + G * most - 1) / (G * most) : 0;
+    const long long skip = r < capped ? r : capped;
+    s = skip * G * most;
+    r -= skip;
+    long long len = 0;
+    for (;;) {
+        len = (U - s + 2 * G - 1) / (2 * G);
+        if (skip < capped || len > most) len = most;
+        if (len < least) {
+            len = least;  // from here on every round is the same
+            s += r * G * len;
+            break;
+        }
+        if (r == 0) break;
+        --r;
+        s += G * len;
+    }
+    u0 = s + (c % G) * len;
+    u1 = u0 + len < U ? u0 + len : U;
+}
 
-// NWARP warps per CTA (8: two CTAs per SM, 16: one), HCOPY copies of the
-// shared histogram (warp w adds to copy w HCOPY / NWARP: the privatisation
-// depth, fewer warps contending for each bin).
-template <int NWARP, int HCOPY>
-__global__ void __launch_bounds__(NWARP * 32, 16 / NWARP) k_pairs_cellw(const CellwLaunch C,
-                                                                        int win_cap, int hist_cap)
+// NWARP warps per CTA, HCOPY copies of the shared histogram (warp w adds to
+// copy w HCOPY / NWARP: the privatisation depth, fewer warps contending for
+// each bin), MODE the bin map's (RadialMap).
+template <int NWARP, int HCOPY, int MODE>
+__global__ void __launch_bounds__(NWARP * 32, 32 / NWARP) k_pairs_cellw(const CellwLaunch C)
 {
     constexpr int NT = NWARP * 32;
     extern __shared__ __align__(128) unsigned char smem[];
+    const PairLaunch &P = C.pair;
+    const int nbin = P.nbin, nrow = nbin + 1;  // histogram row: nbin bins and an unread cell
+    const int hist_cap = P.nch * nrow + 1;      // the first row has its cell -1, too
     WarpArea *const areas = reinterpret_cast<WarpArea *>(smem);
-    float2 *const win = reinterpret_cast<float2 *>(areas + NWARP);
-    unsigned *const hist = reinterpret_cast<unsigned *>(win + win_cap);
+    unsigned *const hist = reinterpret_cast<unsigned *>(areas + NWARP);
     unsigned short *const chtab = reinterpret_cast<unsigned short *>(hist + HCOPY * hist_cap);
-    __shared__ int s_next, s_abort;
-    __shared__ unsigned long long s_pairs;  // pairs evaluated in the current item
+    __shared__ int s_next, s_full;
+    __shared__ long long s_u0, s_u1;
+    __shared__ unsigned long long s_pairs;  // pairs evaluated since the last flush
     __shared__ float4 s_shift[CELLW_NSHIFT];
     __shared__ int2 s_ny[3], s_nx[15];
 
-    const PairLaunch &P = C.pair;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const unsigned lt = (1u << lane) - 1u;  // the lanes below this one
     WarpArea &A = areas[warp];
-    const int hlen = P.nch * P.nbin;
-    unsigned *const whist = hist + (warp * HCOPY / NWARP) * hist_cap;  // this warp's copy
+    const int hlen = P.nch * nbin;
+    unsigned *const whist = hist + (warp * HCOPY / NWARP) * hist_cap + 1;  // this warp's row 0
+    // row address of channel ch as bin_pair2 takes it: row0 + ch * rowb
+    const unsigned row0 = smem_u32(whist) - 4u * RADIAL_MAGIC_BITS, rowb = 4u * (unsigned)nrow;
     const int half_ch = P.nch / 2;
-    const float hi_f = P.hi_f;
     const int ncx = C.nc[0], ncy = C.nc[1], ncz = C.nc[2];
     const int ncell = ncx * ncy * ncz;
     const int nwx = C.nw[0], nwy = C.nw[1], nwz = C.nw[2];
     const int nwb = nwx * nwy * nwz;
     const long long NP = P.NP;
+    const float qnan = __int_as_float(0x7fc00000);
 
-    for (int i = tid; i < P.nbin; i += NT) win[i] = P.win[i];
-    for (int c = 0; c < HCOPY; ++c)
-        for (int i = tid; i < hlen; i += NT) hist[c * hist_cap + i] = 0u;
+    for (int i = tid; i < HCOPY * hist_cap; i += NT) hist[i] = 0u;
     for (int i = tid; i < P.ntypes * P.ntypes; i += NT) chtab[i] = P.chtab[i];
     for (int i = tid; i < CELLW_NSHIFT; i += NT) s_shift[i] = C.shift[i];
     if (tid < 3) s_ny[tid] = make_int2(C.ny_lo[tid], C.ny_hi[tid]);
     if (tid < 15) s_nx[tid] = make_int2(C.nx_lo[tid], C.nx_hi[tid]);
-    if (lane == 0) {
-        mbar_init(&A.bar[0], 1);
-        mbar_init(&A.bar[1], 1);
-        A.qn = 0;
-        fence_mbar_init();
-    }
-    if (tid == 0) s_abort = 0;
-    __syncthreads();
+    if (tid == 0) s_pairs = 0ull;
 
-    unsigned ph0 = 0u, ph1 = 0u;      // mbarrier phases of the two buffers
-    bool dead = false;                // a bounded wait of this warp ran out
-    unsigned long long n_cand = 0, n_rech = 0, n_eval = 0;
+    int nn = 0, qn = 0;  // entries of the warp's two queues (the same in every lane)
+    unsigned long long n_cand = 0, n_rech = 0, n_eval = 0;  // n_cand: counts flushed
+    bool lost = false;                                      // a u32 bin could have overflowed
 
-    for (long long g = blockIdx.x; g < P.n_items; g += gridDim.x) {
-        // item = (lag, origin, part): lag slowest
-        const long long per_lag = (long long)P.n_orig * C.parts;
-        const int lag_idx = (int)(g / per_lag);
-        const long long rem = g - (long long)lag_idx * per_lag;
-        const int k = (int)(rem / C.parts);
-        const int part = (int)(rem - (long long)k * C.parts);
-        const int wb0 = (int)((long long)part * nwb / C.parts);
-        const int wb1 = (int)((long long)(part + 1) * nwb / C.parts);
-        const long long fo = P.primo + (long long)k * P.skip;
-        const long long fl = fo + (long long)lag_idx * P.every;
-        const int *st_o = C.start + fo * (long long)(ncell + 1);
-        const int *st_l = C.start + fl * (long long)(ncell + 1);
-        const float4 *rec_o = C.wpos + fo * NP;
-        const float4 *rec_l = C.wpos + fl * NP;
-        if (tid == 0) {
-            s_next = wb0;
-            s_pairs = 0ull;
+    // Adds the CTA's histogram copies to the counts of lag index lag_idx and
+    // clears them (all threads; every warp is done with its pairs).  A u32 bin
+    // holds its hits exactly only while fewer than 2^32 pairs were evaluated
+    // (the host keeps chunks far below).
+    auto flush = [&](int lag_idx) {
+        if (s_pairs > 0xffffffffull) lost = true;
+        for (int i = tid; i < hlen; i += NT) {
+            const int at = (i / nbin) * nrow + i % nbin + 1;
+            unsigned v = 0;  // modulo 2^32: a copy may hold the self pairs another one counted
+#pragma unroll
+            for (int c = 0; c < HCOPY; ++c) v += hist[c * hist_cap + at];
+#pragma unroll
+            for (int c = 0; c < HCOPY; ++c) hist[c * hist_cap + at] = 0u;
+            n_cand += v;
+            if (v && !lost)
+                atomicAdd(P.counts + (long long)lag_idx * P.every * hlen + i,
+                          (unsigned long long)v);
         }
         __syncthreads();
+        if (tid == 0) s_pairs = 0ull;
+        __syncthreads();
+    };
 
-        // the reference's d2 of a pair in FP64 (its minimum image for the box kind)
-        auto ref_d2_box = [&](const double *xi64, const double *xj64, const double *box) {
-            return P.tric ? ref_d2<true>(xi64[0], xi64[1], xi64[2], xj64[0], xj64[1], xj64[2],
-                                         box, P.err)
-                          : ref_d2<false>(xi64[0], xi64[1], xi64[2], xj64[0], xj64[1], xj64[2],
-                                          box, P.err);
+    // units: (lag, origin, warp block), the warp block fastest
+    const long long per_lag = (long long)P.n_orig * nwb, U = per_lag * P.n_lags;
+    int cur_lag = -1;
+    while (!lost) {
+        __syncthreads();  // every warp has read the last chunk's range
+        if (tid == 0) {
+            const long long c = (long long)atomicAdd(C.queue, 1u);
+            long long u0 = 0, u1 = 0;
+            chunk_range(c, gridDim.x, U, C.most, NWARP, u0, u1);
+            s_u0 = u0;
+            s_u1 = u1;
+            s_next = 0;
+            s_full = s_pairs > 0x7fffffffull;
+        }
+        __syncthreads();
+        const long long c0 = s_u0, c1 = s_u1;
+        if (c0 >= c1) break;
+        for (long long g0 = c0; g0 < c1 && !lost;) {
+        const int lag_idx = (int)(g0 / per_lag);
+        const long long g1 = min(c1, (lag_idx + 1) * per_lag);
+        if (g0 != c0) {
+            __syncthreads();  // the warps are done with the chunk's last lag
+            if (tid == 0) {
+                s_next = 0;
+                s_full = s_pairs > 0x7fffffffull;
+            }
+            __syncthreads();
+        }
+        if (cur_lag >= 0 && (lag_idx != cur_lag || s_full)) flush(cur_lag);
+        cur_lag = lag_idx;
+        int k = -1;  // origin of the warp's queues
+        long long fo = 0, fl = 0;
+        const int *st_o = nullptr, *st_l = nullptr;
+        const float4 *rec_o = nullptr, *rec_l = nullptr;
+        const long long seg_orig = (g0 - lag_idx * per_lag) / nwb;  // the segment's first origin
+        const long long seg_off = (g0 - lag_idx * per_lag) - seg_orig * nwb;
+
+        // Recomputes queued pairs [0, n) in exact FP64 (reference arithmetic),
+        // one per lane; into the channel of distinct atoms, like every pair.
+        auto recheck = [&](int n) {
+            __syncwarp();
+            if (lane < n) {
+                const uint2 e = A.q[lane];
+                const double *xi = P.pos64 + (fo * P.N + (int)(e.x & 0xffffffu)) * 3;
+                const double *xj = P.pos64 + (fl * P.N + (int)(e.y & 0xffffffu)) * 3;
+                const double *box = P.box64 + fo * 9;
+                const double d2 = P.tric ? ref_d2<true>(xi[0], xi[1], xi[2], xj[0], xj[1], xj[2],
+                                                        box, P.err)
+                                         : ref_d2<false>(xi[0], xi[1], xi[2], xj[0], xj[1], xj[2],
+                                                         box, P.err);
+                const int b = ref_bin(d2, P.rmin, P.dr, P.rmin2, P.rmax2, nbin);
+                const int ch = chtab[(int)(e.x >> 24) * P.ntypes + (int)(e.y >> 24)];
+                if (b >= 0 && GOFR_CHECK(ch < P.nch && b < nbin, P.err))
+                    atomicAdd(whist + ch * nrow + b, 1u);
+                ++n_rech;
+            }
+            __syncwarp();
         };
-        // Bins the warp's queued candidates 32 at a time.  An entry's FP32 d2
-        // is recomputed from the first atom and the chunk buffer's record
-        // with the pair loop's operations (one difference per axis, a
-        // multiply, two FMAs: the same value); pairs outside their bin's
-        // certified window are flagged per round and recomputed in FP64
-        // after the rounds.
-        int cn = 0;  // entries in the queue (the same in every lane)
-        auto flush_q = [&](const float4 *bufp) {
-            __syncwarp();  // every lane's entries and first atoms visible
-            unsigned needm = 0u;  // rounds whose entry of this lane goes to the recheck
-            // each round's entry, first atom and record are loaded a round ahead
-            // (a lane past the queue's end reads entry 0's: valid addresses, unused)
-            bool vn = lane < cn;
-            unsigned en = vn ? (unsigned)A.cq[lane] : 0u;
-            float4 fin = A.fi[en >> 8], fjn = bufp[en & 0xffu];
-            for (int g0 = 0; g0 < cn; g0 += 32) {
-                const bool v = vn;
-                const float4 fi = fin, fj = fjn;
-                vn = g0 + 32 + lane < cn;
-                en = vn ? (unsigned)A.cq[g0 + 32 + lane] : 0u;
-                fin = A.fi[en >> 8];
-                fjn = bufp[en & 0xffu];
-                const float dx = __fsub_rn(fi.x, fj.x), dy = __fsub_rn(fi.y, fj.y),
-                            dz = __fsub_rn(fi.z, fj.z);
-                float d2 = __fmul_rn(dx, dx);
-                d2 = __fmaf_rn(dy, dy, d2);
-                d2 = __fmaf_rn(dz, dz, d2);
-                const unsigned iv = __float_as_uint(fi.w), jv = __float_as_uint(fj.w);
-                const int ch = chtab[(int)(iv >> 24) * P.ntypes + (int)(jv >> 24)] +
-                               (((iv ^ jv) & 0xffffffu) == 0u ? half_ch : 0);
-                // bin guess (the window test decides): (sqrt(d2) - rmin) / dr as one
-                // FMA, negative guesses clamped to the last bin (whose window fails)
-                const int b_ = __float2int_rd(
-                    __fmaf_rn(sqrt_guess(d2), P.inv_dr_f, -P.rmin_f * P.inv_dr_f));
-                const int bi = (int)min((unsigned)b_, (unsigned)(P.nbin - 1));
-                const float2 w = win[bi];
-                const bool test = v && d2 >= P.lo_f;
-                const bool inw = d2 >= w.x && d2 <= w.y;
-                red_shared_add1_if(smem_u32(whist + ch * P.nbin + bi),
-                                   test && inw &&
-                                       GOFR_CHECK(ch >= 0 && ch < P.nch && bi >= 0 && bi < P.nbin,
-                                                  P.err));
-                needm |= (test && !inw) ? 1u << (g0 >> 5) : 0u;
-            }
-            if (__any_sync(0xffffffffu, needm != 0u)) {
-                while (needm) {
-                    const int it = __ffs(needm) - 1;
-                    needm &= needm - 1u;
-                    const unsigned e = A.cq[it * 32 + lane];
-                    const unsigned iv = __float_as_uint(A.fi[e >> 8].w),
-                                   jv = __float_as_uint(bufp[e & 0xffu].w);
-                    const int ia = (int)(iv & 0xffffffu), ja = (int)(jv & 0xffffffu);
-                    const int ch = chtab[(int)(iv >> 24) * P.ntypes + (int)(jv >> 24)] +
-                                   (ia == ja ? half_ch : 0);
-                    ++n_rech;
-                    const int slot = atomicAdd(&A.qn, 1);
-                    if (slot < QW) {
-                        A.q[slot] = make_uint4((unsigned)ia, (unsigned)ja, (unsigned)ch, 0u);
-                    } else {
-                        const double *xi64 = P.pos64 + (fo * P.N + ia) * 3;
-                        const double *xj64 = P.pos64 + (fl * P.N + ja) * 3;
-                        const double d2d = ref_d2_box(xi64, xj64, P.box64 + fo * 9);
-                        const int bb = ref_bin(d2d, P.rmin, P.dr, P.rmin2, P.rmax2, P.nbin);
-                        if (bb >= 0) atomicAdd(whist + ch * P.nbin + bb, 1u);
-                    }
-                }
-            }
-            if (lane == 0) n_cand += (unsigned)cn;
-            cn = 0;
-            __syncwarp();  // every lane done with the entries before they are rewritten
-        };
-        // Recomputes the warp's queued pairs in exact FP64 (reference arithmetic).
-        auto drain_queue = [&]() {
+        // Takes entries [0, n) of `near`, one per lane: the pair's bin again with
+        // the pair loop's operations (the same value), out of the cell it was
+        // added to, and into the recheck queue where it can be within the
+        // window.
+        auto resolve = [&](int n) {
             __syncwarp();
-            const int nq = min(A.qn, QW);
-            for (int q = lane; q < nq; q += 32) {
-                const uint4 e = A.q[q];
-                const double *xi64 = P.pos64 + (fo * P.N + (int)e.x) * 3;
-                const double *xj64 = P.pos64 + (fl * P.N + (int)e.y) * 3;
-                const double d2d = ref_d2_box(xi64, xj64, P.box64 + fo * 9);
-                const int bb = ref_bin(d2d, P.rmin, P.dr, P.rmin2, P.rmax2, P.nbin);
-                if (bb >= 0) atomicAdd(whist + (int)e.z * P.nbin + bb, 1u);
+            bool need = false;
+            unsigned wi = 0u, wj = 0u;
+            if (lane < n) {
+                const uint2 e = A.near[lane];
+                const ulonglong2 u0 = A.fa[e.x][0], u1 = A.fa[e.x][1];
+                const float4 v = rec_l[e.y & SLOT_MASK];
+                const float4 sh = s_shift[e.y >> 25];
+                wi = (unsigned)u1.y;
+                wj = __float_as_uint(v.w);
+                const float dx = __fsub_rn(__uint_as_float((unsigned)u0.x), __fadd_rn(v.x, sh.x)),
+                            dy = __fsub_rn(__uint_as_float((unsigned)u0.y), __fadd_rn(v.y, sh.y)),
+                            dz = __fsub_rn(__uint_as_float((unsigned)u1.x), __fadd_rn(v.z, sh.z));
+                const float q = radial_q(
+                    __fmaf_rn(dz, dz, __fmaf_rn(dy, dy, __fmaf_rn(dx, dx, RADIAL_TINY))), P.rm);
+                const float t = __fadd_rn(q, RADIAL_MAGIC);
+                need = t <= P.rm.t_hi && t >= P.rm.t_lo;
+                const int b = (int)(__float_as_uint(t) - RADIAL_MAGIC_BITS);
+                if (need && b >= 0 && b < nbin)
+                    atomicSub(whist + chtab[(int)(wi >> 24) * P.ntypes + (int)(wj >> 24)] * nrow + b,
+                              1u);
             }
-            __syncwarp();
-            if (lane == 0) A.qn = 0;
-            __syncwarp();
+            const unsigned m = __ballot_sync(0xffffffffu, need);
+            if (need) A.q[qn + __popc(m & lt)] = make_uint2(wi, wj);
+            qn += __popc(m);
+            if (qn >= 32) {
+                recheck(32);
+                qn -= 32;
+                if (lane < qn) A.q[lane] = A.q[32 + lane];
+                __syncwarp();
+            }
         };
 
-        while (!dead) {
-            int wb = 0;
-            if (lane == 0) wb = atomicAdd(&s_next, 1);
-            wb = __shfl_sync(0xffffffffu, wb, 0);
-            if (wb >= wb1) break;
+        for (;;) {
+            int nx = 0;
+            if (lane == 0) nx = atomicAdd(&s_next, 1);
+            nx = __shfl_sync(0xffffffffu, nx, 0);
+            if (g0 + nx >= g1) break;
+            const long long uo = seg_off + nx;
+            const int kk = (int)(seg_orig + uo / nwb), wb = (int)(uo % nwb);
+            if (kk != k) {
+                recheck(qn);  // the queue names the last origin's frames
+                qn = 0;
+                k = kk;
+                fo = P.primo + (long long)k * P.skip;
+                fl = fo + (long long)lag_idx * P.every;
+                st_o = C.start + fo * (long long)(ncell + 1);
+                st_l = C.start + fl * (long long)(ncell + 1);
+                rec_o = C.wpos + fo * NP;
+                rec_l = C.wpos + fl * NP;
+            }
             const int wz = wb / (nwx * nwy), wy = (wb / nwx) % nwy, wx = wb % nwx;
             const int cx0 = wx * C.w[0], cy0 = wy * C.w[1], cz0 = wz * C.w[2];
             const int cnx = min(C.w[0], ncx - cx0), cny = min(C.w[1], ncy - cy0),
@@ -310,89 +337,72 @@ __global__ void __launch_bounds__(NWARP * 32, 16 / NWARP) k_pairs_cellw(const Ce
             // the neighbourhood: layers uz (image sz), in each the rows uy
             // (image sy), each row the cells ux in one or two sorted ranges
             // (two when the row wraps the box: images sx and sx + 1); the
-            // layer's row slots beyond its own rows stay empty
+            // ranges that hold records, back to back, are the flat list the
+            // chunks take their records from
             const int jny = cny + C.ny_span;
             const int nrows = (cnz + C.nz_hi - C.nz_lo + 1) * jny;
-            for (int rr = lane; rr < nrows; rr += 32) {
-                const int lz = rr / jny, k = rr - lz * jny;
+            int nseg = 0, n_j = 0;
+            for (int r0 = 0; r0 < nrows; r0 += 32) {
+                const int rr = r0 + lane;
+                const int lz = rr / jny, ky = rr - lz * jny;
                 const int uz = cz0 + C.nz_lo + lz;
                 const int sz = floordiv(uz, ncz), cz = uz - sz * ncz;
-                int2 s0 = make_int2(0, 0), s1 = make_int2(0, 0);
-                // the host keeps every image reached inside the tables and every
-                // row within one wrap of the box; a row outside them is reported
-                // and left empty (no access outside the tables or the frame)
-                bool ok = sz >= -1 && sz <= 1;
-                const int2 yr = ok ? s_ny[sz + 1] : make_int2(0, -1 - cny);
-                if (k <= cny + yr.y - yr.x) {
-                    const int uy = cy0 + yr.x + k;
-                    const int sy = floordiv(uy, ncy), cy = uy - sy * ncy;
-                    ok = sy >= -2 && sy <= 2;
-                    const int2 xr = ok ? s_nx[(sz + 1) * 5 + sy + 2] : make_int2(0, 0);
-                    const int ux = cx0 + xr.x, len = cnx + xr.y - xr.x + 1;
-                    const int sx = floordiv(ux, ncx), a = ux - sx * ncx, b = a + len;
-                    ok = ok && sx >= -2 && len >= 0 && len <= ncx && (b <= ncx ? sx <= 2 : sx <= 1);
-                    if (ok) {
-                        const int base = (cz * ncy + cy) * ncx;
-                        const unsigned code =
-                            (unsigned)((sx + 2) + 5 * (sy + 2) + 25 * (sz + 1)) << 25;
-                        if (b <= ncx) {
-                            s0 = make_int2((int)((unsigned)st_l[base + a] | code), st_l[base + b]);
-                        } else {
-                            s0 = make_int2((int)((unsigned)st_l[base + a] | code),
-                                           st_l[base + ncx]);
-                            s1 = make_int2((int)((unsigned)st_l[base] | (code + (1u << 25))),
-                                           st_l[base + b - ncx]);
+                int beg0 = 0, len0 = 0, beg1 = 0, len1 = 0, code = 0;
+                if (rr < nrows) {
+                    // the host keeps every image reached inside the tables and every
+                    // row within one wrap of the box; a row outside them is reported
+                    // and left empty (no access outside the tables or the frame)
+                    bool ok = sz >= -1 && sz <= 1;
+                    const int2 yr = ok ? s_ny[sz + 1] : make_int2(0, -1 - cny);
+                    if (ky <= cny + yr.y - yr.x) {
+                        const int uy = cy0 + yr.x + ky;
+                        const int sy = floordiv(uy, ncy), cy = uy - sy * ncy;
+                        ok = sy >= -2 && sy <= 2;
+                        const int2 xr = ok ? s_nx[(sz + 1) * 5 + sy + 2] : make_int2(0, 0);
+                        const int ux = cx0 + xr.x, len = cnx + xr.y - xr.x + 1;
+                        const int sx = floordiv(ux, ncx), a = ux - sx * ncx, b = a + len;
+                        ok = ok && sx >= -2 && len >= 0 && len <= ncx &&
+                             (b <= ncx ? sx <= 2 : sx <= 1);
+                        if (ok) {
+                            const int base = (cz * ncy + cy) * ncx;
+                            code = (sx + 2) + 5 * (sy + 2) + 25 * (sz + 1);
+                            beg0 = st_l[base + a];
+                            len0 = st_l[base + min(b, ncx)] - beg0;
+                            if (b > ncx) {
+                                beg1 = st_l[base];
+                                len1 = st_l[base + b - ncx] - beg1;
+                            }
                         }
                     }
+                    if (!ok) atomicOr(P.err, ERRW_BOUNDS);
                 }
-                if (!ok) atomicOr(P.err, ERRW_BOUNDS);
-                A.seg[2 * rr] = s0;
-                A.seg[2 * rr + 1] = s1;
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const int beg = h ? beg1 : beg0, len = h ? len1 : len0;
+                    const unsigned m = __ballot_sync(0xffffffffu, len > 0);
+                    if (!m) continue;
+                    int incl = len;
+#pragma unroll
+                    for (int o = 1; o < 32; o <<= 1) {
+                        const int v = __shfl_up_sync(0xffffffffu, incl, o);
+                        if (lane >= o) incl += v;
+                    }
+                    const int at = nseg + __popc(m & lt), f = n_j + incl - len;
+                    if (len > 0 && GOFR_CHECK(at < MAXSEG, P.err)) {
+                        A.pre[at] = f;
+                        A.src[at] = make_int2(beg - f, code + h);
+                    }
+                    nseg += __popc(m);
+                    n_j += __shfl_sync(0xffffffffu, incl, 31);
+                }
             }
-            __syncwarp();
-            int n_j = 0;
-            for (int s = lane; s < 2 * nrows; s += 32)
-                n_j += A.seg[s].y - (int)((unsigned)A.seg[s].x & SEG_BEGIN);
-            n_j = __reduce_add_sync(0xffffffffu, n_j);
-            // Fills buffer b with the next records of the neighbourhood: up to CH
-            // records from up to MAXP pieces (every lane walks the segments
-            // alike); lane 0 then expects their bytes on the buffer's mbarrier
-            // and issues one bulk copy per piece.  False at the end of the
-            // neighbourhood (nothing issued).
-            auto issue = [&](Walk &w, int b) -> bool {
-                int filled = 0, np = 0;
-                while (w.row < nrows && filled < CH && np < MAXP) {
-                    const int2 sg = A.seg[2 * w.row + w.half];
-                    const int beg = (int)((unsigned)sg.x & SEG_BEGIN);
-                    const int len = sg.y - beg;
-                    if (w.off < len) {
-                        const int n = min(CH - filled, len - w.off);
-                        if (lane == 0)
-                            A.pc[b][np] = make_int4(filled, beg + w.off, n,
-                                                    (int)((unsigned)sg.x >> 25));
-                        ++np;
-                        filled += n;
-                        w.off += n;
-                        continue;
-                    }
-                    w.off = 0;
-                    if (++w.half == 2) { w.half = 0; ++w.row; }
-                }
-                if (filled == 0) return false;
-                if (lane == 0) {
-                    A.n[b] = filled;
-                    A.np[b] = np;
-                    mbar_arrive_expect_tx(&A.bar[b], (unsigned)(filled * 16));
-                    for (int p = 0; p < np; ++p) {
-                        const int4 pc = A.pc[b][p];
-                        bulk_g2s(&A.buf[b][pc.x], rec_l + pc.y, (unsigned)(pc.z * 16), &A.bar[b]);
-                    }
-                }
-                return true;
-            };
+            A.pre[nseg + lane] = 0x7fffffff;
+            if (lane == 0) A.pre[nseg + 32] = 0x7fffffff;
 
-            for (int ibase = 0; ibase < n_i && !dead; ibase += FA) {
-                // first atoms ibase .. ibase + na - 1 of the block
+            for (int ibase = 0; ibase < n_i; ibase += FA) {
+                // first atoms ibase .. ibase + na - 1 of the block, each group of
+                // 32 in the order of their types (the row addresses of a lane's
+                // records change only with the first atom's type)
                 const int na = min(FA, n_i - ibase);
                 for (int q0 = 0; q0 < na; q0 += 32) {
                     const int q = q0 + lane;
@@ -403,133 +413,153 @@ __global__ void __launch_bounds__(NWARP * 32, 16 / NWARP) k_pairs_cellw(const Ce
                         row += (qq >= __shfl_sync(0xffffffffu, ipre, rr)) ? 1 : 0;
                     const int rb = __shfl_sync(0xffffffffu, ib, row);
                     const int rp = __shfl_sync(0xffffffffu, ipre - ilen, row);
-                    if (q < na) A.fi[q] = rec_o[rb + (qq - rp)];
+                    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+                    if (q < na) v = rec_o[rb + (qq - rp)];
+                    const unsigned w = __float_as_uint(v.w), ti = w >> 24;
+                    unsigned left = __ballot_sync(0xffffffffu, q < na);
+                    int at = q0, end = q0;  // its place, the end of its type's run
+                    for (int base = q0; left;) {
+                        const unsigned t = __shfl_sync(0xffffffffu, ti, __ffs(left) - 1);
+                        const unsigned m = __ballot_sync(0xffffffffu, q < na && ti == t);
+                        if (q < na && ti == t) {
+                            at = base + __popc(m & lt);
+                            end = base + __popc(m);
+                        }
+                        base += __popc(m);
+                        left &= ~m;
+                    }
+                    if (q < na) {
+                        const f2 z = f2pk(v.z, v.z);
+                        A.fa[at][0] = make_ulonglong2(f2pk(v.x, v.x), f2pk(v.y, v.y));
+                        A.fa[at][1] = make_ulonglong2(
+                            z, (unsigned long long)((unsigned)end << 8 | ti) << 32 | w);
+                        // the atom's pair with itself: from the channel of distinct
+                        // atoms, where the loop below counts it, to its own
+                        const int ia = (int)(w & 0xffffffu);
+                        const int b = P.tric ? self_bin<true>(P, fo, fl, ia)
+                                             : self_bin<false>(P, fo, fl, ia);
+                        if (b >= 0) {
+                            const int ch = chtab[(int)ti * P.ntypes + (int)ti];
+                            atomicSub(whist + ch * nrow + b, 1u);
+                            atomicAdd(whist + (ch + half_ch) * nrow + b, 1u);
+                        }
+                    }
                 }
                 if (lane == 0) {
                     const unsigned long long pe = (unsigned long long)na * (unsigned long long)n_j;
                     n_eval += pe;
                     atomicAdd(&s_pairs, pe);
                 }
-                // earlier generic accesses of both buffers (records moved to their
-                // image, padding, reads) before the bulk copies that refill them
-                fence_proxy_async_smem();
                 __syncwarp();
-                Walk w{0, 0, 0};
-                bool have0 = issue(w, 0);
-                bool have1 = have0 && issue(w, 1);
-                for (int c = 0; (c & 1) ? have1 : have0; ++c) {
-                    const int b = c & 1;
-                    const bool ok = mbar_wait_bounded(&A.bar[b], b ? ph1 : ph0);
-                    if (!__all_sync(0xffffffffu, ok)) {
-                        // give the other buffer's copy a bounded chance to land,
-                        // then stop this warp's work (the CTA ends at the item)
-                        if (lane == 0 && (b ? have0 : have1))
-                            mbar_wait_bounded(&A.bar[b ^ 1], b ? ph0 : ph1);
-                        if (lane == 0) {
-                            atomicOr(P.err, ERRW_WAIT_TIMEOUT);
-                            s_abort = 1;
-                        }
-                        dead = true;
-                        break;
-                    }
-                    if (b) ph1 ^= 1u; else ph0 ^= 1u;
-                    const int n = A.n[b], np = A.np[b];
-                    float4 *const bufp = A.buf[b];
-                    // this lane's records lane + 32 t (consecutive lanes, consecutive
-                    // records: no bank conflict): moved to their piece's image
-                    // (image (0, 0, 0) adds zeros: x + 0 = x) and written back for
-                    // the binning; records past n are NaN (never a candidate)
-                    float rx[4], ry[4], rz[4];
+                const f2 inv = f2pk(P.rm.inv_dr, P.rm.inv_dr), off = f2pk(P.rm.q_off, P.rm.q_off),
+                         tiny = f2pk(RADIAL_TINY, RADIAL_TINY);
+                int seg = 0;  // the segment that holds flat record f0 (or the one before it)
+                for (int f0 = 0; f0 < n_j; f0 += CH) {
+                    // this lane's records f0 + lane + 32 t: the starts of the
+                    // segments after `seg` that fall into a group of 32, as bits,
+                    // give each lane its segment by a count of the bits up to it
+                    float x[4], y[4], z[4];
+                    unsigned tj[4], sj[4];  // type; image << 25 | sorted slot
 #pragma unroll
                     for (int t = 0; t < 4; ++t) {
-                        const int k = lane + 32 * t;
-                        float4 v = make_float4(__int_as_float(0x7fc00000), __int_as_float(0x7fc00000),
-                                               __int_as_float(0x7fc00000),
-                                               __uint_as_float(0xffffffffu));
-                        if (k < n) {
-                            int code = A.pc[b][0].w;
-                            for (int p = 1; p < np; ++p) {
-                                const int4 pc = A.pc[b][p];
-                                if (pc.x <= k) code = pc.w;
+                        const int fb = f0 + 32 * t;
+                        const unsigned rel = (unsigned)(A.pre[seg + 1 + lane] - fb);
+                        const unsigned m =
+                            __reduce_or_sync(0xffffffffu, rel < 32u ? 1u << rel : 0u);
+                        const int mine = seg + __popc(m & (lt | 1u << lane));
+                        seg += __popc(m);
+                        x[t] = y[t] = z[t] = qnan;  // no record: never within rmax
+                        tj[t] = sj[t] = 0u;
+                        if (fb + lane < n_j) {
+                            const int2 sc = A.src[mine];
+                            const float4 v = rec_l[sc.x + fb + lane];
+                            sj[t] = (unsigned)(sc.x + fb + lane) | (unsigned)sc.y << 25;
+                            // moved to its image ((0, 0, 0) adds zeros: x + 0 = x)
+                            const float4 sh = s_shift[sc.y];
+                            x[t] = __fadd_rn(v.x, sh.x);
+                            y[t] = __fadd_rn(v.y, sh.y);
+                            z[t] = __fadd_rn(v.z, sh.z);
+                            tj[t] = __float_as_uint(v.w) >> 24;
+                        }
+                    }
+                    const f2 xa = f2pk(x[0], x[1]), xb = f2pk(x[2], x[3]);
+                    const f2 ya = f2pk(y[0], y[1]), yb = f2pk(y[2], y[3]);
+                    const f2 za = f2pk(z[0], z[1]), zb = f2pk(z[2], z[3]);
+                    for (int q0 = 0; q0 < na; q0 += 32) {
+                        const int q1 = min(na, q0 + 32);
+                        unsigned mk[4] = {0u, 0u, 0u, 0u}, bit = 1u;
+                        // one first atom (broadcast) against the lane's four records
+                        auto four = [&](f2 fx, f2 fy, f2 fz, const unsigned *row) {
+                            // one difference per axis, three FMAs
+                            const f2 dxa = f2sub(fx, xa), dya = f2sub(fy, ya), dza = f2sub(fz, za);
+                            const f2 dxb = f2sub(fx, xb), dyb = f2sub(fy, yb), dzb = f2sub(fz, zb);
+                            const f2 da = f2fma(dza, dza, f2fma(dya, dya, f2fma(dxa, dxa, tiny)));
+                            const f2 db = f2fma(dzb, dzb, f2fma(dyb, dyb, f2fma(dxb, dxb, tiny)));
+                            bin_pair2<MODE>(da, inv, off, P.rm, row[0], row[1], bit, mk[0], mk[1]);
+                            bin_pair2<MODE>(db, inv, off, P.rm, row[2], row[3], bit, mk[2], mk[3]);
+                        };
+                        // first atoms of one type at a time; one a turn: the loop is
+                        // small (unrolled by two it measured 3 % slower, by four
+                        // 50 %: instruction fetches)
+                        for (int i = q0; i < q1;) {
+                            const unsigned hi = (unsigned)(A.fa[i][1].y >> 32);
+                            const int e = (int)(hi >> 8);
+                            const unsigned short *ct = chtab + (int)(hi & 0xffu) * P.ntypes;
+                            unsigned row[4];
+#pragma unroll
+                            for (int t = 0; t < 4; ++t) row[t] = row0 + rowb * ct[tj[t]];
+                            for (; i < e; ++i) {
+                                const ulonglong2 u0 = A.fa[i][0];
+                                four(u0.x, u0.y, A.fa[i][1].x, row);
+                                bit <<= 1;
                             }
-                            const float4 sh = s_shift[code];
-                            v = bufp[k];
-                            v.x = __fadd_rn(v.x, sh.x);
-                            v.y = __fadd_rn(v.y, sh.y);
-                            v.z = __fadd_rn(v.z, sh.z);
                         }
-                        bufp[k] = v;
-                        rx[t] = v.x; ry[t] = v.y; rz[t] = v.z;
-                    }
-                    __syncwarp();
-                    const unsigned eb0 = (unsigned)lane;
-                    for (int i = 0; i < na; ++i) {
-                        // first atom i (broadcast) against this lane's four records
-                        const float4 fv = A.fi[i];
-                        float dd[4];
+                        // pairs within the margin of a bin edge, one per lane and
+                        // round, into their queue; it is taken 32 at a time
+                        while (__any_sync(0xffffffffu, (mk[0] | mk[1] | mk[2] | mk[3]) != 0u)) {
+                            unsigned bits = 0u, sl = 0u;
 #pragma unroll
-                        for (int t = 0; t < 4; ++t) {
-                            // one difference per axis, a multiply, two FMAs (the
-                            // binning recomputes d2 with the same operations)
-                            const float ex = __fsub_rn(fv.x, rx[t]), ey = __fsub_rn(fv.y, ry[t]),
-                                        ez = __fsub_rn(fv.z, rz[t]);
-                            float s2 = __fmul_rn(ex, ex);
-                            s2 = __fmaf_rn(ey, ey, s2);
-                            dd[t] = __fmaf_rn(ez, ez, s2);
+                            for (int t = 3; t >= 0; --t)
+                                if (mk[t]) { bits = mk[t]; sl = sj[t]; }
+                            const bool have = bits != 0u;
+                            bool first = have;
+#pragma unroll
+                            for (int t = 0; t < 4; ++t)
+                                if (first && mk[t]) { mk[t] &= mk[t] - 1u; first = false; }
+                            const unsigned m = __ballot_sync(0xffffffffu, have);
+                            if (have)
+                                A.near[nn + __popc(m & lt)] =
+                                    make_uint2((unsigned)(q0 + __ffs(bits) - 1), sl);
+                            nn += __popc(m);
+                            if (nn >= 32) {
+                                resolve(32);
+                                nn -= 32;
+                                if (lane < nn) A.near[lane] = A.near[32 + lane];
+                                __syncwarp();
+                            }
                         }
-                        const float d0 = dd[0], d1 = dd[1], d2v = dd[2], d3 = dd[3];
-                        // entries i << 8 | record, compacted by one ballot per record slot
-                        const unsigned eb = (unsigned)i << 8 | eb0;
-                        const bool p0 = d0 <= hi_f, p1 = d1 <= hi_f, p2 = d2v <= hi_f,
-                                   p3 = d3 <= hi_f;
-                        const unsigned b0 = __ballot_sync(0xffffffffu, p0),
-                                       b1 = __ballot_sync(0xffffffffu, p1),
-                                       b2 = __ballot_sync(0xffffffffu, p2),
-                                       b3 = __ballot_sync(0xffffffffu, p3);
-                        const int c1 = cn + __popc(b0), c2 = c1 + __popc(b1),
-                                  c3 = c2 + __popc(b2);
-                        if (p0) A.cq[cn + __popc(b0 & lt)] = (unsigned short)eb;
-                        if (p1) A.cq[c1 + __popc(b1 & lt)] = (unsigned short)(eb + 32u);
-                        if (p2) A.cq[c2 + __popc(b2 & lt)] = (unsigned short)(eb + 64u);
-                        if (p3) A.cq[c3 + __popc(b3 & lt)] = (unsigned short)(eb + 96u);
-                        cn = c3 + __popc(b3);
-                        if (!GOFR_CHECK(cn <= CQ, P.err)) cn = CQ;
-                        // room for the next first atom's entries
-                        if (cn > CQ - CQ_ROOM) flush_q(bufp);
                     }
-                    // the entries name records of this buffer: bin them before it is refilled
-                    if (cn > 0) flush_q(bufp);
-                    fence_proxy_async_smem();
-                    __syncwarp();  // every lane done with buffer b
-                    if (b) have1 = issue(w, 1);
-                    else have0 = issue(w, 0);
                 }
-                if (A.qn > QW / 2) drain_queue();
+                resolve(nn);  // the entries name first atoms of this batch
+                nn = 0;
+                __syncwarp();  // every lane done with the first atoms and segments
             }
         }
-        if (!dead) drain_queue();
-        __syncthreads();  // every warp done with this item
-        // a u32 shared bin holds the item's hits exactly only while the item
-        // evaluated fewer than 2^32 pairs (the host sizes items far below)
-        if (tid == 0 && s_pairs > 0xffffffffull) {
-            atomicOr(P.err, ERRW_HIST_OVERFLOW);
-            s_abort = 1;
+        recheck(qn);
+        qn = 0;
+        g0 = g1;
         }
-        __syncthreads();
-        const bool abort = s_abort != 0;
-        // add the item's histogram copies to its lag's counts, then clear them
-        for (int i = tid; i < hlen; i += NT) {
-            unsigned long long v = 0;
-#pragma unroll
-            for (int c = 0; c < HCOPY; ++c) {
-                v += hist[c * hist_cap + i];
-                hist[c * hist_cap + i] = 0u;
-            }
-            if (v && !abort)
-                atomicAdd(P.counts + (long long)lag_idx * P.every * hlen + i, v);
+    }
+    __syncthreads();
+    if (cur_lag >= 0 && !lost) flush(cur_lag);
+    if (tid == 0) {
+        if (lost) atomicOr(P.err, ERRW_HIST_OVERFLOW);
+        // the last CTA leaves the queue as the next launch on the stream takes it
+        __threadfence();
+        if (atomicAdd(C.queue + 1, 1u) == gridDim.x - 1) {
+            C.queue[0] = 0u;
+            C.queue[1] = 0u;
         }
-        __syncthreads();
-        if (abort) break;
     }
     for (int o = 16; o > 0; o >>= 1) {
         n_cand += __shfl_xor_sync(0xffffffffu, n_cand, o);
@@ -548,14 +578,14 @@ __global__ void __launch_bounds__(NWARP * 32, 16 / NWARP) k_pairs_cellw(const Ce
 int cellw_smem_bytes(int nch, int nbin, int ntypes, int cta_warps, int hcopy)
 {
     using namespace cellw;
-    size_t b = sizeof(WarpArea) * cta_warps + (size_t)nbin * 8 +
-               (size_t)hcopy * nch * nbin * 4 + (size_t)ntypes * ntypes * 2;
+    const size_t hist_cap = (size_t)nch * (nbin + 1) + 1;
+    size_t b = sizeof(WarpArea) * cta_warps + (size_t)hcopy * hist_cap * 4 +
+               (size_t)ntypes * ntypes * 2;
     return (int)((b + 127) / 128 * 128);
 }
 
 int cellw_chunk_records() { return cellw::CH; }
 int cellw_batch_atoms() { return cellw::FA; }
-int cellw_chunk_pieces() { return cellw::MAXP; }
 
 // Sorted AoS copy of every frame: {x, y, z, type << 24 | id} with the block
 // kernel's coordinates (w = x - n L, n = floor((x - xlo) / L), one FMA in
@@ -616,12 +646,12 @@ int launch_cell_scatter_w(const double *pos64, const unsigned char *types8, size
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
-template <int NWARP, int HCOPY>
+template <int NWARP, int HCOPY, int MODE>
 static int launch_cellw_shape(const CellwLaunch &C, int num_sms, cudaStream_t s)
 {
     using namespace cellw;
     constexpr int NT = NWARP * 32;
-    auto kern = k_pairs_cellw<NWARP, HCOPY>;
+    auto kern = k_pairs_cellw<NWARP, HCOPY, MODE>;
     const int smem = cellw_smem_bytes(C.pair.nch, C.pair.nbin, C.pair.ntypes, NWARP, HCOPY);
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) !=
         cudaSuccess)
@@ -630,21 +660,33 @@ static int launch_cellw_shape(const CellwLaunch &C, int num_sms, cudaStream_t s)
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, NT, smem) != cudaSuccess)
         return -1;
     if (per_sm < 1) return -2;
+    // at least a warp block a warp
+    const long long units = C.pair.n_items * C.nw[0] * C.nw[1] * C.nw[2];
     long long grid = (long long)num_sms * per_sm;
-    if (grid > C.pair.n_items) grid = C.pair.n_items;
-    kern<<<(unsigned)grid, NT, smem, s>>>(C, C.pair.nbin, C.pair.nch * C.pair.nbin);
+    if (grid > (units + NWARP - 1) / NWARP) grid = (units + NWARP - 1) / NWARP;
+    kern<<<(unsigned)grid, NT, smem, s>>>(C);
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
+}
+
+template <int MODE>
+static int launch_cellw_mode(const CellwLaunch &C, int num_sms, cudaStream_t s)
+{
+    if (C.cta_warps == 16) {
+        return C.hcopy == 2 ? launch_cellw_shape<16, 2, MODE>(C, num_sms, s)
+                            : launch_cellw_shape<16, 1, MODE>(C, num_sms, s);
+    }
+    return C.hcopy == 2 ? launch_cellw_shape<8, 2, MODE>(C, num_sms, s)
+                        : launch_cellw_shape<8, 1, MODE>(C, num_sms, s);
 }
 
 int launch_cellw_pairs(const CellwLaunch &C, int num_sms, cudaStream_t s)
 {
     if (C.pair.n_items <= 0) return 0;
-    if (C.cta_warps == 16) {
-        return C.hcopy == 2 ? launch_cellw_shape<16, 2>(C, num_sms, s)
-                            : launch_cellw_shape<16, 1>(C, num_sms, s);
+    switch (C.pair.rm.mode) {
+    case 0: return launch_cellw_mode<0>(C, num_sms, s);
+    case 1: return launch_cellw_mode<1>(C, num_sms, s);
+    default: return launch_cellw_mode<2>(C, num_sms, s);
     }
-    return C.hcopy == 2 ? launch_cellw_shape<8, 2>(C, num_sms, s)
-                        : launch_cellw_shape<8, 1>(C, num_sms, s);
 }
 
 }  // namespace gofr

@@ -97,6 +97,130 @@ __device__ __forceinline__ void red_shared_add1_if(unsigned addr, bool p)
 }
 
 // ---------------------------------------------------------------------------
+// packed f32x2 arithmetic (PTX ISA add/sub/mul/fma .f32x2, sm_100+)
+// ---------------------------------------------------------------------------
+typedef unsigned long long f2;
+
+__device__ __forceinline__ f2 f2pk(float a, float b)
+{
+    f2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void f2up(f2 v, float &a, float &b)
+{
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+}
+__device__ __forceinline__ f2 f2add(f2 a, f2 b)
+{
+    f2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f2 f2sub(f2 a, f2 b)
+{
+    f2 r;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f2 f2mul(f2 a, f2 b)
+{
+    f2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f2 f2fma(f2 a, f2 b, f2 c)
+{
+    f2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+
+
+// ---------------------------------------------------------------------------
+// Binning a pair where it is found
+// ---------------------------------------------------------------------------
+//
+// Every pair whose d2 is formed is added to a histogram cell at once: two
+// pairs of a lane (FP32 d2 in one f32x2) take rs = rsqrt(d2) (hardware
+// approximation, relative error <= 2^-22.9), q' = (d2 inv_dr) rs + q_off =
+// r / dr - rmin / dr - 1/2, t = q' + 1.5 2^23, whose low mantissa bits are
+// n = rint(q'), and fr = q' - n.  The cell is n, with t clamped into the
+// histogram row: a row has nbin cells and an unread one, and a pair beyond
+// rmax ends in the unread cell, one below rmin in that of the row before (the
+// lanes of a warp that add to one cell are merged: an unread cell for every lane
+// took a quarter more shared-memory wavefronts).  A pair with |fr| > lim may belong to
+// the next bin (lim leaves out what r, d2 and the reference's own rounding can
+// move a pair by; host: radial_map): `bit` is set in the lane's mask, and the
+// caller takes the pair out of its cell again and recomputes it in FP64.
+//
+// Eleven and a half issue slots per 32 pairs with d2's own (packed: 5 1/2;
+// rsqrt, clamp, address, reduction, compare, mask), whatever share of the
+// pairs is within rmax.  Queueing the candidates and binning the queue 32 at a
+// time cost ~45 (a queue entry ~80 lane instructions).  The reduction is not
+// predicated: a predicated red.shared is compiled into a branch around it
+// (three more slots and a divergence each), which measured 5 % slower than
+// letting every lane add somewhere.
+constexpr float RADIAL_MAGIC = 12582912.0f;       // 1.5 * 2^23
+constexpr unsigned RADIAL_MAGIC_BITS = 0x4b400000u;
+// start of the sum d2: d2 = 0 would make rsqrt infinite and q' NaN (adds 1e-15 to r at most)
+constexpr float RADIAL_TINY = 1e-30f;
+
+__device__ __forceinline__ float rsqrt_bin(float x)
+{
+    float r;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+
+// q' of one pair's d2, with bin_pair2's operations.
+__device__ __forceinline__ float radial_q(float d2, const RadialMap &m)
+{
+    return __fmaf_rn(__fmul_rn(d2, m.inv_dr), rsqrt_bin(d2), m.q_off);
+}
+
+// row: shared-memory address of the pair's histogram row minus 4 times the
+// bits of 1.5 2^23, so cell n is t's bits shifted by two plus it.
+template <int MODE>
+__device__ __forceinline__ void bin_one(float t, float fr, const RadialMap &m, unsigned row,
+                                        unsigned bit, unsigned &mask)
+{
+    float c = fminf(t, m.t_end);  // no record (NaN): the unread cell
+    if (MODE != 0) c = fmaxf(c, RADIAL_MAGIC - 1.0f);
+    asm volatile("red.shared.add.u32 [%0], 1;" ::"r"((__float_as_uint(c) << 2) + row) : "memory");
+    if (MODE == 2) {
+        asm("{\n\t.reg .pred p;\n\t.reg .f32 a;\n\tabs.f32 a, %1;\n\t"
+            "setp.lt.f32 p, %4, %5;\n\tsetp.gt.or.f32 p, a, %2, p;\n\t@p or.b32 %0, %0, %3;\n\t}"
+            : "+r"(mask)
+            : "f"(fr), "f"(m.lim), "r"(bit), "f"(t), "f"(m.t_ok));
+    } else {
+        asm("{\n\t.reg .pred p;\n\t.reg .f32 a;\n\tabs.f32 a, %1;\n\t"
+            "setp.gt.f32 p, a, %2;\n\t@p or.b32 %0, %0, %3;\n\t}"
+            : "+r"(mask)
+            : "f"(fr), "f"(m.lim), "r"(bit));
+    }
+}
+
+// d2 of two pairs into their histogram rows; inv, off: inv_dr and q_off in both lanes.
+template <int MODE>
+__device__ __forceinline__ void bin_pair2(f2 d2, f2 inv, f2 off, const RadialMap &m, unsigned row0,
+                                          unsigned row1, unsigned bit, unsigned &mask0,
+                                          unsigned &mask1)
+{
+    const f2 MAG = f2pk(RADIAL_MAGIC, RADIAL_MAGIC);
+    float a, b;
+    f2up(d2, a, b);
+    const f2 q = f2fma(f2mul(d2, inv), f2pk(rsqrt_bin(a), rsqrt_bin(b)), off);
+    const f2 t = f2add(q, MAG);
+    const f2 fr = f2sub(q, f2sub(t, MAG));
+    float t0, t1, f0, f1;
+    f2up(t, t0, t1);
+    f2up(fr, f0, f1);
+    bin_one<MODE>(t0, f0, m, row0, bit, mask0);
+    bin_one<MODE>(t1, f1, m, row1, bit, mask1);
+}
+
+// ---------------------------------------------------------------------------
 // FP64 restatement of the reference pair arithmetic.
 // Every operation is an explicitly rounded IEEE intrinsic, so nvcc cannot
 // contract a multiply and an add into an FMA: the result is bit-identical to
@@ -197,6 +321,35 @@ __device__ __forceinline__ void wrap_tric64(const double p[3], const double lo[3
     const double x2 = __fma_rn(-ny, tilt[0], x1);
     const double nx = floor(__ddiv_rn(__dsub_rn(x2, lo[0]), L[0]));
     w[0] = __fma_rn(-nx, L[0], x2);
+}
+
+// The reference's bin of atom ia with itself, frame fo against frame fl (-1:
+// not counted).  The pair kernels bin an atom's pair with itself like any
+// other, into the channel of distinct atoms (an index compare per pair would
+// cost a tenth of their inner loop); this bin is where that count went, to be
+// moved to the channel of the same atom.  FP32 on the frames' own coordinates
+// where the difference needs no minimum image and lies off every bin edge by
+// the all-pairs kernel's bound, else the reference's FP64.
+template <bool TRI>
+__device__ __forceinline__ int self_bin(const PairLaunch &P, long long fo, long long fl, int ia)
+{
+    const float *a = P.pos32 + fo * 3 * (long long)P.NP + ia;
+    const float *b = P.pos32 + fl * 3 * (long long)P.NP + ia;
+    const float dx = __fsub_rn(a[0], b[0]), dy = __fsub_rn(a[P.NP], b[P.NP]),
+                dz = __fsub_rn(a[2 * (long long)P.NP], b[2 * (long long)P.NP]);
+    if (fmaxf(fabsf(dx), fmaxf(fabsf(dy), fabsf(dz))) <= P.rm.self_max) {
+        const float q = radial_q(
+            __fmaf_rn(dz, dz, __fmaf_rn(dy, dy, __fmaf_rn(dx, dx, RADIAL_TINY))), P.rm);
+        const float t = __fadd_rn(q, RADIAL_MAGIC);
+        if (fabsf(__fsub_rn(q, __fsub_rn(t, RADIAL_MAGIC))) <= P.rm.lim_self &&
+            (P.rm.mode != 2 || t >= P.rm.t_ok || t < P.rm.t_lo)) {
+            const int n = (int)(__float_as_uint(t) - RADIAL_MAGIC_BITS);
+            return t <= P.rm.t_hi && t >= P.rm.t_lo && n >= 0 && n < P.nbin ? n : -1;
+        }
+    }
+    const double *xi = P.pos64 + (fo * P.N + ia) * 3, *xj = P.pos64 + (fl * P.N + ia) * 3;
+    const double d2 = ref_d2<TRI>(xi[0], xi[1], xi[2], xj[0], xj[1], xj[2], P.box64 + fo * 9, P.err);
+    return ref_bin(d2, P.rmin, P.dr, P.rmin2, P.rmax2, P.nbin);
 }
 
 }  // namespace gofr

@@ -27,7 +27,8 @@ enum : unsigned {
 #endif
 
 // Stats slots (unsigned long long) on the device.
-enum : int { ST_CANDIDATES = 0, ST_RECHECKS = 1, ST_EVALUATED = 2, ST_COUNT = 4 };
+// ST_QUEUE: the two words of the warp-streamed kernel's chunk queue.
+enum : int { ST_CANDIDATES = 0, ST_RECHECKS = 1, ST_EVALUATED = 2, ST_QUEUE = 3, ST_COUNT = 4 };
 
 // Per-frame FP32 box parameters for the FP32 kernels (12 floats, 48 B).
 //   L[3]    full edges 2*lh rounded to float
@@ -38,6 +39,22 @@ struct Box32 {
     float invL[3];
     float tilt[3];
     float pad[3];
+};
+
+// Bin map of the kernels that bin a pair where they find it (the comment at
+// bin_pair2 in gofr_device.cuh): q' = sqrt(d2) inv_dr + q_off, n = rint(q'); the
+// pair is in bin n for certain when |q' - n| <= lim (t_lo and t_hi: the n, plus
+// 1.5 2^23, that a pair of the window can come out at).
+//   mode 0: rmin = 0 (n is never negative); 1: rmin > 0; 2: rmin < 0 (only
+//   pairs beyond -rmin count: n < t_ok - 1.5 2^23 is never certain)
+struct RadialMap {
+    float inv_dr, q_off;
+    float t_end;      // nbin + 1.5 2^23: the unread cell
+    float t_hi, t_lo, t_ok;
+    float lim;        // negative: no pair is certain
+    float lim_self;   // the same for an unwrapped difference of the FP32 frames
+    float self_max;   // |component| up to which that difference needs no image
+    int mode;
 };
 
 // One launch of an all-pairs kernel over (lag, i-tile, origin) items.
@@ -63,6 +80,7 @@ struct PairLaunch {
     float rmin_f, inv_dr_f;   // bin guess
     float wlim;               // wrap check: |frac| > wlim flags a recheck
     double rmin, rmax, dr, rmin2, rmax2;  // reference binning constants
+    RadialMap rm;
     int tric;
     int wchk;                 // batched kernel: per-pair wrap-decision check on
     int ghist;                // histogram too large for shared memory: atomics go
@@ -93,8 +111,8 @@ struct CellLaunch {
 };
 
 // One launch of the warp-streamed cell-list kernel (gofr_cellw.cu): items
-// are (lag, origin, part), pair.n_items = n_lags * n_orig * parts; each warp
-// takes blocks of w[0] x w[1] x w[2] cells of the part's range.
+// are (lag, origin), pair.n_items = n_lags * n_orig, each of nw[0] nw[1] nw[2]
+// warp blocks of w[0] x w[1] x w[2] cells; a warp takes one block at a time.
 //
 // Cells are an axis-aligned grid of the box [lo, lo + L) (triclinic: the
 // upper-triangular cell's axis-aligned fundamental domain).  A warp block's
@@ -120,7 +138,8 @@ struct CellwLaunch {
     int nw[3];                     // warp blocks per axis
     int reach;                     // neighbour cells per side
     int r;                         // records per lane (4; kept in plans and tuner keys)
-    int parts;                     // parts of the warp blocks per (lag, origin)
+    long long most;                // warp blocks of a CTA's chunk at most
+    unsigned *queue;               // {next chunk, CTAs done}, zero before and after a launch
     int cta_warps;                 // warps per CTA: 8 (two CTAs per SM) or 16 (one)
     int hcopy;                     // copies of the shared histogram (privatisation depth: 1, 2)
     int nz_lo, nz_hi;              // neighbourhood layers (see above)
@@ -132,7 +151,6 @@ struct CellwLaunch {
 int cellw_smem_bytes(int nch, int nbin, int ntypes, int cta_warps = 8, int hcopy = 1);
 int cellw_chunk_records();  // neighbour records per chunk (4 per lane)
 int cellw_batch_atoms();    // first atoms per batch (each batch streams the neighbourhood)
-int cellw_chunk_pieces();   // bulk copies per chunk at most
 // box_internal {xlo, ylo, zlo, lx/2, ly/2, lz/2, xy, xz, yz}; tric: the
 // coordinates are reduced into the axis-aligned cell by the lattice (z, then
 // y, then x), else per axis.

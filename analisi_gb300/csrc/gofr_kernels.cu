@@ -110,46 +110,6 @@ __device__ __forceinline__ void recheck_pair(const double *__restrict__ pos64,
     if (b >= 0 && GOFR_CHECK(b < nbin && ch >= 0, err)) hist_add(hist, gcounts, ch, nbin, b);
 }
 
-// ---------------------------------------------------------------------------
-// packed f32x2 arithmetic (PTX ISA add/sub/mul/fma .f32x2, sm_100+)
-// ---------------------------------------------------------------------------
-typedef unsigned long long f2;
-
-__device__ __forceinline__ f2 f2pk(float a, float b)
-{
-    f2 r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-    return r;
-}
-__device__ __forceinline__ void f2up(f2 v, float &a, float &b)
-{
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
-}
-__device__ __forceinline__ f2 f2add(f2 a, f2 b)
-{
-    f2 r;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ f2 f2sub(f2 a, f2 b)
-{
-    f2 r;
-    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ f2 f2mul(f2 a, f2 b)
-{
-    f2 r;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ f2 f2fma(f2 a, f2 b, f2 c)
-{
-    f2 r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
-
 // Box constants of one origin frame, duplicated into both f32x2 lanes.
 struct Box2 {
     f2 invL[3], negL[3];

@@ -29,7 +29,7 @@ EXPORTED = [
     "gofr_batch_output_layout", "gofr_batch_run", "gofr_measure_peaks",
     "gofr_run_f64_noalloc", "gofr_run_windows", "gofr_set_centres", "gofr_msd_output_size",
     "gofr_msd_run", "gofr_neigh_layout", "gofr_neigh_run", "gofr_run_normalized",
-    "gofr_run_streamed", "gofr_cellw_tables", "gofr_plan_query",
+    "gofr_run_streamed", "gofr_cellw_tables", "gofr_plan_query", "gofr_radial_query",
 ]
 
 
@@ -156,6 +156,8 @@ def load_library(path=None):
                                     ctypes.POINTER(ctypes.c_float), dp]
     L.gofr_plan_query.argtypes = [dp, ctypes.c_int, dp, dp, ctypes.c_size_t, ctypes.c_uint,
                                   ctypes.POINTER(Params), ip]
+    L.gofr_radial_query.argtypes = [dp, ctypes.c_int, dp, dp, ctypes.c_size_t, ctypes.c_uint,
+                                    ctypes.POINTER(Params), dp]
     L.gofr_batch_set.argtypes = [vp, ctypes.POINTER(TrajDesc), ctypes.c_uint]
     L.gofr_batch_output_layout.argtypes = [vp, ctypes.c_uint, ctypes.POINTER(ctypes.c_size_t),
                                            ctypes.POINTER(ctypes.c_size_t)]
@@ -182,7 +184,7 @@ def load_library(path=None):
                  "gofr_bin_thresholds", "gofr_batch_set", "gofr_batch_output_layout",
                  "gofr_batch_run", "gofr_measure_peaks", "gofr_run_f64_noalloc",
                  "gofr_run_windows", "gofr_run_normalized", "gofr_run_streamed",
-                 "gofr_cellw_tables", "gofr_plan_query"):
+                 "gofr_cellw_tables", "gofr_plan_query", "gofr_radial_query"):
         getattr(L, name).restype = ctypes.c_int
     if path is None:
         _lib = L
@@ -237,6 +239,22 @@ def plan_query(box, triclinic, coord_min, coord_max, natoms, ntypes, params):
     return {"kernel": int(out[0]), "reach": int(out[1]), "cells": tuple(int(v) for v in out[2:5]),
             "block": tuple(int(v) for v in out[5:8]), "cta_warps": int(out[8]),
             "wrapcheck": bool(out[9])}
+
+
+def radial_query(box, triclinic, coord_min, coord_max, natoms, ntypes, params):
+    """The bin map of the kernel plan_query names (host code, no GPU): a dict
+    {inv_dr, q_off, lim, lim_self, t_lo, t_hi, t_ok, self_max} of float32."""
+    L = load_library()
+    b = np.ascontiguousarray(box, dtype=np.float64)
+    lo = np.ascontiguousarray(coord_min, dtype=np.float64)
+    hi = np.ascontiguousarray(coord_max, dtype=np.float64)
+    out = np.zeros(8)
+    rc = L.gofr_radial_query(_dp(b), BOX_TRICLINIC if triclinic else BOX_ORTHO, _dp(lo), _dp(hi),
+                             int(natoms), int(ntypes), ctypes.byref(params), _dp(out))
+    if rc != GOFR_OK:
+        raise GofrError(rc, "no FP32 bin map for these parameters")
+    return dict(zip(("inv_dr", "q_off", "lim", "lim_self", "t_lo", "t_hi", "t_ok", "self_max"),
+                    out.astype(np.float32)))
 
 
 def cellw_tables(box, triclinic, coord_min, coord_max, rmax, nc):

@@ -111,7 +111,8 @@ typedef struct gofr_params {
 typedef struct gofr_stats {
     unsigned long long pairs;        /* ordered pairs of the reference loop (N^2 per lag/origin) */
     unsigned long long evaluated;    /* pairs whose distance was computed on the GPU */
-    unsigned long long candidates;   /* FP32 pairs inside the accept window (+ its error bound) */
+    unsigned long long candidates;   /* FP32 pairs inside the accept window (+ its error bound;
+                                        warp-streamed kernel: pairs counted) */
     unsigned long long rechecks;     /* pairs recomputed in FP64 */
     double kernel_ms;                /* device time of the pair kernel(s), CUDA events */
     double total_ms;                 /* device time of the whole run incl. copies */
@@ -253,6 +254,21 @@ int gofr_bin_thresholds(double rmin, double rmax, unsigned nbin, double *th);
 int gofr_plan_query(const double *box, int box_kind, const double *coord_min,
                     const double *coord_max, size_t natoms, unsigned ntypes,
                     const gofr_params *p, int *out);
+
+/* The bin map of the kernel that gofr_plan_query names (host only; arguments as
+ * there; FP32 kernels): a pair's FP32 d2 goes to bin rint(q), q = (d2 inv_dr)
+ * rsqrt(d2) + q_off, for certain when |q - rint(q)| <= lim, and is recomputed
+ * in FP64 otherwise.  out (8 doubles): inv_dr, q_off, lim, the lim of an
+ * atom's pair with itself, the smallest and largest bin + 1.5 2^23 that a pair
+ * of the window can come out at, the first bin + 1.5 2^23 that can be certain
+ * (rmin < 0), and the |component| up to which an atom's pair with itself takes
+ * no minimum image.  GOFR_ERR_UNSUPPORTED when the plan is the FP64 kernel or
+ * no pair can count.  No reference counterpart (its binning is
+ * lib/src/gofrt.cpp:104,114-118): it lets the margin be checked without a
+ * GPU. */
+int gofr_radial_query(const double *box, int box_kind, const double *coord_min,
+                      const double *coord_max, size_t natoms, unsigned ntypes,
+                      const gofr_params *p, double *out);
 
 /* Neighbourhood tables of the warp-streamed cell-list kernel (host only, no
  * device work) for one box (internal format, 6 or 9 doubles), the
