@@ -111,6 +111,8 @@ struct gofr_ctx {
     size_t cap_gofr = 0;
     double *d_chfac = nullptr;
     size_t cap_chfac = 0;
+    long long *d_primos = nullptr;      // first frames of a run's windows
+    size_t cap_primos = 0;
     size_t batch_total = 0;
     unsigned long long launches = 0;  // kernels launched on this context
     // batched trajectories (gofr_batch_set / gofr_batch_run)
@@ -118,7 +120,7 @@ struct gofr_ctx {
         std::vector<PairLaunch> launches;       // one per trajectory (FP32 path)
         std::vector<WorkDesc> work[2];          // descriptors, orthorhombic / triclinic
         std::vector<int> f64_trajs;             // trajectories that need the FP64 kernel
-        int max_nbin = 1, max_nch = 1, max_ntypes = 1;
+        int max_cells = 1, max_ntypes = 1, mode = 0;
         PairLaunch *d_launches = nullptr;
         WorkDesc *d_work[2] = {nullptr, nullptr};
         unsigned *d_head = nullptr;             // queue heads [2]
@@ -403,6 +405,38 @@ Bound error_bound(const TrajDev &t)
     return b;
 }
 
+// Component bound of the all-pairs kernel in orthorhombic boxes, whose atoms are
+// moved into the box before the difference (u = 2^-24, per axis; maxima over
+// frames):
+//   w = fl32(a - k fl32(L)), k = rint(a / L), |k| <= kw:  |w - (x - shift - k L)| <=
+//       eps + kw |fl32(L) - L| + u W, |w| <= W = L/2 + what a quotient next to a
+//       half-integer leaves
+//   d = fl32(w_i - w_j):                  u 2 W
+//   |d| or fl32(fl32(L) - |d|):           |fl32(L) - L| (and u of itself, counted with
+//                                         the component in radial_margin)
+// plus the reference's own rounding as in error_bound.  Its image is the
+// nearest, |d_ref| = min(|d|, L - |d|), wherever that is certain.
+Bound error_bound_boxed(const TrajDev &t)
+{
+    Bound b = error_bound(t);  // kmax, and the fields a triclinic box keeps
+    if (t.tric) return b;
+    const double u24 = std::ldexp(1.0, -24), u53 = std::ldexp(1.0, -53);
+    const BoxStats &s = t.bs;
+    for (int k = 0; k < 3; ++k) {
+        const double eps = t.M[k] * u24 * (1.0 + std::ldexp(1.0, -20)) +
+                           t.M[k] * std::ldexp(1.0, -52);
+        const double A = t.M[k] + eps;
+        const double kw = std::floor(A / s.Lmin[k] * (1.0 + 1e-6) + 0.5 + 1e-6);
+        const double W = 0.5 * s.Lmax[k] * (1.0 + 1e-6) + (A + s.Lmax[k]) * 4.0 * u24;
+        const double ew = eps + kw * s.eL[k] + u24 * W;
+        const double D = 2.0 * t.M[k] * (1.0 + std::ldexp(1.0, -40));
+        b.e[k] = (2.0 * ew + 2.0 * u24 * W + s.eL[k] + u53 * D +
+                  b.kmax[k] * u53 * (D + s.Lmax[k])) * (1.0 + std::ldexp(1.0, -20));
+    }
+    b.enorm = std::sqrt(b.e[0] * b.e[0] + b.e[1] * b.e[1] + b.e[2] * b.e[2]);
+    return b;
+}
+
 // Per-axis error bound of the cell-list kernel's FP32 differences, for an
 // orthorhombic box that is the same in every frame (u = 2^-24, v = 2^-53,
 // per axis: xlo, L, L32 = fl32(L), c = fl64(xlo + L/2)).
@@ -666,6 +700,17 @@ Bound radial_bound_cells(const TrajDev &t, const CellwGeom &g, double R)
     return b;
 }
 
+// |component| short of L/2 by this much or less: the image is not certain (the
+// component's error, its own rounding and that of the limit).
+float wrap_tolerance(const TrajDev &t)
+{
+    const Bound b = error_bound_boxed(t);
+    double tol = 0.0;
+    for (int k = 0; k < 3; ++k)
+        tol = std::max(tol, 1.01 * b.e[k] + t.bs.eL[k] + 4.0 * std::ldexp(1.0, -24) * t.bs.Lmax[k]);
+    return f_up(tol);
+}
+
 inline double Efun(const Bound &b, double s)
 {
     if (s < 0) s = 0;
@@ -746,7 +791,7 @@ RadialMap radial_map(const TrajDev &t, const Bound &b, const Bound &b1, const go
     m.t_end = (float)(magic + p.nbin);
     m.t_hi = (float)(magic + p.nbin + wide);
     m.t_lo = (float)(magic + (m.mode == 2 ? edge - 1.0 : (m.mode == 1 ? -1.0 : 0.0)) - wide);
-    m.t_ok = (float)(magic + edge + 1.0);
+    m.t_ok = m.mode == 2 ? (float)(magic + edge + 1.0) : 0.0f;
     m.self_max = f_down(0.25 * std::min(t.bs.Lmin[0], std::min(t.bs.Lmin[1], t.bs.Lmin[2])));
     return m;
 }
@@ -966,8 +1011,8 @@ RadialMap plan_radial_map(const TrajDev &t, const gofr_params &p, const Plan &pl
 {
     const BinMap bm(p.rmin, p.rmax, p.nbin);
     const Bound b1 = error_bound(t);
-    return radial_map(t, pl.cellw ? radial_bound_cells(t, pl.geom, bm.rmax + 2.0 * bm.dr) : b1, b1,
-                      p, pl.th);
+    return radial_map(t, pl.cellw ? radial_bound_cells(t, pl.geom, bm.rmax + 2.0 * bm.dr)
+                                  : error_bound_boxed(t), b1, p, pl.th);
 }
 
 // One cell-list configuration: cells of edge >= rmax (1 + 1e-6) / reach, so
@@ -1293,7 +1338,8 @@ int make_plan(gofr_ctx *ctx, const TrajDev &t, const gofr_params &p, Plan &pl,
                     "the FP32 kernel needs finite rmin < rmax and nbin < 2^24");
     pl.b = error_bound(t);
     certify(pl.b, pl.th.data(), p.nbin, pl.w);
-    const double emax = std::max(pl.b.e[0], std::max(pl.b.e[1], pl.b.e[2]));
+    const Bound bb = error_bound_boxed(t);
+    const double emax = std::max({pl.b.e[0], pl.b.e[1], pl.b.e[2], bb.e[0], bb.e[1], bb.e[2]});
     const double reach = std::sqrt((double)pl.w.hi_f) * (1.0 + std::ldexp(1.0, -20)) +
                          2.0 * emax + 1e-9;
     pl.kind = 0;
@@ -1384,6 +1430,79 @@ void set_cellw_geometry(CellwLaunch &C, const CellwGeom &g)
     for (int k = 0; k < CELLW_NSHIFT; ++k) C.shift[k] = g.shift[k];
 }
 
+// A unit of the all-pairs kernel: gs first atoms against jc chunks of second
+// atoms, ng groups and nj parts of n_i and N atoms.  A unit loads its first
+// atoms once (about 250 instructions per 32) and each chunk once (about 150),
+// and a first atom against a chunk is about 80: 64 atoms against the whole
+// frame unless that makes fewer than `want` units of `frames` (lag, origin)
+// pairs; then 32 atoms, then fewer chunks, and fewer atoms only when one chunk
+// is left.
+struct AllpairsUnit {
+    int gs = ALLPAIRS_GROUP, ng = 1, jc = 1, nj = 1;
+};
+
+AllpairsUnit allpairs_unit(size_t n_i, size_t N, double frames, double want)
+{
+    AllpairsUnit a;
+    const int chunks = (int)((N + ALLPAIRS_CHUNK - 1) / ALLPAIRS_CHUNK);
+    auto groups = [&](int gs) { return std::ceil((double)n_i / gs); };
+    a.jc = chunks;
+    if (frames * groups(a.gs) < want) a.gs = 32;
+    const double units = frames * groups(a.gs);
+    if (units < want)
+        a.jc = (int)std::max(1.0, std::floor(chunks / std::ceil(want / std::max(units, 1.0))));
+    while (a.gs > 8 && frames * groups(a.gs) * chunks < want) a.gs /= 2;
+    a.nj = (chunks + a.jc - 1) / a.jc;
+    a.ng = (int)groups(a.gs);
+    return a;
+}
+
+// Units of a CTA's chunk at most: fewer than 2^31 pairs between two flushes (or
+// a unit a warp), so that no u32 shared bin overflows (the kernel checks).
+long long allpairs_most(size_t N, const AllpairsUnit &a)
+{
+    const double pairs = std::min((double)N, (double)a.jc * ALLPAIRS_CHUNK) * a.gs;
+    return (long long)std::max(8.0, std::floor(2147483648.0 / pairs));
+}
+
+// The unit of a batched member, so that a descriptor of `target` pairs holds 32
+// units or more (four for each of a CTA's warps).
+AllpairsUnit batch_unit(size_t N, unsigned long long target)
+{
+    const double n2 = (double)N * (double)N;
+    return allpairs_unit(N, N, 1.0, 32.0 * n2 / (double)target);
+}
+
+// Work descriptors of trajectory k, each of about `target` pairs (never more
+// than 2^30 unless eight units have more), appended to out with their pairs.
+struct WorkCost {
+    unsigned long long c;
+    WorkDesc w;
+    bool tri;
+};
+
+void add_descriptors(int k, const TrajDev &t, const RunShape &rs, const AllpairsUnit &a,
+                     unsigned long long target, std::vector<WorkCost> &out)
+{
+    const unsigned long long units =
+        (unsigned long long)a.ng * a.nj * rs.n_orig * rs.n_lags;
+    const unsigned long long one =
+        std::min<unsigned long long>(t.N, (unsigned long long)a.jc * ALLPAIRS_CHUNK) * a.gs;
+    const unsigned long long per = std::min<unsigned long long>(target, 1ull << 30) / one;
+    const unsigned long long len = std::max<unsigned long long>(8, (per + 7) / 8 * 8);
+    for (unsigned long long u = 0; u < units; u += len) {
+        const unsigned long long e = std::min(units, u + len);
+        out.push_back({(e - u) * one, WorkDesc{k, 0, (long long)u, (long long)e}, t.tric != 0});
+    }
+}
+
+// Pairs per descriptor: about sixteen descriptors per CTA of the grid (four per
+// SM), so that the last ones end together.
+unsigned long long batch_target(unsigned long long total, int num_sms)
+{
+    return std::max<unsigned long long>(total / ((unsigned long long)num_sms * 4 * 16), 1ull << 19);
+}
+
 // Warp blocks of a CTA's chunk at most: chunks of fewer than 2^31 all-pairs-
 // equivalent pairs (or a block a warp), so that no u32 shared bin overflows
 // between two flushes (the kernel checks the pairs it evaluated).
@@ -1459,8 +1578,11 @@ int ensure_cells(gofr_ctx *ctx, const TrajDev &t, const Plan &pl)
 
 // Queue every launch of one trajectory's calculate on the stream; counts is
 // a device pointer to data_length*(nparts>1?nparts:1) zeroed counts.
+// nwin > 1 or d_primos: calculate(d_primos[w]) for each window, counts of one
+// after the other's (the all-pairs kernel only).
 int enqueue_run(gofr_ctx *ctx, const TrajDev &t, const gofr_params &p, const RunShape &rs,
-                const Plan &pl, unsigned long long *counts, unsigned long long *pairs_out)
+                const Plan &pl, unsigned long long *counts, unsigned long long *pairs_out,
+                unsigned nwin = 1, const long long *d_primos = nullptr)
 {
     *pairs_out = 0;
     if (pl.empty || rs.n_lags == 0 || rs.n_orig == 0 || t.N == 0) return GOFR_OK;
@@ -1469,22 +1591,19 @@ int enqueue_run(gofr_ctx *ctx, const TrajDev &t, const gofr_params &p, const Run
     if (rc) return rc;
     CK(cudaMemcpyAsync(ctx->d_chtab, tab.data(), tab.size() * sizeof(unsigned short),
                        cudaMemcpyHostToDevice, ctx->stream));
-    if (pl.kind == 0) {
-        rc = ensure(ctx, ctx->d_win, ctx->cap_win, pl.w.win.size());
-        if (rc) return rc;
-        CK(cudaMemcpyAsync(ctx->d_win, pl.w.win.data(), pl.w.win.size() * sizeof(float2),
-                           cudaMemcpyHostToDevice, ctx->stream));
-    }
     int max_smem = 0;
     CK(cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device));
     // a histogram that would not leave room for one CTA (with headroom) per SM
     // goes to global memory: slower atomics, same counts
-    const bool ghist = pairs_smem_bytes(pl.kind, (int)rs.nch, (int)p.nbin, (int)t.ntypes) >
-                       max_smem - 8192;
-    const int smem = pairs_smem_bytes(pl.kind, (int)rs.nch, (int)p.nbin, (int)t.ntypes, ghist);
-    if (smem > max_smem)
-        return fail(ctx, GOFR_ERR_UNSUPPORTED, "kernel needs %d B of shared memory (max %d)",
-                    smem, max_smem);
+    bool ghist = (pl.kind == 0 ? allpairs_smem_bytes((int)rs.nch, (int)p.nbin, (int)t.ntypes)
+                               : (size_t)pairs_smem_bytes(1, (int)rs.nch, (int)p.nbin,
+                                                          (int)t.ntypes)) >
+                 (size_t)max_smem - 8192;
+    // the windows of the block cell-list kernel and of the global-memory histogram form
+    if (pl.kind == 0) {
+        rc = ensure(ctx, ctx->d_win, ctx->cap_win, pl.w.win.size());
+        if (rc) return rc;
+    }
     PairLaunch L{};
     L.pos32 = t.pos32;
     L.types8 = t.types8;
@@ -1506,7 +1625,6 @@ int enqueue_run(gofr_ctx *ctx, const TrajDev &t, const gofr_params &p, const Run
     L.skip = (int)rs.skip;
     L.primo = (long long)p.primo;
     L.tric = t.tric;
-    L.ghist = ghist ? 1 : 0;
 #ifdef GOFR_DEBUG_BOUNDS
     {
         // test hook of the debug build: ANALISI_GB300_DEBUG_STALL=1 makes the
@@ -1514,8 +1632,15 @@ int enqueue_run(gofr_ctx *ctx, const TrajDev &t, const gofr_params &p, const Run
         // flight; the run must end with GOFR_ERR_DEVICE and a usable context
         const char *st = std::getenv("ANALISI_GB300_DEBUG_STALL");
         L.dbg_stall = (st && std::strcmp(st, "1") == 0) ? 1 : 0;
+        // the form that waits for copies is the one with global-memory histograms
+        if (L.dbg_stall && pl.kind == 0 && !pl.cells) ghist = true;
     }
 #endif
+    L.ghist = ghist ? 1 : 0;
+    const int smem = pairs_smem_bytes(pl.kind, (int)rs.nch, (int)p.nbin, (int)t.ntypes, ghist);
+    if ((pl.kind == 1 || ghist) && smem > max_smem)
+        return fail(ctx, GOFR_ERR_UNSUPPORTED, "kernel needs %d B of shared memory (max %d)",
+                    smem, max_smem);
     BinMap bm(p.rmin, p.rmax, p.nbin);
     L.rmin = bm.rmin; L.rmax = bm.rmax; L.dr = bm.dr; L.rmin2 = bm.rmin2; L.rmax2 = bm.rmax2;
     if (pl.kind == 0) {
@@ -1524,8 +1649,12 @@ int enqueue_run(gofr_ctx *ctx, const TrajDev &t, const gofr_params &p, const Run
         L.rmin_f = (float)p.rmin;
         L.inv_dr_f = (float)(1.0 / bm.dr);
         L.wlim = (float)(0.5 - pl.b.eta);
+        L.wtol = wrap_tolerance(t);
         L.rm = plan_radial_map(t, p, pl);
     }
+    if (pl.kind == 0 && (ghist || (pl.cells && !pl.cellw)))
+        CK(cudaMemcpyAsync(ctx->d_win, pl.w.win.data(), pl.w.win.size() * sizeof(float2),
+                           cudaMemcpyHostToDevice, ctx->stream));
     if (pl.cells && pl.cellw && !ghist) {
         int brc = ensure_cells(ctx, t, pl);
         if (brc) return brc;
@@ -1580,8 +1709,35 @@ int enqueue_run(gofr_ctx *ctx, const TrajDev &t, const gofr_params &p, const Run
         return GOFR_OK;
     }
     const unsigned nparts = p.nparts > 1 ? p.nparts : 1;
-    const int TI = pairs_tile_atoms(pl.kind);
     const size_t per = t.N / nparts;
+    if (pl.kind == 0 && !ghist) {
+        // every window and partition in one launch
+        const size_t longest = t.N - (nparts - 1) * per;
+        L.nwin = (int)nwin;
+        L.primos = d_primos;
+        L.nparts = (int)nparts;
+        L.part_stride = (long long)rs.data_length;
+        L.win_stride = (long long)(rs.data_length * nparts);
+        // sixteen units per warp slot (32 per SM): the last round of a job leaves
+        // half a unit a warp idle
+        const AllpairsUnit a = allpairs_unit(longest, t.N,
+                                             (double)nwin * nparts * rs.n_lags * rs.n_orig,
+                                             512.0 * ctx->num_sms);
+        L.gs = a.gs;
+        L.ng = a.ng;
+        L.jc = a.jc;
+        L.nj = a.nj;
+        L.most = allpairs_most(t.N, a);
+        L.queue = reinterpret_cast<unsigned *>(ctx->d_stats + ST_QUEUE);
+        L.counts = counts;
+        ++ctx->launches;
+        if (launch_allpairs(L, pl.wrapcheck, ctx->num_sms, ctx->stream))
+            return fail(ctx, GOFR_ERR_CUDA, "pair kernel launch failed: %s",
+                        cudaGetErrorString(cudaGetLastError()));
+        *pairs_out = (unsigned long long)nwin * rs.n_lags * rs.n_orig * t.N * t.N;
+        return GOFR_OK;
+    }
+    const int TI = pairs_tile_atoms(pl.kind);
     for (unsigned q = 0; q < nparts; ++q) {
         size_t a0 = q * per, a1 = (q == nparts - 1) ? t.N : (q + 1) * per;
         if (a1 <= a0) continue;
@@ -1685,8 +1841,6 @@ void tune_log(const std::string &key, const TuneChoice &c, double ms)
     out << " ms=" << ms << "\n";
 }
 
-int enqueue_run(gofr_ctx *ctx, const TrajDev &t, const gofr_params &p, const RunShape &rs,
-                const Plan &pl, unsigned long long *counts, unsigned long long *pairs_out);
 
 // Times one plan on the sample parameters; returns milliseconds (or < 0).
 double tune_time(gofr_ctx *ctx, const TrajDev &t, const gofr_params &q, const Plan &pl)
@@ -1952,7 +2106,6 @@ void free_batch(gofr_ctx *ctx)
 int build_batch(gofr_ctx *ctx)
 {
     auto &B = ctx->batch;
-    const int TI = pairs_tile_atoms(0);
     std::vector<float2> wins;
     std::vector<unsigned short> tabs;
     std::vector<size_t> win_off(ctx->trajs.size(), 0), tab_off(ctx->trajs.size(), 0);
@@ -2027,10 +2180,8 @@ int build_batch(gofr_ctx *ctx)
             B.allpairs_pairs += (unsigned long long)work[k];
         }
     }
-    const unsigned long long target =
-        std::max<unsigned long long>(total / ((unsigned long long)ctx->num_sms * 2 * 24), 1ull << 24);
-    struct Cost { unsigned long long c; WorkDesc w; bool tri; };
-    std::vector<Cost> all;
+    const unsigned long long target = batch_target(B.allpairs_pairs, ctx->num_sms);
+    std::vector<WorkCost> all;
     B.launches.resize(ctx->trajs.size());
     for (size_t k = 0; k < ctx->trajs.size(); ++k) {
         TrajDev &t = ctx->trajs[k];
@@ -2050,26 +2201,14 @@ int build_batch(gofr_ctx *ctx)
             B.cell_max_ntypes = std::max(B.cell_max_ntypes, (int)t.ntypes);
             continue;
         }
-        B.max_nbin = std::max(B.max_nbin, (int)t.params.nbin);
-        B.max_nch = std::max(B.max_nch, (int)rs.nch);
+        B.max_cells = std::max(B.max_cells, (int)rs.nch * ((int)t.params.nbin + 1) + 1);
         B.max_ntypes = std::max(B.max_ntypes, (int)t.ntypes);
-        const int n_itiles = (int)((t.N + TI - 1) / TI);
-        for (unsigned l = 0; l < rs.n_lags; ++l)
-            for (int it = 0; it < n_itiles; ++it) {
-                const unsigned long long tile = std::min<size_t>(TI, t.N - (size_t)it * TI);
-                const unsigned long long per_item = tile * t.N;
-                unsigned long long chunk = std::max<unsigned long long>(1, target / per_item);
-                chunk = std::min<unsigned long long>(chunk, std::max<unsigned long long>(
-                                                                1, (1ull << 31) / per_item));
-                for (unsigned k0 = 0; k0 < rs.n_orig; k0 += (unsigned)chunk) {
-                    const unsigned k1 = (unsigned)std::min<unsigned long long>(k0 + chunk, rs.n_orig);
-                    WorkDesc w{(int)k, (int)l, it, (int)k0, (int)k1, 0, 0, 0};
-                    all.push_back({(k1 - k0) * per_item, w, t.tric != 0});
-                }
-            }
+        if (t.params.rmin != 0.0) B.mode = 2;
+        add_descriptors((int)k, t, rs, batch_unit(t.N, target), target, all);
     }
-    std::stable_sort(all.begin(), all.end(), [](const Cost &a, const Cost &b) { return a.c > b.c; });
-    for (auto &c : all) B.work[c.tri ? 1 : 0].push_back(c.w);
+    std::stable_sort(all.begin(), all.end(),
+                     [](const WorkCost &a, const WorkCost &b) { return a.c > b.c; });
+    for (auto &e : all) B.work[e.tri ? 1 : 0].push_back(e.w);
     CK(dev_malloc(&B.d_win, std::max<size_t>(wins.size(), 1) * sizeof(float2)));
     CK(dev_malloc(&B.d_chtab, std::max<size_t>(tabs.size(), 1) * sizeof(unsigned short)));
     if (!wins.empty())
@@ -2106,7 +2245,11 @@ int build_batch(gofr_ctx *ctx)
         L.n_orig = (int)rs.n_orig;
         L.skip = (int)rs.skip;
         L.primo = (long long)t.params.primo;
-        L.n_itiles = (int)((t.N + TI - 1) / TI);
+        const AllpairsUnit a = batch_unit(t.N, target);
+        L.gs = a.gs;
+        L.ng = a.ng;
+        L.jc = a.jc;
+        L.nj = a.nj;
         BinMap bm(t.params.rmin, t.params.rmax, t.params.nbin);
         L.rmin = bm.rmin; L.rmax = bm.rmax; L.dr = bm.dr; L.rmin2 = bm.rmin2; L.rmax2 = bm.rmax2;
         L.hi_f = pl.w.hi_f;
@@ -2114,6 +2257,8 @@ int build_batch(gofr_ctx *ctx)
         L.rmin_f = (float)t.params.rmin;
         L.inv_dr_f = (float)(1.0 / bm.dr);
         L.wlim = (float)(0.5 - pl.b.eta);
+        L.wtol = wrap_tolerance(t);
+        L.rm = plan_radial_map(t, t.params, pl);
         L.tric = t.tric;
         L.wchk = pl.wrapcheck ? 1 : 0;
     }
@@ -2202,14 +2347,14 @@ int build_batch(gofr_ctx *ctx)
     }
     CK(dev_malloc(&B.d_head, 2 * sizeof(unsigned)));
     CK(cudaMallocHost(&B.h_stage, std::max<size_t>(ctx->batch_total, 1) * sizeof(unsigned long long)));
-    const int smem = batch_smem_bytes(B.max_nbin, B.max_nch, B.max_ntypes);
     int max_smem = 0;
     CK(cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device));
-    if (smem > max_smem)
-        return fail(ctx, GOFR_ERR_UNSUPPORTED, "batch histograms need %d B of shared memory", smem);
+    const size_t smem = allpairs_smem_bytes(1, B.max_cells - 2, B.max_ntypes);
+    if (smem > (size_t)max_smem)
+        return fail(ctx, GOFR_ERR_UNSUPPORTED, "batch histograms need %zu B of shared memory", smem);
     for (int v = 0; v < 2; ++v) {
         if (B.work[v].empty()) continue;
-        if (prepare_batch(B.max_nbin, B.max_nch, B.max_ntypes, v == 1, ctx->num_sms,
+        if (prepare_batch(B.max_cells, B.max_ntypes, v == 1, B.mode, ctx->num_sms,
                           (int)B.work[v].size(), &B.grid[v]))
             return fail(ctx, GOFR_ERR_CUDA, "batched kernel setup failed");
     }
@@ -2249,7 +2394,7 @@ int enqueue_batch(gofr_ctx *ctx)
         if (B.work[v].empty()) continue;
         ++ctx->launches;
         if (launch_batch_grid(B.d_launches, B.d_work[v], (int)B.work[v].size(), B.d_head + v,
-                              B.max_nbin, B.max_nch, B.max_ntypes, v == 1, ctx->d_err,
+                              B.max_cells, B.max_ntypes, v == 1, B.mode, ctx->d_err,
                               ctx->d_stats, B.grid[v], ctx->stream))
             return fail(ctx, GOFR_ERR_CUDA, "batched kernel launch failed: %s",
                         cudaGetErrorString(cudaGetLastError()));
@@ -2339,6 +2484,7 @@ void gofr_ctx_destroy(gofr_ctx *ctx)
         cudaFree(ctx->d_counts);
         cudaFree(ctx->d_gofr);
         cudaFree(ctx->d_chfac);
+        cudaFree(ctx->d_primos);
         cudaFree(ctx->d_win);
         cudaFree(ctx->d_chtab);
         cudaFree(ctx->d_err);
@@ -2452,13 +2598,11 @@ int run_windows_impl(gofr_ctx *ctx, const gofr_params *p, unsigned nwin,
     if (n_out) CK(cudaMemsetAsync(ctx->d_counts, 0, n_out * sizeof(unsigned long long), ctx->stream));
     CK(cudaEventRecord(ctx->ev[1], ctx->stream));
     unsigned long long pairs = 0;
-    PairLaunch *d_l = nullptr;
-    WorkDesc *d_w = nullptr;
-    unsigned *d_head = nullptr;
     int max_smem = 0;
     CK(cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device));
     bool one_launch = pl.kind == 0 && !pl.cells && !pl.empty && rs.n_lags > 0 && rs.n_orig > 0 &&
-                      batch_smem_bytes((int)p->nbin, (int)rs.nch, (int)t.ntypes) <= max_smem - 8192;
+                      allpairs_smem_bytes((int)rs.nch, (int)p->nbin, (int)t.ntypes) <=
+                          (size_t)max_smem - 8192;
     if (!one_launch) {
         for (unsigned w = 0; w < nwin && rc == GOFR_OK; ++w) {
             gofr_params q = *p;
@@ -2469,83 +2613,12 @@ int run_windows_impl(gofr_ctx *ctx, const gofr_params *p, unsigned nwin,
         }
         if (rc) return rc;
     } else {
-        // one parameter record per (window, partition), descriptors over all of them
-        const int TI = pairs_tile_atoms(0);
-        std::vector<unsigned short> tab = channel_table(t.ntypes);
-        rc = ensure(ctx, ctx->d_chtab, ctx->cap_chtab, tab.size());
-        if (rc == GOFR_OK) rc = ensure(ctx, ctx->d_win, ctx->cap_win, pl.w.win.size());
+        rc = ensure(ctx, ctx->d_primos, ctx->cap_primos, nwin);
         if (rc) return rc;
-        CK(cudaMemcpyAsync(ctx->d_chtab, tab.data(), tab.size() * sizeof(unsigned short),
+        const std::vector<long long> first(primos, primos + nwin);
+        CK(cudaMemcpyAsync(ctx->d_primos, first.data(), nwin * sizeof(long long),
                            cudaMemcpyHostToDevice, ctx->stream));
-        CK(cudaMemcpyAsync(ctx->d_win, pl.w.win.data(), pl.w.win.size() * sizeof(float2),
-                           cudaMemcpyHostToDevice, ctx->stream));
-        BinMap bm(p->rmin, p->rmax, p->nbin);
-        std::vector<PairLaunch> ls;
-        struct Cost { unsigned long long c; WorkDesc w; };
-        std::vector<Cost> all;
-        const size_t per = t.N / nparts;
-        const unsigned long long target = 1ull << 26;
-        for (unsigned w = 0; w < nwin; ++w)
-            for (unsigned q = 0; q < nparts; ++q) {
-                const size_t a0 = q * per, a1 = (q == nparts - 1) ? t.N : (q + 1) * per;
-                if (a1 <= a0) continue;
-                PairLaunch L{};
-                L.pos32 = t.pos32; L.types8 = t.types8; L.pos64 = t.pos64; L.box64 = t.box64;
-                L.box32 = t.box32; L.win = ctx->d_win; L.chtab = ctx->d_chtab;
-                L.counts = ctx->d_counts + w * per_win + q * rs.data_length;
-                L.err = ctx->d_err; L.stats = ctx->d_stats;
-                L.N = (int)t.N; L.NP = (int)padded_natoms(t.N);
-                L.nbin = (int)p->nbin; L.nch = (int)rs.nch; L.ntypes = (int)t.ntypes;
-                L.a0 = (int)a0; L.a1 = (int)a1;
-                L.n_lags = (int)rs.n_lags; L.every = (int)rs.every;
-                L.n_orig = (int)rs.n_orig; L.skip = (int)rs.skip; L.primo = (long long)primos[w];
-                L.n_itiles = (int)((a1 - a0 + TI - 1) / TI);
-                L.rmin = bm.rmin; L.rmax = bm.rmax; L.dr = bm.dr; L.rmin2 = bm.rmin2;
-                L.rmax2 = bm.rmax2;
-                L.hi_f = pl.w.hi_f; L.lo_f = pl.w.lo_f; L.rmin_f = (float)p->rmin;
-                L.inv_dr_f = (float)(1.0 / bm.dr); L.wlim = (float)(0.5 - pl.b.eta);
-                L.tric = t.tric; L.wchk = pl.wrapcheck ? 1 : 0;
-                const int li = (int)ls.size();
-                ls.push_back(L);
-                for (unsigned l = 0; l < rs.n_lags; ++l)
-                    for (int it = 0; it < L.n_itiles; ++it) {
-                        const unsigned long long tile =
-                            std::min<size_t>(TI, a1 - a0 - (size_t)it * TI);
-                        const unsigned long long per_item = tile * t.N;
-                        unsigned long long chunk = std::max<unsigned long long>(1, target / per_item);
-                        chunk = std::min<unsigned long long>(
-                            chunk, std::max<unsigned long long>(1, (1ull << 31) / per_item));
-                        for (unsigned k0 = 0; k0 < rs.n_orig; k0 += (unsigned)chunk) {
-                            const unsigned k1 =
-                                (unsigned)std::min<unsigned long long>(k0 + chunk, rs.n_orig);
-                            all.push_back({(k1 - k0) * per_item, WorkDesc{li, (int)l, it, (int)k0,
-                                                                       (int)k1, 0, 0, 0}});
-                        }
-                    }
-            }
-        std::stable_sort(all.begin(), all.end(),
-                         [](const Cost &a, const Cost &b) { return a.c > b.c; });
-        std::vector<WorkDesc> work;
-        for (auto &c : all) work.push_back(c.w);
-        int grid = 0;
-        if (prepare_batch((int)p->nbin, (int)rs.nch, (int)t.ntypes, t.tric != 0, ctx->num_sms,
-                          (int)work.size(), &grid))
-            return fail(ctx, GOFR_ERR_CUDA, "batched kernel setup failed");
-        CK(dev_malloc(&d_l, ls.size() * sizeof(PairLaunch)));
-        CK(dev_malloc(&d_w, std::max<size_t>(work.size(), 1) * sizeof(WorkDesc)));
-        CK(dev_malloc(&d_head, sizeof(unsigned)));
-        CK(cudaMemcpyAsync(d_l, ls.data(), ls.size() * sizeof(PairLaunch), cudaMemcpyHostToDevice,
-                           ctx->stream));
-        CK(cudaMemcpyAsync(d_w, work.data(), work.size() * sizeof(WorkDesc),
-                           cudaMemcpyHostToDevice, ctx->stream));
-        CK(cudaMemsetAsync(d_head, 0, sizeof(unsigned), ctx->stream));
-        ++ctx->launches;
-        if (launch_batch_grid(d_l, d_w, (int)work.size(), d_head, (int)p->nbin, (int)rs.nch,
-                              (int)t.ntypes, t.tric != 0, ctx->d_err, ctx->d_stats, grid,
-                              ctx->stream))
-            rc = fail(ctx, GOFR_ERR_CUDA, "windows launch failed: %s",
-                      cudaGetErrorString(cudaGetLastError()));
-        pairs = (unsigned long long)nwin * rs.n_lags * rs.n_orig * t.N * t.N;
+        rc = enqueue_run(ctx, t, *p, rs, pl, ctx->d_counts, &pairs, nwin, ctx->d_primos);
     }
     if (rc == GOFR_OK) {
         CK(cudaEventRecord(ctx->ev[2], ctx->stream));
@@ -2564,9 +2637,6 @@ int run_windows_impl(gofr_ctx *ctx, const gofr_params *p, unsigned nwin,
         rc = gofr_sync(ctx);
     }
     cudaStreamSynchronize(ctx->stream);
-    cudaFree(d_l);
-    cudaFree(d_w);
-    cudaFree(d_head);
     return rc;
 }
 

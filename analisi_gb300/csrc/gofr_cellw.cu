@@ -99,36 +99,6 @@ struct WarpArea {
     int pre[MAXSEG + 33];        // flat index of each segment's first record (INT_MAX past the last)
 };
 
-// Units [u0, u1) of chunk c of a launch of G CTAs over U units: every round of G
-// chunks takes half of what is left (a CTA meets few chunk ends, and the last
-// chunks are small enough for the CTAs to finish together), no chunk more
-// than `most` units or fewer than `least`.
-__device__ __forceinline__ void chunk_range(long long c, long long G, long long U, long long most,
-                                            long long least, long long &u0, long long &u1)
-{
-    long long r = c / G, s = 0;
-    // rounds of full chunks, while half of the rest is more than G of them
-    const long long capped = U > 2 * G * most ? (U - 2 * G * most + G * most - 1) / (G * most) : 0;
-    const long long skip = r < capped ? r : capped;
-    s = skip * G * most;
-    r -= skip;
-    long long len = 0;
-    for (;;) {
-        len = (U - s + 2 * G - 1) / (2 * G);
-        if (skip < capped || len > most) len = most;
-        if (len < least) {
-            len = least;  // from here on every round is the same
-            s += r * G * len;
-            break;
-        }
-        if (r == 0) break;
-        --r;
-        s += G * len;
-    }
-    u0 = s + (c % G) * len;
-    u1 = u0 + len < U ? u0 + len : U;
-}
-
 // NWARP warps per CTA, HCOPY copies of the shared histogram (warp w adds to
 // copy w HCOPY / NWARP: the privatisation depth, fewer warps contending for
 // each bin), MODE the bin map's (RadialMap).
@@ -279,7 +249,7 @@ __global__ void __launch_bounds__(NWARP * 32, 32 / NWARP) k_pairs_cellw(const Ce
                 const float t = __fadd_rn(q, RADIAL_MAGIC);
                 need = t <= P.rm.t_hi && t >= P.rm.t_lo;
                 const int b = (int)(__float_as_uint(t) - RADIAL_MAGIC_BITS);
-                if (need && b >= 0 && b < nbin)
+                if (b >= 0 && b < nbin)
                     atomicSub(whist + chtab[(int)(wi >> 24) * P.ntypes + (int)(wj >> 24)] * nrow + b,
                               1u);
             }

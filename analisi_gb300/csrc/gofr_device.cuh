@@ -220,6 +220,36 @@ __device__ __forceinline__ void bin_pair2(f2 d2, f2 inv, f2 off, const RadialMap
     bin_one<MODE>(t1, f1, m, row1, bit, mask1);
 }
 
+// Units [u0, u1) of chunk c of a launch of G CTAs over U units: every round of G
+// chunks takes half of what is left (a CTA meets few chunk ends, and the last
+// chunks are small enough for the CTAs to finish together), no chunk more
+// than `most` units or fewer than `warps`, and every chunk a multiple of
+// `warps`, so that equal units leave no warp of a CTA idle at its end (chunks
+// of 9 units for 8 warps kept 44 % of them waiting).
+__device__ __forceinline__ void chunk_range(long long c, long long G, long long U, long long most,
+                                            long long warps, long long &u0, long long &u1)
+{
+    most = most < warps ? warps : most / warps * warps;
+    long long r = c / G;
+    // rounds of full chunks, while half of the rest is more than G of them
+    const long long capped = U > 2 * G * most ? (U - 2 * G * most + G * most - 1) / (G * most) : 0;
+    const long long full = r < capped ? r : capped;
+    long long s = full * G * most, len = most;
+    r -= full;
+    if (full == capped) {
+        for (;; --r) {
+            len = (U - s + 2 * G * warps - 1) / (2 * G * warps) * warps;
+            if (len < warps) len = warps;
+            if (len > most) len = most;
+            if (len == warps) s += r * G * len;  // from here on every round is the same
+            if (len == warps || r == 0) break;
+            s += G * len;
+        }
+    }
+    u0 = s + (c % G) * len;
+    u1 = u0 + len < U ? u0 + len : U;
+}
+
 // ---------------------------------------------------------------------------
 // FP64 restatement of the reference pair arithmetic.
 // Every operation is an explicitly rounded IEEE intrinsic, so nvcc cannot

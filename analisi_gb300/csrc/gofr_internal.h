@@ -71,6 +71,16 @@ struct PairLaunch {
     unsigned long long *stats;
     int N, NP, nbin, nch, ntypes;
     int a0, a1;               // first-atom range [a0, a1) (one reference thread partition)
+    // gofr_allpairs.cu: every window and partition in one launch
+    int nwin;                 // calculate(primos[w]) windows (primos null: one, primo)
+    const long long *primos;
+    long long win_stride;     // counts of a window
+    int nparts;               // first atom a belongs to partition min(a / (N / nparts), nparts - 1)
+    long long part_stride;    // counts of a partition
+    int gs, ng;               // first atoms per unit, groups of them per partition
+    int jc, nj;               // chunks of second atoms per unit, parts of the frame they make
+    long long most;           // units of a CTA's chunk at most
+    unsigned *queue;          // {next chunk, CTAs done}, zero before and after a launch
     int n_lags, every;        // lags t = l*every, l < n_lags
     int n_orig, skip;         // origins primo + k*skip, k < n_orig
     long long primo;
@@ -78,7 +88,9 @@ struct PairLaunch {
     long long n_items;        // n_lags * n_itiles * n_orig
     float hi_f, lo_f;         // certain reject above hi_f / below lo_f
     float rmin_f, inv_dr_f;   // bin guess
-    float wlim;               // wrap check: |frac| > wlim flags a recheck
+    float wlim;               // wrap check: |frac| > wlim flags a recheck (triclinic; the
+                              // global-memory histogram form)
+    float wtol;               // orthorhombic: |component| > L / 2 - wtol flags a recheck
     double rmin, rmax, dr, rmin2, rmax2;  // reference binning constants
     RadialMap rm;
     int tric;
@@ -90,11 +102,16 @@ struct PairLaunch {
                               // bounded wait runs out (test of that path)
 };
 
-// One work descriptor of the batched kernel: origins [k0, k1) of one
-// (trajectory, lag, first-atom tile).
+// One work descriptor of the batched kernel: units [u0, u1) of one trajectory
+// (units as the single launch's: lag, origin, group of first atoms, part of the
+// second atoms).
 struct WorkDesc {
-    int traj, lag_idx, itile, k0, k1, pad0, pad1, pad2;
+    int traj, pad;
+    long long u0, u1;
 };
+
+constexpr int ALLPAIRS_GROUP = 64;   // first atoms of a warp's unit at most (gofr_allpairs.cu)
+constexpr int ALLPAIRS_CHUNK = 128;  // second atoms a warp holds at a time: 4 per lane
 
 // One launch of the cell-list pair kernel (gofr_cells.cu): items are
 // (lag, block of cells, origin), pair.n_items = n_lags * nblocks * n_orig.
@@ -259,11 +276,14 @@ int launch_pairs(const PairLaunch &P, int kind, bool wrapcheck, int num_sms, cud
                  size_t *smem_bytes_out);
 int pairs_smem_bytes(int kind, int nch, int nbin, int ntypes, bool ghist = false);
 int pairs_tile_atoms(int kind);
-int batch_smem_bytes(int max_nbin, int max_nch, int max_ntypes);
-int prepare_batch(int max_nbin, int max_nch, int max_ntypes, bool tric, int num_sms, int n_work,
-                  int *grid_out);
+size_t allpairs_smem_bytes(int nch, int nbin, int ntypes);
+int launch_allpairs(const PairLaunch &P, bool wrapcheck, int num_sms, cudaStream_t s);
+// cells: nch (nbin + 1) + 1 of the member with the most; mode: 0 when every
+// member's bin map is of mode 0, else 2.
+int prepare_batch(int max_cells, int max_ntypes, bool tric, int mode, int num_sms, int n_work,
+                  int *grid);
 int launch_batch_grid(const PairLaunch *d_trajs, const WorkDesc *d_work, int n_work,
-                      unsigned *d_head, int max_nbin, int max_nch, int max_ntypes, bool tric,
+                      unsigned *d_head, int max_cells, int max_ntypes, bool tric, int mode,
                       unsigned *d_err, unsigned long long *d_stats, int grid, cudaStream_t s);
 int launch_zero_u64(unsigned long long *p, size_t n, cudaStream_t s);
 

@@ -1,4 +1,6 @@
-// Gofrt pair/histogram kernels for GB300 (sm_103a).
+// Gofrt pair/histogram kernels for GB300 (sm_103a): the plain FP64 kernel, the
+// FP32 + FP64-recheck kernel for histograms too large for shared memory, and
+// the kernels that make frames resident.
 //
 // Replaces the reference's hot loop Gofrt::calc_single_th
 // (lib/src/gofrt.cpp:96-122, with the inlined geometry of
@@ -7,20 +9,20 @@
 //
 // Work decomposition: one launch covers every (lag, first-atom tile, origin)
 // item of a Gofrt::calculate.  A persistent grid of CTAs takes contiguous,
-// lag-major ranges of items, so consecutive items of a CTA share the lag and
-// its shared-memory histogram [nch][nbin] is flushed to the global u64 counts
-// only when the lag changes (or before a u32 bin could overflow).
+// lag-major ranges of items.
 //
-// FP32 kernel, per item: each thread holds R first atoms (frame `origin`)
-// in registers, duplicated into f32x2 pairs; the CTA streams the second atoms
-// (frame `origin+lag`, SoA x|y|z blocks plus u8 types) through shared memory
-// in tiles of TJ atoms, double buffered with 1-D TMA bulk copies completed on
+// FP32 kernel (histograms that fit shared memory: gofr_allpairs.cu), per
+// item: each thread holds R first atoms (frame `origin`) in registers,
+// duplicated into f32x2 pairs; the CTA streams the second atoms (frame
+// `origin+lag`, SoA x|y|z blocks plus u8 types) through shared memory in
+// tiles of TJ atoms, double buffered with 1-D TMA bulk copies completed on
 // mbarriers.  Distances are computed two second-atoms per packed f32x2
-// instruction.  The rare pairs that land inside the accept window (plus its
-// error bound) are appended to per-thread slots in shared memory and binned
-// later by the whole warp, so the hot loop never diverges; pairs whose FP32
-// bin cannot be certified go to a per-CTA queue recomputed in FP64 by all
-// threads together at the end of the item.
+// instruction.  The pairs that land inside the accept window (plus its error
+// bound) are appended to per-thread slots in shared memory and binned later
+// by the whole warp into the u64 counts in global memory, whose atomics the
+// hot loop does not wait for; pairs whose FP32 bin cannot be certified go to a
+// per-CTA queue recomputed in FP64 by all threads together at the end of the
+// item.
 #include <cstdint>
 #include <cstdio>
 #include <cuda_runtime.h>
@@ -193,8 +195,8 @@ __device__ __forceinline__ f2 pair2(f2 xi, f2 yi, f2 zi, f2 xj, f2 yj, f2 zj, co
 
 // Shared-memory layout of the FP32 kernel (byte offsets).
 struct F32Smem {
-    int jx, jt, bars, flag, rqn, win, hist, chtab, slots, rq, total;
-    __host__ __device__ F32Smem(int nbin, int nch, int ntypes, bool ghist = false)
+    int jx, jt, bars, flag, rqn, win, chtab, slots, rq, total;
+    __host__ __device__ F32Smem(int nbin, int ntypes)
     {
         int o = 0;
         jx = o;    o += 2 * 3 * TJ32 * 4;        // [2][3][TJ] floats
@@ -205,7 +207,6 @@ struct F32Smem {
         slots = o; o += SLOTS * NT * 8;          // [SLOTS][NT] uint2
         rq = o;    o += QCAP * 16;               // [QCAP] uint4
         win = o;   o += nbin * 8;                // [nbin] float2
-        hist = o;  o += ghist ? 0 : nch * nbin * 4;  // [nch][nbin] u32
         chtab = o; o += ntypes * ntypes * 2;     // [ntypes][ntypes] u16
         total = (o + 127) / 128 * 128;
     }
@@ -232,7 +233,6 @@ struct F32Views {
     uint2 *slots;
     uint4 *rq;
     float2 *win;
-    unsigned *hist;
     unsigned short *chtab;
     __device__ F32Views(unsigned char *smem, const F32Smem &L)
         : jx(reinterpret_cast<float *>(smem + L.jx)), jt(smem + L.jt),
@@ -242,7 +242,6 @@ struct F32Views {
           slots(reinterpret_cast<uint2 *>(smem + L.slots)),
           rq(reinterpret_cast<uint4 *>(smem + L.rq)),
           win(reinterpret_cast<float2 *>(smem + L.win)),
-          hist(reinterpret_cast<unsigned *>(smem + L.hist)),
           chtab(reinterpret_cast<unsigned short *>(smem + L.chtab))
     {
     }
@@ -287,7 +286,7 @@ __device__ __forceinline__ void f32_abort(const F32Views &V, const F32Thread &th
 #endif
 
 // One item: the first atoms of tile `itile` at origin k against every second
-// atom at lag lag_idx, binned into V.hist.  Returns false if a bounded wait
+// atom at lag lag_idx, binned into the lag's counts.  Returns false if a bounded wait
 // ran out (the caller aborts the CTA).  All threads of the CTA call it.
 template <bool TRI, bool WCHK>
 __device__ __forceinline__ bool f32_item(const PairLaunch &P, const F32Views &V, F32Thread &th,
@@ -301,8 +300,7 @@ __device__ __forceinline__ bool f32_item(const PairLaunch &P, const F32Views &V,
     uint2 *const my_slots = V.slots + tid;
     const long long fo = P.primo + (long long)k * P.skip;
     const long long fl = fo + (long long)lag_idx * P.every;
-    unsigned long long *const gc =
-        P.ghist ? P.counts + (long long)lag_idx * P.every * P.nch * P.nbin : nullptr;
+    unsigned long long *const gc = P.counts + (long long)lag_idx * P.every * P.nch * P.nbin;
     Box2 bx;
     {
         const Box32 b = P.box32[fo];
@@ -376,9 +374,8 @@ __device__ __forceinline__ bool f32_item(const PairLaunch &P, const F32Views &V,
 
         // Bins every slot of this warp's lanes (all lanes take part; each
         // processes its own slots, two per round so that their shared-memory
-        // load chains overlap), then empties them.  Shared-histogram updates
-        // are predicated reductions; the rare FP64 rechecks sit behind one
-        // warp-uniform branch.
+        // load chains overlap), then empties them.  The rare FP64 rechecks sit
+        // behind one warp-uniform branch.
         auto warp_flush = [&]() {
             const int maxc = __reduce_max_sync(0xffffffffu, (unsigned)cnt);
             for (int q0 = 0; q0 < maxc; q0 += 2) {
@@ -414,15 +411,9 @@ __device__ __forceinline__ bool f32_item(const PairLaunch &P, const F32Views &V,
                                        P.err);
                     need[u] = (v[u] && wrap) || (test && !inw);
                 }
-                if (gc) {
 #pragma unroll
-                    for (int u = 0; u < 2; ++u)
-                        if (ok[u]) atomicAdd(gc + ch[u] * P.nbin + bi[u], 1ull);
-                } else {
-#pragma unroll
-                    for (int u = 0; u < 2; ++u)
-                        red_shared_add1_if(smem_u32(V.hist + ch[u] * P.nbin + bi[u]), ok[u]);
-                }
+                for (int u = 0; u < 2; ++u)
+                    if (ok[u]) atomicAdd(gc + ch[u] * P.nbin + bi[u], 1ull);
                 if (__any_sync(0xffffffffu, need[0] || need[1])) {
 #pragma unroll
                     for (int u = 0; u < 2; ++u) {
@@ -433,7 +424,7 @@ __device__ __forceinline__ bool f32_item(const PairLaunch &P, const F32Views &V,
                             V.rq[slot] =
                                 make_uint4((unsigned)ia[u], (unsigned)ja[u], (unsigned)ch[u], 0u);
                         } else {
-                            recheck_pair<TRI>(P.pos64, P.box64, N, fo, fl, ia[u], ja[u], V.hist,
+                            recheck_pair<TRI>(P.pos64, P.box64, N, fo, fl, ia[u], ja[u], nullptr,
                                               ch[u], P.nbin, P.rmin, P.dr, P.rmin2, P.rmax2, P.err,
                                               gc);
                         }
@@ -487,7 +478,7 @@ __device__ __forceinline__ bool f32_item(const PairLaunch &P, const F32Views &V,
             const int n = min(*V.rqn, QCAP);
             for (int q = tid; q < n; q += NT) {
                 const uint4 e = V.rq[q];
-                recheck_pair<TRI>(P.pos64, P.box64, N, fo, fl, (int)e.x, (int)e.y, V.hist,
+                recheck_pair<TRI>(P.pos64, P.box64, N, fo, fl, (int)e.x, (int)e.y, nullptr,
                                   (int)e.z, P.nbin, P.rmin, P.dr, P.rmin2, P.rmax2, P.err, gc);
             }
             __syncthreads();
@@ -499,7 +490,7 @@ __device__ __forceinline__ bool f32_item(const PairLaunch &P, const F32Views &V,
     const int n = min(*V.rqn, QCAP);
     for (int q = tid; q < n; q += NT) {
         const uint4 e = V.rq[q];
-        recheck_pair<TRI>(P.pos64, P.box64, N, fo, fl, (int)e.x, (int)e.y, V.hist, (int)e.z,
+        recheck_pair<TRI>(P.pos64, P.box64, N, fo, fl, (int)e.x, (int)e.y, nullptr, (int)e.z,
                           P.nbin, P.rmin, P.dr, P.rmin2, P.rmax2, P.err, gc);
     }
     __syncthreads();
@@ -512,11 +503,9 @@ template <bool TRI, bool WCHK>
 __global__ void __launch_bounds__(NT, 2) k_pairs_f32(const PairLaunch P)
 {
     extern __shared__ __align__(128) unsigned char smem[];
-    const F32Views V(smem, F32Smem(P.nbin, P.nch, P.ntypes, P.ghist != 0));
+    const F32Views V(smem, F32Smem(P.nbin, P.ntypes));
     const int tid = threadIdx.x;
-    const int hlen = P.ghist ? 0 : P.nch * P.nbin;
     for (int i = tid; i < P.nbin; i += NT) V.win[i] = P.win[i];
-    for (int i = tid; i < hlen; i += NT) V.hist[i] = 0u;
     for (int i = tid; i < P.ntypes * P.ntypes; i += NT) V.chtab[i] = P.chtab[i];
     f32_init_barriers(V);
     __syncthreads();
@@ -524,85 +513,16 @@ __global__ void __launch_bounds__(NT, 2) k_pairs_f32(const PairLaunch P)
     const long long per = (P.n_items + gridDim.x - 1) / gridDim.x;
     const long long it0 = (long long)blockIdx.x * per;
     const long long it1 = min(it0 + per, P.n_items);
-    const long long flush_every = items_per_flush(TI32, P.N);
-    int cur_lag = -1;
-    long long since_flush = 0;
     F32Thread th;
     for (long long item = it0; item < it1; ++item) {
         int lag_idx, itile, k;
         decompose(item, P, lag_idx, itile, k);
-        if (lag_idx != cur_lag || since_flush >= flush_every) {
-            if (cur_lag >= 0 && hlen)
-                flush_hist(V.hist, hlen, P.counts + (long long)cur_lag * P.every * hlen);
-            cur_lag = lag_idx;
-            since_flush = 0;
-        }
-        ++since_flush;
         if (!f32_item<TRI, WCHK>(P, V, th, lag_idx, itile, k)) {
             f32_abort(V, th, P.err, GOFR_STALL(P) ? DBG_WAIT_CAP : WAIT_CAP);
             return;
         }
     }
-    if (cur_lag >= 0 && hlen)
-        flush_hist(V.hist, hlen, P.counts + (long long)cur_lag * P.every * hlen);
     add_stats(P.stats, th.n_cand, th.n_rech);
-}
-
-// Many trajectories in one persistent launch.  Each CTA pulls work
-// descriptors (trajectory, lag, first-atom tile, origin range) from a device
-// queue (one atomic counter; descriptors sorted by decreasing cost on the
-// host), switches the shared tables when the trajectory changes, and flushes
-// its histogram into that trajectory's counts at the end of every descriptor.
-template <bool TRI>
-__global__ void __launch_bounds__(NT, 2) k_pairs_batch(const PairLaunch *__restrict__ trajs,
-                                                       const WorkDesc *__restrict__ work,
-                                                       int n_work, unsigned *head, int max_nbin,
-                                                       int max_nch, int max_ntypes, unsigned *err,
-                                                       unsigned long long *stats)
-{
-    extern __shared__ __align__(128) unsigned char smem[];
-    __shared__ int s_next;
-    // the current trajectory's parameters live in shared memory: a register
-    // copy of the whole struct would crowd out the hot loop
-    __shared__ __align__(16) PairLaunch sP;
-    const F32Views V(smem, F32Smem(max_nbin, max_nch, max_ntypes));
-    const int tid = threadIdx.x;
-    for (int i = tid; i < max_nch * max_nbin; i += NT) V.hist[i] = 0u;
-    f32_init_barriers(V);
-    __syncthreads();
-    const PairLaunch &P = sP;
-    int cur = -1;
-    F32Thread th;
-    for (;;) {
-        if (tid == 0) s_next = (int)atomicAdd(head, 1u);
-        __syncthreads();
-        const int idx = s_next;
-        __syncthreads();
-        if (idx >= n_work) break;
-        const WorkDesc w = work[idx];
-        if (w.traj != cur) {
-            constexpr int words = (int)(sizeof(PairLaunch) / 4);
-            const unsigned *src = reinterpret_cast<const unsigned *>(trajs + w.traj);
-            for (int i = tid; i < words; i += NT) reinterpret_cast<unsigned *>(&sP)[i] = src[i];
-            __syncthreads();
-            for (int i = tid; i < P.nbin; i += NT) V.win[i] = P.win[i];
-            for (int i = tid; i < P.ntypes * P.ntypes; i += NT) V.chtab[i] = P.chtab[i];
-            cur = w.traj;
-            __syncthreads();
-        }
-        const bool wchk = P.wchk != 0;
-        for (int k = w.k0; k < w.k1; ++k) {
-            const bool ok = wchk ? f32_item<TRI, true>(P, V, th, w.lag_idx, w.itile, k)
-                                 : f32_item<TRI, false>(P, V, th, w.lag_idx, w.itile, k);
-            if (!ok) {
-                f32_abort(V, th, err);
-                return;
-            }
-        }
-        const int hlen = P.nch * P.nbin;
-        flush_hist(V.hist, hlen, P.counts + (long long)w.lag_idx * P.every * hlen);
-    }
-    add_stats(stats, th.n_cand, th.n_rech);
 }
 
 // ---------------------------------------------------------------------------
@@ -798,7 +718,7 @@ int launch_zero_u64(unsigned long long *p, size_t n, cudaStream_t s)
 
 int pairs_smem_bytes(int kind, int nch, int nbin, int ntypes, bool ghist)
 {
-    if (kind == 0) return F32Smem(nbin, nch, ntypes, ghist).total;
+    if (kind == 0) return F32Smem(nbin, ntypes).total;
     size_t b = (size_t)TJ64 * (3 * 8 + 4) + (ghist ? 0 : (size_t)nch * nbin * 4) +
                (size_t)ntypes * ntypes * 2;
     return (int)((b + 127) / 128 * 128);
@@ -820,41 +740,6 @@ static int launch_persistent(K kernel, const PairLaunch &P, int smem, int num_sm
     if (grid > P.n_items) grid = P.n_items;
     if (grid < 1) grid = 1;
     kernel<<<(unsigned)grid, NT, smem, s>>>(P);
-    return cuda_ok(cudaGetLastError());
-}
-
-int batch_smem_bytes(int max_nbin, int max_nch, int max_ntypes)
-{
-    return F32Smem(max_nbin, max_nch, max_ntypes).total;
-}
-
-int prepare_batch(int max_nbin, int max_nch, int max_ntypes, bool tric, int num_sms, int n_work,
-                  int *grid_out)
-{
-    const int smem = batch_smem_bytes(max_nbin, max_nch, max_ntypes);
-    auto kernel = tric ? k_pairs_batch<true> : k_pairs_batch<false>;
-    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) !=
-        cudaSuccess)
-        return -1;
-    int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, NT, smem) != cudaSuccess)
-        return -1;
-    if (per_sm < 1) return -2;
-    long long grid = (long long)num_sms * per_sm;
-    if (grid > n_work) grid = n_work;
-    *grid_out = (int)(grid < 1 ? 1 : grid);
-    return 0;
-}
-
-int launch_batch_grid(const PairLaunch *d_trajs, const WorkDesc *d_work, int n_work,
-                      unsigned *d_head, int max_nbin, int max_nch, int max_ntypes, bool tric,
-                      unsigned *d_err, unsigned long long *d_stats, int grid, cudaStream_t s)
-{
-    if (n_work <= 0) return 0;
-    const int smem = batch_smem_bytes(max_nbin, max_nch, max_ntypes);
-    auto kernel = tric ? k_pairs_batch<true> : k_pairs_batch<false>;
-    kernel<<<(unsigned)grid, NT, smem, s>>>(d_trajs, d_work, n_work, d_head, max_nbin, max_nch,
-                                            max_ntypes, d_err, d_stats);
     return cuda_ok(cudaGetLastError());
 }
 

@@ -2,7 +2,8 @@
 the CPU: pairs placed within a few margins of bin edges are put through the
 kernel's FP32 operations in numpy (the warp-streamed kernel's: coordinates
 reduced into the cell, the neighbour moved by the FP32 image vector; the
-all-pairs kernel's: FP32 minimum image), with the hardware rsqrt at both ends of
+all-pairs kernel's: both atoms moved into the box, |d| or L - |d|; triclinic, the
+FP32 minimum image), with the hardware rsqrt at both ends of
 its stated error and at its centre.  Every pair the map calls certain must be
 in the reference's bin (lib/src/gofrt.cpp:104,114-118 on its FP64 minimum
 image), and every pair the reference counts must come out inside the map's
@@ -36,24 +37,33 @@ CASES = [
 ]
 
 
-def allpairs_d(xi, xj, lo3, hi3, L, tilt):
+def allpairs_d(xi, xj, lo3, hi3, L, tilt, tric):
     shift = 0.5 * lo3 + 0.5 * hi3
-    d = ((xi - shift).astype(f32) - (xj - shift).astype(f32)).astype(f32)
     L32, inv = L.astype(f32), (1.0 / L).astype(f32)
     t32 = np.array(tilt, dtype=f32)
-    one = np.ones(len(d), dtype=f32)
+    one = np.ones(len(xi), dtype=f32)
 
-    def wrap(ax):
-        return (fma32(d[:, ax], inv[ax] * one, MAGIC * one) - MAGIC).astype(f32)
+    def wrap(v, ax):
+        return (fma32(v, inv[ax] * one, MAGIC * one) - MAGIC).astype(f32)
 
-    k = wrap(2)
+    ai, aj = (xi - shift).astype(f32), (xj - shift).astype(f32)
+    if not tric:  # both atoms into the box, then |d| or L - |d|
+        d = np.empty_like(ai)
+        for ax in range(3):
+            wi = fma32(wrap(ai[:, ax], ax), -L32[ax] * one, ai[:, ax])
+            wj = fma32(wrap(aj[:, ax], ax), -L32[ax] * one, aj[:, ax])
+            a = np.abs((wi - wj).astype(f32))
+            d[:, ax] = np.minimum(a, (L32[ax] - a).astype(f32))
+        return d
+    d = (ai - aj).astype(f32)
+    k = wrap(d[:, 2], 2)
     d[:, 2] = fma32(k, -L32[2] * one, d[:, 2])
     d[:, 1] = fma32(k, -t32[2] * one, d[:, 1])
     d[:, 0] = fma32(k, -t32[1] * one, d[:, 0])
-    k = wrap(1)
+    k = wrap(d[:, 1], 1)
     d[:, 1] = fma32(k, -L32[1] * one, d[:, 1])
     d[:, 0] = fma32(k, -t32[0] * one, d[:, 0])
-    k = wrap(0)
+    k = wrap(d[:, 0], 0)
     d[:, 0] = fma32(k, -L32[0] * one, d[:, 0])
     return d
 
@@ -108,7 +118,7 @@ def test_certain_pairs_are_in_the_reference_bin(built_engine, case):
         tab = engine.cellw_tables(*args, rmax, list(plan["cells"]))
         d = cellw_d(xi, xj, d_ref, tab, lo, L, tilt)
     else:
-        d = allpairs_d(xi, xj, allx.min(0), allx.max(0), L, tilt)
+        d = allpairs_d(xi, xj, allx.min(0), allx.max(0), L, tilt, tric)
     one = np.ones(len(d), dtype=f32)
     d2 = fma32(d[:, 2], d[:, 2], fma32(d[:, 1], d[:, 1], fma32(d[:, 0], d[:, 0], f32(1e-30) * one)))
     for s in (-1.0, 0.0, 1.0):
