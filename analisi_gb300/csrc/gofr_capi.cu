@@ -998,6 +998,7 @@ struct Plan {
     bool cellw = false;          // the warp-streamed form of the cell-list kernel
     int wblk[3] = {1, 1, 1}, nw[3] = {1, 1, 1};  // its warp blocks
     int cta_warps = 8, hcopy = 1;  // its CTA size and histogram privatisation depth
+    int pg = 1, npg = 1;           // partitions per histogram, groups of them
     CellwGeom geom;                // its neighbourhood tables and image vectors
     bool wrapcheck = false;
     bool empty = false;        // accepted window empty: nothing can be counted
@@ -1019,6 +1020,8 @@ RadialMap plan_radial_map(const TrajDev &t, const gofr_params &p, const Plan &pl
 // two atoms at minimum-image distance <= rmax are at most `reach` cells apart
 // on every axis (periodically); at least 2 reach + 1 cells per axis.  A CTA
 // takes a block of bx*by*bz cells with r first atoms per thread.
+constexpr double kAllpairsPair = 1.23;
+
 struct CellCand {
     int reach = 1, r = 4;
     int nc[3] = {0, 0, 0};
@@ -1029,11 +1032,13 @@ struct CellCand {
 };
 
 // Cell lists need a box that is the same in every frame (the frames share
-// one grid) and one reference thread partition; the block kernel also an
-// orthorhombic box (the warp-streamed kernel takes triclinic ones).
-bool cell_eligible(const TrajDev &t, const gofr_params &p, bool allow_tric = false)
+// one grid); the block kernel also an orthorhombic box and one reference
+// thread partition, the warp-streamed kernel (`warp`) takes triclinic boxes and,
+// where the planner chooses it, counts per partition.
+bool cell_eligible(const TrajDev &t, const gofr_params &p, bool warp = false)
 {
-    if ((t.tric && !allow_tric) || !t.box_constant || p.nparts > 1) return false;
+    if ((t.tric && !warp) || !t.box_constant) return false;
+    if (p.nparts > 1 && !(warp && p.kernel == GOFR_KERNEL_AUTO && p.nparts <= t.N)) return false;
     if (!(p.rmax > 0.0)) return false;
     if (t.N >= (1u << 24)) return false;  // sorted slots pack type << 24 | atom id
     // large histograms use the global-memory form of the all-pairs kernel
@@ -1061,10 +1066,10 @@ bool cell_grid(const TrajDev &t, const gofr_params &p, int reach, int nc[3])
 // whole tiles of 256 r, with room for three standard deviations of density
 // fluctuation) times the atoms of its neighbourhood, relative to the N^2
 // pairs of the all-pairs kernel.  The time model weighs each evaluated pair
-// and each candidate (d <= rmax, binned in the warp flush): measured on the
-// 16k- and 131k-atom workloads, a candidate costs ~6.8 pair evaluations in
-// the all-pairs kernel and ~6.5 in the cell kernel, whose pairs (no wrap
-// arithmetic) cost ~0.62 of an all-pairs evaluation.
+// and each candidate (d <= rmax, binned in the warp flush), measured on the
+// 16k- and 131k-atom workloads in units of 95 SM-quarter cycles per 128 pairs:
+// ~0.62 a pair and ~6.5 a candidate here; a pair of the all-pairs kernel
+// costs 1.23, within rmax or not.
 std::vector<CellCand> cell_candidates(const TrajDev &t, const gofr_params &p)
 {
     std::vector<CellCand> all;
@@ -1099,7 +1104,7 @@ std::vector<CellCand> cell_candidates(const TrajDev &t, const gofr_params &p)
                                               ((nc[1] + by - 1) / by) * ((nc[2] + bz - 1) / bz);
                         c.cost = blocks * slots * nbhd * per_cell / ((double)t.N * t.N);
                         const double f_cell = std::min(1.0, f_all / std::max(c.fraction, 1e-9));
-                        c.time = c.cost * (0.62 + 6.5 * f_cell) / (1.0 + 6.8 * f_all);
+                        c.time = c.cost * (0.62 + 6.5 * f_cell) / kAllpairsPair;
                         all.push_back(c);
                     }
                 }
@@ -1184,12 +1189,26 @@ struct CellwCand {
     double cost = 1e300;    // lane-pair slots evaluated / N^2 (+ per-chunk overhead)
 };
 
+// Partitions whose channels share one histogram of the warp-streamed kernel
+// beside its warps' areas (16 warps, one CTA per SM), at most 65535 classes.
+int cellw_partitions(const TrajDev &t, const gofr_params &p)
+{
+    const int nch = (int)(t.ntypes * (t.ntypes + 1));
+    int pg = (int)std::max(1u, p.nparts);
+    while (pg > 1 && (cellw_smem_bytes(nch * pg, (int)p.nbin, (int)t.ntypes, 16, 1) > 220 * 1024 ||
+                      pg * (int)t.ntypes > 65535))
+        pg = (pg + 1) / 2;
+    return pg;
+}
+
 // Every configuration, cheapest first.  The cost counts, over all warp
 // blocks, the block's first atoms times the record slots of its
-// neighbourhood's chunks (rows packed 128 records to a chunk, at most 8
-// pieces each, so short rows fill chunks less), plus a fixed overhead per
-// chunk streamed (one per batch of 64 first atoms; atoms with room for two
-// standard deviations of density fluctuation), relative to N^2.  Triclinic
+// neighbourhood's chunks of 128, plus what a chunk (2.3 first atoms, once per
+// batch of 64; atoms with room for two standard deviations of density
+// fluctuation) and a block (46 first atoms against a chunk: its rows, its
+// atoms, its last rechecks) cost beside, relative to N^2: in units of a pair
+// of this kernel, 95 SM-quarter cycles per 128 (fitted to 300 plans of 1000 to
+// 131072 atoms, rmax of a tenth to a third of the box).  Triclinic
 // neighbourhoods take the widest row and cell ranges of their geometry (one
 // more than the orthorhombic 2 reach where a tilt shifts them).
 std::vector<CellwCand> cellw_candidates(const TrajDev &t, const gofr_params &p)
@@ -1201,6 +1220,8 @@ std::vector<CellwCand> cellw_candidates(const TrajDev &t, const gofr_params &p)
     if (cellw_smem_bytes(nch, (int)p.nbin, (int)t.ntypes, 16, 1) > 220 * 1024 &&
         cellw_smem_bytes(nch, (int)p.nbin, (int)t.ntypes, 8, 1) > 110 * 1024)
         return all;
+    const int pg = cellw_partitions(t, p);
+    const double npg = std::ceil((double)std::max(1u, p.nparts) / pg);
     for (int m = 1; m <= 3; ++m) {
         int nc[3];
         CellwGeom g;
@@ -1226,15 +1247,13 @@ std::vector<CellwCand> cellw_candidates(const TrajDev &t, const gofr_params &p)
                     const double batches =
                         std::ceil(std::max(atoms + 2.0 * std::sqrt(atoms), 1.0) /
                                   cellw_batch_atoms());
-                    // a chunk's fixed work (wait, image moves, padding, the last
-                    // flush) is about that of six first atoms against its records
                     CellwCand c;
                     c.reach = m;
                     c.r = 4;
                     for (int k = 0; k < 3; ++k) c.nc[k] = nc[k];
                     c.w = {{wx, wy, wz}};
                     c.fraction = rows * (wx + g.nx_span) / ncell;
-                    c.cost = blocks * (atoms + 6.0 * batches) * chunks * chr /
+                    c.cost = blocks * ((atoms + 2.3 * batches * npg) * chunks + 46.0 * npg) * chr /
                              ((double)t.N * t.N);
                     all.push_back(c);
                 }
@@ -1298,18 +1317,46 @@ bool make_cellw_plan(const TrajDev &t, const gofr_params &p, Plan &pl, const Cel
                       ? 16
                       : 8;
     q.hcopy = 1;
+    q.pg = cellw_partitions(t, p);
+    q.npg = ((int)std::max(1u, p.nparts) + q.pg - 1) / q.pg;
     pl = q;
     return true;
 }
 
-// AUTO takes the cell-list form when its modelled time is below this share of
-// the all-pairs kernel's (a margin for the model's error).
+// AUTO takes the block cell-list form when its modelled time is below this
+// share of the all-pairs kernel's (a margin for the model's error), where the
+// warp-streamed form cannot run.
 constexpr double kCellAutoTime = 0.85;
-// ... and the warp-streamed form where the block form is not taken (a
-// triclinic box, or a box too small for the block form to pay) when its
-// modelled lane work is below this share of the all-pairs kernel's pairs (an
-// evaluated pair costs it about twice an all-pairs one).
-constexpr double kCellwAuto = 0.4;
+// AUTO takes the warp-streamed form when its modelled cost is below this many
+// pairs of its own (an all-pairs pair is kAllpairsPair = 1.23 of them).
+// Measured, 20 lags x 10 origins: 3575 atoms, L = 3.3 rmax, cost 0.81: 1.11 ms
+// against 1.96; 2149 atoms, L = 2.8 rmax, cost 1.20: 0.66 against 0.76; 1715
+// atoms, L = 2.6 rmax, cost 1.3: 0.56 against 0.55; between 0.9 and 1.2 the
+// gain is a tenth to a quarter of a run, less than the lists of new frames
+// cost) ...
+constexpr double kCellwAuto = 0.9;
+// ... and the trajectory has this many atoms: below, the first pass on new
+// frames pays more for building the lists (allocations, three kernels and a
+// synchronisation: 0.5 ms) than runs on them gain (1000 atoms, 20 lags x 10
+// origins: 0.08 ms against 0.23).
+constexpr size_t kCellMinAtoms = 2048;
+
+// The cell-list plan AUTO takes for the all-pairs plan pl, if any.
+bool auto_cell_plan(const TrajDev &t, const gofr_params &p, Plan &pl)
+{
+    if (pl.kind != 0 || pl.wrapcheck || pl.empty || t.N < kCellMinAtoms) return false;
+    CellwCand c;
+    Plan q = pl;
+    if (cellw_choice(t, p, c) && make_cellw_plan(t, p, q, c)) {
+        if (!(c.cost < kCellwAuto)) return false;
+        pl = q;
+        return true;
+    }
+    q = pl;
+    if (!cell_plan(t, p, q) || !(q.cell_time < kCellAutoTime)) return false;
+    pl = q;
+    return true;
+}
 
 int make_plan(gofr_ctx *ctx, const TrajDev &t, const gofr_params &p, Plan &pl,
               bool allow_cells = true)
@@ -1349,25 +1396,15 @@ int make_plan(gofr_ctx *ctx, const TrajDev &t, const gofr_params &p, Plan &pl,
         return fail(ctx, GOFR_ERR_UNSUPPORTED,
                     "coordinates too far outside the box for a certified FP32 wrap");
     }
-    if (allow_cells && (req == GOFR_KERNEL_CELL || req == GOFR_KERNEL_AUTO) && !pl.wrapcheck) {
-        Plan c = pl;
-        if (cell_plan(t, p, c) && (req == GOFR_KERNEL_CELL || c.cell_time < kCellAutoTime))
-            pl = c;
-    }
-    // the warp-streamed form: on request, and for AUTO wherever the block
-    // cell-list form was taken and the warp form is eligible (measured faster
-    // on every workload where both run), and elsewhere (triclinic boxes,
-    // boxes where the block form does not pay) when its modelled lane work is
-    // below kCellwAuto of the all-pairs pairs
-    if (allow_cells && !pl.wrapcheck &&
-        (req == GOFR_KERNEL_CELL_WARP || req == GOFR_KERNEL_AUTO)) {
-        CellwCand c;
-        Plan q = pl;
-        q.cells = false;
-        if (cellw_choice(t, p, c) &&
-            (req != GOFR_KERNEL_AUTO || pl.cells || c.cost < kCellwAuto) &&
-            make_cellw_plan(t, p, q, c))
-            pl = q;
+    if (allow_cells && !pl.wrapcheck) {
+        if (req == GOFR_KERNEL_AUTO) {
+            auto_cell_plan(t, p, pl);
+        } else if (req == GOFR_KERNEL_CELL) {
+            cell_plan(t, p, pl);
+        } else if (req == GOFR_KERNEL_CELL_WARP) {
+            CellwCand c;
+            if (cellw_choice(t, p, c)) make_cellw_plan(t, p, pl, c);
+        }
     }
     if (req == GOFR_KERNEL_CELL && !pl.cells)
         return fail(ctx, GOFR_ERR_UNSUPPORTED,
@@ -1674,7 +1711,11 @@ int enqueue_run(gofr_ctx *ctx, const TrajDev &t, const gofr_params &p, const Run
         C.cta_warps = pl.cta_warps;
         C.hcopy = pl.hcopy;
         set_cellw_geometry(C, pl.geom);
-        if (cellw_smem_bytes(L.nch, L.nbin, L.ntypes, C.cta_warps, C.hcopy) > max_smem)
+        C.pg = pl.pg;
+        C.npg = pl.npg;
+        C.pair.nparts = (int)std::max(1u, p.nparts);
+        C.pair.part_stride = (long long)rs.data_length;
+        if (cellw_smem_bytes(L.nch * C.pg, L.nbin, L.ntypes, C.cta_warps, C.hcopy) > max_smem)
             return fail(ctx, GOFR_ERR_UNSUPPORTED, "cell-list histogram does not fit shared memory");
         ++ctx->launches;
         if (launch_cellw_pairs(C, ctx->num_sms, ctx->stream))
@@ -2114,6 +2155,7 @@ int build_batch(gofr_ctx *ctx)
     std::vector<RunShape> shapes(ctx->trajs.size());
     std::vector<std::vector<CellCand>> cands(ctx->trajs.size());
     std::vector<double> work(ctx->trajs.size(), 0.0);
+    std::vector<char> is_cell(ctx->trajs.size(), 0);
     for (size_t k = 0; k < ctx->trajs.size(); ++k) {
         TrajDev &t = ctx->trajs[k];
         gofr_params p = t.params;
@@ -2126,13 +2168,22 @@ int build_batch(gofr_ctx *ctx)
         const unsigned long long pk = (unsigned long long)shapes[k].n_lags * shapes[k].n_orig * t.N * t.N;
         total += pk;
         work[k] = (double)pk;
-        if (plans[k].kind == 0 && !plans[k].wrapcheck && !plans[k].empty)
-            cands[k] = cell_candidates(t, p);
+        // cell lists as AUTO takes them for a single trajectory
+        Plan q = plans[k];
+        if (auto_cell_plan(t, p, q)) {
+            if (q.cellw) {
+                plans[k] = q;
+                is_cell[k] = 1;
+            } else {
+                cands[k] = cell_candidates(t, p);
+            }
+        }
     }
     B.pairs = total;
-    // One cell-list launch serves every member that gains from cell lists; it
-    // has one first-atoms-per-thread count R, the one with the least modelled
-    // time over the batch.
+    // One launch of the block cell-list kernel serves every member that gains
+    // from cell lists but cannot run the warp-streamed form; it has one
+    // first-atoms-per-thread count R, the one with the least modelled time over
+    // the batch.
     auto best_of = [&](size_t k, int r) -> const CellCand * {
         for (const CellCand &c : cands[k])
             if (c.r == r) return c.time < kCellAutoTime ? &c : nullptr;
@@ -2149,26 +2200,13 @@ int build_batch(gofr_ctx *ctx)
             if (tot < best_total) { best_total = tot; B.cell_r = r; }
         }
     }
-    std::vector<char> is_cell(ctx->trajs.size(), 0);
     for (size_t k = 0; k < ctx->trajs.size(); ++k) {
+        if (is_cell[k]) continue;
         const CellCand *c = best_of(k, B.cell_r);
         gofr_params p = ctx->trajs[k].params;
         p.nparts = 1;
         if (!c) {
-            // the warp-streamed form where the block form does not pay, as AUTO
-            // takes it for a single trajectory
-            CellwCand cw;
-            Plan q = plans[k];
-            q.cells = false;
-            p.kernel = GOFR_KERNEL_AUTO;
-            if (plans[k].kind == 0 && !plans[k].wrapcheck && !plans[k].empty &&
-                cellw_choice(ctx->trajs[k], p, cw) && cw.cost < kCellwAuto &&
-                make_cellw_plan(ctx->trajs[k], p, q, cw)) {
-                plans[k] = q;
-                is_cell[k] = 1;
-            } else {
-                B.allpairs_pairs += (unsigned long long)work[k];
-            }
+            B.allpairs_pairs += (unsigned long long)work[k];
             continue;
         }
         Plan q = plans[k];
@@ -2298,6 +2336,8 @@ int build_batch(gofr_ctx *ctx)
         C.cta_warps = q.cta_warps;  // as a single run of the member
         C.hcopy = 1;
         set_cellw_geometry(C, q.geom);
+        C.pg = C.npg = 1;
+        C.pair.nparts = 1;
         wl.push_back({(unsigned long long)work[k], C});
         B.launches[k] = PairLaunch{};  // not in the all-pairs queue
     }

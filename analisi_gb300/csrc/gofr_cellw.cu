@@ -51,6 +51,11 @@
 // first atom and record, then taken out of their cell and recomputed in FP64,
 // 32 at a time.
 //
+// Counts per reference thread partition of the first atoms take a histogram
+// of as many partitions as fit shared memory, and the first atoms of a block
+// in the order of (partition, type); the blocks are streamed once per such
+// group of partitions.
+//
 // Work is a list of (lag, origin, warp block) units, dealt to the CTAs in
 // chunks of decreasing size from one counter; the warps of a CTA take the
 // chunk's units one by one and never wait for one another inside a chunk.
@@ -81,6 +86,7 @@ constexpr int MAXROWS = CELLW_MAX_ROWS;  // neighbourhood rows of a warp block
 constexpr int MAXSEG = 2 * MAXROWS;      // sorted ranges of them (two when a row wraps the box)
 constexpr int QW = 64;         // FP64 recheck queue of a warp
 static_assert(CH == 4 * 32, "four records per lane");
+static_assert(FA == 64, "two groups of first atoms");
 static_assert(QW >= 64, "a round adds at most 32 entries to a queue drained at 32");
 
 constexpr unsigned SLOT_MASK = 0x1ffffffu;  // a sorted slot below its image's index
@@ -90,9 +96,10 @@ __device__ __forceinline__ int floordiv(int a, int n) { return a >= 0 ? a / n : 
 
 // Shared memory of one warp.
 struct WarpArea {
-    ulonglong2 fa[FA][2];        // first atoms {x x | y y}, {z z | w, run end << 8 | type}: coordinates
-                                 // duplicated for f32x2, w = type << 24 | id, and the end of the run
-                                 // of first atoms of the same type
+    ulonglong2 fa[FA][2];        // first atoms {x x | y y}, {z z | w, run end << 16 | class}:
+                                 // coordinates duplicated for f32x2, w = type << 24 | id, the class
+                                 // partition ntypes + type (the partition's place in the histogram)
+                                 // and the end of the run of first atoms of the class
     uint2 near[QW];              // pairs near a bin edge: {first atom, image << 25 | sorted slot}
     uint2 q[QW];                 // FP64 recheck queue: w of both atoms
     int2 src[MAXSEG];            // {sorted slot of the segment's first record - its flat index, image}
@@ -101,15 +108,17 @@ struct WarpArea {
 
 // NWARP warps per CTA, HCOPY copies of the shared histogram (warp w adds to
 // copy w HCOPY / NWARP: the privatisation depth, fewer warps contending for
-// each bin), MODE the bin map's (RadialMap).
-template <int NWARP, int HCOPY, int MODE>
+// each bin), MODE the bin map's (RadialMap), PARTS: counts per partition (apart:
+// the first atoms' partitions cost the form without them 2 % in registers).
+template <int NWARP, int HCOPY, int MODE, bool PARTS>
 __global__ void __launch_bounds__(NWARP * 32, 32 / NWARP) k_pairs_cellw(const CellwLaunch C)
 {
     constexpr int NT = NWARP * 32;
     extern __shared__ __align__(128) unsigned char smem[];
     const PairLaunch &P = C.pair;
     const int nbin = P.nbin, nrow = nbin + 1;  // histogram row: nbin bins and an unread cell
-    const int hist_cap = P.nch * nrow + 1;      // the first row has its cell -1, too
+    const int nch = PARTS ? P.nch * C.pg : P.nch;  // rows: C.pg partitions' channels
+    const int hist_cap = nch * nrow + 1;        // the first row has its cell -1, too
     WarpArea *const areas = reinterpret_cast<WarpArea *>(smem);
     unsigned *const hist = reinterpret_cast<unsigned *>(areas + NWARP);
     unsigned short *const chtab = reinterpret_cast<unsigned short *>(hist + HCOPY * hist_cap);
@@ -122,7 +131,7 @@ __global__ void __launch_bounds__(NWARP * 32, 32 / NWARP) k_pairs_cellw(const Ce
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const unsigned lt = (1u << lane) - 1u;  // the lanes below this one
     WarpArea &A = areas[warp];
-    const int hlen = P.nch * nbin;
+    const int per_part = PARTS ? P.N / P.nparts : 1;  // first atom a: partition min(a / per_part, nparts - 1)
     unsigned *const whist = hist + (warp * HCOPY / NWARP) * hist_cap + 1;  // this warp's row 0
     // row address of channel ch as bin_pair2 takes it: row0 + ch * rowb
     const unsigned row0 = smem_u32(whist) - 4u * RADIAL_MAGIC_BITS, rowb = 4u * (unsigned)nrow;
@@ -145,32 +154,37 @@ __global__ void __launch_bounds__(NWARP * 32, 32 / NWARP) k_pairs_cellw(const Ce
     unsigned long long n_cand = 0, n_rech = 0, n_eval = 0;  // n_cand: counts flushed
     bool lost = false;                                      // a u32 bin could have overflowed
 
-    // Adds the CTA's histogram copies to the counts of lag index lag_idx and
-    // clears them (all threads; every warp is done with its pairs).  A u32 bin
-    // holds its hits exactly only while fewer than 2^32 pairs were evaluated
-    // (the host keeps chunks far below).
-    auto flush = [&](int lag_idx) {
+    // Adds the CTA's histogram copies to the counts of plane (partition group,
+    // lag) and clears them (all threads; every warp is done with its pairs).  A
+    // u32 bin holds its hits exactly only while fewer than 2^32 pairs were
+    // evaluated (the host keeps chunks far below).
+    auto flush = [&](int plane) {
         if (s_pairs > 0xffffffffull) lost = true;
-        for (int i = tid; i < hlen; i += NT) {
-            const int at = (i / nbin) * nrow + i % nbin + 1;
+        const int grp = PARTS ? plane / P.n_lags : 0, lag_idx = plane - grp * P.n_lags;
+        unsigned long long *const out = P.counts + (PARTS ? grp * C.pg * P.part_stride : 0) +
+                                        (long long)lag_idx * P.every * P.nch * nbin;
+        for (int i = tid; i < nch * nbin; i += NT) {
+            const int row = i / nbin, b = i - row * nbin, at = row * nrow + b + 1;
             unsigned v = 0;  // modulo 2^32: a copy may hold the self pairs another one counted
 #pragma unroll
             for (int c = 0; c < HCOPY; ++c) v += hist[c * hist_cap + at];
 #pragma unroll
             for (int c = 0; c < HCOPY; ++c) hist[c * hist_cap + at] = 0u;
             n_cand += v;
-            if (v && !lost)
-                atomicAdd(P.counts + (long long)lag_idx * P.every * hlen + i,
+            if (v && !lost) {
+                const int part = PARTS ? row / P.nch : 0;
+                atomicAdd(out + part * P.part_stride + (row - part * P.nch) * nbin + b,
                           (unsigned long long)v);
+            }
         }
         __syncthreads();
         if (tid == 0) s_pairs = 0ull;
         __syncthreads();
     };
 
-    // units: (lag, origin, warp block), the warp block fastest
-    const long long per_lag = (long long)P.n_orig * nwb, U = per_lag * P.n_lags;
-    int cur_lag = -1;
+    // units: (partition group, lag, origin, warp block), the warp block fastest
+    const long long per_plane = (long long)P.n_orig * nwb, U = per_plane * P.n_lags * (PARTS ? C.npg : 1);
+    int cur = -1;  // plane (partition group, lag) of the histogram
     while (!lost) {
         __syncthreads();  // every warp has read the last chunk's range
         if (tid == 0) {
@@ -186,25 +200,32 @@ __global__ void __launch_bounds__(NWARP * 32, 32 / NWARP) k_pairs_cellw(const Ce
         const long long c0 = s_u0, c1 = s_u1;
         if (c0 >= c1) break;
         for (long long g0 = c0; g0 < c1 && !lost;) {
-        const int lag_idx = (int)(g0 / per_lag);
-        const long long g1 = min(c1, (lag_idx + 1) * per_lag);
+        const int plane = (int)(g0 / per_plane);
+        const int lag_idx = PARTS ? plane % P.n_lags : plane;
+        const int part0 = PARTS ? plane / P.n_lags * C.pg : 0;
+        const long long g1 = min(c1, (plane + 1) * per_plane);
         if (g0 != c0) {
-            __syncthreads();  // the warps are done with the chunk's last lag
+            __syncthreads();  // the warps are done with the chunk's last plane
             if (tid == 0) {
                 s_next = 0;
                 s_full = s_pairs > 0x7fffffffull;
             }
             __syncthreads();
         }
-        if (cur_lag >= 0 && (lag_idx != cur_lag || s_full)) flush(cur_lag);
-        cur_lag = lag_idx;
+        if (cur >= 0 && (plane != cur || s_full)) flush(cur);
+        cur = plane;
         int k = -1;  // origin of the warp's queues
         long long fo = 0, fl = 0;
         const int *st_o = nullptr, *st_l = nullptr;
         const float4 *rec_o = nullptr, *rec_l = nullptr;
-        const long long seg_orig = (g0 - lag_idx * per_lag) / nwb;  // the segment's first origin
-        const long long seg_off = (g0 - lag_idx * per_lag) - seg_orig * nwb;
+        const long long seg_orig = (g0 - plane * per_plane) / nwb;  // the segment's first origin
+        const long long seg_off = (g0 - plane * per_plane) - seg_orig * nwb;
 
+        // First row of the histogram of atom ia's partition (negative, or C.pg
+        // partitions on: not one of the histogram's).
+        auto part_row = [&](int ia) {
+            return PARTS ? (min(ia / per_part, P.nparts - 1) - part0) * P.nch : 0;
+        };
         // Recomputes queued pairs [0, n) in exact FP64 (reference arithmetic),
         // one per lane; into the channel of distinct atoms, like every pair.
         auto recheck = [&](int n) {
@@ -219,8 +240,9 @@ __global__ void __launch_bounds__(NWARP * 32, 32 / NWARP) k_pairs_cellw(const Ce
                                          : ref_d2<false>(xi[0], xi[1], xi[2], xj[0], xj[1], xj[2],
                                                          box, P.err);
                 const int b = ref_bin(d2, P.rmin, P.dr, P.rmin2, P.rmax2, nbin);
-                const int ch = chtab[(int)(e.x >> 24) * P.ntypes + (int)(e.y >> 24)];
-                if (b >= 0 && GOFR_CHECK(ch < P.nch && b < nbin, P.err))
+                const int ch = part_row((int)(e.x & 0xffffffu)) +
+                               chtab[(int)(e.x >> 24) * P.ntypes + (int)(e.y >> 24)];
+                if (b >= 0 && GOFR_CHECK(ch >= 0 && ch < nch && b < nbin, P.err))
                     atomicAdd(whist + ch * nrow + b, 1u);
                 ++n_rech;
             }
@@ -250,7 +272,8 @@ __global__ void __launch_bounds__(NWARP * 32, 32 / NWARP) k_pairs_cellw(const Ce
                 need = t <= P.rm.t_hi && t >= P.rm.t_lo;
                 const int b = (int)(__float_as_uint(t) - RADIAL_MAGIC_BITS);
                 if (b >= 0 && b < nbin)
-                    atomicSub(whist + chtab[(int)(wi >> 24) * P.ntypes + (int)(wj >> 24)] * nrow + b,
+                    atomicSub(whist + (part_row((int)(wi & 0xffffffu)) +
+                                       chtab[(int)(wi >> 24) * P.ntypes + (int)(wj >> 24)]) * nrow + b,
                               1u);
             }
             const unsigned m = __ballot_sync(0xffffffffu, need);
@@ -370,12 +393,18 @@ __global__ void __launch_bounds__(NWARP * 32, 32 / NWARP) k_pairs_cellw(const Ce
             if (lane == 0) A.pre[nseg + 32] = 0x7fffffff;
 
             for (int ibase = 0; ibase < n_i; ibase += FA) {
-                // first atoms ibase .. ibase + na - 1 of the block, each group of
-                // 32 in the order of their types (the row addresses of a lane's
-                // records change only with the first atom's type)
-                const int na = min(FA, n_i - ibase);
-                for (int q0 = 0; q0 < na; q0 += 32) {
-                    const int q = q0 + lane;
+                // first atoms ibase .. ibase + n - 1 of the block, those of the
+                // histogram's partitions, each group of 32 in the order of their
+                // classes (the row addresses of a lane's records change only with
+                // the first atom's class)
+                const int n = min(FA, n_i - ibase);
+                int nag[FA / 32];  // first atoms of each group (slots 32 g ...)
+                int na = 0;
+#pragma unroll
+                for (int g = 0; g < FA / 32; ++g) {
+                    const int q0 = 32 * g, q = q0 + lane;
+                    nag[g] = 0;
+                    if (q0 >= n) continue;
                     // row of atom ibase + q (every lane takes part in the shuffles)
                     const int qq = min(ibase + q, n_i - 1);
                     int row = 0;
@@ -384,37 +413,43 @@ __global__ void __launch_bounds__(NWARP * 32, 32 / NWARP) k_pairs_cellw(const Ce
                     const int rb = __shfl_sync(0xffffffffu, ib, row);
                     const int rp = __shfl_sync(0xffffffffu, ipre - ilen, row);
                     float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-                    if (q < na) v = rec_o[rb + (qq - rp)];
-                    const unsigned w = __float_as_uint(v.w), ti = w >> 24;
-                    unsigned left = __ballot_sync(0xffffffffu, q < na);
-                    int at = q0, end = q0;  // its place, the end of its type's run
+                    if (q < n) v = rec_o[rb + (qq - rp)];
+                    const unsigned w = __float_as_uint(v.w);
+                    const int ia = (int)(w & 0xffffffu), prow = part_row(ia);
+                    const bool have = q < n && (!PARTS || (prow >= 0 && prow < nch));
+                    const int ti = (int)(w >> 24),
+                              cls = PARTS ? prow / P.nch * P.ntypes + ti : ti;
+                    unsigned left = __ballot_sync(0xffffffffu, have);
+                    nag[g] = __popc(left);
+                    na += nag[g];
+                    int at = q0, end = q0;  // its place, the end of its class's run
                     for (int base = q0; left;) {
-                        const unsigned t = __shfl_sync(0xffffffffu, ti, __ffs(left) - 1);
-                        const unsigned m = __ballot_sync(0xffffffffu, q < na && ti == t);
-                        if (q < na && ti == t) {
+                        const int c = __shfl_sync(0xffffffffu, cls, __ffs(left) - 1);
+                        const unsigned m = __ballot_sync(0xffffffffu, have && cls == c);
+                        if (have && cls == c) {
                             at = base + __popc(m & lt);
                             end = base + __popc(m);
                         }
                         base += __popc(m);
                         left &= ~m;
                     }
-                    if (q < na) {
+                    if (have) {
                         const f2 z = f2pk(v.z, v.z);
                         A.fa[at][0] = make_ulonglong2(f2pk(v.x, v.x), f2pk(v.y, v.y));
                         A.fa[at][1] = make_ulonglong2(
-                            z, (unsigned long long)((unsigned)end << 8 | ti) << 32 | w);
+                            z, (unsigned long long)((unsigned)end << 16 | (unsigned)cls) << 32 | w);
                         // the atom's pair with itself: from the channel of distinct
                         // atoms, where the loop below counts it, to its own
-                        const int ia = (int)(w & 0xffffffu);
                         const int b = P.tric ? self_bin<true>(P, fo, fl, ia)
                                              : self_bin<false>(P, fo, fl, ia);
                         if (b >= 0) {
-                            const int ch = chtab[(int)ti * P.ntypes + (int)ti];
+                            const int ch = prow + chtab[ti * P.ntypes + ti];
                             atomicSub(whist + ch * nrow + b, 1u);
                             atomicAdd(whist + (ch + half_ch) * nrow + b, 1u);
                         }
                     }
                 }
+                if (na == 0) continue;
                 if (lane == 0) {
                     const unsigned long long pe = (unsigned long long)na * (unsigned long long)n_j;
                     n_eval += pe;
@@ -455,8 +490,8 @@ __global__ void __launch_bounds__(NWARP * 32, 32 / NWARP) k_pairs_cellw(const Ce
                     const f2 xa = f2pk(x[0], x[1]), xb = f2pk(x[2], x[3]);
                     const f2 ya = f2pk(y[0], y[1]), yb = f2pk(y[2], y[3]);
                     const f2 za = f2pk(z[0], z[1]), zb = f2pk(z[2], z[3]);
-                    for (int q0 = 0; q0 < na; q0 += 32) {
-                        const int q1 = min(na, q0 + 32);
+                    for (int g = 0; g < FA / 32; ++g) {
+                        const int q0 = 32 * g, q1 = q0 + (g ? nag[1] : nag[0]);
                         unsigned mk[4] = {0u, 0u, 0u, 0u}, bit = 1u;
                         // one first atom (broadcast) against the lane's four records
                         auto four = [&](f2 fx, f2 fy, f2 fz, const unsigned *row) {
@@ -468,16 +503,18 @@ __global__ void __launch_bounds__(NWARP * 32, 32 / NWARP) k_pairs_cellw(const Ce
                             bin_pair2<MODE>(da, inv, off, P.rm, row[0], row[1], bit, mk[0], mk[1]);
                             bin_pair2<MODE>(db, inv, off, P.rm, row[2], row[3], bit, mk[2], mk[3]);
                         };
-                        // first atoms of one type at a time; one a turn: the loop is
+                        // first atoms of one class at a time; one a turn: the loop is
                         // small (unrolled by two it measured 3 % slower, by four
                         // 50 %: instruction fetches)
                         for (int i = q0; i < q1;) {
                             const unsigned hi = (unsigned)(A.fa[i][1].y >> 32);
-                            const int e = (int)(hi >> 8);
-                            const unsigned short *ct = chtab + (int)(hi & 0xffu) * P.ntypes;
+                            const int e = (int)(hi >> 16), cls = (int)(hi & 0xffffu);
+                            const int part = PARTS ? cls / P.ntypes : 0;
+                            const unsigned short *ct = chtab + (cls - part * P.ntypes) * P.ntypes;
+                            const unsigned rowp = row0 + rowb * (unsigned)(part * P.nch);
                             unsigned row[4];
 #pragma unroll
-                            for (int t = 0; t < 4; ++t) row[t] = row0 + rowb * ct[tj[t]];
+                            for (int t = 0; t < 4; ++t) row[t] = rowp + rowb * ct[tj[t]];
                             for (; i < e; ++i) {
                                 const ulonglong2 u0 = A.fa[i][0];
                                 four(u0.x, u0.y, A.fa[i][1].x, row);
@@ -521,7 +558,7 @@ __global__ void __launch_bounds__(NWARP * 32, 32 / NWARP) k_pairs_cellw(const Ce
         }
     }
     __syncthreads();
-    if (cur_lag >= 0 && !lost) flush(cur_lag);
+    if (cur >= 0 && !lost) flush(cur);
     if (tid == 0) {
         if (lost) atomicOr(P.err, ERRW_HIST_OVERFLOW);
         // the last CTA leaves the queue as the next launch on the stream takes it
@@ -616,13 +653,13 @@ int launch_cell_scatter_w(const double *pos64, const unsigned char *types8, size
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
-template <int NWARP, int HCOPY, int MODE>
+template <int NWARP, int HCOPY, int MODE, bool PARTS>
 static int launch_cellw_shape(const CellwLaunch &C, int num_sms, cudaStream_t s)
 {
     using namespace cellw;
     constexpr int NT = NWARP * 32;
-    auto kern = k_pairs_cellw<NWARP, HCOPY, MODE>;
-    const int smem = cellw_smem_bytes(C.pair.nch, C.pair.nbin, C.pair.ntypes, NWARP, HCOPY);
+    auto kern = k_pairs_cellw<NWARP, HCOPY, MODE, PARTS>;
+    const int smem = cellw_smem_bytes(C.pair.nch * C.pg, C.pair.nbin, C.pair.ntypes, NWARP, HCOPY);
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) !=
         cudaSuccess)
         return -1;
@@ -631,7 +668,7 @@ static int launch_cellw_shape(const CellwLaunch &C, int num_sms, cudaStream_t s)
         return -1;
     if (per_sm < 1) return -2;
     // at least a warp block a warp
-    const long long units = C.pair.n_items * C.nw[0] * C.nw[1] * C.nw[2];
+    const long long units = C.pair.n_items * C.npg * C.nw[0] * C.nw[1] * C.nw[2];
     long long grid = (long long)num_sms * per_sm;
     if (grid > (units + NWARP - 1) / NWARP) grid = (units + NWARP - 1) / NWARP;
     kern<<<(unsigned)grid, NT, smem, s>>>(C);
@@ -641,12 +678,16 @@ static int launch_cellw_shape(const CellwLaunch &C, int num_sms, cudaStream_t s)
 template <int MODE>
 static int launch_cellw_mode(const CellwLaunch &C, int num_sms, cudaStream_t s)
 {
-    if (C.cta_warps == 16) {
-        return C.hcopy == 2 ? launch_cellw_shape<16, 2, MODE>(C, num_sms, s)
-                            : launch_cellw_shape<16, 1, MODE>(C, num_sms, s);
+    if (C.pair.nparts > 1) {
+        return C.cta_warps == 16 ? launch_cellw_shape<16, 1, MODE, true>(C, num_sms, s)
+                                 : launch_cellw_shape<8, 1, MODE, true>(C, num_sms, s);
     }
-    return C.hcopy == 2 ? launch_cellw_shape<8, 2, MODE>(C, num_sms, s)
-                        : launch_cellw_shape<8, 1, MODE>(C, num_sms, s);
+    if (C.cta_warps == 16) {
+        return C.hcopy == 2 ? launch_cellw_shape<16, 2, MODE, false>(C, num_sms, s)
+                            : launch_cellw_shape<16, 1, MODE, false>(C, num_sms, s);
+    }
+    return C.hcopy == 2 ? launch_cellw_shape<8, 2, MODE, false>(C, num_sms, s)
+                        : launch_cellw_shape<8, 1, MODE, false>(C, num_sms, s);
 }
 
 int launch_cellw_pairs(const CellwLaunch &C, int num_sms, cudaStream_t s)

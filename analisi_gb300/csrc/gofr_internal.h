@@ -155,6 +155,7 @@ struct CellwLaunch {
     int nw[3];                     // warp blocks per axis
     int reach;                     // neighbour cells per side
     int r;                         // records per lane (4; kept in plans and tuner keys)
+    int pg, npg;                   // partitions per histogram, groups of them (pair.nparts)
     long long most;                // warp blocks of a CTA's chunk at most
     unsigned *queue;               // {next chunk, CTAs done}, zero before and after a launch
     int cta_warps;                 // warps per CTA: 8 (two CTAs per SM) or 16 (one)

@@ -83,9 +83,9 @@ enum gofr_kernel {
                                     the cell-list conditions, a histogram and channel
                                     table that fit shared memory, and tilts
                                     that keep the images a block reaches within two box
-                                    edges).  AUTO takes it wherever it would take the block
-                                    cell-list form, and for a triclinic box when it
-                                    evaluates under half of the pairs.
+                                    edges).  AUTO takes it for 2048 atoms or more
+                                    where its modelled cost is below the all-pairs
+                                    kernel's.
                                     ANALISI_GB300_CELLW_PLAN="reach,4,wx,wy,wz" pins its
                                     configuration (4: the records a lane holds) */
 };

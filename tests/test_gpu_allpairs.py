@@ -85,3 +85,30 @@ def test_batch_of_every_kind(gpu_engine, oracle_mod, rmin):
     for use_graph in (True, False):
         for got, (w, p) in zip(gpu_engine.batch_run(use_graph=use_graph), members):
             np.testing.assert_array_equal(got, _ref(oracle_mod, w, p))
+
+
+# N, L, types, triclinic, rmax, bins, partitions, kernel (40: more partitions than
+# one histogram holds, in a box where the all-pairs kernel is the cheaper one
+# then, and in one where it is not; 700: more partitions than atoms of a warp block)
+@pytest.mark.parametrize("case", [(2300, 27.0, 3, False, 5.0, 37, 4, 5),
+                                  (2301, 27.0, 3, False, 5.0, 400, 40, 1),
+                                  (6001, 45.0, 3, False, 5.0, 400, 40, 5),
+                                  (2099, 26.0, 1, False, 4.0, 20, 700, 5),
+                                  (4100, 33.0, 2, True, 6.0, 50, 3, 5)],
+                         ids=["4", "40-allpairs", "40", "700", "tric"])
+def test_cell_lists_per_partition(gpu_engine, oracle_mod, case):
+    N, L, nt, tric, rmax, nbin, parts, kernel = case
+    w = _case(N, L, nt, tric)
+    p = _p(0.0, rmax, nbin=nbin)
+    gpu_engine.set_frames(w["positions"], w["boxes"], w["type_ids"], w["ntypes"], triclinic=tric)
+    args = [p[k] for k in ("rmin", "rmax", "nbin", "tmax", "skip", "every", "ntimesteps", "primo")]
+    got = gpu_engine.run(*args, nparts=parts)
+    assert gpu_engine.stats()["kernel_used"] == kernel
+    np.testing.assert_array_equal(got, _ref(oracle_mod, w, p, parts, True))
+    got = gpu_engine.run_windows(p["rmin"], rmax, nbin, 2, 2, 1, 3, [3, 0], nparts=parts)
+    for k, first in enumerate([3, 0]):
+        np.testing.assert_array_equal(
+            got[k], _ref(oracle_mod, w, dict(p, tmax=2, ntimesteps=3, primo=first), parts, True))
+    # a forced cell-list kernel still refuses partitions
+    with pytest.raises(engine.GofrError):
+        gpu_engine.run(*args, kernel="cellw", nparts=parts)
