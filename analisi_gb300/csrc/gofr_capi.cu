@@ -2050,6 +2050,41 @@ int tune_plan(gofr_ctx *ctx, const TrajDev &t, const gofr_params &p, Plan &pl)
     return GOFR_OK;
 }
 
+// The plan of a run on the resident frames: make_plan's, the tuner's where
+// asked for or known, with the cell lists built.
+int choose_plan(gofr_ctx *ctx, const TrajDev &t, const gofr_params &p, Plan &pl)
+{
+    // the tuner starts from the all-pairs plan and decides on cells itself;
+    // AUTO takes the tuner's choice when it has one for this job's key
+    const bool tuned = p.nparts <= 1 &&
+                       (p.kernel == GOFR_KERNEL_TUNED ||
+                        (p.kernel == GOFR_KERNEL_AUTO && tune_known(t, p)));
+    int rc = make_plan(ctx, t, p, pl, !tuned);
+    if (rc) return rc;
+    if (tuned) {
+        rc = tune_plan(ctx, t, p, pl);
+        if (rc) return rc;
+    }
+    if (pl.cells && p.kernel != GOFR_KERNEL_CELL && p.kernel != GOFR_KERNEL_CELL_WARP) {
+        // a plan the engine chose (AUTO / TUNED) whose cell lists do not fit
+        // the device: the all-pairs form gives the same counts
+        const int crc = ensure_cells(ctx, t, pl);
+        if (crc == GOFR_ERR_NOMEM) {
+            ctx->err.clear();
+            (void)cudaGetLastError();
+            gofr_params q = p;
+            q.kernel = GOFR_KERNEL_AUTO;
+            Plan ap;
+            rc = make_plan(ctx, t, q, ap, false);
+            if (rc) return rc;
+            pl = ap;
+        } else if (crc) {
+            return crc;
+        }
+    }
+    return GOFR_OK;
+}
+
 int run_common(gofr_ctx *ctx, const gofr_params *p, unsigned long long *counts_dev,
                unsigned long long *counts_host)
 {
@@ -2061,34 +2096,8 @@ int run_common(gofr_ctx *ctx, const gofr_params *p, unsigned long long *counts_d
     int rc = shape_of(ctx, t, *p, rs);
     if (rc) return rc;
     Plan pl;
-    // the tuner starts from the all-pairs plan and decides on cells itself;
-    // AUTO takes the tuner's choice when it has one for this job's key
-    const bool tuned = p->nparts <= 1 &&
-                       (p->kernel == GOFR_KERNEL_TUNED ||
-                        (p->kernel == GOFR_KERNEL_AUTO && tune_known(t, *p)));
-    rc = make_plan(ctx, t, *p, pl, !tuned);
+    rc = choose_plan(ctx, t, *p, pl);
     if (rc) return rc;
-    if (tuned) {
-        rc = tune_plan(ctx, t, *p, pl);
-        if (rc) return rc;
-    }
-    if (pl.cells && p->kernel != GOFR_KERNEL_CELL && p->kernel != GOFR_KERNEL_CELL_WARP) {
-        // a plan the engine chose (AUTO / TUNED) whose cell lists do not fit
-        // the device: the all-pairs form gives the same counts
-        const int crc = ensure_cells(ctx, t, pl);
-        if (crc == GOFR_ERR_NOMEM) {
-            ctx->err.clear();
-            (void)cudaGetLastError();
-            gofr_params q = *p;
-            q.kernel = GOFR_KERNEL_AUTO;
-            Plan ap;
-            rc = make_plan(ctx, t, q, ap, false);
-            if (rc) return rc;
-            pl = ap;
-        } else if (crc) {
-            return crc;
-        }
-    }
     const unsigned nparts = p->nparts > 1 ? p->nparts : 1;
     const size_t n_out = rs.data_length * nparts;
     unsigned long long *out = counts_dev;
@@ -2626,7 +2635,7 @@ int run_windows_impl(gofr_ctx *ctx, const gofr_params *p, unsigned nwin,
         if (rc) return rc;
     }
     Plan pl;
-    int rc = make_plan(ctx, t, *p, pl);
+    int rc = choose_plan(ctx, t, *p, pl);
     if (rc) return rc;
     const size_t per_win = rs.data_length * nparts;
     const size_t n_out = per_win * nwin;

@@ -142,16 +142,24 @@ public:
             uploaded_version = ~0ull;  // the context holds the last chunk's frames
         } else {
             check(gofr_output_size(ctx, &p, &n));
-            counts.resize(n ? n : 1);
-            check(gofr_run(ctx, &p, counts.data()));
         }
         const size_t dl = vdata.size();
-        if (n == 0 || dl == 0) return;
         std::vector<double> tmp;
         double *dst = nullptr;
         if constexpr (sizeof(TFLOAT) == sizeof(double)) dst = reinterpret_cast<double *>(vdata.data());
         else { tmp.resize(dl); dst = tmp.data(); }
-        check(gofr_counts_to_buffer(counts.data(), dl, nthreads, ntimesteps, skip, dst));
+        if (!stream && dl > 0 && n == dl * nthreads) {
+            // the counts stay on the GPU, which folds the partitions and adds incr
+            // as the reference's threads do: only the result comes back
+            check(gofr_run_normalized(ctx, &p, 0, nullptr, 0, dst, nullptr));
+        } else {
+            if (!stream) {
+                counts.resize(n ? n : 1);
+                check(gofr_run(ctx, &p, counts.data()));
+            }
+            if (n == 0 || dl == 0) return;
+            check(gofr_counts_to_buffer(counts.data(), dl, nthreads, ntimesteps, skip, dst));
+        }
         if constexpr (sizeof(TFLOAT) != sizeof(double))
             for (size_t i = 0; i < dl; ++i) vdata[i] = (TFLOAT)tmp[i];
         if (debug) dump();
