@@ -72,6 +72,7 @@ struct TrajDev {
     std::vector<int> h_perm, h_tbegin, h_types;
     int *d_perm = nullptr, *d_tbegin = nullptr;
     double *d_cm = nullptr;          // [T][ntypes][3]
+    double cm_max = 0.0;             // largest |component| of them
 };
 
 }  // namespace
@@ -3199,6 +3200,9 @@ int gofr_set_centres(gofr_ctx *ctx, const double *centres, size_t nframes, unsig
     t.d_cm = nullptr;
     const size_t n = nframes * ntypes * 3;
     CK(dev_malloc(&t.d_cm, n * sizeof(double)));
+    t.cm_max = 0.0;
+    for (size_t i = 0; i < n; ++i)
+        t.cm_max = std::max(t.cm_max, std::isfinite(centres[i]) ? std::fabs(centres[i]) : INFINITY);
     CK(cudaMemcpyAsync(t.d_cm, centres, n * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
     return GOFR_OK;
@@ -3241,16 +3245,11 @@ int gofr_msd_run(gofr_ctx *ctx, const gofr_msd_params *p, double *out_host)
         std::memset(out_host, 0, nout * sizeof(double));
         return GOFR_OK;
     }
-    int rc = ensure(ctx, ctx->d_msd_partial, ctx->cap_msd_partial, nout * n_orig);
-    if (rc) return rc;
-    rc = ensure(ctx, ctx->d_msd_out, ctx->cap_msd_out, nout);
-    if (rc) return rc;
     MsdLaunch M{};
     M.pos64 = t.pos64;
     M.cm = t.d_cm;
     M.perm = t.d_perm;
     M.tbegin = t.d_tbegin;
-    M.partial = ctx->d_msd_partial;
     M.N = (int)t.N;
     M.ntypes = (int)t.ntypes;
     M.leff = (int)leff;
@@ -3259,23 +3258,59 @@ int gofr_msd_run(gofr_ctx *ctx, const gofr_msd_params *p, double *out_host)
     M.primo = (long long)p->primo;
     M.cm_msd = p->center_of_mass ? 1 : 0;
     M.cm_self = p->in_center_of_mass_frame ? 1 : 0;
-    CK(cudaEventRecord(ctx->ev[0], ctx->stream));
-    CK(cudaMemsetAsync(ctx->d_err, 0, sizeof(unsigned), ctx->stream));
-    CK(cudaMemsetAsync(ctx->d_stats, 0, ST_COUNT * sizeof(unsigned long long), ctx->stream));
-    CK(cudaEventRecord(ctx->ev[1], ctx->stream));
-    ctx->launches += 2;
-    if (launch_msd(M, ctx->d_msd_out, ctx->num_sms, ctx->stream))
-        return fail(ctx, GOFR_ERR_CUDA, "MSD kernel launch failed: %s",
-                    cudaGetErrorString(cudaGetLastError()));
-    CK(cudaEventRecord(ctx->ev[2], ctx->stream));
-    CK(cudaMemcpyAsync(out_host, ctx->d_msd_out, nout * sizeof(double), cudaMemcpyDeviceToHost,
-                       ctx->stream));
-    CK(cudaEventRecord(ctx->ev[3], ctx->stream));
-    // one squared displacement per (lag, origin, atom)
-    ctx->stats.pairs = (unsigned long long)leff * n_orig * t.N;
-    ctx->stats.evaluated = ctx->stats.pairs;
-    ctx->stats.kernel_used = -1;
-    return gofr_sync(ctx);
+    // |x| (and |x - centre|) below 2^e; centres that are not finite take the
+    // FP64 form, which carries them into the result
+    double bound = 0.0;
+    for (int k = 0; k < 3; ++k) bound = std::max(bound, std::fabs(t.shift[k]) + t.M[k]);
+    if (M.cm_self) bound += t.cm_max;
+    bound *= 1.0 + std::ldexp(1.0, -40);
+    MsdFixed X{};
+    const bool fixed =
+        std::isfinite(bound) && msd_fixed_plan(M, t.h_tbegin.data(), ctx->num_sms, X);
+    int rc = ensure(ctx, ctx->d_msd_partial, ctx->cap_msd_partial,
+                    fixed ? msd_fixed_partial(M, X) : nout * n_orig);
+    if (rc) return rc;
+    rc = ensure(ctx, ctx->d_msd_out, ctx->cap_msd_out, nout);
+    if (rc) return rc;
+    M.partial = ctx->d_msd_partial;
+    if (fixed) {
+        int e = 0;
+        std::frexp(bound, &e);
+        X.shift = std::max(-900, std::min(900, MSD_FIXED_BITS - e));
+        X.partial = reinterpret_cast<long long *>(ctx->d_msd_partial);
+        X.inexact = reinterpret_cast<int *>(X.partial + msd_fixed_partial(M, X) -
+                                            (X.grid + M.ntypes));
+        X.suspect = ctx->d_stats + ST_CANDIDATES;  // unused by this calculation
+    }
+    for (bool exact = fixed;; exact = false) {
+        if (!exact) {
+            rc = ensure(ctx, ctx->d_msd_partial, ctx->cap_msd_partial, nout * n_orig);
+            if (rc) return rc;
+            M.partial = ctx->d_msd_partial;
+        }
+        CK(cudaEventRecord(ctx->ev[0], ctx->stream));
+        CK(cudaMemsetAsync(ctx->d_err, 0, sizeof(unsigned), ctx->stream));
+        CK(cudaMemsetAsync(ctx->d_stats, 0, ST_COUNT * sizeof(unsigned long long), ctx->stream));
+        CK(cudaEventRecord(ctx->ev[1], ctx->stream));
+        ctx->launches += 2;
+        if (exact ? launch_msd_fixed(M, X, ctx->d_msd_out, ctx->stream)
+                  : launch_msd(M, ctx->d_msd_out, ctx->num_sms, ctx->stream))
+            return fail(ctx, GOFR_ERR_CUDA, "MSD kernel launch failed: %s",
+                        cudaGetErrorString(cudaGetLastError()));
+        CK(cudaEventRecord(ctx->ev[2], ctx->stream));
+        CK(cudaMemcpyAsync(out_host, ctx->d_msd_out, nout * sizeof(double), cudaMemcpyDeviceToHost,
+                           ctx->stream));
+        CK(cudaEventRecord(ctx->ev[3], ctx->stream));
+        // one squared displacement per (lag, origin, atom)
+        ctx->stats.pairs = (unsigned long long)leff * n_orig * t.N;
+        ctx->stats.evaluated = ctx->stats.pairs;
+        ctx->stats.kernel_used = -1;
+        rc = gofr_sync(ctx);
+        if (rc) return rc;
+        const bool suspect = ctx->stats.candidates != 0;
+        ctx->stats.candidates = 0;
+        if (!suspect) return GOFR_OK;  // else the FP64 form over again
+    }
 }
 
 int gofr_neigh_layout(const gofr_ctx *ctx_c, const gofr_neigh_spec *spec, unsigned nspec,

@@ -207,6 +207,22 @@ struct MsdLaunch {
     int cm_msd, cm_self;
 };
 int launch_msd(const MsdLaunch &M, double *out_device, int num_sms, cudaStream_t s);
+// The same in exact integer sums (k_msd_fixed).
+struct MsdFixed {
+    int atoms, origins, tiles;  // atoms and origins of a chunk, tiles of origins
+    int frames;                 // frames of a chunk (its row length in shared memory)
+    int lags, phases, passes;   // lags and origin phases of a CTA's threads, CTAs per chunk range
+    long long chunks, per;      // chunks, chunks per CTA
+    int grid;
+    int shift;                  // coordinates are rint(x 2^shift)
+    long long *partial;         // [grid + ntypes][leff][6]
+    int *inexact;               // [grid + ntypes] a coordinate is not held exactly
+    unsigned long long *suspect;  // set when that could show in a result
+};
+constexpr int MSD_FIXED_BITS = 56;  // coordinates below 2^56
+bool msd_fixed_plan(const MsdLaunch &M, const int *h_tbegin, int num_sms, MsdFixed &X);
+size_t msd_fixed_partial(const MsdLaunch &M, const MsdFixed &X);  // 8-byte words of both
+int launch_msd_fixed(const MsdLaunch &M, const MsdFixed &X, double *out_device, cudaStream_t s);
 
 // Neighbour lists (gofr_neigh.cu)
 constexpr int NEIGH_MAXT = 32;

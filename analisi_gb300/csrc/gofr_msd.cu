@@ -4,13 +4,34 @@
 // The reference loops lag -> origin -> atom and keeps, per (lag, type), a
 // running mean of |x_i(o) - x_i(o+t)|^2 (optionally minus the type's
 // centre-of-mass displacement), and of the centres' own squared displacement.
-// Here every (origin, lag) item is one CTA: it forms each atom's displacement
-// with the reference's FP64 operations, adds its squared components into the
-// type's sum with FMAs (atoms visited in type-sorted order, one block
-// reduction per type) and writes one partial sum per (lag, origin, type).  A second kernel adds the origins of each
-// (lag, type) in a fixed order and divides by the count.  Items are ordered
-// origin-major so that consecutive CTAs share the origin frame and slide the
-// lagged frame, which keeps the frames they read in L2.
+//
+// k_msd_fixed: FP64 instructions issue at 1/64 of the FP32 rate here, so the
+// sums are taken in integers, exactly.  A coordinate (minus its type's centre
+// where asked for) is the 64-bit integer rint(x 2^s), s so that every
+// coordinate is below 2^56: three bits finer than FP64 resolves the largest
+// coordinates, so all but those within an eighth of zero are held exactly (and
+// those to 2^-57 of the largest).  A displacement is one 64-bit subtraction, its
+// square three 29-bit products (64-bit multiply-adds), whose sums are combined
+// in 128 bits and rounded once per (lag, type): no term is rounded at all,
+// where the FP64 sums rounded every one.  Where some coordinate is not held
+// exactly and a displacement is so small that this could show (2^42 units rms:
+// a relative error of 5e-13 at most above), the caller runs the FP64 form.  A CTA holds the frames of a few atoms of one type in
+// shared memory, so each coordinate is read from HBM once and every (origin,
+// lag) pair comes from shared memory: thread = (lag, phase of the origins),
+// consecutive lags reading consecutive frames.
+//   Bound by the 32-bit integer multiplier.  16384 atoms in
+// three types, 100 origins x 100 lags: 0.46 ms against 2.79 for the FP64 form;
+// 5003 atoms with both centre-of-mass options, 60 x 80: 0.12 against 0.48.
+//
+// k_msd_partial: the FP64 form, for windows of lags whose frames of one atom
+// do not fit shared memory (more than about 4000 lags).  Every (origin, lag)
+// item is one CTA: it forms each atom's displacement with the reference's FP64
+// operations, adds its squared components into the type's sum with FMAs
+// (atoms visited in type-sorted order, one block reduction per type) and
+// writes one partial sum per (lag, origin, type).  A second kernel adds the
+// origins of each (lag, type) in a fixed order and divides by the count.
+// Items are ordered origin-major so that consecutive CTAs share the origin
+// frame and slide the lagged frame, which keeps the frames they read in L2.
 #include <cstdint>
 #include <cuda_runtime.h>
 
@@ -109,6 +130,234 @@ __global__ void k_msd_final(const MsdLaunch M, double *out)
     }
 }
 
+// ---------------------------------------------------------------------------
+// exact integer sums
+// ---------------------------------------------------------------------------
+constexpr int FT = 512;    // threads per CTA
+constexpr int NACC = 6;    // sums h h, h l, l l: low 32 bits and the rest of each
+constexpr int TERMS = 8;   // squared displacements (three axes each) between two carries
+constexpr int PLANE = 105 * 1024 / 24;  // (atom, frame) entries of an axis in shared memory: a
+                                        // constant, so the axes are offsets of one address
+constexpr int BITS = MSD_FIXED_BITS;  // coordinates are below 2^BITS
+static_assert(BITS == 56, "the products of add_square");
+
+// Sums of the products of d = h 2^29 + l (|d| < 2^57, h signed, l in [0,
+// 2^29)): hh < 2^56, |hl| < 2^57 and ll < 2^58 in 64 bits, carried into the
+// sums of the high words every TERMS displacements (24 products of 2^58 and a
+// low word stay below 2^63).
+struct Acc {
+    long long p[3], hi[3];
+};
+
+// rint(x 2^shift) for |x| 2^shift < 2^BITS, halves away from zero: integer
+// instructions alone (a product and a conversion of the FP64 pipe took a
+// fifth of the kernel's time).  lost collects whether any bit was rounded off.
+__device__ __forceinline__ long long to_fixed(double x, int shift, bool &lost)
+{
+    const long long u = __double_as_longlong(x);
+    const int e = (int)(u >> 52 & 0x7ff);
+    const long long m = (u & 0xfffffffffffffll) | 0x10000000000000ll;
+    const int r = 1075 - shift - e;  // bits below the point
+    if (r > 53 || e == 0) {          // less than half a unit (and below 2^-1022)
+        lost = lost || x != 0.0;
+        return 0;
+    }
+    lost = lost || (r > 0 && (m & ((1ll << r) - 1)) != 0);
+    const long long v = r <= 0 ? m << -r : (m + (1ll << (r - 1))) >> r;
+    return u < 0 ? -v : v;
+}
+
+__device__ __forceinline__ void mad_wide(long long &a, int x, int y)
+{
+    asm("mad.wide.s32 %0, %1, %2, %0;" : "+l"(a) : "r"(x), "r"(y));
+}
+
+__device__ __forceinline__ void add_square(Acc &a, long long d)
+{
+    const int h = (int)(d >> 29), l = (int)d & 0x1fffffff;
+    mad_wide(a.p[0], h, h);
+    mad_wide(a.p[1], h, l);
+    mad_wide(a.p[2], l, l);
+}
+
+// p keeps its low 32 bits; the rest goes to hi.
+__device__ __forceinline__ void carry(Acc &a)
+{
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        a.hi[i] += a.p[i] >> 32;
+        a.p[i] &= 0xffffffffll;
+    }
+}
+
+// Chunks of type k: tiles of origins of groups of `atoms` atoms.
+__device__ __forceinline__ long long chunks_of(const MsdLaunch &M, const MsdFixed &X, int k)
+{
+    return (long long)((M.tbegin[k + 1] - M.tbegin[k] + X.atoms - 1) / X.atoms) * X.tiles;
+}
+
+// CTA b takes chunks [b per, (b + 1) per) of the types' chunks back to back.  The sums of the CTA's
+// chunks of type k go to partial[b + k] (CTAs and types both ascend, so the
+// entry is one (CTA, type)'s own).
+__global__ void __launch_bounds__(FT, 2) k_msd_fixed(const MsdLaunch M, const MsdFixed X)
+{
+    extern __shared__ __align__(16) long long smem[];
+    const int tid = threadIdx.x, F = X.frames;
+    const int l0 = blockIdx.y * X.lags, nl = min(X.lags, M.leff - l0);
+    const int lag = l0 + tid % X.lags, phase = tid / X.lags;
+    const bool busy = phase < X.phases && lag < l0 + nl;
+    const long long c0 = (long long)blockIdx.x * X.per, c1 = min(c0 + X.per, X.chunks);
+    Acc acc{};
+    bool lost = false;  // a coordinate of the type is not held exactly
+    const int step = X.phases * M.skip;
+    // loading: thread = (frame phase lf, atom la, axis lx)
+    const int per_frame = 3 * X.atoms, lstep = FT / per_frame, lf = tid / per_frame,
+              la = (tid - lf * per_frame) / 3, lx = tid - lf * per_frame - 3 * la;
+    int k = 0;
+    long long kb = 0, ke = chunks_of(M, X, 0);  // chunks of type k
+    auto to_type_of = [&](long long c) {
+        while (c >= ke) {
+            kb = ke;
+            ke += chunks_of(M, X, ++k);
+        }
+    };
+    to_type_of(c0);
+    // the sums of the CTA's chunks of type k, every phase's, to their entry
+    auto flush = [&]() {
+        long long *out = X.partial + ((long long)(blockIdx.x + k) * M.leff + l0) * NACC;
+        carry(acc);
+#pragma unroll
+        for (int i = 0; i < NACC; ++i) {
+            __syncthreads();  // the tile, or the last sum, is no longer read
+            smem[tid] = busy ? (i < 3 ? acc.p[i] : acc.hi[i - 3]) : 0;
+            __syncthreads();
+            if (tid < nl) {
+                long long v = 0;
+                for (int ph = 0; ph < X.phases; ++ph) v += smem[ph * X.lags + tid];
+                out[tid * NACC + i] = v;
+            }
+        }
+        acc = Acc{};
+        const int any = __syncthreads_or(lost);
+        if (tid == 0) X.inexact[blockIdx.x + k] = any;
+        lost = false;
+    };
+    for (long long c = c0; c < c1; ++c) {
+        if (c >= ke) {
+            flush();
+            to_type_of(c);
+        }
+        const int group = (int)((c - kb) / X.tiles),
+                  tile = (int)((c - kb) - (long long)group * X.tiles);
+        const int a0 = M.tbegin[k] + group * X.atoms, na = min(X.atoms, M.tbegin[k + 1] - a0);
+        const int o0 = tile * X.origins, no = min(X.origins, M.n_orig - o0);
+        const long long f0 = M.primo + (long long)o0 * M.skip;
+        const int nf = (no - 1) * M.skip + M.leff;
+        __syncthreads();  // the last tile is no longer read
+        if (la < na && lf < lstep) {
+            const double *x = M.pos64 + ((f0 + lf) * M.N + M.perm[a0 + la]) * 3 + lx;
+            const double *cm = M.cm_self ? M.cm + ((f0 + lf) * M.ntypes + k) * 3 + lx : nullptr;
+            long long *out = smem + lx * PLANE + la * F;
+#pragma unroll 4
+            for (int f = lf; f < nf; f += lstep) {
+                long long v = to_fixed(*x, X.shift, lost);
+                x += (long long)lstep * M.N * 3;
+                if (cm) {
+                    v -= to_fixed(*cm, X.shift, lost);
+                    cm += (long long)lstep * M.ntypes * 3;
+                }
+                out[f] = v;
+            }
+        }
+        __syncthreads();
+        if (busy) {
+            for (int a = 0; a < na; ++a) {
+                int i = a * F + phase * M.skip;
+                for (int o = phase; o < no;) {
+                    // TERMS origins between two carries
+                    const int oe = min(no, o + TERMS * X.phases);
+#pragma unroll 2
+                    for (; o < oe; o += X.phases, i += step) {
+                        const int j = i + lag;
+                        add_square(acc, smem[j] - smem[i]);
+                        add_square(acc, smem[j + PLANE] - smem[i + PLANE]);
+                        add_square(acc, smem[j + 2 * PLANE] - smem[i + 2 * PLANE]);
+                    }
+                    carry(acc);
+                }
+            }
+        }
+    }
+    flush();
+}
+
+__device__ __forceinline__ double to_double(__int128 v)  // v >= 0, one rounding of each half
+{
+    return __dadd_rn(__dmul_rn((double)(long long)(v >> 64), 18446744073709551616.0),
+                     __ull2double_rn((unsigned long long)v));
+}
+
+// One warp per result: the sums of a (lag, type) over its entries, exactly, or
+// the centres' squared displacement over the origins.
+__global__ void k_msd_fixed_final(const MsdLaunch M, const MsdFixed X, double *out)
+{
+    const int lane = threadIdx.x & 31;
+    const int fk = M.cm_msd ? 2 * M.ntypes : M.ntypes;
+    const int g = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (g >= M.leff * fk) return;
+    const int lag = g / fk, c = g - lag * fk;
+    if (c >= M.ntypes) {
+        const int k = c - M.ntypes;
+        double s = 0.0;
+        for (int o = lane; o < M.n_orig; o += 32) {
+            const long long fo = M.primo + (long long)o * M.skip;
+            const double *co = M.cm + (fo * M.ntypes + k) * 3;
+            const double *cl = M.cm + ((fo + lag) * M.ntypes + k) * 3;
+            s = __dadd_rn(s, sq3(__dsub_rn(co[0], cl[0]), __dsub_rn(co[1], cl[1]),
+                                 __dsub_rn(co[2], cl[2])));
+        }
+        for (int o = 16; o > 0; o >>= 1) s = __dadd_rn(s, __shfl_xor_sync(0xffffffffu, s, o));
+        if (lane == 0) out[g] = __ddiv_rn(s, (double)M.n_orig);
+        return;
+    }
+    __int128 hi = 0, lo = 0;  // the sum is hi 2^64 + lo
+    bool inexact = false;
+    long long kb = 0;
+    for (int k = 0; k < c; ++k) kb += chunks_of(M, X, k);
+    const long long ke = kb + chunks_of(M, X, c);
+    if (ke > kb) {
+        const long long b0 = kb / X.per, b1 = (ke - 1) / X.per;
+        for (long long b = b0 + lane; b <= b1; b += 32) {
+            const long long *v = X.partial + ((b + c) * M.leff + lag) * NACC;
+            inexact = inexact || X.inexact[b + c] != 0;
+            // h h 2^58 + 2 h l 2^29 + l l, each sum high 2^32 + low
+            hi += ((__int128)v[3] << 26) + (v[4] >> 2);
+            lo += ((__int128)v[0] << 58) + ((__int128)v[1] << 30) + v[2] +
+                  ((__int128)(v[4] & 3) << 62) + ((__int128)v[5] << 32);
+        }
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+        const unsigned long long h0 = __shfl_xor_sync(0xffffffffu, (unsigned long long)hi, o),
+                                 l0 = __shfl_xor_sync(0xffffffffu, (unsigned long long)lo, o);
+        const long long h1 = __shfl_xor_sync(0xffffffffu, (long long)(hi >> 64), o),
+                        l1 = __shfl_xor_sync(0xffffffffu, (long long)(lo >> 64), o);
+        hi += ((__int128)h1 << 64) + h0;
+        lo += ((__int128)l1 << 64) + l0;
+    }
+    inexact = __any_sync(0xffffffffu, inexact);
+    if (lane) return;
+    hi += lo >> 64;
+    const double sum = __dadd_rn(__dmul_rn(to_double(hi), 18446744073709551616.0),
+                                 __ull2double_rn((unsigned long long)lo));
+    const double count = (double)M.n_orig * (double)(M.tbegin[c + 1] - M.tbegin[c]);
+    const double mean = __ddiv_rn(sum, count);
+    out[g] = scalbn(mean, -2 * X.shift);
+    // coordinates near zero beside large ones are held to half a unit: a
+    // displacement of d units rms has a relative error of 2 / d at most (and far
+    // less in the mean over many).  Below 2^42 units the caller takes the FP64 form.
+    if (inexact && lag > 0 && mean < 19342813113834066795298816.0) *X.suspect = 1ull;  // 2^84
+}
+
 }  // namespace msd
 
 int launch_msd(const MsdLaunch &M, double *out_device, int num_sms, cudaStream_t s)
@@ -123,6 +372,70 @@ int launch_msd(const MsdLaunch &M, double *out_device, int num_sms, cudaStream_t
     long long g2 = (nout + NT - 1) / NT;
     if (g2 > (long long)num_sms * 8) g2 = (long long)num_sms * 8;
     k_msd_final<<<(unsigned)g2, NT, 0, s>>>(M, out_device);
+    return cudaGetLastError() == cudaSuccess ? 0 : -1;
+}
+
+size_t msd_fixed_partial(const MsdLaunch &M, const MsdFixed &X)
+{
+    return (size_t)(X.grid + M.ntypes) * ((size_t)M.leff * msd::NACC + 1);
+}
+
+// Atoms, origins and threads of a CTA of k_msd_fixed, for the type counts in
+// h_tbegin; false when the frames of one atom's lags do not fit shared memory
+// (two CTAs of 512 threads per SM).
+bool msd_fixed_plan(const MsdLaunch &M, const int *h_tbegin, int num_sms, MsdFixed &X)
+{
+    using namespace msd;
+    const long long budget = PLANE;
+    const long long all = (long long)(M.n_orig - 1) * M.skip + M.leff;
+    auto count = [&](int atoms, int tiles) {
+        long long c = 0;
+        for (int k = 0; k < M.ntypes; ++k)
+            c += (long long)((h_tbegin[k + 1] - h_tbegin[k] + atoms - 1) / atoms) * tiles;
+        return c;
+    };
+    X.atoms = 0;
+    for (int a = 16; a >= 1 && !X.atoms; a /= 2)  // every origin in one tile
+        if (all * a <= budget && (a <= 2 || count(a, 1) >= 16LL * num_sms)) X.atoms = a;
+    X.origins = M.n_orig;
+    for (int a = 8; a >= 1 && !X.atoms; a /= 2) {
+        // tiles of origins: each reads its lags' frames again, so three times
+        // as many frames as lags where more than one atom fits
+        const long long f = budget / a;
+        if (f < (a > 1 ? 3LL * M.leff : (long long)M.leff + M.skip)) continue;
+        X.atoms = a;
+        X.origins = (int)((f - M.leff) / M.skip + 1);
+    }
+    if (!X.atoms) return false;
+    X.origins = X.origins < M.n_orig ? X.origins : M.n_orig;
+    X.tiles = (M.n_orig + X.origins - 1) / X.origins;
+    X.frames = (X.origins - 1) * M.skip + M.leff;
+    X.lags = M.leff < FT ? M.leff : FT;
+    X.passes = (M.leff + X.lags - 1) / X.lags;
+    X.phases = FT / X.lags < M.n_orig ? FT / X.lags : M.n_orig;
+    X.chunks = count(X.atoms, X.tiles);
+    // contiguous chunks per CTA, two CTAs per SM; no 64-bit sum of 2^17 squares
+    // of three axes overflows
+    long long per = (X.chunks + 2LL * num_sms - 1) / (2LL * num_sms);
+    const long long most = (1LL << 17) / ((long long)X.atoms * X.origins);
+    if (most < 1) return false;
+    X.per = per < most ? (per > 0 ? per : 1) : most;
+    const long long grid = (X.chunks + X.per - 1) / X.per;
+    if (grid > (1LL << 30) || X.chunks == 0) return false;
+    X.grid = (int)grid;
+    return true;
+}
+
+int launch_msd_fixed(const MsdLaunch &M, const MsdFixed &X, double *out_device, cudaStream_t s)
+{
+    using namespace msd;
+    const size_t smem = (size_t)3 * PLANE * 8;
+    if (cudaFuncSetAttribute(k_msd_fixed, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
+        cudaSuccess)
+        return -1;
+    k_msd_fixed<<<dim3((unsigned)X.grid, (unsigned)X.passes), FT, smem, s>>>(M, X);
+    const long long warps = (long long)M.leff * (M.cm_msd ? 2 : 1) * M.ntypes;
+    k_msd_fixed_final<<<(unsigned)((warps + 7) / 8), 256, 0, s>>>(M, X, out_device);
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
