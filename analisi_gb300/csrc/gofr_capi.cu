@@ -554,6 +554,8 @@ struct CellwGeom {
     int nx_lo[15] = {}, nx_hi[15] = {};
     int nz_span = 0, ny_span = 0, nx_span = 0;  // widest layer range, row range, cell range
     float4 shift[CELLW_NSHIFT] = {};
+    double rm = 0.0;           // reach of a first atom: rmax and the FP64 slop (the largest axis)
+    double oy[3] = {}, ox[15] = {};  // image offsets in cells
     double S[3] = {0, 0, 0};   // max |FP32 image vector| per axis over the images reached
     double eT[3] = {0, 0, 0};  // max |FP32 image vector - lattice vector| per axis
 };
@@ -585,6 +587,7 @@ bool cellw_geometry(const TrajDev &t, const gofr_params &p, const int nc[3], Cel
                            8.0 * v * (std::fabs(t.h_box[k]) + 2.0 * L[k])) *
                           (1.0 + std::ldexp(1.0, -40));
         rho[k] = rm / h[k];
+        g.rm = std::max(g.rm, rm);
     }
     const double xy = t.tric ? t.h_box[6] : 0.0, xz = t.tric ? t.h_box[7] : 0.0,
                  yz = t.tric ? t.h_box[8] : 0.0;
@@ -598,6 +601,7 @@ bool cellw_geometry(const TrajDev &t, const gofr_params &p, const int nc[3], Cel
     int sx_lo = 0, sx_hi = 0, sy_lo = 0, sy_hi = 0;
     for (int sz = sz_lo; sz <= sz_hi; ++sz) {
         const double oy = sz * yz / h[1];
+        g.oy[sz + 1] = oy;
         const int a = (int)std::floor(-rho[1] - oy - tiny), b = (int)std::floor(rho[1] - oy + tiny);
         g.ny_lo[sz + 1] = a;
         g.ny_hi[sz + 1] = b;
@@ -611,6 +615,7 @@ bool cellw_geometry(const TrajDev &t, const gofr_params &p, const int nc[3], Cel
             const int c0 = (int)std::floor(-rho[0] - ox - tiny),
                       c1 = (int)std::floor(rho[0] - ox + tiny);
             const int k = (sz + 1) * 5 + sy + 2;
+            g.ox[k] = ox;
             g.nx_lo[k] = c0;
             g.nx_hi[k] = c1;
             g.nx_span = std::max(g.nx_span, c1 - c0 + 1);
@@ -993,6 +998,8 @@ struct Plan {
     int kind = 1;              // 0 = FP32+recheck, 1 = FP64
     bool cells = false;        // FP32 kernel in its cell-list form
     int nc[3] = {0, 0, 0}, blk[3] = {1, 1, 1}, nb[3] = {1, 1, 1};
+    int grid[3] = {0, 0, 0};     // the cell grid of the sorted frames (nc; in x fx times nc)
+    int fx = 1;
     int reach = 1, cell_r = 4;   // neighbour reach in cells, first atoms per thread
     double cell_fraction = 1.0;  // neighbourhood cells / all cells
     double cell_time = 1e300;    // modelled time / the all-pairs kernel's
@@ -1120,7 +1127,7 @@ void apply_cell(Plan &pl, const CellCand &c)
     pl.reach = c.reach;
     pl.cell_r = c.r;
     for (int k = 0; k < 3; ++k) {
-        pl.nc[k] = c.nc[k];
+        pl.nc[k] = pl.grid[k] = c.nc[k];
         pl.blk[k] = c.blk[k];
         pl.nb[k] = (c.nc[k] + c.blk[k] - 1) / c.blk[k];
     }
@@ -1284,6 +1291,18 @@ bool cellw_choice(const TrajDev &t, const gofr_params &p, CellwCand &out)
     return true;
 }
 
+// Cells per planner's cell in x: an eighth of the reach where the sorted frames
+// keep at most two cells per atom (a row's ends then follow the sphere to an
+// eighth of rmax: 8 % fewer pairs than whole cells at reach 2).
+int cellw_refine(const TrajDev &t, const CellwCand &c)
+{
+    int fx = 1;
+    while (c.reach * fx * 2 <= 8 && c.nc[0] * fx * 2 <= 1024 &&
+           (double)c.nc[0] * c.nc[1] * c.nc[2] * fx * 2 <= 2.0 * (double)t.N)
+        fx *= 2;
+    return fx;
+}
+
 // Turns an FP32 plan into the warp-streamed cell-list form (the block cell
 // kernel's certified bound and windows: the same wrapped coordinates and
 // image moves).
@@ -1295,8 +1314,12 @@ bool make_cellw_plan(const TrajDev &t, const gofr_params &p, Plan &pl, const Cel
     for (int k = 0; k < 3; ++k) cc.nc[k] = c.nc[k];
     cc.fraction = c.fraction;
     cc.time = c.cost;
+    // finer cells in x for the trimmed rows
     CellwGeom g;
-    if (!cellw_geometry(t, p, c.nc, g)) return false;
+    int grid[3] = {c.nc[0], c.nc[1], c.nc[2]};
+    const int fx = cellw_refine(t, c);
+    grid[0] *= fx;
+    if (!cellw_geometry(t, p, grid, g)) return false;
     Plan q = pl;
     if (t.tric) {
         const Bound b = error_bound_cells_tric(t, g);
@@ -1306,6 +1329,8 @@ bool make_cellw_plan(const TrajDev &t, const gofr_params &p, Plan &pl, const Cel
     }
     q.cellw = true;
     q.geom = g;
+    q.fx = fx;
+    q.grid[0] = grid[0];
     for (int k = 0; k < 3; ++k) {
         q.wblk[k] = c.w[k];
         q.nw[k] = (c.nc[k] + c.w[k] - 1) / c.w[k];
@@ -1458,13 +1483,30 @@ int check_device_error(gofr_ctx *ctx)
     return GOFR_OK;
 }
 
-void set_cellw_geometry(CellwLaunch &C, const CellwGeom &g)
+// The plan's grid and neighbourhood.
+void set_cellw_grid(CellwLaunch &C, const TrajDev &t, const Plan &pl)
 {
+    const CellwGeom &g = pl.geom;
+    for (int k = 0; k < 3; ++k) {
+        C.nc[k] = pl.grid[k];
+        C.w[k] = pl.wblk[k] * (k == 0 ? pl.fx : 1);
+        C.nw[k] = pl.nw[k];
+        C.ny_lo[k] = g.ny_lo[k];
+        C.ny_hi[k] = g.ny_hi[k];
+        C.oy[k] = (float)g.oy[k];
+    }
     C.nz_lo = g.nz_lo;
     C.nz_hi = g.nz_hi;
-    for (int k = 0; k < 3; ++k) { C.ny_lo[k] = g.ny_lo[k]; C.ny_hi[k] = g.ny_hi[k]; }
-    for (int k = 0; k < 15; ++k) { C.nx_lo[k] = g.nx_lo[k]; C.nx_hi[k] = g.nx_hi[k]; }
+    for (int k = 0; k < 15; ++k) {
+        C.nx_lo[k] = g.nx_lo[k];
+        C.nx_hi[k] = g.nx_hi[k];
+        C.ox[k] = (float)g.ox[k];
+    }
     C.ny_span = g.ny_span;
+    C.hy = (float)(2.0 * t.h_box[4] / pl.grid[1]);
+    C.hz = (float)(2.0 * t.h_box[5] / pl.grid[2]);
+    C.inv_hx = (float)(pl.grid[0] / (2.0 * t.h_box[3]));
+    C.rm2 = (float)(g.rm * g.rm * (1.0 + 2e-5));
     for (int k = 0; k < CELLW_NSHIFT; ++k) C.shift[k] = g.shift[k];
 }
 
@@ -1560,7 +1602,7 @@ int ensure_cells(gofr_ctx *ctx, const TrajDev &t, const Plan &pl)
     const bool aos = pl.cellw;  // the warp-streamed kernel's records, else the SoA frames
     if (t.tric && !aos)
         return fail(ctx, GOFR_ERR_UNSUPPORTED, "the block cell-list kernel is orthorhombic");
-    if (tm.cell_nc[0] == pl.nc[0] && tm.cell_nc[1] == pl.nc[1] && tm.cell_nc[2] == pl.nc[2] &&
+    if (tm.cell_nc[0] == pl.grid[0] && tm.cell_nc[1] == pl.grid[1] && tm.cell_nc[2] == pl.grid[2] &&
         (aos ? tm.d_wpos != nullptr : tm.d_spos != nullptr))
         return GOFR_OK;
     auto drop_kept = [&tm]() {
@@ -1569,7 +1611,7 @@ int ensure_cells(gofr_ctx *ctx, const TrajDev &t, const Plan &pl)
         tm.cell_nc[0] = tm.cell_nc[1] = tm.cell_nc[2] = 0;
     };
     drop_kept();
-    const size_t ncell = (size_t)pl.nc[0] * pl.nc[1] * pl.nc[2];
+    const size_t ncell = (size_t)pl.grid[0] * pl.grid[1] * pl.grid[2];
     const size_t NP = padded_natoms(t.N);
     int *cell_of = nullptr, *rank_of = nullptr, *count = nullptr;
     auto drop_temp = [&]() {
@@ -1596,11 +1638,11 @@ int ensure_cells(gofr_ctx *ctx, const TrajDev &t, const Plan &pl)
     ctx->launches += 3;
     double centre[3];
     for (int k = 0; k < 3; ++k) centre[k] = t.h_box[k] + t.h_box[3 + k];  // xlo + L/2
-    int brc = launch_cell_build(t.pos64, t.types8, t.T, t.N, &t.h_box[0], centre, pl.nc,
+    int brc = launch_cell_build(t.pos64, t.types8, t.T, t.N, &t.h_box[0], centre, pl.grid,
                                 t.tric != 0, cell_of, rank_of, count, tm.d_cstart, tm.d_spos,
                                 tm.d_sidt, ctx->stream);
     if (!brc && aos)
-        brc = launch_cell_scatter_w(t.pos64, t.types8, t.T, t.N, &t.h_box[0], centre, pl.nc,
+        brc = launch_cell_scatter_w(t.pos64, t.types8, t.T, t.N, &t.h_box[0], centre, pl.grid,
                                     t.tric != 0, cell_of, rank_of, tm.d_cstart, tm.d_wpos,
                                     ctx->stream);
     const cudaError_t se = cudaStreamSynchronize(ctx->stream);
@@ -1610,7 +1652,7 @@ int ensure_cells(gofr_ctx *ctx, const TrajDev &t, const Plan &pl)
         return fail(ctx, GOFR_ERR_CUDA, "cell-list build failed: %s",
                     cudaGetErrorString(se != cudaSuccess ? se : cudaGetLastError()));
     }
-    for (int k = 0; k < 3; ++k) tm.cell_nc[k] = pl.nc[k];
+    for (int k = 0; k < 3; ++k) tm.cell_nc[k] = pl.grid[k];
     return GOFR_OK;
 }
 
@@ -1706,12 +1748,11 @@ int enqueue_run(gofr_ctx *ctx, const TrajDev &t, const gofr_params &p, const Run
         C.queue = reinterpret_cast<unsigned *>(ctx->d_stats + ST_QUEUE);
         C.start = t.d_cstart;
         C.wpos = t.d_wpos;
-        for (int k = 0; k < 3; ++k) { C.nc[k] = pl.nc[k]; C.w[k] = pl.wblk[k]; C.nw[k] = pl.nw[k]; }
+        set_cellw_grid(C, t, pl);
         C.reach = pl.reach;
         C.r = pl.cell_r;
         C.cta_warps = pl.cta_warps;
         C.hcopy = pl.hcopy;
-        set_cellw_geometry(C, pl.geom);
         C.pg = pl.pg;
         C.npg = pl.npg;
         C.pair.nparts = (int)std::max(1u, p.nparts);
@@ -2340,12 +2381,11 @@ int build_batch(gofr_ctx *ctx)
         C.queue = reinterpret_cast<unsigned *>(ctx->d_stats + ST_QUEUE);
         C.start = t.d_cstart;
         C.wpos = t.d_wpos;
-        for (int a = 0; a < 3; ++a) { C.nc[a] = q.nc[a]; C.w[a] = q.wblk[a]; C.nw[a] = q.nw[a]; }
+        set_cellw_grid(C, t, q);
         C.reach = q.reach;
         C.r = q.cell_r;
         C.cta_warps = q.cta_warps;  // as a single run of the member
         C.hcopy = 1;
-        set_cellw_geometry(C, q.geom);
         C.pg = C.npg = 1;
         C.pair.nparts = 1;
         wl.push_back({(unsigned long long)work[k], C});
@@ -2991,14 +3031,14 @@ int gofr_radial_query(const double *box, int box_kind, const double *coord_min,
     return GOFR_OK;
 }
 
-int gofr_cellw_tables(const double *box, int box_kind, const double *coord_min,
-                      const double *coord_max, double rmax, const int *nc, int *tables,
-                      float *shifts, double *bound)
+// The neighbourhood of a grid from host arguments.
+static int host_geometry(const double *box, int box_kind, const double *coord_min,
+                         const double *coord_max, double rmax, const int *nc, TrajDev &t,
+                         CellwGeom &g)
 {
-    if (!box || !coord_min || !coord_max || !nc || !tables) return GOFR_ERR_ARG;
+    if (!box || !coord_min || !coord_max || !nc) return GOFR_ERR_ARG;
     if (box_kind != GOFR_BOX_ORTHO && box_kind != GOFR_BOX_TRICLINIC) return GOFR_ERR_ARG;
     if (!(rmax > 0.0) || !std::isfinite(rmax)) return GOFR_ERR_ARG;
-    TrajDev t;
     t.T = 1;
     t.N = 1;
     t.tric = box_kind == GOFR_BOX_TRICLINIC;
@@ -3012,8 +3052,18 @@ int gofr_cellw_tables(const double *box, int box_kind, const double *coord_min,
     }
     gofr_params p{};
     p.rmax = rmax;
+    return cellw_geometry(t, p, nc, g) ? GOFR_OK : GOFR_ERR_UNSUPPORTED;
+}
+
+int gofr_cellw_tables(const double *box, int box_kind, const double *coord_min,
+                      const double *coord_max, double rmax, const int *nc, int *tables,
+                      float *shifts, double *bound)
+{
+    if (!tables) return GOFR_ERR_ARG;
+    TrajDev t;
     CellwGeom g;
-    if (!cellw_geometry(t, p, nc, g)) return GOFR_ERR_UNSUPPORTED;
+    const int rc = host_geometry(box, box_kind, coord_min, coord_max, rmax, nc, t, g);
+    if (rc) return rc;
     tables[0] = g.nz_lo;
     tables[1] = g.nz_hi;
     for (int k = 0; k < 3; ++k) { tables[2 + k] = g.ny_lo[k]; tables[5 + k] = g.ny_hi[k]; }
@@ -3028,6 +3078,31 @@ int gofr_cellw_tables(const double *box, int box_kind, const double *coord_min,
         const Bound b = t.tric ? error_bound_cells_tric(t, g) : error_bound_cells(t);
         for (int k = 0; k < 3; ++k) bound[k] = b.e[k];
     }
+    return GOFR_OK;
+}
+
+int gofr_cellw_row(const double *box, int box_kind, const double *coord_min,
+                   const double *coord_max, double rmax, const int *nc, const int *cn,
+                   const int *row, int *range)
+{
+    if (!cn || !row || !range) return GOFR_ERR_ARG;
+    TrajDev t;
+    Plan pl;
+    const int rc = host_geometry(box, box_kind, coord_min, coord_max, rmax, nc, t, pl.geom);
+    if (rc) return rc;
+    const int lz = row[0], ry = row[1], sz = row[2], sy = row[3];
+    if (sz < -1 || sz > 1 || sy < -2 || sy > 2 || cn[0] < 1 || cn[1] < 1 || cn[2] < 1)
+        return GOFR_ERR_ARG;
+    for (int k = 0; k < 3; ++k) pl.grid[k] = nc[k];
+    CellwLaunch C{};
+    set_cellw_grid(C, t, pl);
+    const int im = (sz + 1) * 5 + sy + 2;
+    range[0] = C.nx_lo[im];
+    range[1] = C.nx_hi[im];
+    if (!cellw_row(C.rm2, C.hy, C.hz, C.inv_hx, ry, C.oy[sz + 1], cn[1], lz, cn[2], C.ox[im],
+                   range[0], range[1]) ||
+        cn[0] + range[1] < range[0])
+        range[1] = range[0] - 1 - cn[0];
     return GOFR_OK;
 }
 
@@ -3426,7 +3501,7 @@ int gofr_neigh_run(gofr_ctx *ctx, const gofr_neigh_spec *spec, unsigned nspec, s
         if (!allpairs && L.prefilter && !t.tric && t.box_constant && t.N < (1u << 24) &&
             q.rmax > 0.0 && cell_grid(t, q, 1, nc)) {
             Plan pl;
-            for (int k = 0; k < 3; ++k) pl.nc[k] = nc[k];
+            for (int k = 0; k < 3; ++k) pl.nc[k] = pl.grid[k] = nc[k];
             const int crc = ensure_cells(ctx, t, pl);
             if (crc == GOFR_OK) {
                 const size_t ncell = (size_t)nc[0] * nc[1] * nc[2];

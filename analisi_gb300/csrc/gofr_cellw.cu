@@ -45,6 +45,15 @@
 // more cell where the shift is not whole), together with the FP32 lattice
 // vector of each image.
 //
+// A row keeps only the cells within reach of the block at the row's distance
+// in y and z (cellw_row), and cells are up to eight to the reach in x, so the
+// rows' ends follow the sphere around the block: at reach 2, 3.43 times the
+// sphere's volume instead of 3.73 for whole cells (66.3 to 60.9 ms at 16k
+// atoms, 20.3 to 17.8 at 32k triclinic, 8.4 to 7.8 at 131k).  Finer rows in y
+// and z would leave 3.13 but are four times as many to list; leaving out
+// (first atom, chunk) pairs by the chunk's bounding box would save another 4 %
+// of the pairs, less than the boxes cost.
+//
 // Every evaluated pair goes straight into the CTA's shared histogram
 // (bin_pair2, gofr_device.cuh), and the pairs near a bin edge (the radial
 // margin of gofr_capi.cu; 0.13 % of them at 16k atoms) are noted in a bit per
@@ -66,10 +75,10 @@
 // Bound by instruction issue: 73 instructions per 128 pairs (46 of them the
 // pairs' own), 77 % of the issue slots used, the shared-memory pipe 57 %
 // busy, the FP32 pipe 59 %, no DRAM traffic to speak of.  16384 atoms, 25
-// origins x 100 lags (17 % of N^2 evaluated, 26 % of those within rmax): 66.0
+// origins x 100 lags (16 % of N^2 evaluated, 28 % of those within rmax): 60.9
 // ms, where the form that queued its candidates and binned the queue took
-// 178.9; 131072 atoms, 5 x 10: 8.6 ms against 21.7; 32768 atoms, triclinic,
-// 10 x 20: 20.8 ms against 59.8.  64 registers, 32 warps per SM: with 128
+// 178.9; 131072 atoms, 5 x 10: 7.8 ms against 21.7; 32768 atoms, triclinic,
+// 10 x 20: 17.8 ms against 59.8.  64 registers, 32 warps per SM: with 128
 // registers and 16 warps 74.9 ms.
 #include <cstdint>
 #include <cuda_runtime.h>
@@ -127,6 +136,7 @@ __global__ void __launch_bounds__(NWARP * 32, 32 / NWARP) k_pairs_cellw(const Ce
     __shared__ unsigned long long s_pairs;  // pairs evaluated since the last flush
     __shared__ float4 s_shift[CELLW_NSHIFT];
     __shared__ int2 s_ny[3], s_nx[15];
+    __shared__ float s_oy[3], s_ox[15];
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const unsigned lt = (1u << lane) - 1u;  // the lanes below this one
@@ -146,8 +156,14 @@ __global__ void __launch_bounds__(NWARP * 32, 32 / NWARP) k_pairs_cellw(const Ce
     for (int i = tid; i < HCOPY * hist_cap; i += NT) hist[i] = 0u;
     for (int i = tid; i < P.ntypes * P.ntypes; i += NT) chtab[i] = P.chtab[i];
     for (int i = tid; i < CELLW_NSHIFT; i += NT) s_shift[i] = C.shift[i];
-    if (tid < 3) s_ny[tid] = make_int2(C.ny_lo[tid], C.ny_hi[tid]);
-    if (tid < 15) s_nx[tid] = make_int2(C.nx_lo[tid], C.nx_hi[tid]);
+    if (tid < 3) {
+        s_ny[tid] = make_int2(C.ny_lo[tid], C.ny_hi[tid]);
+        s_oy[tid] = C.oy[tid];
+    }
+    if (tid < 15) {
+        s_nx[tid] = make_int2(C.nx_lo[tid], C.nx_hi[tid]);
+        s_ox[tid] = C.ox[tid];
+    }
     if (tid == 0) s_pairs = 0ull;
 
     int nn = 0, qn = 0;  // entries of the warp's two queues (the same in every lane)
@@ -351,7 +367,15 @@ __global__ void __launch_bounds__(NWARP * 32, 32 / NWARP) k_pairs_cellw(const Ce
                         const int uy = cy0 + yr.x + ky;
                         const int sy = floordiv(uy, ncy), cy = uy - sy * ncy;
                         ok = sy >= -2 && sy <= 2;
-                        const int2 xr = ok ? s_nx[(sz + 1) * 5 + sy + 2] : make_int2(0, 0);
+                        int2 xr = make_int2(0, -1 - cnx);
+                        if (ok) {
+                            const int im = (sz + 1) * 5 + sy + 2;
+                            xr = s_nx[im];
+                            if (!cellw_row(C.rm2, C.hy, C.hz, C.inv_hx, yr.x + ky, s_oy[sz + 1],
+                                           cny, C.nz_lo + lz, cnz, s_ox[im], xr.x, xr.y) ||
+                                cnx + xr.y < xr.x)
+                                xr.y = xr.x - 1 - cnx;  // no cell
+                        }
                         const int ux = cx0 + xr.x, len = cnx + xr.y - xr.x + 1;
                         const int sx = floordiv(ux, ncx), a = ux - sx * ncx, b = a + len;
                         ok = ok && sx >= -2 && len >= 0 && len <= ncx &&

@@ -1,6 +1,7 @@
 // Internal declarations shared by the host side (gofr_capi.cu) and the
 // kernels (gofr_kernels.cu).  Not part of the C ABI.
 #pragma once
+#include <cmath>
 #include <cstddef>
 #include <cstdint>
 #include <cuda_runtime.h>
@@ -146,12 +147,40 @@ struct CellLaunch {
 constexpr int CELLW_MAX_ROWS = 64;  // neighbourhood rows of a warp block (all its layers)
 constexpr int CELLW_NSHIFT = 75;    // images sx, sy in -2..2, sz in -1..1
 constexpr int CELLW_SHIFT0 = 37;    // index of the image (0, 0, 0)
+// A row of a neighbourhood holds the cells that come within the reach of the
+// warp block at the row's distance in y and z, so that the rows' ends follow
+// the sphere around the block; cells are finer in x (Plan::fx) for it.
+//
+// Gap along an axis between the cell [r + o, r + o + 1) and the block [0, c),
+// in cells, less a thousandth of a cell for the FP32 rounding and the cells'.
+__host__ __device__ inline float cellw_gap(int r, float o, int c)
+{
+    const float below = -(float)(r + 1) - o, above = (float)r + o - (float)c;
+    return fmaxf(fmaxf(below, above) - 1e-3f, 0.0f);
+}
+// Trims the cells [lo, hi] (from the block's first and last cell) of row ry,
+// layer lz (from the block's first; images oy, ox cells off; the block is
+// cny, cnz cells) to those within the radius; false when the row has none.
+__host__ __device__ inline bool cellw_row(float rm2, float hy, float hz, float inv_hx, int ry,
+                                          float oy, int cny, int lz, int cnz, float ox, int &lo,
+                                          int &hi)
+{
+    const float gy = hy * cellw_gap(ry, oy, cny), gz = hz * cellw_gap(lz, 0.0f, cnz);
+    const float e2 = rm2 - gy * gy - gz * gz;
+    if (!(e2 > 0.0f)) return false;
+    const float rho = sqrtf(e2) * inv_hx * 1.00001f + 1e-3f;
+    const int a = (int)floorf(-rho - ox), b = (int)floorf(rho - ox);
+    if (a > lo) lo = a;
+    if (b < hi) hi = b;
+    return true;
+}
+
 struct CellwLaunch {
     PairLaunch pair;
     const int *start;              // [T][ncell+1] sorted-record offset of each cell
     const float4 *wpos;            // [T][NP] {x, y, z, type << 24 | atom id} sorted by cell
-    int nc[3];                     // cells per axis
-    int w[3];                      // cells per warp block per axis
+    int nc[3];                     // cells per axis (fx times the planner's in x)
+    int w[3];                      // cells per warp block per axis (the same)
     int nw[3];                     // warp blocks per axis
     int reach;                     // neighbour cells per side
     int r;                         // records per lane (4; kept in plans and tuner keys)
@@ -164,6 +193,8 @@ struct CellwLaunch {
     int ny_lo[3], ny_hi[3];        // rows, per layer image sz + 1
     int nx_lo[15], nx_hi[15];      // cells, per row images (sz + 1) 5 + sy + 2
     int ny_span;                   // max over sz of ny_hi - ny_lo + 1
+    float oy[3], ox[15];           // image offsets in cells: rows of layer image sz + 1, cells
+    float hy, hz, inv_hx, rm2;     // cell edges, 1 / edge, radius^2 (with room for rounding)
     float4 shift[CELLW_NSHIFT];    // FP32 lattice vector {x, y, z, 0} of each image
 };
 int cellw_smem_bytes(int nch, int nbin, int ntypes, int cta_warps = 8, int hcopy = 1);

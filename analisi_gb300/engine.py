@@ -29,7 +29,8 @@ EXPORTED = [
     "gofr_batch_output_layout", "gofr_batch_run", "gofr_measure_peaks",
     "gofr_run_f64_noalloc", "gofr_run_windows", "gofr_set_centres", "gofr_msd_output_size",
     "gofr_msd_run", "gofr_neigh_layout", "gofr_neigh_run", "gofr_run_normalized",
-    "gofr_run_streamed", "gofr_cellw_tables", "gofr_plan_query", "gofr_radial_query",
+    "gofr_run_streamed", "gofr_cellw_tables", "gofr_cellw_row",
+    "gofr_plan_query", "gofr_radial_query",
 ]
 
 
@@ -154,6 +155,7 @@ def load_library(path=None):
     L.gofr_bin_thresholds.argtypes = [ctypes.c_double, ctypes.c_double, ctypes.c_uint, dp]
     L.gofr_cellw_tables.argtypes = [dp, ctypes.c_int, dp, dp, ctypes.c_double, ip, ip,
                                     ctypes.POINTER(ctypes.c_float), dp]
+    L.gofr_cellw_row.argtypes = [dp, ctypes.c_int, dp, dp, ctypes.c_double, ip, ip, ip, ip]
     L.gofr_plan_query.argtypes = [dp, ctypes.c_int, dp, dp, ctypes.c_size_t, ctypes.c_uint,
                                   ctypes.POINTER(Params), ip]
     L.gofr_radial_query.argtypes = [dp, ctypes.c_int, dp, dp, ctypes.c_size_t, ctypes.c_uint,
@@ -184,7 +186,7 @@ def load_library(path=None):
                  "gofr_bin_thresholds", "gofr_batch_set", "gofr_batch_output_layout",
                  "gofr_batch_run", "gofr_measure_peaks", "gofr_run_f64_noalloc",
                  "gofr_run_windows", "gofr_run_normalized", "gofr_run_streamed",
-                 "gofr_cellw_tables", "gofr_plan_query", "gofr_radial_query"):
+                 "gofr_cellw_tables", "gofr_cellw_row", "gofr_plan_query", "gofr_radial_query"):
         getattr(L, name).restype = ctypes.c_int
     if path is None:
         _lib = L
@@ -284,6 +286,26 @@ def cellw_tables(box, triclinic, coord_min, coord_max, rmax, nc):
             "nx": {(sz, sy): (int(t[8 + (sz + 1) * 5 + sy + 2]), int(t[23 + (sz + 1) * 5 + sy + 2]))
                    for sz in (-1, 0, 1) for sy in range(-2, 3)},
             "shift": sh, "bound": e}
+
+
+def cellw_row(box, triclinic, coord_min, coord_max, rmax, nc, cn, row):
+    """Cells (lo, hi) that the warp-streamed cell-list kernel keeps of one row
+    of a warp block's neighbourhood (host code): cn the block's cells, row =
+    (layer, row) from the block's first and their images (sz, sy); the cells
+    are [cx0 + lo, cx0 + cn[0] + hi]."""
+    L = load_library()
+    b = np.ascontiguousarray(box, dtype=np.float64)
+    lo = np.ascontiguousarray(coord_min, dtype=np.float64)
+    hi = np.ascontiguousarray(coord_max, dtype=np.float64)
+    ip = ctypes.POINTER(ctypes.c_int)
+    a = [np.ascontiguousarray(v, dtype=np.int32) for v in (nc, cn, row)]
+    out = np.zeros(2, dtype=np.int32)
+    rc = L.gofr_cellw_row(_dp(b), BOX_TRICLINIC if triclinic else BOX_ORTHO, _dp(lo), _dp(hi),
+                          float(rmax), *[v.ctypes.data_as(ip) for v in a],
+                          out.ctypes.data_as(ip))
+    if rc != GOFR_OK:
+        raise GofrError(rc, "invalid box, extent, rmax, grid or row")
+    return int(out[0]), int(out[1])
 
 
 def counts_to_buffer(counts, ntimesteps, skip, nparts=0):

@@ -293,6 +293,17 @@ int gofr_cellw_tables(const double *box, int box_kind, const double *coord_min,
                       const double *coord_max, double rmax, const int *nc, int *tables,
                       float *shifts, double *bound);
 
+/* Host-only (no context, no GPU): the cells that a row of that neighbourhood
+ * keeps within the radius.  cn[3]: the warp block's cells; row[4]: the
+ * layer and the row relative to the block's first (uz - cz0, uy - cy0), and
+ * their images sz, sy.  range[2]: cells [cx0 + range[0], cx0 + cn[0] +
+ * range[1]] (none when that is empty).  Every pair the reference counts is
+ * inside them (lib/src/gofrt.cpp:101-117 evaluates all); this lets that be
+ * checked without a GPU. */
+int gofr_cellw_row(const double *box, int box_kind, const double *coord_min,
+                   const double *coord_max, double rmax, const int *nc, const int *cn,
+                   const int *row, int *range);
+
 /* Measures, on `device`, the two peaks that bound the FP32 pair kernel: the
  * FP32 lane-operation rate (one FFMA = one operation, the unit of the kernel's
  * 16/19 operations per pair) and the shared-memory u32 atomic rate.  No
