@@ -391,7 +391,7 @@ __global__ void __launch_bounds__(NT, 4) k_allpairs(const PairLaunch P)
     const int tid = threadIdx.x, lane = tid & 31;
     WarpArea &A = areas[tid >> 5];
     for (int i = tid; i < hcells; i += NT) hist[i] = 0u;
-    for (int i = tid; i < P.ntypes * P.ntypes; i += NT) chtab[i] = P.chtab[i];
+    for (int i = tid; i < P.ntypes * P.ntypes; i += NT) chtab[i] = type_channel(i, P.ntypes);
     if (tid == 0) s_pairs = 0ull;
 
     const int per = P.N / P.nparts;
@@ -519,7 +519,7 @@ __global__ void __launch_bounds__(NT, 4) k_allpairs_batch(const PairLaunch *__re
             const unsigned *src = reinterpret_cast<const unsigned *>(trajs + w.traj);
             for (int i = tid; i < words; i += NT) reinterpret_cast<unsigned *>(&sP)[i] = src[i];
             __syncthreads();
-            for (int i = tid; i < P.ntypes * P.ntypes; i += NT) chtab[i] = P.chtab[i];
+            for (int i = tid; i < P.ntypes * P.ntypes; i += NT) chtab[i] = type_channel(i, P.ntypes);
             cur = w.traj;
             __syncthreads();
         }

