@@ -2849,7 +2849,7 @@ int gofr_run_normalized(gofr_ctx *ctx, const gofr_params *p, unsigned nwin,
     L.nbin = (int)p->nbin;
     L.nch = (int)rs.nch;
     L.mode = norm;
-    L.incr = (rs.ntimesteps / rs.skip > 0) ? 1.0 / (int)(rs.ntimesteps / rs.skip) : 1.0;
+    L.fold = fold_table((rs.ntimesteps / rs.skip > 0) ? 1.0 / (int)(rs.ntimesteps / rs.skip) : 1.0);
     L.r0 = p->rmin;
     L.dr = (p->rmax - p->rmin) / p->nbin;
     L.c43pi = 4.0 * 3.141592653589793 / 3.0;  // numpy: 4 * np.pi / 3
@@ -3139,36 +3139,6 @@ int gofr_cellw_row(const double *box, int box_kind, const double *coord_min,
     return GOFR_OK;
 }
 
-// incr added k times in sequence (lib/src/gofrt.cpp:118), in O(number of
-// binades): within one binade of the running sum the rounded step is the
-// same for every addition until the sum reaches the binade's upper end, so
-// those additions are taken in one exact multiplication.  Exact ties (the
-// step is half an ulp) are taken one at a time; they end in a fixed point.
-static double repeated_sum(unsigned long long k, double incr)
-{
-    double s = 0.0;
-    while (k > 0) {
-        double n1 = s + incr;
-        if (n1 == s) return s;  // the sum no longer moves
-        if (s == 0.0 || !std::isfinite(n1)) { s = n1; --k; continue; }
-        int e;
-        std::frexp(s, &e);                     // s in [2^(e-1), 2^e)
-        double top = std::ldexp(1.0, e);       // upper end of the binade
-        double u = std::ldexp(1.0, e - 53);    // ulp in the binade
-        double r = incr / u;                   // exact (power-of-two scaling)
-        double fr = r - std::floor(r);
-        if (fr == 0.5 || !(top - s > incr)) { s = n1; --k; continue; }
-        double delta = n1 - s;                 // exact: same binade, Sterbenz
-        // additions from s + j*delta stay exact steps while s + j*delta + incr <= top
-        double jm = std::floor((top - s - incr) / delta) - 2.0;
-        if (jm < 1.0) { s = n1; --k; continue; }
-        unsigned long long j = jm >= (double)k ? k : (unsigned long long)jm;
-        s = s + (double)j * delta;
-        k -= j;
-    }
-    return s;
-}
-
 int gofr_counts_to_buffer(const unsigned long long *counts, size_t n, unsigned nparts,
                           unsigned ntimesteps, unsigned skip, double *out)
 {
@@ -3179,9 +3149,10 @@ int gofr_counts_to_buffer(const unsigned long long *counts, size_t n, unsigned n
         for (size_t i = 0; i < n; ++i) out[i] = (double)counts[i] * incr;
         return GOFR_OK;
     }
+    const FoldTable fold = fold_table(incr);
     for (size_t i = 0; i < n; ++i) {
-        double acc = repeated_sum(counts[i], incr);
-        for (unsigned q = 1; q < nparts; ++q) acc += repeated_sum(counts[(size_t)q * n + i], incr);
+        double acc = fold_sum(fold, counts[i]);
+        for (unsigned q = 1; q < nparts; ++q) acc += fold_sum(fold, counts[(size_t)q * n + i]);
         out[i] = acc;
     }
     return GOFR_OK;

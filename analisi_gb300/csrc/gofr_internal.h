@@ -217,6 +217,37 @@ int launch_cell_scatter_w(const double *pos64, const unsigned char *types8, size
 int launch_cellw_pairs(const CellwLaunch &C, int num_sms, cudaStream_t s);
 
 // FP64 normalisation of window counts on the device (gofr_norm.cu).
+// s(k), the FP64 sum of k additions of incr from 0 (lib/src/gofrt.cpp:118), as
+// the runs of equal steps it consists of: within one binade the rounded step
+// is the same for every addition (but for the first, where the step is half
+// an ulp off an odd sum), so s(k) = s0 + (k - k0) delta exactly from each run's
+// first addition k0 on.  At most a tie, a run and a step over the end per
+// binade, and the sum stands still 54 binades above incr.
+constexpr int FOLD_RUNS = 176;
+struct FoldTable {
+    unsigned long long k0[FOLD_RUNS];
+    double s0[FOLD_RUNS], delta[FOLD_RUNS];
+    unsigned char first[64];  // the run that holds 2^b
+    int n;
+};
+FoldTable fold_table(double incr);
+__host__ __device__ inline double fold_sum(const FoldTable &t, unsigned long long k)
+{
+    if (k == 0) return 0.0;
+#ifdef __CUDA_ARCH__
+    int i = t.first[63 - __clzll((long long)k)];
+#else
+    int i = t.first[63 - __builtin_clzll(k)];
+#endif
+    while (i + 1 < t.n && t.k0[i + 1] <= k) ++i;
+    const double j = (double)(k - t.k0[i]);
+#ifdef __CUDA_ARCH__
+    return __dadd_rn(t.s0[i], __dmul_rn(j, t.delta[i]));  // both exact
+#else
+    return t.s0[i] + j * t.delta[i];
+#endif
+}
+
 struct NormLaunch {
     const unsigned long long *counts;  // [nwin][nparts][n] exact counts
     double *out;                       // [nwin][n]
@@ -224,9 +255,9 @@ struct NormLaunch {
     size_t n;                          // leff * nch * nbin
     int nwin, nparts, nbin, nch;
     int mode;                          // 0 buffer, 1 / shell volume, 2 / shell volume / density
-    double incr;                       // 1 / int(ntimesteps / skip)
     double r0, dr;                     // bin b spans [b dr + r0, (b + 1) dr + r0)
     double c43pi;                      // fl(fl(4 pi) / 3)
+    FoldTable fold;                    // of 1 / int(ntimesteps / skip)
 };
 int launch_counts_to_gofr(const NormLaunch &L, int num_sms, cudaStream_t s);
 
