@@ -30,7 +30,7 @@
 // copies and per-thread candidate slots binned by the warp took 26.1; with the
 // rounded quotient of the triclinic form 8.2.  5488 atoms to 9 A in four
 // partitions, 20 x 40: 18.3 ms against 32.7; 1000 atoms to 3.5 A (1.7 %
-// counted), 18 x 20: 0.34 against 0.44; 300 atoms, 6 x 6: 27 us against 78.  64
+// counted), 18 x 20: 0.34 against 0.44; 300 atoms, 6 x 6: 23 us against 78.  64
 // registers (spilling 60 bytes outside the loops): with 80 and three CTAs per
 // SM within 2 %.
 #include <cstdint>
@@ -202,7 +202,14 @@ __device__ __forceinline__ void unit(const PairLaunch &P, WarpArea &A, unsigned 
             // the atom's pair with itself: from the channel of distinct atoms,
             // where the loop below counts it, to its own (in the unit that counts
             // it: a cell is never below zero when it is flushed)
-            const int b = ia / (P.jc * CH) == jp ? self_bin<TRI>(P, fo, fl, ia) : -1;
+            // At lag 0 the distance is exactly zero, which lies on a bin edge when
+            // rmin is 0: given here, and in `resolve`, since every atom took the
+            // FP64 arithmetic twice otherwise (68 us a call of 300 atoms against 63;
+            // the cell-list kernel loses 1 % to the test and has less of lag 0)
+            const int s0 = jp * P.jc * CH;
+            const int b = ia < s0 || ia >= s0 + P.jc * CH ? -1
+                          : fo == fl                      ? P.self0
+                                                          : self_bin<TRI>(P, fo, fl, ia);
             if (b >= 0) {
                 const int ch = chtab[(int)ti * P.ntypes + (int)ti];
                 atomicSub(whist + ch * nrow + b, 1u);
@@ -254,9 +261,13 @@ __device__ __forceinline__ void unit(const PairLaunch &P, WarpArea &A, unsigned 
             const float t = __fadd_rn(radial_q(d2, P.rm), RADIAL_MAGIC);
             const int b = (int)(__float_as_uint(t) - RADIAL_MAGIC_BITS);
             need = (t <= P.rm.t_hi && t >= P.rm.t_lo) || (WCHK && w0);
-            if (b >= 0 && b < nbin)
-                atomicSub(whist + chtab[(int)(u1.y >> 32 & 0xffu) * P.ntypes +
-                                        (int)P.types8[e.y]] * nrow + b, 1u);
+            unsigned *const row =
+                whist + chtab[(int)(u1.y >> 32 & 0xffu) * P.ntypes + (int)P.types8[e.y]] * nrow;
+            if (b >= 0 && b < nbin) atomicSub(row + b, 1u);
+            if (fo == fl && ia == e.y) {
+                need = false;
+                if (P.self0 >= 0) atomicAdd(row + P.self0, 1u);
+            }
         }
         const unsigned m = __ballot_sync(0xffffffffu, need);
         if (need) A.q[qn + __popc(m & lt)] = make_uint2(ia, e.y);

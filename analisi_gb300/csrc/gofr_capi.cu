@@ -1056,6 +1056,14 @@ RadialMap plan_radial_map(const TrajDev &t, const gofr_params &p, const Plan &pl
                                   : error_bound_boxed(t), b1, p, pl.th);
 }
 
+// The reference's bin of distance zero, -1 when it is not counted.
+int bin_of_zero(const Plan &pl)
+{
+    int b = -1;
+    for (size_t k = 0; !pl.empty && k + 1 < pl.th.size() && pl.th[k] <= 0.0; ++k) b = (int)k;
+    return b;
+}
+
 // One cell-list configuration: cells of edge >= rmax (1 + 1e-6) / reach, so
 // two atoms at minimum-image distance <= rmax are at most `reach` cells apart
 // on every axis (periodically); at least 2 reach + 1 cells per axis.  A CTA
@@ -1788,6 +1796,7 @@ int enqueue_run(gofr_ctx *ctx, const TrajDev &t, const gofr_params &p, const Run
         L.wlim = (float)(0.5 - pl.b.eta);
         L.wtol = wrap_tolerance(t);
         L.rm = plan_radial_map(t, p, pl);
+        L.self0 = bin_of_zero(pl);
     }
     if (pl.kind == 0 && (ghist || (pl.cells && !pl.cellw)))
         CK(cudaMemcpyAsync(ctx->d_win, pl.w.win.data(), pl.w.win.size() * sizeof(float2),
@@ -2395,6 +2404,7 @@ int build_batch(gofr_ctx *ctx)
         L.wlim = (float)(0.5 - pl.b.eta);
         L.wtol = wrap_tolerance(t);
         L.rm = plan_radial_map(t, t.params, pl);
+        L.self0 = bin_of_zero(pl);
         L.tric = t.tric;
         L.wchk = pl.wrapcheck ? 1 : 0;
     }

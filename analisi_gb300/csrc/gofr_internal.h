@@ -100,6 +100,7 @@ struct PairLaunch {
                               // global-memory histogram form)
     float wtol;               // orthorhombic: |component| > L / 2 - wtol flags a recheck
     double rmin, rmax, dr, rmin2, rmax2;  // reference binning constants
+    int self0;                   // the reference's bin of distance zero (-1: not counted)
     RadialMap rm;
     int tric;
     int wchk;                 // batched kernel: per-pair wrap-decision check on
