@@ -78,8 +78,8 @@
 // origins x 100 lags (16 % of N^2 evaluated, 28 % of those within rmax): 60.9
 // ms, where the form that queued its candidates and binned the queue took
 // 178.9; 131072 atoms, 5 x 10: 7.8 ms against 21.7; 32768 atoms, triclinic,
-// 10 x 20: 17.8 ms against 59.8.  64 registers, 32 warps per SM: with 128
-// registers and 16 warps 74.9 ms.
+// 10 x 20: 17.8 ms against 59.8.  64 registers, 32 warps per SM (two CTAs of
+// 16, one of 32 for a large histogram): with 128 registers and 16 warps 74.9 ms.
 #include <cstdint>
 #include <cuda_runtime.h>
 
@@ -699,9 +699,32 @@ static int launch_cellw_shape(const CellwLaunch &C, int num_sms, cudaStream_t s)
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
+// Whether one CTA of 32 warps takes the place of the CTAs of 16: where the
+// histogram lets only one of those on an SM, and 32 warps' areas fit beside it
+// (half the warps left the SM waiting on latencies: 5488 atoms, 4 partitions
+// of 14 KB, 5.55 to 4.67 ms; 16384 atoms, 4 types, 800 bins, 3.71 to 3.06).
+static bool cellw_wide(const CellwLaunch &C)
+{
+    if (C.cta_warps != 16 || C.hcopy != 1 || C.most < 32) return false;
+    int dev = 0, sm = 0, cta = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev) !=
+            cudaSuccess ||
+        cudaDeviceGetAttribute(&cta, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess)
+        return false;
+    auto bytes = [&C](int warps) {  // with the static shared memory
+        return cellw_smem_bytes(C.pair.nch * C.pg, C.pair.nbin, C.pair.ntypes, warps, 1) + 2048;
+    };
+    const int reserved = sm - cta;  // per CTA
+    return 2 * (bytes(16) + reserved) > sm && bytes(32) <= cta;
+}
+
 template <int MODE>
 static int launch_cellw_mode(const CellwLaunch &C, int num_sms, cudaStream_t s)
 {
+    if (cellw_wide(C))
+        return C.pair.nparts > 1 ? launch_cellw_shape<32, 1, MODE, true>(C, num_sms, s)
+                                 : launch_cellw_shape<32, 1, MODE, false>(C, num_sms, s);
     if (C.pair.nparts > 1) {
         return C.cta_warps == 16 ? launch_cellw_shape<16, 1, MODE, true>(C, num_sms, s)
                                  : launch_cellw_shape<8, 1, MODE, true>(C, num_sms, s);

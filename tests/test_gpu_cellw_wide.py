@@ -1,0 +1,33 @@
+"""Histograms that leave the warp-streamed cell-list kernel one CTA per SM: the
+CTA of 32 warps every kind of rmin, counts
+per partition, orthorhombic and triclinic.  Counts equal the oracle's."""
+import numpy as np
+import pytest
+
+from analisi_gb300 import engine, workloads
+
+pytestmark = pytest.mark.gpu
+
+# types, bins, rmin, triclinic, partitions
+CASES = [
+    (5, 500, 0.0, False, 1),    # 60 KB of cells: one CTA of 32 warps
+    (5, 500, 0.8, True, 1),
+    (5, 500, -0.6, False, 1),
+    (3, 301, 0.0, False, 5),    # five partitions of 14 KB in one histogram
+]
+
+
+@pytest.mark.parametrize("case", CASES, ids=lambda c: "-".join(str(x) for x in c))
+def test_large_histograms(gpu_engine, oracle_mod, case):
+    nt, nbin, rmin, tric, nparts = case
+    N, L, rmax = 2600, 30.0, 5.0
+    counts = [N // nt] * nt
+    counts[0] += N - sum(counts)
+    w = workloads.small_case(nt + nbin, N, 7, L, 0.2, counts, tric=tric, wrap_into_cell=tric)
+    gpu_engine.set_frames(w["positions"], w["boxes"], w["type_ids"], w["ntypes"], triclinic=tric)
+    args = (rmin, rmax, nbin, 2, 2, 1, 5, 1)
+    got = gpu_engine.run(*args, nparts=nparts)
+    assert gpu_engine.stats()["kernel_used"] == 5
+    want = oracle_mod.gofrt_counts(w["positions"], w["boxes"], w["type_ids"], nt, rmin, rmax, nbin,
+                                   2, nparts, 2, 1, 5, 1, tric=tric, per_thread=nparts > 1)
+    np.testing.assert_array_equal(got, want)
