@@ -1089,7 +1089,10 @@ bool cell_eligible(const TrajDev &t, const gofr_params &p, bool warp = false)
     if (p.nparts > 1 && !(warp && p.kernel == GOFR_KERNEL_AUTO && p.nparts <= t.N)) return false;
     if (!(p.rmax > 0.0)) return false;
     if (t.N >= (1u << 24)) return false;  // sorted slots pack type << 24 | atom id
-    // large histograms use the global-memory form of the all-pairs kernel
+    // AUTO takes any histogram that the warp-streamed kernel has room for (6 types,
+    // 600 bins, 32768 atoms: 152 ms all-pairs); the block kernel's, which needs more
+    // beside it, and a forced or tuned one keep to what that has room for
+    if (warp && p.kernel == GOFR_KERNEL_AUTO) return true;
     return cell_smem_bytes((int)(t.ntypes * (t.ntypes + 1)), (int)p.nbin, (int)t.ntypes) <=
            160 * 1024;
 }

@@ -1,5 +1,5 @@
 """Histograms that leave the warp-streamed cell-list kernel one CTA per SM: the
-CTA of 32 warps every kind of rmin, counts
+CTA of 32 warps (and, past its room, the CTA of 16), every kind of rmin, counts
 per partition, orthorhombic and triclinic.  Counts equal the oracle's."""
 import numpy as np
 import pytest
@@ -14,6 +14,9 @@ CASES = [
     (5, 500, 0.8, True, 1),
     (5, 500, -0.6, False, 1),
     (3, 301, 0.0, False, 5),    # five partitions of 14 KB in one histogram
+    (6, 600, 0.0, False, 1),    # 101 KB: one CTA of 16 warps
+    (6, 870, 0.0, False, 1),    # 146 KB: the last of them
+    (6, 960, 0.0, False, 1),    # 161 KB: no room for 16 warps, the all-pairs kernel
 ]
 
 
@@ -27,7 +30,15 @@ def test_large_histograms(gpu_engine, oracle_mod, case):
     gpu_engine.set_frames(w["positions"], w["boxes"], w["type_ids"], w["ntypes"], triclinic=tric)
     args = (rmin, rmax, nbin, 2, 2, 1, 5, 1)
     got = gpu_engine.run(*args, nparts=nparts)
-    assert gpu_engine.stats()["kernel_used"] == 5
+    assert gpu_engine.stats()["kernel_used"] == (1 if nbin == 960 else 5)
     want = oracle_mod.gofrt_counts(w["positions"], w["boxes"], w["type_ids"], nt, rmin, rmax, nbin,
                                    2, nparts, 2, 1, 5, 1, tric=tric, per_thread=nparts > 1)
     np.testing.assert_array_equal(got, want)
+
+
+def test_forced_kernel_keeps_its_limit(gpu_engine):
+    """kernel="cellw" refuses a histogram it refused before AUTO took it."""
+    w = workloads.small_case(3, 2600, 3, 30.0, 0.2, [434, 434, 433, 433, 433, 433])
+    gpu_engine.set_frames(w["positions"], w["boxes"], w["type_ids"], w["ntypes"])
+    with pytest.raises(engine.GofrError):
+        gpu_engine.run(0.0, 5.0, 600, 1, 1, 1, 2, 0, kernel="cellw")
