@@ -324,6 +324,11 @@ __device__ __forceinline__ void unit(const PairLaunch &P, WarpArea &A, unsigned 
                     bit <<= 1;
                 }
             }
+            if (P.rm.lim < 0.0f) {  // every pair is noted: not those without an atom
+#pragma unroll
+                for (int t = 0; t < 4; ++t)
+                    if (j0 + t >= P.N) mk[t] = 0u;
+            }
             while (__any_sync(0xffffffffu, (mk[0] | mk[1] | mk[2] | mk[3]) != 0u)) {
                 unsigned bits = 0u, j = 0u;
 #pragma unroll

@@ -826,7 +826,7 @@ RadialMap radial_map(const TrajDev &t, const Bound &b, const Bound &b1, const go
     m.lim_self = md1 < 0.25 ? f_down(0.5 - md1) : -1.0f;
     const double wide = md < 0.25 ? 0.0 : std::min(std::ceil(md), 1048576.0);
     const double magic = 12582912.0;
-    m.t_end = (float)(magic + p.nbin);
+    m.q_end = (float)p.nbin;
     m.t_hi = (float)(magic + p.nbin + wide);
     m.t_lo = (float)(magic + (m.mode == 2 ? edge - 1.0 : (m.mode == 1 ? -1.0 : 0.0)) - wide);
     m.t_ok = m.mode == 2 ? (float)(magic + edge + 1.0) : 0.0f;

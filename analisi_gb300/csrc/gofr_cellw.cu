@@ -75,10 +75,10 @@
 // Bound by instruction issue: 73 instructions per 128 pairs (46 of them the
 // pairs' own), 77 % of the issue slots used, the shared-memory pipe 57 %
 // busy, the FP32 pipe 59 %, no DRAM traffic to speak of.  16384 atoms, 25
-// origins x 100 lags (16 % of N^2 evaluated, 28 % of those within rmax): 60.9
+// origins x 100 lags (16 % of N^2 evaluated, 28 % of those within rmax): 59.7
 // ms, where the form that queued its candidates and binned the queue took
-// 178.9; 131072 atoms, 5 x 10: 7.8 ms against 21.7; 32768 atoms, triclinic,
-// 10 x 20: 17.8 ms against 59.8.  64 registers, 32 warps per SM (two CTAs of
+// 178.9; 131072 atoms, 5 x 10: 7.6 ms against 21.7; 32768 atoms, triclinic,
+// 10 x 20: 17.3 ms against 59.8.  64 registers, 32 warps per SM (two CTAs of
 // 16, one of 32 for a large histogram): with 128 registers and 16 warps 74.9 ms.
 #include <cstdint>
 #include <cuda_runtime.h>
@@ -544,6 +544,11 @@ __global__ void __launch_bounds__(NWARP * 32, 32 / NWARP) k_pairs_cellw(const Ce
                                 four(u0.x, u0.y, A.fa[i][1].x, row);
                                 bit <<= 1;
                             }
+                        }
+                        if (P.rm.lim < 0.0f) {  // every pair is noted: not those without a record
+#pragma unroll
+                            for (int t = 0; t < 4; ++t)
+                                if (f0 + 32 * t + lane >= n_j) mk[t] = 0u;
                         }
                         // pairs within the margin of a bin edge, one per lane and
                         // round, into their queue; it is taken 32 at a time

@@ -58,7 +58,7 @@ struct Box32 {
 //   pairs beyond -rmin count: n < t_ok - 1.5 2^23 is never certain)
 struct RadialMap {
     float inv_dr, q_off;
-    float t_end;      // nbin + 1.5 2^23: the unread cell
+    float q_end;      // nbin: the unread cell
     float t_hi, t_lo, t_ok;
     float lim;        // negative: no pair is certain
     float lim_self;   // the same for an unwrapped difference of the FP32 frames

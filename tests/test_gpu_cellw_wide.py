@@ -42,3 +42,18 @@ def test_forced_kernel_keeps_its_limit(gpu_engine):
     gpu_engine.set_frames(w["positions"], w["boxes"], w["type_ids"], w["ntypes"])
     with pytest.raises(engine.GofrError):
         gpu_engine.run(0.0, 5.0, 600, 1, 1, 1, 2, 0, kernel="cellw")
+
+
+@pytest.mark.parametrize("N,L,kernel,rmin,rmax", [
+    (129, 10.0, "f32", 4.0, 4.004), (250, 10.0, "f32", 4.0, 4.004), (129, 10.0, "f32", -1e-4, 1e-4),
+    (250, 10.0, "f32", -1e-4, 1e-4), (2600, 30.0, "cellw", 4.0, 4.004)])
+def test_bins_finer_than_the_margin(gpu_engine, oracle_mod, N, L, kernel, rmin, rmax):
+    """Bins so fine that every pair is recomputed: the lanes without an atom of
+    the last chunk are not, the pairs clamped to the row's ends are."""
+    w = workloads.small_case(N, N, 5, L, 0.2, [N - N // 3, N // 3])
+    gpu_engine.set_frames(w["positions"], w["boxes"], w["type_ids"], w["ntypes"])
+    got = gpu_engine.run(rmin, rmax, 500, 2, 1, 1, 4, 0, kernel=kernel)
+    want = oracle_mod.gofrt_counts(w["positions"], w["boxes"], w["type_ids"], 2, rmin, rmax, 500,
+                                   2, 1, 1, 1, 4, 0)
+    np.testing.assert_array_equal(got, want)
+    assert want.sum() > 0 or rmin < 0
