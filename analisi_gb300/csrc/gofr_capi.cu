@@ -5,8 +5,9 @@
 //     into HBM and converted there to FP32 {x,y,z,type} records;
 //   * calc_init semantics (lib/src/gofrt.cpp:41-93): leff, the trajectory
 //     length check, origins/lags grid, incr;
-//   * exact bin thresholds in d2 space (gofr_bin_thresholds) and the certified
-//     FP32 error bound that turns them into FP32 windows (certify());
+//   * exact bin thresholds in d2 space (gofr_bin_thresholds), the certified
+//     FP32 error bound and the radial margin of the kernels that bin in place
+//     (radial_map()), or the FP32 windows of the other two (certify());
 //   * kernel selection (the planner's cost models, the cell grids and the
 //     warp-streamed kernel's neighbourhood geometry, orthorhombic and
 //     triclinic, with their certified bounds; the autotuner), launches,

@@ -195,7 +195,7 @@ struct CellwLaunch {
     int pg, npg;                   // partitions per histogram, groups of them (pair.nparts)
     long long most;                // warp blocks of a CTA's chunk at most
     unsigned *queue;               // {next chunk, CTAs done}, zero before and after a launch
-    int cta_warps;                 // warps per CTA: 8 (two CTAs per SM) or 16 (one)
+    int cta_warps;                 // warps per CTA: 8 or 16 (one CTA of 32 where 16 leave half an SM)
     int hcopy;                     // copies of the shared histogram (privatisation depth: 1, 2)
     int nz_lo, nz_hi;              // neighbourhood layers (see above)
     int ny_lo[3], ny_hi[3];        // rows, per layer image sz + 1

@@ -258,10 +258,10 @@ class Clocks:
                 "samples": len(rows)}
 
 
-KERNEL_NAMES = {1: "k_pairs_f32 (all pairs)", 2: "k_pairs_f64 (all pairs)",
+KERNEL_NAMES = {1: "k_allpairs (all pairs)", 2: "k_pairs_f64 (all pairs)",
                 3: "k_pairs_cell (block cell lists)",
                 5: "k_pairs_cellw (warp-streamed cell lists)"}
-PROFILE_OF = {1: "k_pairs_f32_c2_n16384.md", 3: "k_pairs_cell_c2_n16384.md",
+PROFILE_OF = {1: "k_allpairs_c2_n16384.md", 3: "k_pairs_cell_c2_n16384.md",
               5: "k_pairs_cellw_c2_n16384.md"}
 
 
@@ -335,7 +335,7 @@ def bench_batch(engine, workloads, device, origins=0, reps=2):
             "pairs": st["pairs"], "value": round(batch_rate, 2), "unit": UNIT,
             "ms": round(sum(ms) / len(ms), 1),
             "kernel": "one graph: k_pairs_cellw per cell-list member (second stream) + "
-                      "k_pairs_batch (all-pairs members, persistent work queue)",
+                      "k_allpairs_batch (all-pairs members, persistent work queue)",
             "evaluated_fraction": round(st["evaluated"] / st["pairs"], 4),
             "sequential_same_plans": round(seq["auto"][0], 2),
             "best_single_same_plans": round(seq["auto"][1], 2),
@@ -366,7 +366,7 @@ def bench_allpairs(eng, prm, args, flush, steps=2):
             pairs += st["pairs"]
             ms += st["kernel_ms"]
     return {"value": round(pairs / ms / 1e6, 3), "unit": UNIT, "steps": steps,
-            "kernel": "k_pairs_f32 (all pairs)"}
+            "kernel": "k_allpairs (all pairs)"}
 
 
 def bench_msd(eng, w, p, reps=3):
@@ -650,9 +650,9 @@ def run_gpu(args):
                      "ordered pair of the reference loop (N^2 per origin and lag) / mean kernel "
                      "time: the all-pairs unit of the metric.  The cell-list kernel evaluates "
                      "only the pairs of neighbouring cells at 7 operations each (three "
-                     "differences, a multiply, two FMAs, the candidate test; neighbours moved "
+                     "differences, three FMAs, the edge test; neighbours moved "
                      "to their image once per chunk); frac_evaluated_pairs is that issue rate "
-                     "against the same peak.  Candidate binning is counted in neither.  "
+                     "against the same peak.  Binning is counted in neither.  "
                      "traffic = ncu dram bytes per launch (profiles/)",
             "frac_evaluated_pairs": round(achieved_eval / peak, 4),
             "achieved_evaluated_pairs": round(achieved_eval, 3),

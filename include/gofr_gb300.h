@@ -83,9 +83,10 @@ enum gofr_kernel {
                                     the cell-list conditions, a histogram and channel
                                     table that fit shared memory, and tilts
                                     that keep the images a block reaches within two box
-                                    edges).  AUTO takes it for 2048 atoms or more
-                                    where its modelled cost is below the all-pairs
-                                    kernel's.
+                                    edges, nparts <= 1).  AUTO takes it for 2048 atoms
+                                    or more where its modelled cost is below the
+                                    all-pairs kernel's, for any nparts and any
+                                    histogram that its warps leave room for.
                                     ANALISI_GB300_CELLW_PLAN="reach,4,wx,wy,wz" pins its
                                     configuration (4: the records a lane holds) */
 };
@@ -411,10 +412,11 @@ int gofr_msd_output_size(const gofr_ctx *ctx, const gofr_msd_params *p, size_t *
  * mean over origins and atoms of type k of |x(o) - x(o+t)|^2 (optionally
  * minus the type's centre-of-mass displacement); (t, 1, k) the mean over
  * origins of the centre-of-mass |cm_k(o) - cm_k(o+t)|^2.  Each displacement is
- * the reference's FP64 value; its squared components are added into FP64 sums
- * (fused multiply-adds, a fixed order) divided by the count, where the
- * reference keeps a running mean: the two agree to rounding (relative ~1e-13
- * for 1e7 terms).  Errors as
+ * formed from integers that hold the coordinates as finely as FP64 does, its
+ * squares are summed exactly and rounded once (FP64 sums where the coordinates
+ * or the window of lags do not allow it), where the reference keeps a running
+ * mean: the two agree to the reference's rounding (relative ~1e-13 for 1e7
+ * terms).  Errors as
  * lib/src/msd.cpp:57-68 (GOFR_ERR_RANGE: trajectory too short). */
 int gofr_msd_run(gofr_ctx *ctx, const gofr_msd_params *p, double *out_host);
 
