@@ -72,7 +72,7 @@
 // (lag, origin) dealt round-robin, a barrier and a flush after each, left 10 % of
 // the 16k-atom job idle in the last round and 18 % of the 131k-atom one.)
 //
-// Bound by instruction issue: 73 instructions per 128 pairs (46 of them the
+// Bound by instruction issue: 71 instructions per 128 pairs (46 of them the
 // pairs' own), 77 % of the issue slots used, the shared-memory pipe 57 %
 // busy, the FP32 pipe 59 %, no DRAM traffic to speak of.  16384 atoms, 25
 // origins x 100 lags (16 % of N^2 evaluated, 28 % of those within rmax): 59.7
