@@ -2735,8 +2735,11 @@ int run_windows_impl(gofr_ctx *ctx, const gofr_params *p, unsigned nwin,
         const int rc = shape_of(ctx, t, q, rs);
         if (rc) return rc;
     }
+    // p->primo is no window's: the tuner samples the first one
+    gofr_params first_win = *p;
+    first_win.primo = primos[0];
     Plan pl;
-    int rc = choose_plan(ctx, t, *p, pl);
+    int rc = choose_plan(ctx, t, first_win, pl);
     if (rc) return rc;
     const size_t per_win = rs.data_length * nparts;
     const size_t n_out = per_win * nwin;

@@ -112,3 +112,25 @@ def test_cell_lists_per_partition(gpu_engine, oracle_mod, case):
     # a forced cell-list kernel still refuses partitions
     with pytest.raises(engine.GofrError):
         gpu_engine.run(*args, kernel="cellw", nparts=parts)
+
+
+def test_tuned_windows_sample_the_first_window(gpu_engine, oracle_mod):
+    """The tuner of a run over windows samples the first window: the parameters'
+    own first frame, here past the end, is not one of them."""
+    import ctypes
+    w = workloads.small_case(83, 6000, 6, 42.0, 0.1, [4000, 2000], rmin=0.0, rmax=4.0, nbin=37,
+                             tmax=2, skip=1, every=1, ntimesteps=3, primo=0)
+    gpu_engine.set_frames(w["positions"], w["boxes"], w["type_ids"], 2)
+    p = engine.make_params(0.0, 4.0, 37, 2, 1, 1, 3, 1 << 40, "tuned")
+    primos = np.array([2, 0], dtype=np.uint64)
+    out = np.zeros(2 * 2 * 6 * 37, dtype=np.uint64)
+    as_u64 = ctypes.POINTER(ctypes.c_ulonglong)
+    gpu_engine._check(gpu_engine.L.gofr_run_windows(
+        gpu_engine._ctx, ctypes.byref(p), 2, primos.ctypes.data_as(as_u64),
+        out.ctypes.data_as(as_u64)))
+    # an eightieth of the pairs is near: all pairs would be an order slower
+    assert gpu_engine.stats()["kernel_used"] in (3, 5)
+    for k, primo in enumerate((2, 0)):
+        want = oracle_mod.gofrt_counts(w["positions"], w["boxes"], w["type_ids"], 2, 0.0, 4.0, 37,
+                                       2, 8, 1, 1, 3, primo)
+        np.testing.assert_array_equal(out.reshape(2, *want.shape)[k], want)
