@@ -1405,16 +1405,29 @@ constexpr double kCellAutoTime = 0.85;
 // gain is a tenth to a quarter of a run, less than the lists of new frames
 // cost) ...
 constexpr double kCellwAuto = 0.9;
-// ... and the trajectory has this many atoms: below, the first pass on new
-// frames pays more for building the lists (allocations, three kernels and a
-// synchronisation: 0.5 ms) than runs on them gain (1000 atoms, 20 lags x 10
-// origins: 0.08 ms against 0.23).
+// ... and the trajectory has this many atoms, or half as many and a job of this
+// many ordered pairs.  A small job gains less from the lists than building them
+// on new frames costs (0.1 to 0.5 ms).  Repeated call / first call on new frames,
+// us, all pairs against cell lists: 2000 atoms, 6e7 pairs 163 / 174, 145 / 404;
+// 1200 atoms, 2.9e8 pairs 396 / 413, 153 / 326; 1500 atoms, 5.4e9 pairs 4178 /
+// 4207, 928 / 1407; 2000 atoms triclinic, 8e8 pairs 846 / 874, 245 / 521.
 constexpr size_t kCellMinAtoms = 2048;
+constexpr double kCellSmallPairs = 268435456.0;
+
+bool pays_for_lists(const TrajDev &t, const gofr_params &p)
+{
+    if (t.N >= kCellMinAtoms) return true;
+    if (t.N < kCellMinAtoms / 2) return false;
+    const unsigned leff = (p.ntimesteps < p.tmax || p.tmax == 0) ? p.ntimesteps : p.tmax;
+    const double lags = std::ceil((double)leff / std::max(1u, p.every)),
+                 origins = std::ceil((double)p.ntimesteps / std::max(1u, p.skip));
+    return lags * origins * (double)t.N * (double)t.N >= kCellSmallPairs;
+}
 
 // The cell-list plan AUTO takes for the all-pairs plan pl, if any.
 bool auto_cell_plan(const TrajDev &t, const gofr_params &p, Plan &pl)
 {
-    if (pl.kind != 0 || pl.wrapcheck || pl.empty || t.N < kCellMinAtoms) return false;
+    if (pl.kind != 0 || pl.wrapcheck || pl.empty || !pays_for_lists(t, p)) return false;
     CellwCand c;
     Plan q = pl;
     if (cellw_choice(t, p, c) && make_cellw_plan(t, p, q, c)) {

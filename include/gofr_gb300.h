@@ -84,7 +84,7 @@ enum gofr_kernel {
                                     table that fit shared memory, and tilts
                                     that keep the images a block reaches within two box
                                     edges, nparts <= 1).  AUTO takes it for 2048 atoms
-                                    or more where its modelled cost is below the
+                                    or more (1024 for jobs of 2^28 pairs) where its modelled cost is below the
                                     all-pairs kernel's, for any nparts and any
                                     histogram that its warps leave room for.
                                     ANALISI_GB300_CELLW_PLAN="reach,4,wx,wy,wz" pins its
