@@ -177,7 +177,8 @@ int fail(gofr_ctx *ctx, int code, const char *fmt, ...)
 // ANALISI_GB300_FAIL_ALLOC=<tag> only the allocations made with that tag
 // (e.g. "cells": the cell-sorted frames), so that the error paths and the
 // fallbacks can be run without a real shortage; they must leave the context
-// usable.
+// usable.  With ANALISI_GB300_FILL_ALLOC=<byte> every allocation is filled with
+// that byte, so that a test does not depend on what the memory held before.
 template <class T>
 cudaError_t dev_malloc(T **p, size_t bytes, const char *tag = nullptr)
 {
@@ -186,7 +187,12 @@ cudaError_t dev_malloc(T **p, size_t bytes, const char *tag = nullptr)
         *p = nullptr;
         return cudaErrorMemoryAllocation;
     }
-    return cudaMalloc(reinterpret_cast<void **>(p), bytes);
+    const cudaError_t rc = cudaMalloc(reinterpret_cast<void **>(p), bytes);
+    const char *f = std::getenv("ANALISI_GB300_FILL_ALLOC");
+    if (!f || rc != cudaSuccess) return rc;
+    const cudaError_t fill = cudaMemset(*p, std::atoi(f) & 0xff, bytes);
+    // the engine's streams do not wait for the default one
+    return fill == cudaSuccess ? cudaStreamSynchronize(nullptr) : fill;
 }
 
 struct DevGuard {
@@ -2008,7 +2014,9 @@ void tune_log(const std::string &key, const TuneChoice &c, double ms)
 }
 
 
-// Times one plan on the sample parameters; returns milliseconds (or < 0).
+// Times one plan on the sample parameters; returns milliseconds (or < 0: it
+// did not run, or a kernel reported an error).  The pair kernels deal their work
+// from counters beside the statistics, which have to be zero at their launch.
 double tune_time(gofr_ctx *ctx, const TrajDev &t, const gofr_params &q, const Plan &pl)
 {
     RunShape rs;
@@ -2016,7 +2024,8 @@ double tune_time(gofr_ctx *ctx, const TrajDev &t, const gofr_params &q, const Pl
     if (ensure(ctx, ctx->d_counts, ctx->cap_counts, rs.data_length)) return -1.0;
     double best = -1.0;
     for (int rep = 0; rep < 2; ++rep) {  // the first run also builds cell lists
-        if (cudaMemsetAsync(ctx->d_counts, 0, rs.data_length * 8, ctx->stream) != cudaSuccess)
+        if (cudaMemsetAsync(ctx->d_counts, 0, rs.data_length * 8, ctx->stream) != cudaSuccess ||
+            clear_stats(ctx) != cudaSuccess)
             return -1.0;
         cudaEventRecord(ctx->ev[1], ctx->stream);
         unsigned long long pairs = 0;
@@ -2026,7 +2035,12 @@ double tune_time(gofr_ctx *ctx, const TrajDev &t, const gofr_params &q, const Pl
             return -1.0;
         }
         cudaEventRecord(ctx->ev[2], ctx->stream);
-        if (cudaStreamSynchronize(ctx->stream) != cudaSuccess) return -1.0;
+        if (queue_stats(ctx) != cudaSuccess) return -1.0;
+        if (check_device_error(ctx)) {
+            ctx->err.clear();
+            (void)cudaGetLastError();
+            return -1.0;
+        }
         float ms = 0.f;
         cudaEventElapsedTime(&ms, ctx->ev[1], ctx->ev[2]);
         best = ms;
@@ -2624,6 +2638,8 @@ int gofr_ctx_create(gofr_ctx **out, int device)
         ok = ok && cudaEventCreateWithFlags(&ctx->ev_join, cudaEventDisableTiming) == cudaSuccess;
         ok = ok && dev_malloc(&ctx->d_stats, ST_COUNT * sizeof(unsigned long long)) == cudaSuccess;
         ok = ok && cudaMallocHost(&ctx->h_stats, ST_COUNT * sizeof(unsigned long long)) == cudaSuccess;
+        // the counters and the error word are zero before the first run, too
+        ok = ok && clear_stats(ctx) == cudaSuccess;
         if (ok) ctx->d_err = reinterpret_cast<unsigned *>(ctx->d_stats + ST_ERR);
         ok = ok && dev_malloc(&ctx->d_minmax, 256 * 6 * sizeof(double)) == cudaSuccess;
         ok = ok && dev_malloc(&ctx->d_nonfinite, sizeof(unsigned)) == cudaSuccess;
