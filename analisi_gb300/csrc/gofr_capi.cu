@@ -1096,10 +1096,10 @@ bool cell_eligible(const TrajDev &t, const gofr_params &p, bool warp = false)
     if (p.nparts > 1 && !(warp && p.kernel == GOFR_KERNEL_AUTO && p.nparts <= t.N)) return false;
     if (!(p.rmax > 0.0)) return false;
     if (t.N >= (1u << 24)) return false;  // sorted slots pack type << 24 | atom id
-    // AUTO takes any histogram that the warp-streamed kernel has room for (6 types,
-    // 600 bins, 32768 atoms: 152 ms all-pairs); the block kernel's, which needs more
-    // beside it, and a forced or tuned one keep to what that has room for
-    if (warp && p.kernel == GOFR_KERNEL_AUTO) return true;
+    // AUTO and the tuner take any histogram that the warp-streamed kernel has room
+    // for (6 types, 600 bins, 32768 atoms: 152 ms all-pairs); the block kernel, which
+    // needs more beside it, and a forced one keep to what that has room for
+    if (warp && (p.kernel == GOFR_KERNEL_AUTO || p.kernel == GOFR_KERNEL_TUNED)) return true;
     return cell_smem_bytes((int)(t.ntypes * (t.ntypes + 1)), (int)p.nbin, (int)t.ntypes) <=
            160 * 1024;
 }
@@ -1944,8 +1944,9 @@ std::mutex g_tune_mutex;
 std::map<std::string, TuneChoice> g_tune;
 bool g_tune_loaded = false;
 
-std::string tune_key(const TrajDev &t, const gofr_params &p)
+std::string tune_key(const TrajDev &t, gofr_params p)
 {
+    p.kernel = GOFR_KERNEL_TUNED;  // AUTO looks for the tuner's choices under the same key
     int lg = 0;
     while ((1ull << (lg + 1)) <= (unsigned long long)t.N) ++lg;
     std::ostringstream k;

@@ -35,3 +35,26 @@ def test_trials_on_a_new_context_do_the_whole_sample(built_engine, tmp_path, fil
     assert len(ms) == 1 and ms[0] > 0.6
     assert all(float(line.rsplit("ms=", 1)[1]) > 0.0 for line in open(log))
     assert {**tuned, "kernel_used": 0} == {**plain, "kernel_used": 0}
+
+
+# 3 types x 1500 bins: a histogram the warp-streamed kernel has room for and the
+# block cell-list kernel has not
+WIDE = dict(seed=91, counts=[2000, 1500, 1000], frames=24, edge=36.0,
+            params=dict(rmin=0.0, rmax=4.0, nbin=1500, tmax=8, skip=2, every=1, ntimesteps=16,
+                        primo=0))
+
+
+def test_large_histograms_are_tuned_and_found_again(built_engine, tmp_path):
+    """The tuner tries the warp-streamed kernel wherever AUTO takes it, and AUTO
+    finds its choice (one changed to the all-pairs kernel shows that it does)."""
+    cache, log = str(tmp_path / "cache.txt"), str(tmp_path / "log.txt")
+    auto, = _child(WIDE, ["auto"], {})
+    tuned, = _child(WIDE, ["tuned"], {"ANALISI_GB300_TUNE_CACHE": cache,
+                                      "ANALISI_GB300_TUNE_LOG": log})
+    assert auto["kernel_used"] == 5
+    assert " warp-cells " in open(log).read() and tuned == auto
+    key = open(cache).read().split()[0]
+    with open(cache, "w") as f:
+        f.write(f"{key} 0 1 4 1 1 1 8 1\n")
+    again, = _child(WIDE, ["auto"], {"ANALISI_GB300_TUNE_CACHE": cache})
+    assert again == {**auto, "kernel_used": 1}
