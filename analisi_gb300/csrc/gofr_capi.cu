@@ -1950,7 +1950,9 @@ std::string tune_key(const TrajDev &t, gofr_params p)
     int lg = 0;
     while ((1ull << (lg + 1)) <= (unsigned long long)t.N) ++lg;
     std::ostringstream k;
-    k << "n2^" << lg << "_bins" << p.nbin << "_types" << t.ntypes << (t.tric ? "_tric" : "_ortho");
+    // v2: the kernels that bin a pair where they find it.  Choices stored without a
+    // version were timed with kernels that are gone.
+    k << "v2_n2^" << lg << "_bins" << p.nbin << "_types" << t.ntypes << (t.tric ? "_tric" : "_ortho");
     int nc[3];
     if (cell_eligible(t, p, true) && cell_grid(t, p, 2, nc))
         k << "_halfcells" << nc[0] << "x" << nc[1] << "x" << nc[2];
@@ -1959,9 +1961,8 @@ std::string tune_key(const TrajDev &t, gofr_params p)
     return k.str();
 }
 
-// Cache file lines: key kind reach r b0 b1 b2 cta_warps hcopy (lines of an
-// older form, key cells reach r b0 b1 b2, are read as kinds 0/1; other lines
-// are skipped).
+// Cache file lines: key kind reach r b0 b1 b2 cta_warps hcopy (other lines are
+// skipped; keys of older kernels are never asked for).
 void tune_load_file()
 {
     if (g_tune_loaded) return;

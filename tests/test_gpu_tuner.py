@@ -58,3 +58,15 @@ def test_large_histograms_are_tuned_and_found_again(built_engine, tmp_path):
         f.write(f"{key} 0 1 4 1 1 1 8 1\n")
     again, = _child(WIDE, ["auto"], {"ANALISI_GB300_TUNE_CACHE": cache})
     assert again == {**auto, "kernel_used": 1}
+
+
+def test_choices_stored_for_older_kernels_are_not_taken(built_engine, tmp_path):
+    """A stored choice compares the kernels of its time: lines whose key starts at
+    the job's size, as all did before the key named a version, are left alone."""
+    cache = str(tmp_path / "cache.txt")
+    tuned, = _child(WIDE, ["tuned"], {"ANALISI_GB300_TUNE_CACHE": cache})
+    key = open(cache).read().split()[0]
+    with open(cache, "w") as f:
+        f.write(f"{key[key.index('n2^'):]} 0 1 4 1 1 1 8 1\n")
+    auto, = _child(WIDE, ["auto"], {"ANALISI_GB300_TUNE_CACHE": cache})
+    assert auto["kernel_used"] == 5 and auto == tuned
