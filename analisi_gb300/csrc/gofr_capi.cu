@@ -1610,29 +1610,33 @@ void set_cellw_grid(CellwLaunch &C, const TrajDev &t, const Plan &pl)
 // and a first atom against a chunk is about 80: 64 atoms against the whole
 // frame unless that makes fewer than `want` units of `frames` (lag, origin)
 // pairs; then 32 atoms, then fewer chunks, and fewer atoms only when one chunk
-// is left.
+// is left.  Never more than kAllpairsChunks of them (4.2 million atoms): the
+// eight warps' units of a CTA hold fewer than 2^31 pairs, which a u32 shared bin
+// counts.
 struct AllpairsUnit {
     int gs = ALLPAIRS_GROUP, ng = 1, jc = 1, nj = 1;
 };
+constexpr int kAllpairsChunks = 0x7fffffff / (8 * ALLPAIRS_GROUP * ALLPAIRS_CHUNK);
 
 AllpairsUnit allpairs_unit(size_t n_i, size_t N, double frames, double want)
 {
     AllpairsUnit a;
     const int chunks = (int)((N + ALLPAIRS_CHUNK - 1) / ALLPAIRS_CHUNK);
     auto groups = [&](int gs) { return std::ceil((double)n_i / gs); };
-    a.jc = chunks;
+    a.jc = std::min(chunks, kAllpairsChunks);
     if (frames * groups(a.gs) < want) a.gs = 32;
     const double units = frames * groups(a.gs);
     if (units < want)
-        a.jc = (int)std::max(1.0, std::floor(chunks / std::ceil(want / std::max(units, 1.0))));
+        a.jc = (int)std::max(1.0, std::min((double)a.jc, std::floor(chunks / std::ceil(
+                                                             want / std::max(units, 1.0)))));
     while (a.gs > 8 && frames * groups(a.gs) * chunks < want) a.gs /= 2;
     a.nj = (chunks + a.jc - 1) / a.jc;
     a.ng = (int)groups(a.gs);
     return a;
 }
 
-// Units of a CTA's chunk at most: fewer than 2^31 pairs between two flushes (or
-// a unit a warp), so that no u32 shared bin overflows (the kernel checks).
+// Units of a CTA's chunk at most: 2^31 pairs between two flushes, so that no u32
+// shared bin overflows (the kernel checks); a unit a warp always fits.
 long long allpairs_most(size_t N, const AllpairsUnit &a)
 {
     const double pairs = std::min((double)N, (double)a.jc * ALLPAIRS_CHUNK) * a.gs;
@@ -3109,6 +3113,20 @@ int gofr_radial_query(const double *box, int box_kind, const double *coord_min,
     const RadialMap m = plan_radial_map(t, *p, pl);
     const float f[8] = {m.inv_dr, m.q_off, m.lim, m.lim_self, m.t_lo, m.t_hi, m.t_ok, m.self_max};
     for (int k = 0; k < 8; ++k) out[k] = f[k];
+    return GOFR_OK;
+}
+
+int gofr_allpairs_query(size_t natoms, unsigned nparts, double frames, int num_sms, long long *out)
+{
+    if (!out || natoms == 0 || nparts == 0 || nparts > natoms || !(frames >= 1.0) || num_sms < 1)
+        return GOFR_ERR_ARG;
+    const size_t longest = natoms - (nparts - 1) * (natoms / nparts);
+    const AllpairsUnit a = allpairs_unit(longest, natoms, frames * nparts, 512.0 * num_sms);
+    out[0] = a.gs;
+    out[1] = a.ng;
+    out[2] = a.jc;
+    out[3] = a.nj;
+    out[4] = allpairs_most(natoms, a);
     return GOFR_OK;
 }
 

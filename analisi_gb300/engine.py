@@ -30,7 +30,7 @@ EXPORTED = [
     "gofr_run_f64_noalloc", "gofr_run_windows", "gofr_set_centres", "gofr_msd_output_size",
     "gofr_msd_run", "gofr_neigh_layout", "gofr_neigh_run", "gofr_run_normalized",
     "gofr_run_streamed", "gofr_cellw_tables", "gofr_cellw_row",
-    "gofr_plan_query", "gofr_radial_query",
+    "gofr_plan_query", "gofr_radial_query", "gofr_allpairs_query",
 ]
 
 
@@ -160,6 +160,8 @@ def load_library(path=None):
                                   ctypes.POINTER(Params), ip]
     L.gofr_radial_query.argtypes = [dp, ctypes.c_int, dp, dp, ctypes.c_size_t, ctypes.c_uint,
                                     ctypes.POINTER(Params), dp]
+    L.gofr_allpairs_query.argtypes = [ctypes.c_size_t, ctypes.c_uint, ctypes.c_double,
+                                      ctypes.c_int, ctypes.POINTER(ctypes.c_longlong)]
     L.gofr_batch_set.argtypes = [vp, ctypes.POINTER(TrajDesc), ctypes.c_uint]
     L.gofr_batch_output_layout.argtypes = [vp, ctypes.c_uint, ctypes.POINTER(ctypes.c_size_t),
                                            ctypes.POINTER(ctypes.c_size_t)]
@@ -186,7 +188,8 @@ def load_library(path=None):
                  "gofr_bin_thresholds", "gofr_batch_set", "gofr_batch_output_layout",
                  "gofr_batch_run", "gofr_measure_peaks", "gofr_run_f64_noalloc",
                  "gofr_run_windows", "gofr_run_normalized", "gofr_run_streamed",
-                 "gofr_cellw_tables", "gofr_cellw_row", "gofr_plan_query", "gofr_radial_query"):
+                 "gofr_cellw_tables", "gofr_cellw_row", "gofr_plan_query", "gofr_radial_query",
+                 "gofr_allpairs_query"):
         getattr(L, name).restype = ctypes.c_int
     if path is None:
         _lib = L
@@ -257,6 +260,17 @@ def radial_query(box, triclinic, coord_min, coord_max, natoms, ntypes, params):
         raise GofrError(rc, "no FP32 bin map for these parameters")
     return dict(zip(("inv_dr", "q_off", "lim", "lim_self", "t_lo", "t_hi", "t_ok", "self_max"),
                     out.astype(np.float32)))
+
+
+def allpairs_query(natoms, nparts, frames, num_sms=152):
+    """How the all-pairs kernel splits a run (host code, no GPU): a dict
+    {first, groups, chunks, parts, most}."""
+    L = load_library()
+    out = (ctypes.c_longlong * 5)()
+    rc = L.gofr_allpairs_query(int(natoms), int(nparts), float(frames), int(num_sms), out)
+    if rc != GOFR_OK:
+        raise GofrError(rc, "invalid atoms, partitions, frames or multiprocessors")
+    return dict(zip(("first", "groups", "chunks", "parts", "most"), [int(v) for v in out]))
 
 
 def cellw_tables(box, triclinic, coord_min, coord_max, rmax, nc):

@@ -271,6 +271,15 @@ int gofr_radial_query(const double *box, int box_kind, const double *coord_min,
                       const double *coord_max, size_t natoms, unsigned ntypes,
                       const gofr_params *p, double *out);
 
+/* How the all-pairs kernel splits a run over `frames` (lag, origin) pairs of
+ * natoms atoms in nparts partitions on num_sms multiprocessors (host only):
+ * out (5 values): first atoms of a unit, groups of them per partition, chunks
+ * of 128 second atoms of a unit, parts of the frame they make, units of a CTA's
+ * chunk at most.  Between two flushes a CTA counts fewer than 2^32 pairs into its
+ * 32-bit bins (no reference counterpart: it counts in 64 bits). */
+int gofr_allpairs_query(size_t natoms, unsigned nparts, double frames, int num_sms,
+                        long long *out);
+
 /* Neighbourhood tables of the warp-streamed cell-list kernel (host only, no
  * device work) for one box (internal format, 6 or 9 doubles), the
  * coordinates' extent per axis [coord_min, coord_max], rmax and a cell grid
