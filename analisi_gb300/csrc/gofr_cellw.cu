@@ -68,7 +68,9 @@
 // Work is a list of (lag, origin, warp block) units, dealt to the CTAs in
 // chunks of decreasing size from one counter; the warps of a CTA take the
 // chunk's units one by one and never wait for one another inside a chunk.
-// The histogram is added to the counts when the lag changes.  (Items of one
+// The histogram is added to the counts when the lag changes, and before 2^32
+// pairs were evaluated since (a u32 bin could overflow): a warp whose unit finds
+// no room for its pairs keeps it for after the flush.  (Items of one
 // (lag, origin) dealt round-robin, a barrier and a flush after each, left 10 % of
 // the 16k-atom job idle in the last round and 18 % of the 131k-atom one.)
 //
@@ -113,6 +115,7 @@ struct WarpArea {
     uint2 q[QW];                 // FP64 recheck queue: w of both atoms
     int2 src[MAXSEG];            // {sorted slot of the segment's first record - its flat index, image}
     int pre[MAXSEG + 33];        // flat index of each segment's first record (INT_MAX past the last)
+    int held;                    // unit left for after the next flush (-1: none)
 };
 
 // NWARP warps per CTA, HCOPY copies of the shared histogram (warp w adds to
@@ -165,6 +168,7 @@ __global__ void __launch_bounds__(NWARP * 32, 32 / NWARP) k_pairs_cellw(const Ce
         s_ox[tid] = C.ox[tid];
     }
     if (tid == 0) s_pairs = 0ull;
+    if (lane == 0) A.held = -1;
 
     int nn = 0, qn = 0;  // entries of the warp's two queues (the same in every lane)
     unsigned long long n_cand = 0, n_rech = 0, n_eval = 0;  // n_cand: counts flushed
@@ -173,7 +177,7 @@ __global__ void __launch_bounds__(NWARP * 32, 32 / NWARP) k_pairs_cellw(const Ce
     // Adds the CTA's histogram copies to the counts of plane (partition group,
     // lag) and clears them (all threads; every warp is done with its pairs).  A
     // u32 bin holds its hits exactly only while fewer than 2^32 pairs were
-    // evaluated (the host keeps chunks far below).
+    // evaluated: only a single unit can have more.
     auto flush = [&](int plane) {
         if (s_pairs > 0xffffffffull) lost = true;
         const int grp = PARTS ? plane / P.n_lags : 0, lag_idx = plane - grp * P.n_lags;
@@ -215,12 +219,13 @@ __global__ void __launch_bounds__(NWARP * 32, 32 / NWARP) k_pairs_cellw(const Ce
         __syncthreads();
         const long long c0 = s_u0, c1 = s_u1;
         if (c0 >= c1) break;
+        bool again = false;  // a warp holds a unit of this segment back: a flush, then the rest
         for (long long g0 = c0; g0 < c1 && !lost;) {
         const int plane = (int)(g0 / per_plane);
         const int lag_idx = PARTS ? plane % P.n_lags : plane;
         const int part0 = PARTS ? plane / P.n_lags * C.pg : 0;
         const long long g1 = min(c1, (plane + 1) * per_plane);
-        if (g0 != c0) {
+        if (g0 != c0 && !again) {
             __syncthreads();  // the warps are done with the chunk's last plane
             if (tid == 0) {
                 s_next = 0;
@@ -228,7 +233,7 @@ __global__ void __launch_bounds__(NWARP * 32, 32 / NWARP) k_pairs_cellw(const Ce
             }
             __syncthreads();
         }
-        if (cur >= 0 && (plane != cur || s_full)) flush(cur);
+        if (cur >= 0 && (plane != cur || s_full || again)) flush(cur);
         cur = plane;
         int k = -1;  // origin of the warp's queues
         long long fo = 0, fl = 0;
@@ -305,7 +310,11 @@ __global__ void __launch_bounds__(NWARP * 32, 32 / NWARP) k_pairs_cellw(const Ce
 
         for (;;) {
             int nx = 0;
-            if (lane == 0) nx = atomicAdd(&s_next, 1);
+            if (lane == 0) {
+                nx = A.held;
+                if (nx < 0) nx = atomicAdd(&s_next, 1);
+                A.held = -1;
+            }
             nx = __shfl_sync(0xffffffffu, nx, 0);
             if (g0 + nx >= g1) break;
             const long long uo = seg_off + nx;
@@ -414,7 +423,20 @@ __global__ void __launch_bounds__(NWARP * 32, 32 / NWARP) k_pairs_cellw(const Ce
                 }
             }
             A.pre[nseg + lane] = 0x7fffffff;
-            if (lane == 0) A.pre[nseg + 32] = 0x7fffffff;
+            // room for the unit's pairs in the u32 bins: a unit that finds none waits for
+            // the next flush (the first unit after one always has it)
+            bool room = true;
+            if (lane == 0) {
+                A.pre[nseg + 32] = 0x7fffffff;
+                const unsigned long long pe = (unsigned long long)n_i * (unsigned long long)n_j,
+                                         was = atomicAdd(&s_pairs, pe);
+                room = was == 0ull || was + pe <= 0xffffffffull;
+                if (!room) {
+                    atomicAdd(&s_pairs, 0ull - pe);
+                    A.held = nx;
+                }
+            }
+            if (!__shfl_sync(0xffffffffu, (int)room, 0)) break;
 
             for (int ibase = 0; ibase < n_i; ibase += FA) {
                 // first atoms ibase .. ibase + n - 1 of the block, those of the
@@ -474,11 +496,7 @@ __global__ void __launch_bounds__(NWARP * 32, 32 / NWARP) k_pairs_cellw(const Ce
                     }
                 }
                 if (na == 0) continue;
-                if (lane == 0) {
-                    const unsigned long long pe = (unsigned long long)na * (unsigned long long)n_j;
-                    n_eval += pe;
-                    atomicAdd(&s_pairs, pe);
-                }
+                if (lane == 0) n_eval += (unsigned long long)na * (unsigned long long)n_j;
                 __syncwarp();
                 const f2 inv = f2pk(P.rm.inv_dr, P.rm.inv_dr), off = f2pk(P.rm.q_off, P.rm.q_off),
                          tiny = f2pk(RADIAL_TINY, RADIAL_TINY);
@@ -583,7 +601,8 @@ __global__ void __launch_bounds__(NWARP * 32, 32 / NWARP) k_pairs_cellw(const Ce
         }
         recheck(qn);
         qn = 0;
-        g0 = g1;
+        again = __syncthreads_or(lane == 0 && A.held >= 0) != 0;
+        if (!again) g0 = g1;
         }
     }
     __syncthreads();
