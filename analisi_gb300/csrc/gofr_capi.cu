@@ -72,8 +72,9 @@ struct TrajDev {
     // MSD: atoms sorted by type, type starts, optional centres of mass
     std::vector<int> h_perm, h_tbegin, h_types;
     int *d_perm = nullptr, *d_tbegin = nullptr;
-    double *d_cm = nullptr;          // [T][ntypes][3]
+    double *d_cm = nullptr;          // [T][ntypes][3], then the extent per type [ntypes]
     double cm_max = 0.0;             // largest |component| of them
+    unsigned *d_ext = nullptr;       // [256] largest extent per type over every frame (FP32 bits)
 };
 
 }  // namespace
@@ -237,7 +238,8 @@ void free_traj(TrajDev &t)
     cudaFree(t.d_perm);
     cudaFree(t.d_tbegin);
     cudaFree(t.d_cm);
-    t.d_perm = nullptr; t.d_tbegin = nullptr; t.d_cm = nullptr;
+    cudaFree(t.d_ext);
+    t.d_perm = nullptr; t.d_tbegin = nullptr; t.d_cm = nullptr; t.d_ext = nullptr;
     t.pos64 = nullptr; t.pos32 = nullptr; t.box64 = nullptr; t.box32 = nullptr; t.types = nullptr;
     t.types8 = nullptr;
     t.d_cstart = nullptr; t.d_sidt = nullptr; t.d_spos = nullptr;
@@ -1015,6 +1017,12 @@ int upload_traj(gofr_ctx *ctx, TrajDev &t, const double *positions, const double
     if (launch_convert(t.pos64, t.types, nframes, natoms, t.shift[0], t.shift[1], t.shift[2],
                        t.pos32, t.types8, ctx->stream))
         return fail(ctx, GOFR_ERR_CUDA, "convert kernel launch failed: %s",
+                    cudaGetErrorString(cudaGetLastError()));
+    CK(dev_malloc(&t.d_ext, 256 * sizeof(unsigned)));
+    CK(cudaMemsetAsync(t.d_ext, 0, 256 * sizeof(unsigned), ctx->stream));
+    ++ctx->launches;
+    if (launch_extent(t.pos32, t.types8, natoms, 0, 1, (int)nframes, 0, t.d_ext, ctx->stream))
+        return fail(ctx, GOFR_ERR_CUDA, "extent kernel launch failed: %s",
                     cudaGetErrorString(cudaGetLastError()));
     CK(cudaStreamSynchronize(ctx->stream));
     return GOFR_OK;
@@ -3344,11 +3352,20 @@ int gofr_set_centres(gofr_ctx *ctx, const double *centres, size_t nframes, unsig
     cudaFree(t.d_cm);
     t.d_cm = nullptr;
     const size_t n = nframes * ntypes * 3;
-    CK(dev_malloc(&t.d_cm, n * sizeof(double)));
+    CK(dev_malloc(&t.d_cm, (n + ntypes) * sizeof(double)));
     t.cm_max = 0.0;
-    for (size_t i = 0; i < n; ++i)
+    const size_t row = (size_t)ntypes * 3;
+    std::vector<double> mn(centres, centres + row), mx = mn, ext(ntypes, 0.0);
+    for (size_t i = 0; i < n; ++i) {
         t.cm_max = std::max(t.cm_max, std::isfinite(centres[i]) ? std::fabs(centres[i]) : INFINITY);
+        mn[i % row] = std::min(mn[i % row], centres[i]);
+        mx[i % row] = std::max(mx[i % row], centres[i]);
+    }
+    for (size_t c = 0; c < row; ++c)
+        ext[c / 3] = std::max(ext[c / 3], std::nextafter(mx[c] - mn[c], INFINITY));
     CK(cudaMemcpyAsync(t.d_cm, centres, n * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
+    CK(cudaMemcpyAsync(t.d_cm + n, ext.data(), ntypes * sizeof(double), cudaMemcpyHostToDevice,
+                       ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
     return GOFR_OK;
 }
@@ -3403,28 +3420,47 @@ int gofr_msd_run(gofr_ctx *ctx, const gofr_msd_params *p, double *out_host)
     M.primo = (long long)p->primo;
     M.cm_msd = p->center_of_mass ? 1 : 0;
     M.cm_self = p->in_center_of_mass_frame ? 1 : 0;
-    // |x| (and |x - centre|) below 2^e; centres that are not finite take the
-    // FP64 form, which carries them into the result
-    double bound = 0.0;
-    for (int k = 0; k < 3; ++k) bound = std::max(bound, std::fabs(t.shift[k]) + t.M[k]);
-    if (M.cm_self) bound += t.cm_max;
-    bound *= 1.0 + std::ldexp(1.0, -40);
+    // coordinates (and centres) that the FP32 frames hold to their rounding; the
+    // others, and centres that are not finite, take the FP64 form, which carries
+    // them into the result
+    double bound = 0.0, eps = 0.0;
+    for (int k = 0; k < 3; ++k) {
+        bound = std::max(bound, std::fabs(t.shift[k]) + t.M[k]);
+        eps = std::max(eps, t.M[k]);
+    }
+    if (M.cm_self) bound = std::max(bound, t.cm_max);
     MsdFixed X{};
-    const bool fixed =
-        std::isfinite(bound) && msd_fixed_plan(M, t.h_tbegin.data(), ctx->num_sms, X);
+    const bool fixed = bound < std::ldexp(1.0, 100) &&
+                       msd_fixed_plan(M, t.h_tbegin.data(), ctx->num_sms, X);
     int rc = ensure(ctx, ctx->d_msd_partial, ctx->cap_msd_partial,
                     fixed ? msd_fixed_partial(M, X) : nout * n_orig);
     if (rc) return rc;
-    rc = ensure(ctx, ctx->d_msd_out, ctx->cap_msd_out, nout);
+    // the results, then the extents of this window (256 words)
+    rc = ensure(ctx, ctx->d_msd_out, ctx->cap_msd_out, nout + 128);
     if (rc) return rc;
     M.partial = ctx->d_msd_partial;
     if (fixed) {
-        int e = 0;
-        std::frexp(bound, &e);
-        X.shift = std::max(-900, std::min(900, MSD_FIXED_BITS - e));
+        // the FP32 frames: (|x - c| + 2^-150) 2^-24 and the rounding of x - c, at both ends
+        X.pad = 2.0 * (eps * std::ldexp(1.0, -24) * (1.0 + std::ldexp(1.0, -20)) +
+                       eps * std::ldexp(1.0, -52)) + std::ldexp(1.0, -148);
+        X.cm_ext = t.d_cm ? t.d_cm + t.T * t.ntypes * 3 : nullptr;
+        X.ext = t.d_ext;
+        const long long span = (long long)(n_orig - 1) * skip + leff;
+        if (skip >= 2 * leff || 4 * span < (long long)t.T) {
+            // few of the frames: the extents over this window (or within each origin's
+            // lags, where these lie apart) instead of over every frame
+            unsigned *const ext = reinterpret_cast<unsigned *>(ctx->d_msd_out + nout);
+            CK(cudaMemsetAsync(ext, 0, 256 * sizeof(unsigned), ctx->stream));
+            const bool apart = skip >= 2 * leff;
+            ++ctx->launches;
+            if (launch_extent(t.pos32, t.types8, t.N, M.primo, apart ? (int)n_orig : 1,
+                              apart ? (int)leff : (int)span, (int)skip, ext, ctx->stream))
+                return fail(ctx, GOFR_ERR_CUDA, "extent kernel launch failed: %s",
+                            cudaGetErrorString(cudaGetLastError()));
+            X.ext = ext;
+        }
         X.partial = reinterpret_cast<long long *>(ctx->d_msd_partial);
-        X.inexact = reinterpret_cast<int *>(X.partial + msd_fixed_partial(M, X) -
-                                            (X.grid + M.ntypes));
+        X.lost = X.partial + msd_fixed_partial(M, X) - (X.grid + M.ntypes);
         X.suspect = ctx->d_stats + ST_CANDIDATES;  // unused by this calculation
     }
     for (bool exact = fixed;; exact = false) {

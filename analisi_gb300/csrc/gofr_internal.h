@@ -284,12 +284,17 @@ struct MsdFixed {
     int lags, phases, passes;   // lags and origin phases of a CTA's threads, CTAs per chunk range
     long long chunks, per;      // chunks, chunks per CTA
     int grid;
-    int shift;                  // coordinates are rint(x 2^shift)
+    const unsigned *ext;        // [256] largest extent per type, FP32 bits (launch_extent)
+    const double *cm_ext;       // [ntypes] the same of the centres (cm_self)
+    double pad;                 // what the FP32 frames' rounding can add to an extent
     long long *partial;         // [grid + ntypes][leff][6]
-    int *inexact;               // [grid + ntypes] a coordinate is not held exactly
+    long long *lost;            // [grid + ntypes] values that are not held exactly
     unsigned long long *suspect;  // set when that could show in a result
 };
-constexpr int MSD_FIXED_BITS = 56;  // coordinates below 2^56
+// Largest extent per type over `len` frames from `first` on, or within each of
+// `groups` runs of them; raises ext[256], FP32 bits.
+int launch_extent(const float *pos32, const unsigned char *types8, size_t N, long long first,
+                  int groups, int len, int stride, unsigned *ext, cudaStream_t s);
 bool msd_fixed_plan(const MsdLaunch &M, const int *h_tbegin, int num_sms, MsdFixed &X);
 size_t msd_fixed_partial(const MsdLaunch &M, const MsdFixed &X);  // 8-byte words of both
 int launch_msd_fixed(const MsdLaunch &M, const MsdFixed &X, double *out_device, cudaStream_t s);

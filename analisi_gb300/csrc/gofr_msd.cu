@@ -7,18 +7,22 @@
 //
 // k_msd_fixed: FP64 instructions issue at 1/64 of the FP32 rate here, so the
 // sums are taken in integers, exactly.  A coordinate (minus its type's centre
-// where asked for) is the 64-bit integer rint(x 2^s), s so that every
-// coordinate is below 2^56: three bits finer than FP64 resolves the largest
-// coordinates, so all but those within an eighth of zero are held exactly (and
-// those to 2^-57 of the largest).  A displacement is one 64-bit subtraction, its
+// where asked for) is rint(x 2^s) modulo 2^64, s so that the displacements of
+// its type are below 2^57 (k_extent: the frames' extents, from their FP32
+// copies).  Coordinates of a 32nd of the largest displacement and more are held
+// exactly; those nearer to zero lose what lies below 2^-57 of that displacement,
+// a sixteenth of what FP64 resolves it to.  A displacement is one 64-bit subtraction, its
 // square three 29-bit products (64-bit multiply-adds), whose sums are combined
 // in 128 bits and rounded once per (lag, type): no term is rounded at all,
-// where the FP64 sums rounded every one.  Where some coordinate is not held
-// exactly and a displacement is so small that this could show (2^42 units rms:
-// a relative error of 5e-13 at most above), the caller runs the FP64 form.  A CTA holds the frames of a few atoms of one type in
-// shared memory, so each coordinate is read from HBM once and every (origin,
-// lag) pair comes from shared memory: thread = (lag, phase of the origins),
-// consecutive lags reading consecutive frames.
+// where the FP64 sums rounded every one.  Where coordinates lost bits and the
+// displacements of a (lag, type) are so small that the bound on the result's
+// error (lost_shows) exceeds the FP64 sums' own, the caller runs the FP64 form.
+// (With the unit taken from the largest coordinate instead, a tracer near the
+// origin of a box of 130 had an error of 5.5e-14 against the FP64 sums' 5.5e-16.)
+// A CTA holds the frames of a few atoms of one type in shared memory, so each
+// coordinate is read from HBM once and every (origin, lag) pair comes from
+// shared memory: thread = (lag, phase of the origins), consecutive lags reading
+// consecutive frames.
 //   Bound by the 32-bit integer multiplier.  16384 atoms in
 // three types, 100 origins x 100 lags: 0.46 ms against 2.79 for the FP64 form;
 // 5003 atoms with both centre-of-mass options, 60 x 80: 0.12 against 0.48.
@@ -138,8 +142,7 @@ constexpr int NACC = 6;    // sums h h, h l, l l: low 32 bits and the rest of ea
 constexpr int TERMS = 8;   // squared displacements (three axes each) between two carries
 constexpr int PLANE = 105 * 1024 / 24;  // (atom, frame) entries of an axis in shared memory: a
                                         // constant, so the axes are offsets of one address
-constexpr int BITS = MSD_FIXED_BITS;  // coordinates are below 2^BITS
-static_assert(BITS == 56, "the products of add_square");
+constexpr int BITS = 57;   // displacements are below 2^BITS: the products of add_square
 
 // Sums of the products of d = h 2^29 + l (|d| < 2^57, h signed, l in [0,
 // 2^29)): hh < 2^56, |hl| < 2^57 and ll < 2^58 in 64 bits, carried into the
@@ -149,22 +152,46 @@ struct Acc {
     long long p[3], hi[3];
 };
 
-// rint(x 2^shift) for |x| 2^shift < 2^BITS, halves away from zero: integer
+// rint(x 2^shift) modulo 2^64, halves away from zero: integer
 // instructions alone (a product and a conversion of the FP64 pipe took a
-// fifth of the kernel's time).  lost collects whether any bit was rounded off.
-__device__ __forceinline__ long long to_fixed(double x, int shift, bool &lost)
+// fifth of the kernel's time).  lost counts the values that were rounded.
+__device__ __forceinline__ unsigned long long to_fixed(double x, int shift, unsigned &lost)
 {
     const long long u = __double_as_longlong(x);
     const int e = (int)(u >> 52 & 0x7ff);
-    const long long m = (u & 0xfffffffffffffll) | 0x10000000000000ll;
+    const unsigned long long m = (u & 0xfffffffffffffull) | 0x10000000000000ull;
     const int r = 1075 - shift - e;  // bits below the point
     if (r > 53 || e == 0) {          // less than half a unit (and below 2^-1022)
-        lost = lost || x != 0.0;
+        if (x != 0.0) ++lost;
         return 0;
     }
-    lost = lost || (r > 0 && (m & ((1ll << r) - 1)) != 0);
-    const long long v = r <= 0 ? m << -r : (m + (1ll << (r - 1))) >> r;
-    return u < 0 ? -v : v;
+    if (r > 0 && (m & ((1ull << r) - 1)) != 0) ++lost;
+    const unsigned long long v =
+        r > 0 ? (m + (1ull << (r - 1))) >> r : (r > -64 ? m << -r : 0ull);
+    return u < 0 ? 0ull - v : v;
+}
+
+// s of type k: the bound on its displacements, taken from the FP32 frames with
+// their rounding (pad), and of the centres', is below 2^(BITS - s).
+__device__ __forceinline__ int unit_shift(const MsdLaunch &M, const MsdFixed &X, int k)
+{
+    double d = __dadd_ru((double)__uint_as_float(X.ext[k]), X.pad);
+    if (M.cm_self) d = __dadd_ru(d, X.cm_ext[k]);
+    return BITS - ((int)(__double_as_longlong(d) >> 52) - 1022);
+}
+
+// Whether the bits lost can show in the sum S of a result (units squared; count
+// terms, na atoms).  A value is off by half a unit at most, a displacement by the
+// errors of its two ends (and of their centres), and an end takes part in two
+// terms of a lag, so the squares of the displacements' errors sum up to 2 lost at most
+// and S is off by 2 sqrt(S 2 lost) and less than a millionth of that.  The FP64
+// sums' own bound is more than c 2^-53 of S: a rounded displacement squared (2), the
+// block's sum (8 and more), three FMAs per 256 atoms, an addition per origin.  S is
+// kept where the former is no larger than c 2^-53, c at most 32 (3.6e-15).
+__device__ __forceinline__ bool lost_shows(double S, double lost, int na, int n_orig)
+{
+    const double c = fmin(32.0, 10.0 + n_orig + 3.0 * ((na + NT - 1) / NT));
+    return lost > 0.0 && S * (c * c) < lost * 649037107316853453566312041152512.0;  // 2^109
 }
 
 __device__ __forceinline__ void mad_wide(long long &a, int x, int y)
@@ -178,6 +205,12 @@ __device__ __forceinline__ void add_square(Acc &a, long long d)
     mad_wide(a.p[0], h, h);
     mad_wide(a.p[1], h, l);
     mad_wide(a.p[2], l, l);
+}
+
+// The displacement of two values held modulo 2^64.
+__device__ __forceinline__ long long minus(long long a, long long b)
+{
+    return (long long)((unsigned long long)a - (unsigned long long)b);
 }
 
 // p keeps its low 32 bits; the rest goes to hi.
@@ -208,7 +241,9 @@ __global__ void __launch_bounds__(FT, 2) k_msd_fixed(const MsdLaunch M, const Ms
     const bool busy = phase < X.phases && lag < l0 + nl;
     const long long c0 = (long long)blockIdx.x * X.per, c1 = min(c0 + X.per, X.chunks);
     Acc acc{};
-    bool lost = false;  // a coordinate of the type is not held exactly
+    unsigned lost = 0;  // values of the type that are not held exactly
+    __shared__ unsigned long long s_lost;
+    if (tid == 0) s_lost = 0ull;  // (every flush starts with a barrier)
     const int step = X.phases * M.skip;
     // loading: thread = (frame phase lf, atom la, axis lx)
     const int per_frame = 3 * X.atoms, lstep = FT / per_frame, lf = tid / per_frame,
@@ -222,6 +257,7 @@ __global__ void __launch_bounds__(FT, 2) k_msd_fixed(const MsdLaunch M, const Ms
         }
     };
     to_type_of(c0);
+    int shift = unit_shift(M, X, k);
     // the sums of the CTA's chunks of type k, every phase's, to their entry
     auto flush = [&]() {
         long long *out = X.partial + ((long long)(blockIdx.x + k) * M.leff + l0) * NACC;
@@ -238,14 +274,19 @@ __global__ void __launch_bounds__(FT, 2) k_msd_fixed(const MsdLaunch M, const Ms
             }
         }
         acc = Acc{};
-        const int any = __syncthreads_or(lost);
-        if (tid == 0) X.inexact[blockIdx.x + k] = any;
-        lost = false;
+        if (lost) atomicAdd(&s_lost, (unsigned long long)lost);
+        lost = 0;
+        __syncthreads();
+        if (tid == 0) {
+            X.lost[blockIdx.x + k] = (long long)s_lost;
+            s_lost = 0ull;
+        }
     };
     for (long long c = c0; c < c1; ++c) {
         if (c >= ke) {
             flush();
             to_type_of(c);
+            shift = unit_shift(M, X, k);
         }
         const int group = (int)((c - kb) / X.tiles),
                   tile = (int)((c - kb) - (long long)group * X.tiles);
@@ -260,13 +301,13 @@ __global__ void __launch_bounds__(FT, 2) k_msd_fixed(const MsdLaunch M, const Ms
             long long *out = smem + lx * PLANE + la * F;
 #pragma unroll 4
             for (int f = lf; f < nf; f += lstep) {
-                long long v = to_fixed(*x, X.shift, lost);
+                unsigned long long v = to_fixed(*x, shift, lost);
                 x += (long long)lstep * M.N * 3;
                 if (cm) {
-                    v -= to_fixed(*cm, X.shift, lost);
+                    v -= to_fixed(*cm, shift, lost);
                     cm += (long long)lstep * M.ntypes * 3;
                 }
-                out[f] = v;
+                out[f] = (long long)v;
             }
         }
         __syncthreads();
@@ -279,9 +320,9 @@ __global__ void __launch_bounds__(FT, 2) k_msd_fixed(const MsdLaunch M, const Ms
 #pragma unroll 2
                     for (; o < oe; o += X.phases, i += step) {
                         const int j = i + lag;
-                        add_square(acc, smem[j] - smem[i]);
-                        add_square(acc, smem[j + PLANE] - smem[i + PLANE]);
-                        add_square(acc, smem[j + 2 * PLANE] - smem[i + 2 * PLANE]);
+                        add_square(acc, minus(smem[j], smem[i]));
+                        add_square(acc, minus(smem[j + PLANE], smem[i + PLANE]));
+                        add_square(acc, minus(smem[j + 2 * PLANE], smem[i + 2 * PLANE]));
                     }
                     carry(acc);
                 }
@@ -321,7 +362,7 @@ __global__ void k_msd_fixed_final(const MsdLaunch M, const MsdFixed X, double *o
         return;
     }
     __int128 hi = 0, lo = 0;  // the sum is hi 2^64 + lo
-    bool inexact = false;
+    double lost = 0.0;
     long long kb = 0;
     for (int k = 0; k < c; ++k) kb += chunks_of(M, X, k);
     const long long ke = kb + chunks_of(M, X, c);
@@ -329,7 +370,7 @@ __global__ void k_msd_fixed_final(const MsdLaunch M, const MsdFixed X, double *o
         const long long b0 = kb / X.per, b1 = (ke - 1) / X.per;
         for (long long b = b0 + lane; b <= b1; b += 32) {
             const long long *v = X.partial + ((b + c) * M.leff + lag) * NACC;
-            inexact = inexact || X.inexact[b + c] != 0;
+            lost += (double)X.lost[b + c];
             // h h 2^58 + 2 h l 2^29 + l l, each sum high 2^32 + low
             hi += ((__int128)v[3] << 26) + (v[4] >> 2);
             lo += ((__int128)v[0] << 58) + ((__int128)v[1] << 30) + v[2] +
@@ -343,19 +384,75 @@ __global__ void k_msd_fixed_final(const MsdLaunch M, const MsdFixed X, double *o
                         l1 = __shfl_xor_sync(0xffffffffu, (long long)(lo >> 64), o);
         hi += ((__int128)h1 << 64) + h0;
         lo += ((__int128)l1 << 64) + l0;
+        lost += __shfl_xor_sync(0xffffffffu, lost, o);
     }
-    inexact = __any_sync(0xffffffffu, inexact);
     if (lane) return;
     hi += lo >> 64;
     const double sum = __dadd_rn(__dmul_rn(to_double(hi), 18446744073709551616.0),
                                  __ull2double_rn((unsigned long long)lo));
-    const double count = (double)M.n_orig * (double)(M.tbegin[c + 1] - M.tbegin[c]);
-    const double mean = __ddiv_rn(sum, count);
-    out[g] = scalbn(mean, -2 * X.shift);
-    // coordinates near zero beside large ones are held to half a unit: a
-    // displacement of d units rms has a relative error of 2 / d at most (and far
-    // less in the mean over many).  Below 2^42 units the caller takes the FP64 form.
-    if (inexact && lag > 0 && mean < 19342813113834066795298816.0) *X.suspect = 1ull;  // 2^84
+    const int na = M.tbegin[c + 1] - M.tbegin[c];
+    const double mean = __ddiv_rn(sum, (double)M.n_orig * (double)na);
+    out[g] = scalbn(mean, -2 * unit_shift(M, X, c));
+    if (lag > 0 && lost_shows(sum, lost, na, M.n_orig)) *X.suspect = 1ull;
+}
+
+// The largest extent of a component over the frames, per type of atom, from the
+// FP32 frames: of all `len` frames from `first` on, or (groups > 1) within each of
+// `groups` runs of `len` frames, `stride` apart.  ext: FP32 bits, rounded up; zero
+// before the first launch.  Thread = (four components, phase of the frames or
+// runs).  Bound by the read: 16384 atoms, 398 frames 78 MB.
+__global__ void __launch_bounds__(1024) k_extent(const float *__restrict__ pos32,
+                                                 const unsigned char *__restrict__ types8, int N,
+                                                 int NP, long long first, int groups, int len,
+                                                 int stride, unsigned *ext)
+{
+    __shared__ float4 s_mx[32][33], s_mn[32][33];
+    __shared__ unsigned s_ext[256];
+    const int lane = threadIdx.x & 31, phase = threadIdx.x >> 5;
+    if (threadIdx.x < 256) s_ext[threadIdx.x] = 0u;
+    const unsigned row = 3u * NP / 4u, c4 = blockIdx.x * 32 + lane;  // NP: a multiple of 16
+    const float4 *const src = reinterpret_cast<const float4 *>(pos32);
+    float4 mx = make_float4(-INFINITY, -INFINITY, -INFINITY, -INFINITY),
+           mn = make_float4(INFINITY, INFINITY, INFINITY, INFINITY);
+    auto take = [&](long long f) {
+        const float4 v = src[f * row + c4];
+        mx = make_float4(fmaxf(mx.x, v.x), fmaxf(mx.y, v.y), fmaxf(mx.z, v.z), fmaxf(mx.w, v.w));
+        mn = make_float4(fminf(mn.x, v.x), fminf(mn.y, v.y), fminf(mn.z, v.z), fminf(mn.w, v.w));
+    };
+    if (c4 < row && groups == 1) {
+#pragma unroll 4
+        for (int j = phase; j < len; j += 32) take(first + j);
+    } else if (c4 < row) {
+        float4 e = make_float4(-INFINITY, -INFINITY, -INFINITY, -INFINITY);
+        for (int g = phase; g < groups; g += 32) {
+            mx = make_float4(-INFINITY, -INFINITY, -INFINITY, -INFINITY);
+            mn = make_float4(INFINITY, INFINITY, INFINITY, INFINITY);
+#pragma unroll 4
+            for (int j = 0; j < len; ++j) take(first + (long long)g * stride + j);
+            e = make_float4(fmaxf(e.x, __fsub_ru(mx.x, mn.x)), fmaxf(e.y, __fsub_ru(mx.y, mn.y)),
+                            fmaxf(e.z, __fsub_ru(mx.z, mn.z)), fmaxf(e.w, __fsub_ru(mx.w, mn.w)));
+        }
+        mx = e;
+        mn = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    }
+    s_mx[phase][lane] = mx;
+    s_mn[phase][lane] = mn;
+    __syncthreads();
+    if (threadIdx.x < 128) {
+        const unsigned l = threadIdx.x >> 2, k = threadIdx.x & 3, at = blockIdx.x * 32 + l,
+                       atom = (4u * at + k) % (unsigned)NP;
+        float a = -INFINITY, b = INFINITY;
+        for (int p = 0; p < 32; ++p) {
+            a = fmaxf(a, reinterpret_cast<const float *>(&s_mx[p][l])[k]);
+            b = fminf(b, reinterpret_cast<const float *>(&s_mn[p][l])[k]);
+        }
+        const float v = __fsub_ru(a, b);
+        if (at < row && atom < (unsigned)N && v > 0.0f)
+            atomicMax(s_ext + types8[atom], __float_as_uint(v));
+    }
+    __syncthreads();
+    if (threadIdx.x < 256 && s_ext[threadIdx.x] > ext[threadIdx.x])
+        atomicMax(ext + threadIdx.x, s_ext[threadIdx.x]);
 }
 
 }  // namespace msd
@@ -372,6 +469,16 @@ int launch_msd(const MsdLaunch &M, double *out_device, int num_sms, cudaStream_t
     long long g2 = (nout + NT - 1) / NT;
     if (g2 > (long long)num_sms * 8) g2 = (long long)num_sms * 8;
     k_msd_final<<<(unsigned)g2, NT, 0, s>>>(M, out_device);
+    return cudaGetLastError() == cudaSuccess ? 0 : -1;
+}
+
+int launch_extent(const float *pos32, const unsigned char *types8, size_t N, long long first,
+                  int groups, int len, int stride, unsigned *ext, cudaStream_t s)
+{
+    const size_t NP = padded_natoms(N);
+    const unsigned blocks = (unsigned)((3 * NP / 4 + 31) / 32);
+    msd::k_extent<<<blocks, 1024, 0, s>>>(pos32, types8, (int)N, (int)NP, first, groups, len,
+                                          stride, ext);
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 

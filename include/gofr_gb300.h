@@ -420,11 +420,12 @@ int gofr_msd_output_size(const gofr_ctx *ctx, const gofr_msd_params *p, size_t *
  * result [leff][f_cm][ntypes] to out_host (double).  Element (t, 0, k) is the
  * mean over origins and atoms of type k of |x(o) - x(o+t)|^2 (optionally
  * minus the type's centre-of-mass displacement); (t, 1, k) the mean over
- * origins of the centre-of-mass |cm_k(o) - cm_k(o+t)|^2.  Each displacement is
- * formed from integers that hold the coordinates as finely as FP64 does, its
- * squares are summed exactly and rounded once (FP64 sums where the coordinates
- * or the window of lags do not allow it), where the reference keeps a running
- * mean: the two agree to the reference's rounding (relative ~1e-13 for 1e7
+ * origins of the centre-of-mass |cm_k(o) - cm_k(o+t)|^2.  Coordinates are held
+ * to 2^-58 of the largest displacement of their type or better, their squared
+ * displacements are summed exactly and rounded once, and the result is kept
+ * where what the coordinates lost moves it by at most 3.6e-15 (relative); FP64
+ * sums otherwise, and where the window of lags does not fit.  The reference
+ * keeps a running mean: the two agree to its rounding (relative ~1e-13 for 1e7
  * terms).  Errors as
  * lib/src/msd.cpp:57-68 (GOFR_ERR_RANGE: trajectory too short). */
 int gofr_msd_run(gofr_ctx *ctx, const gofr_msd_params *p, double *out_host);
