@@ -3435,8 +3435,9 @@ int gofr_msd_run(gofr_ctx *ctx, const gofr_msd_params *p, double *out_host)
     int rc = ensure(ctx, ctx->d_msd_partial, ctx->cap_msd_partial,
                     fixed ? msd_fixed_partial(M, X) : nout * n_orig);
     if (rc) return rc;
-    // the results, then the extents of this window (256 words)
-    rc = ensure(ctx, ctx->d_msd_out, ctx->cap_msd_out, nout + 128);
+    // the results, the extents of this window (256 words), the results over again (a
+    // word each)
+    rc = ensure(ctx, ctx->d_msd_out, ctx->cap_msd_out, nout + 128 + (nout + 1) / 2);
     if (rc) return rc;
     M.partial = ctx->d_msd_partial;
     if (fixed) {
@@ -3461,36 +3462,47 @@ int gofr_msd_run(gofr_ctx *ctx, const gofr_msd_params *p, double *out_host)
         }
         X.partial = reinterpret_cast<long long *>(ctx->d_msd_partial);
         X.lost = X.partial + msd_fixed_partial(M, X) - (X.grid + M.ntypes);
-        X.suspect = ctx->d_stats + ST_CANDIDATES;  // unused by this calculation
+        X.entries = reinterpret_cast<int *>(ctx->d_msd_out + nout + 128);
+        X.n_entries = ctx->d_stats + ST_CANDIDATES;  // unused by this calculation
+        X.n_terms = ctx->d_stats + ST_RECHECKS;
     }
-    for (bool exact = fixed;; exact = false) {
-        if (!exact) {
-            rc = ensure(ctx, ctx->d_msd_partial, ctx->cap_msd_partial, nout * n_orig);
-            if (rc) return rc;
-            M.partial = ctx->d_msd_partial;
-        }
-        CK(cudaEventRecord(ctx->ev[0], ctx->stream));
-        CK(clear_stats(ctx));
-        CK(cudaEventRecord(ctx->ev[1], ctx->stream));
+    CK(cudaEventRecord(ctx->ev[0], ctx->stream));
+    CK(clear_stats(ctx));
+    CK(cudaEventRecord(ctx->ev[1], ctx->stream));
+    ctx->launches += 2;
+    if (fixed ? launch_msd_fixed(M, X, ctx->d_msd_out, ctx->stream)
+              : launch_msd(M, ctx->d_msd_out, ctx->num_sms, ctx->stream))
+        return fail(ctx, GOFR_ERR_CUDA, "MSD kernel launch failed: %s",
+                    cudaGetErrorString(cudaGetLastError()));
+    // one squared displacement per (lag, origin, atom)
+    ctx->stats.pairs = (unsigned long long)leff * n_orig * t.N;
+    ctx->stats.evaluated = ctx->stats.pairs;
+    ctx->stats.kernel_used = -1;
+    auto finish = [&]() {
+        CK(cudaEventRecord(ctx->ev[2], ctx->stream));
+        CK(cudaMemcpyAsync(out_host, ctx->d_msd_out, nout * sizeof(double),
+                           cudaMemcpyDeviceToHost, ctx->stream));
+        CK(cudaEventRecord(ctx->ev[3], ctx->stream));
+        return gofr_sync(ctx);
+    };
+    rc = finish();
+    if (rc) return rc;
+    const int again = (int)ctx->stats.candidates;
+    if (again) {
+        // FP64 sums for the results in which lost bits could show
+        rc = ensure(ctx, ctx->d_msd_partial, ctx->cap_msd_partial, (size_t)again * n_orig);
+        if (rc) return rc;
+        M.partial = ctx->d_msd_partial;
         ctx->launches += 2;
-        if (exact ? launch_msd_fixed(M, X, ctx->d_msd_out, ctx->stream)
-                  : launch_msd(M, ctx->d_msd_out, ctx->num_sms, ctx->stream))
+        if (launch_msd_entries(M, X.entries, again, ctx->d_msd_out, ctx->num_sms, ctx->stream))
             return fail(ctx, GOFR_ERR_CUDA, "MSD kernel launch failed: %s",
                         cudaGetErrorString(cudaGetLastError()));
-        CK(cudaEventRecord(ctx->ev[2], ctx->stream));
-        CK(cudaMemcpyAsync(out_host, ctx->d_msd_out, nout * sizeof(double), cudaMemcpyDeviceToHost,
-                           ctx->stream));
-        CK(cudaEventRecord(ctx->ev[3], ctx->stream));
-        // one squared displacement per (lag, origin, atom)
-        ctx->stats.pairs = (unsigned long long)leff * n_orig * t.N;
-        ctx->stats.evaluated = ctx->stats.pairs;
-        ctx->stats.kernel_used = -1;
-        rc = gofr_sync(ctx);
+        rc = finish();
         if (rc) return rc;
-        const bool suspect = ctx->stats.candidates != 0;
-        ctx->stats.candidates = 0;
-        if (!suspect) return GOFR_OK;  // else the FP64 form over again
     }
+    ctx->stats.candidates = 0;
+    if (!fixed) ctx->stats.rechecks = ctx->stats.pairs;
+    return GOFR_OK;
 }
 
 int gofr_neigh_layout(const gofr_ctx *ctx_c, const gofr_neigh_spec *spec, unsigned nspec,

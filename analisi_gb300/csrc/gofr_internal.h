@@ -289,8 +289,13 @@ struct MsdFixed {
     double pad;                 // what the FP32 frames' rounding can add to an extent
     long long *partial;         // [grid + ntypes][leff][6]
     long long *lost;            // [grid + ntypes] values that are not held exactly
-    unsigned long long *suspect;  // set when that could show in a result
+    // results (lag ntypes + type) in which that could show, their number and terms
+    int *entries;
+    unsigned long long *n_entries, *n_terms;
 };
+// FP64 sums for n results (lag ntypes + type) alone; M.partial: [n][n_orig].
+int launch_msd_entries(const MsdLaunch &M, const int *entries, int n, double *out_device,
+                       int num_sms, cudaStream_t s);
 // Largest extent per type over `len` frames from `first` on, or within each of
 // `groups` runs of them; raises ext[256], FP32 bits.
 int launch_extent(const float *pos32, const unsigned char *types8, size_t N, long long first,

@@ -16,7 +16,8 @@
 // in 128 bits and rounded once per (lag, type): no term is rounded at all,
 // where the FP64 sums rounded every one.  Where coordinates lost bits and the
 // displacements of a (lag, type) are so small that the bound on the result's
-// error (lost_shows) exceeds the FP64 sums' own, the caller runs the FP64 form.
+// error (lost_shows) exceeds the FP64 sums' own, the caller has the FP64 sums
+// taken for that (lag, type) alone (k_msd_entries).
 // (With the unit taken from the largest coordinate instead, a tracer near the
 // origin of a box of 130 had an error of 5.5e-14 against the FP64 sums' 5.5e-16.)
 // A CTA holds the frames of a few atoms of one type in shared memory, so each
@@ -65,6 +66,40 @@ __device__ double block_sum(double v, double *red)
     return s;  // valid in thread 0
 }
 
+// Sum over the atoms of type k of their squared displacements between frames fo
+// and fl; valid in thread 0 (all threads of the CTA).
+__device__ __forceinline__ double type_sum(const MsdLaunch &M, long long fo, long long fl, int k,
+                                           double *red)
+{
+    const double *po = M.pos64 + (size_t)fo * M.N * 3;
+    const double *pl = M.pos64 + (size_t)fl * M.N * 3;
+    double cx = 0.0, cy = 0.0, cz = 0.0;
+    if (M.cm_self) {
+        const double *co = M.cm + ((size_t)fo * M.ntypes + k) * 3;
+        const double *cl = M.cm + ((size_t)fl * M.ntypes + k) * 3;
+        cx = __dsub_rn(co[0], cl[0]);
+        cy = __dsub_rn(co[1], cl[1]);
+        cz = __dsub_rn(co[2], cl[2]);
+    }
+    double acc = 0.0;
+    for (int q = M.tbegin[k] + threadIdx.x; q < M.tbegin[k + 1]; q += NT) {
+        const size_t a = (size_t)M.perm[q] * 3;
+        double dx = __dsub_rn(po[a], pl[a]);
+        double dy = __dsub_rn(po[a + 1], pl[a + 1]);
+        double dz = __dsub_rn(po[a + 2], pl[a + 2]);
+        if (M.cm_self) {
+            dx = __dsub_rn(dx, cx);
+            dy = __dsub_rn(dy, cy);
+            dz = __dsub_rn(dz, cz);
+        }
+        // the squares go straight into the sum (three FMAs instead of
+        // three products, two additions and one accumulation: the
+        // kernel is bound by the FP64 pipe)
+        acc = __fma_rn(dz, dz, __fma_rn(dy, dy, __fma_rn(dx, dx, acc)));
+    }
+    return block_sum(acc, red);
+}
+
 __global__ void __launch_bounds__(NT) k_msd_partial(const MsdLaunch M)
 {
     __shared__ double red[NT / 32];
@@ -75,35 +110,9 @@ __global__ void __launch_bounds__(NT) k_msd_partial(const MsdLaunch M)
         const int lag = (int)(item - (long long)o * M.leff);
         const long long fo = (long long)M.primo + (long long)o * M.skip;
         const long long fl = fo + lag;
-        const double *po = M.pos64 + (size_t)fo * M.N * 3;
-        const double *pl = M.pos64 + (size_t)fl * M.N * 3;
         double *out = M.partial + ((size_t)lag * M.n_orig + o) * fk;
         for (int k = 0; k < M.ntypes; ++k) {
-            double cx = 0.0, cy = 0.0, cz = 0.0;
-            if (M.cm_self) {
-                const double *co = M.cm + ((size_t)fo * M.ntypes + k) * 3;
-                const double *cl = M.cm + ((size_t)fl * M.ntypes + k) * 3;
-                cx = __dsub_rn(co[0], cl[0]);
-                cy = __dsub_rn(co[1], cl[1]);
-                cz = __dsub_rn(co[2], cl[2]);
-            }
-            double acc = 0.0;
-            for (int q = M.tbegin[k] + threadIdx.x; q < M.tbegin[k + 1]; q += NT) {
-                const size_t a = (size_t)M.perm[q] * 3;
-                double dx = __dsub_rn(po[a], pl[a]);
-                double dy = __dsub_rn(po[a + 1], pl[a + 1]);
-                double dz = __dsub_rn(po[a + 2], pl[a + 2]);
-                if (M.cm_self) {
-                    dx = __dsub_rn(dx, cx);
-                    dy = __dsub_rn(dy, cy);
-                    dz = __dsub_rn(dz, cz);
-                }
-                // the squares go straight into the sum (three FMAs instead of
-                // three products, two additions and one accumulation: the
-                // kernel is bound by the FP64 pipe)
-                acc = __fma_rn(dz, dz, __fma_rn(dy, dy, __fma_rn(dx, dx, acc)));
-            }
-            const double s = block_sum(acc, red);
+            const double s = type_sum(M, fo, fl, k, red);
             if (threadIdx.x == 0) out[k] = s;
         }
         if (M.cm_msd && threadIdx.x < M.ntypes) {
@@ -114,6 +123,32 @@ __global__ void __launch_bounds__(NT) k_msd_partial(const MsdLaunch M)
                 sq3(__dsub_rn(co[0], cl[0]), __dsub_rn(co[1], cl[1]), __dsub_rn(co[2], cl[2]));
         }
     }
+}
+
+// The same for the n results (lag ntypes + type) of `entries` alone: partial sums
+// [n][n_orig], then the results in their places.
+__global__ void __launch_bounds__(NT) k_msd_entries(const MsdLaunch M, const int *entries, int n)
+{
+    __shared__ double red[NT / 32];
+    const long long n_items = (long long)n * M.n_orig;
+    for (long long item = blockIdx.x; item < n_items; item += gridDim.x) {
+        const int at = entries[item / M.n_orig], o = (int)(item % M.n_orig);
+        const long long fo = (long long)M.primo + (long long)o * M.skip;
+        const double s = type_sum(M, fo, fo + at / M.ntypes, at % M.ntypes, red);
+        if (threadIdx.x == 0) M.partial[item] = s;
+    }
+}
+
+__global__ void k_msd_entries_final(const MsdLaunch M, const int *entries, int n, double *out)
+{
+    const int fk = M.cm_msd ? 2 * M.ntypes : M.ntypes;
+    const int g = blockIdx.x * blockDim.x + threadIdx.x;
+    if (g >= n) return;
+    const int k = entries[g] % M.ntypes;
+    double s = 0.0;
+    for (int o = 0; o < M.n_orig; ++o) s = __dadd_rn(s, M.partial[(size_t)g * M.n_orig + o]);
+    out[(size_t)(entries[g] / M.ntypes) * fk + k] =
+        __ddiv_rn(s, (double)M.n_orig * (double)(M.tbegin[k + 1] - M.tbegin[k]));
 }
 
 // out[lag][c][k] = sum over origins (in order) / count
@@ -393,7 +428,10 @@ __global__ void k_msd_fixed_final(const MsdLaunch M, const MsdFixed X, double *o
     const int na = M.tbegin[c + 1] - M.tbegin[c];
     const double mean = __ddiv_rn(sum, (double)M.n_orig * (double)na);
     out[g] = scalbn(mean, -2 * unit_shift(M, X, c));
-    if (lag > 0 && lost_shows(sum, lost, na, M.n_orig)) *X.suspect = 1ull;
+    if (lag > 0 && lost_shows(sum, lost, na, M.n_orig)) {
+        X.entries[atomicAdd(X.n_entries, 1ull)] = lag * M.ntypes + c;
+        atomicAdd(X.n_terms, (unsigned long long)M.n_orig * na);
+    }
 }
 
 // The largest extent of a component over the frames, per type of atom, from the
@@ -469,6 +507,17 @@ int launch_msd(const MsdLaunch &M, double *out_device, int num_sms, cudaStream_t
     long long g2 = (nout + NT - 1) / NT;
     if (g2 > (long long)num_sms * 8) g2 = (long long)num_sms * 8;
     k_msd_final<<<(unsigned)g2, NT, 0, s>>>(M, out_device);
+    return cudaGetLastError() == cudaSuccess ? 0 : -1;
+}
+
+int launch_msd_entries(const MsdLaunch &M, const int *entries, int n, double *out_device,
+                       int num_sms, cudaStream_t s)
+{
+    using namespace msd;
+    const long long items = (long long)n * M.n_orig;
+    const long long grid = items < num_sms * 16LL ? items : num_sms * 16LL;
+    k_msd_entries<<<(unsigned)grid, NT, 0, s>>>(M, entries, n);
+    k_msd_entries_final<<<(n + 127) / 128, 128, 0, s>>>(M, entries, n, out_device);
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 

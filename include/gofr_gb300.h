@@ -114,7 +114,8 @@ typedef struct gofr_stats {
     unsigned long long evaluated;    /* pairs whose distance was computed on the GPU */
     unsigned long long candidates;   /* FP32 pairs inside the accept window (+ its error bound;
                                         warp-streamed kernel: pairs counted) */
-    unsigned long long rechecks;     /* pairs recomputed in FP64 */
+    unsigned long long rechecks;     /* pairs recomputed in FP64 (MSD: displacements taken in
+                                        FP64 sums) */
     double kernel_ms;                /* device time of the pair kernel(s), CUDA events */
     double total_ms;                 /* device time of the whole run incl. copies */
     int kernel_used;                 /* enum gofr_kernel actually launched */

@@ -87,3 +87,18 @@ def test_held_still_and_other_scales(gpu_engine, scale):
     pos[:, 4:8] = pos[0, 4:8] * 2.0 ** -40
     pos[::2, 4:8] = np.nextafter(pos[::2, 4:8], 1.0)
     _check(gpu_engine, pos * scale, np.arange(12) // 4, 3, 2, 7, 20)
+
+
+def test_fp64_sums_only_where_lost_bits_could_show(gpu_engine):
+    """A type that oscillates by the last bit near zero is summed in FP64; the others,
+    one of which is at rest and one moves by 0.003 a step in a box of 200, are not
+    (the displacements summed in FP64 are in the statistics)."""
+    rng = np.random.default_rng(7)
+    pos = _walk(rng, 30, 40, 0.003) + rng.uniform(-100.0, 100.0, (1, 40, 3))
+    pos[:, :10] = pos[0, :10]
+    _check(gpu_engine, pos, np.arange(40) // 10, 4, 2, 7, 20)
+    assert gpu_engine.stats()["rechecks"] == 0
+    pos[:, 10:20] = pos[0, 10:20] * 2.0 ** -40
+    pos[::2, 10:20] = np.nextafter(pos[::2, 10:20], 1.0)
+    _check(gpu_engine, pos, np.arange(40) // 10, 4, 2, 7, 20)
+    assert gpu_engine.stats()["rechecks"] == 10 * 10 * 6  # its atoms, origins, lags 1 to 6
