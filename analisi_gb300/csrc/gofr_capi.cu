@@ -3447,12 +3447,15 @@ int gofr_msd_run(gofr_ctx *ctx, const gofr_msd_params *p, double *out_host)
         X.cm_ext = t.d_cm ? t.d_cm + t.T * t.ntypes * 3 : nullptr;
         X.ext = t.d_ext;
         const long long span = (long long)(n_orig - 1) * skip + leff;
-        if (skip >= 2 * leff || 4 * span < (long long)t.T) {
-            // few of the frames: the extents over this window (or within each origin's
-            // lags, where these lie apart) instead of over every frame
+        // An atom's extent grows with the frames it is taken over (a random walk's with
+        // their root: over 2000 frames no lag loses bits that show).  Of a longer
+        // trajectory, the extents of this window where it is a small part, or within
+        // each origin's lags where these lie apart.
+        constexpr long long few = 2048;
+        const bool apart = skip >= 2ll * leff || (skip > leff && span > few);
+        if ((long long)t.T > few && (apart || 4 * span < (long long)t.T)) {
             unsigned *const ext = reinterpret_cast<unsigned *>(ctx->d_msd_out + nout);
             CK(cudaMemsetAsync(ext, 0, 256 * sizeof(unsigned), ctx->stream));
-            const bool apart = skip >= 2 * leff;
             ++ctx->launches;
             if (launch_extent(t.pos32, t.types8, t.N, M.primo, apart ? (int)n_orig : 1,
                               apart ? (int)leff : (int)span, (int)skip, ext, ctx->stream))
@@ -3502,6 +3505,27 @@ int gofr_msd_run(gofr_ctx *ctx, const gofr_msd_params *p, double *out_host)
     }
     ctx->stats.candidates = 0;
     if (!fixed) ctx->stats.rechecks = ctx->stats.pairs;
+    return GOFR_OK;
+}
+
+int gofr_msd_plan_query(size_t natoms, unsigned leff, unsigned n_orig, unsigned skip, int num_sms,
+                        int *out)
+{
+    if (!out || natoms == 0 || natoms > (size_t)INT32_MAX / 2 || leff == 0 || n_orig == 0 ||
+        skip == 0 || leff > (unsigned)INT32_MAX || n_orig > (unsigned)INT32_MAX ||
+        skip > (unsigned)INT32_MAX || num_sms < 1)
+        return GOFR_ERR_ARG;
+    const int tbegin[2] = {0, (int)natoms};
+    MsdLaunch M{};
+    M.N = (int)natoms;
+    M.ntypes = 1;
+    M.leff = (int)leff;
+    M.n_orig = (int)n_orig;
+    M.skip = (int)skip;
+    MsdFixed X{};
+    if (!msd_fixed_plan(M, tbegin, num_sms, X)) return GOFR_ERR_UNSUPPORTED;
+    const int v[6] = {X.atoms, X.origins, X.tiles, X.frames, X.lags, X.phases};
+    std::copy(v, v + 6, out);
     return GOFR_OK;
 }
 

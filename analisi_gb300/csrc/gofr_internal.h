@@ -282,6 +282,7 @@ struct MsdFixed {
     int atoms, origins, tiles;  // atoms and origins of a chunk, tiles of origins
     int frames;                 // frames of a chunk (its row length in shared memory)
     int lags, phases, passes;   // lags and origin phases of a CTA's threads, CTAs per chunk range
+    int apart;                  // no frame is in the lags of two origins: phases of the atoms
     long long chunks, per;      // chunks, chunks per CTA
     int grid;
     const unsigned *ext;        // [256] largest extent per type, FP32 bits (launch_extent)

@@ -29,7 +29,8 @@
 // 5003 atoms with both centre-of-mass options, 60 x 80: 0.12 against 0.48.
 //
 // k_msd_partial: the FP64 form, for windows of lags whose frames of one atom
-// do not fit shared memory (more than about 4000 lags).  Every (origin, lag)
+// do not fit shared memory (more than about 4000 lags) and for origins too far
+// apart to share frames (msd_fixed_plan).  Every (origin, lag)
 // item is one CTA: it forms each atom's displacement with the reference's FP64
 // operations, adds its squared components into the type's sum with FMAs
 // (atoms visited in type-sorted order, one block reduction per type) and
@@ -37,6 +38,7 @@
 // origins of each (lag, type) in a fixed order and divides by the count.
 // Items are ordered origin-major so that consecutive CTAs share the origin
 // frame and slide the lagged frame, which keeps the frames they read in L2.
+#include <algorithm>
 #include <cstdint>
 #include <cuda_runtime.h>
 
@@ -267,13 +269,20 @@ __device__ __forceinline__ long long chunks_of(const MsdLaunch &M, const MsdFixe
 // CTA b takes chunks [b per, (b + 1) per) of the types' chunks back to back.  The sums of the CTA's
 // chunks of type k go to partial[b + k] (CTAs and types both ascend, so the
 // entry is one (CTA, type)'s own).
+// APART: no frame is in the lags of two origins.  A tile is then one origin, its
+// threads (lag, lane of the atoms), and a chunk takes as many atoms as fit, so that it
+// reads long pieces of each frame.  A call for 3000 atoms, 40 origins x 10 lags
+// every 500 frames: 79 us; 535 with the origins' phases on the threads and the
+// frames between the origins staged; 97 for the FP64 form.
+template <bool APART>
 __global__ void __launch_bounds__(FT, 2) k_msd_fixed(const MsdLaunch M, const MsdFixed X)
 {
     extern __shared__ __align__(16) long long smem[];
     const int tid = threadIdx.x, F = X.frames;
     const int l0 = blockIdx.y * X.lags, nl = min(X.lags, M.leff - l0);
-    const int lag = l0 + tid % X.lags, phase = tid / X.lags;
-    const bool busy = phase < X.phases && lag < l0 + nl;
+    const int lag = l0 + tid % X.lags, part = tid / X.lags;
+    const int phase = APART ? 0 : part, lane = APART ? part : 0;
+    const bool busy = part < X.phases && lag < l0 + nl;
     const long long c0 = (long long)blockIdx.x * X.per, c1 = min(c0 + X.per, X.chunks);
     Acc acc{};
     unsigned lost = 0;  // values of the type that are not held exactly
@@ -347,7 +356,7 @@ __global__ void __launch_bounds__(FT, 2) k_msd_fixed(const MsdLaunch M, const Ms
         }
         __syncthreads();
         if (busy) {
-            for (int a = 0; a < na; ++a) {
+            for (int a = lane; a < na; a += APART ? X.phases : 1) {
                 int i = a * F + phase * M.skip;
                 for (int o = phase; o < no;) {
                     // TERMS origins between two carries
@@ -438,7 +447,8 @@ __global__ void k_msd_fixed_final(const MsdLaunch M, const MsdFixed X, double *o
 // FP32 frames: of all `len` frames from `first` on, or (groups > 1) within each of
 // `groups` runs of `len` frames, `stride` apart.  ext: FP32 bits, rounded up; zero
 // before the first launch.  Thread = (four components, phase of the frames or
-// runs).  Bound by the read: 16384 atoms, 398 frames 78 MB.
+// runs); a block to a run (gridDim.y of them, groups = 1) where these are few or
+// long.  Bound by the read: 16384 atoms, 398 frames 78 MB.
 __global__ void __launch_bounds__(1024) k_extent(const float *__restrict__ pos32,
                                                  const unsigned char *__restrict__ types8, int N,
                                                  int NP, long long first, int groups, int len,
@@ -448,6 +458,7 @@ __global__ void __launch_bounds__(1024) k_extent(const float *__restrict__ pos32
     __shared__ unsigned s_ext[256];
     const int lane = threadIdx.x & 31, phase = threadIdx.x >> 5;
     if (threadIdx.x < 256) s_ext[threadIdx.x] = 0u;
+    first += (long long)blockIdx.y * stride;
     const unsigned row = 3u * NP / 4u, c4 = blockIdx.x * 32 + lane;  // NP: a multiple of 16
     const float4 *const src = reinterpret_cast<const float4 *>(pos32);
     float4 mx = make_float4(-INFINITY, -INFINITY, -INFINITY, -INFINITY),
@@ -526,8 +537,9 @@ int launch_extent(const float *pos32, const unsigned char *types8, size_t N, lon
 {
     const size_t NP = padded_natoms(N);
     const unsigned blocks = (unsigned)((3 * NP / 4 + 31) / 32);
-    msd::k_extent<<<blocks, 1024, 0, s>>>(pos32, types8, (int)N, (int)NP, first, groups, len,
-                                          stride, ext);
+    const unsigned runs = (groups < 32 || len >= 256) && groups < 65536 ? groups : 1;
+    msd::k_extent<<<dim3(blocks, runs), 1024, 0, s>>>(pos32, types8, (int)N, (int)NP, first,
+                                                      runs > 1 ? 1 : groups, len, stride, ext);
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
@@ -544,6 +556,19 @@ bool msd_fixed_plan(const MsdLaunch &M, const int *h_tbegin, int num_sms, MsdFix
     using namespace msd;
     const long long budget = PLANE;
     const long long all = (long long)(M.n_orig - 1) * M.skip + M.leff;
+    X.lags = M.leff < FT ? M.leff : FT;
+    X.passes = (M.leff + X.lags - 1) / X.lags;
+    X.apart = M.skip >= M.leff || M.n_orig == 1;
+    // Where a frame is in the lags of fewer than 1.6 origins, converting and staging it
+    // costs what the FP64 arithmetic of its one or two displacements does, and a CTA of
+    // long lags waits for its loads: FP64 sums, where their (origin, lag) items fill
+    // the GPU.  us a call, FP64 / integers: 3000 atoms, 200 x 50 every 50 frames 651 /
+    // 976, every 40 649 / 653, every 30 650 / 544; 16384 atoms, 6 x 200 every 300 416 /
+    // 482; 90 x 20 every 20 585 / 544; minus centres, 3000 atoms, 120 x 10 every 100
+    // 156 / 172.
+    if (8ll * M.skip > 5ll * M.leff && (M.leff >= 32 || M.cm_self) &&
+        (long long)M.n_orig * M.leff >= 4ll * num_sms)
+        return false;
     auto count = [&](int atoms, int tiles) {
         long long c = 0;
         for (int k = 0; k < M.ntypes; ++k)
@@ -551,24 +576,31 @@ bool msd_fixed_plan(const MsdLaunch &M, const int *h_tbegin, int num_sms, MsdFix
         return c;
     };
     X.atoms = 0;
-    for (int a = 16; a >= 1 && !X.atoms; a /= 2)  // every origin in one tile
-        if (all * a <= budget && (a <= 2 || count(a, 1) >= 16LL * num_sms)) X.atoms = a;
-    X.origins = M.n_orig;
-    for (int a = 8; a >= 1 && !X.atoms; a /= 2) {
-        // tiles of origins: each reads its lags' frames again, so three times
-        // as many frames as lags where more than one atom fits
-        const long long f = budget / a;
-        if (f < (a > 1 ? 3LL * M.leff : (long long)M.leff + M.skip)) continue;
-        X.atoms = a;
-        X.origins = (int)((f - M.leff) / M.skip + 1);
+    if (X.apart) {
+        // a thread per component when loading; two chunks per CTA or more
+        if (M.leff > budget) return false;
+        X.atoms = (int)std::min<long long>(FT / 3, budget / M.leff);
+        while (X.atoms > 8 && count(X.atoms, M.n_orig) < 4LL * num_sms) X.atoms /= 2;
+        X.origins = 1;
+        X.phases = std::min(FT / X.lags, X.atoms);
+    } else {
+        X.origins = M.n_orig;
+        for (int a = 16; a >= 1 && !X.atoms; a /= 2)  // every origin in one tile
+            if (all * a <= budget && (a <= 2 || count(a, 1) >= 16LL * num_sms)) X.atoms = a;
+        for (int a = 8; a >= 1 && !X.atoms; a /= 2) {
+            // tiles of origins: each reads its lags' frames again, so three times
+            // as many frames as lags where more than one atom fits
+            const long long f = budget / a;
+            if (f < (a > 1 ? 3LL * M.leff : (long long)M.leff + M.skip)) continue;
+            X.atoms = a;
+            X.origins = (int)((f - M.leff) / M.skip + 1);
+        }
+        if (!X.atoms) return false;
+        X.origins = X.origins < M.n_orig ? X.origins : M.n_orig;
+        X.phases = std::min(FT / X.lags, X.origins);
     }
-    if (!X.atoms) return false;
-    X.origins = X.origins < M.n_orig ? X.origins : M.n_orig;
     X.tiles = (M.n_orig + X.origins - 1) / X.origins;
     X.frames = (X.origins - 1) * M.skip + M.leff;
-    X.lags = M.leff < FT ? M.leff : FT;
-    X.passes = (M.leff + X.lags - 1) / X.lags;
-    X.phases = FT / X.lags < M.n_orig ? FT / X.lags : M.n_orig;
     X.chunks = count(X.atoms, X.tiles);
     // contiguous chunks per CTA, two CTAs per SM; no 64-bit sum of 2^17 squares
     // of three axes overflows
@@ -586,10 +618,11 @@ int launch_msd_fixed(const MsdLaunch &M, const MsdFixed &X, double *out_device, 
 {
     using namespace msd;
     const size_t smem = (size_t)3 * PLANE * 8;
-    if (cudaFuncSetAttribute(k_msd_fixed, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
+    auto kernel = X.apart ? k_msd_fixed<true> : k_msd_fixed<false>;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
         cudaSuccess)
         return -1;
-    k_msd_fixed<<<dim3((unsigned)X.grid, (unsigned)X.passes), FT, smem, s>>>(M, X);
+    kernel<<<dim3((unsigned)X.grid, (unsigned)X.passes), FT, smem, s>>>(M, X);
     const long long warps = (long long)M.leff * (M.cm_msd ? 2 : 1) * M.ntypes;
     k_msd_fixed_final<<<(unsigned)((warps + 7) / 8), 256, 0, s>>>(M, X, out_device);
     return cudaGetLastError() == cudaSuccess ? 0 : -1;

@@ -31,6 +31,7 @@ EXPORTED = [
     "gofr_msd_run", "gofr_neigh_layout", "gofr_neigh_run", "gofr_run_normalized",
     "gofr_run_streamed", "gofr_cellw_tables", "gofr_cellw_row",
     "gofr_plan_query", "gofr_radial_query", "gofr_allpairs_query",
+    "gofr_msd_plan_query",
 ]
 
 
@@ -162,6 +163,8 @@ def load_library(path=None):
                                     ctypes.POINTER(Params), dp]
     L.gofr_allpairs_query.argtypes = [ctypes.c_size_t, ctypes.c_uint, ctypes.c_double,
                                       ctypes.c_int, ctypes.POINTER(ctypes.c_longlong)]
+    L.gofr_msd_plan_query.argtypes = [ctypes.c_size_t, ctypes.c_uint, ctypes.c_uint,
+                                      ctypes.c_uint, ctypes.c_int, ip]
     L.gofr_batch_set.argtypes = [vp, ctypes.POINTER(TrajDesc), ctypes.c_uint]
     L.gofr_batch_output_layout.argtypes = [vp, ctypes.c_uint, ctypes.POINTER(ctypes.c_size_t),
                                            ctypes.POINTER(ctypes.c_size_t)]
@@ -189,7 +192,7 @@ def load_library(path=None):
                  "gofr_batch_run", "gofr_measure_peaks", "gofr_run_f64_noalloc",
                  "gofr_run_windows", "gofr_run_normalized", "gofr_run_streamed",
                  "gofr_cellw_tables", "gofr_cellw_row", "gofr_plan_query", "gofr_radial_query",
-                 "gofr_allpairs_query"):
+                 "gofr_allpairs_query", "gofr_msd_plan_query"):
         getattr(L, name).restype = ctypes.c_int
     if path is None:
         _lib = L
@@ -271,6 +274,20 @@ def allpairs_query(natoms, nparts, frames, num_sms=152):
     if rc != GOFR_OK:
         raise GofrError(rc, "invalid atoms, partitions, frames or multiprocessors")
     return dict(zip(("first", "groups", "chunks", "parts", "most"), [int(v) for v in out]))
+
+
+def msd_plan_query(natoms, lags, origins, skip, num_sms=152):
+    """How the integer sums of Engine.msd are laid out (host code, no GPU): a dict
+    {atoms, origins, tiles, frames, lags, phases}, None where FP64 sums run."""
+    L = load_library()
+    out = (ctypes.c_int * 6)()
+    rc = L.gofr_msd_plan_query(int(natoms), int(lags), int(origins), int(skip), int(num_sms), out)
+    if rc == -7:  # GOFR_ERR_UNSUPPORTED
+        return None
+    if rc != GOFR_OK:
+        raise GofrError(rc, "invalid atoms, lags, origins, skip or multiprocessors")
+    return dict(zip(("atoms", "origins", "tiles", "frames", "lags", "phases"),
+                    [int(v) for v in out]))
 
 
 def cellw_tables(box, triclinic, coord_min, coord_max, rmax, nc):

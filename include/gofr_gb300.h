@@ -431,6 +431,15 @@ int gofr_msd_output_size(const gofr_ctx *ctx, const gofr_msd_params *p, size_t *
  * lib/src/msd.cpp:57-68 (GOFR_ERR_RANGE: trajectory too short). */
 int gofr_msd_run(gofr_ctx *ctx, const gofr_msd_params *p, double *out_host);
 
+/* How the integer sums of gofr_msd_run are laid out for natoms atoms of one type,
+ * leff lags and n_orig origins `skip` frames apart on num_sms multiprocessors
+ * (host only, no reference counterpart): out (6 values): atoms and origins of a
+ * tile, tiles of origins, frames of a tile, lags and phases of its origins that
+ * the threads of a CTA are laid out for.  GOFR_ERR_UNSUPPORTED where the FP64
+ * sums run. */
+int gofr_msd_plan_query(size_t natoms, unsigned leff, unsigned n_orig, unsigned skip, int num_sms,
+                        int *out);
+
 /* ------------------------------------------------------------------------
  * Neighbour lists of one resident frame (the reference's Neighbours<T,double>,
  * lib/include/neighbour.h:9-104, lib/src/neighbour.cpp:9-97).
