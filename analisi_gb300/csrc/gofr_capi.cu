@@ -210,14 +210,14 @@ struct DevGuard {
 };
 
 template <typename T>
-int ensure(gofr_ctx *ctx, T *&p, size_t &cap, size_t n)
+int ensure(gofr_ctx *ctx, T *&p, size_t &cap, size_t n, const char *tag = nullptr)
 {
     if (n <= cap && p) return GOFR_OK;
     if (p) cudaFree(p);
     p = nullptr;
     cap = 0;
     size_t bytes = std::max<size_t>(n, 1) * sizeof(T);
-    CK(dev_malloc(&p, bytes));
+    CK(dev_malloc(&p, bytes, tag));
     cap = n;
     return GOFR_OK;
 }
@@ -3430,10 +3430,22 @@ int gofr_msd_run(gofr_ctx *ctx, const gofr_msd_params *p, double *out_host)
     }
     if (M.cm_self) bound = std::max(bound, t.cm_max);
     MsdFixed X{};
-    const bool fixed = bound < std::ldexp(1.0, 100) &&
-                       msd_fixed_plan(M, t.h_tbegin.data(), ctx->num_sms, X);
-    int rc = ensure(ctx, ctx->d_msd_partial, ctx->cap_msd_partial,
-                    fixed ? msd_fixed_partial(M, X) : nout * n_orig);
+    bool fixed = bound < std::ldexp(1.0, 100) &&
+                 msd_fixed_plan(M, t.h_tbegin.data(), ctx->num_sms, X);
+    int rc = GOFR_OK;
+    if (fixed) {
+        rc = ensure(ctx, ctx->d_msd_partial, ctx->cap_msd_partial, msd_fixed_partial(M, X),
+                    "msd_sums");
+        if (rc == GOFR_ERR_NOMEM) {
+            // the FP64 form's sums, one per (lag, origin, type), may fit
+            ctx->err.clear();
+            (void)cudaGetLastError();
+            fixed = false;
+        } else if (rc) {
+            return rc;
+        }
+    }
+    if (!fixed) rc = ensure(ctx, ctx->d_msd_partial, ctx->cap_msd_partial, nout * n_orig);
     if (rc) return rc;
     // the results, the extents of this window (256 words), the results over again (a
     // word each)
