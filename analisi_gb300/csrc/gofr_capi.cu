@@ -63,6 +63,9 @@ struct TrajDev {
     gofr_params params{};       // batch parameters
     size_t out_offset = 0, out_count = 0;
     bool box_constant = true;   // every frame has the same box
+    // cells per atom up to which the planner refines a grid in x, and takes one of
+    // several cells to the reach
+    double refine_cells = 2.0, reach_cells = 6.0;
     // cell lists (built on first use for a grid, kept while the frames stay)
     int cell_nc[3] = {0, 0, 0};
     int *d_cstart = nullptr;
@@ -172,19 +175,36 @@ int fail(gofr_ctx *ctx, int code, const char *fmt, ...)
                         "%s failed: %s", #call, cudaGetErrorString(e_));                     \
     } while (0)
 
+// Whether ANALISI_GB300_MAX_ALLOC leaves no room for an allocation (below).
+bool beyond_max_alloc(size_t bytes)
+{
+    static size_t first = 0;  // free when the variable was first seen
+    const char *m = std::getenv("ANALISI_GB300_MAX_ALLOC");
+    size_t now = 0, all = 0;
+    if (!m || cudaMemGetInfo(&now, &all) != cudaSuccess) return false;
+    if (!first) first = now;
+    return first + bytes > now + (size_t)std::atoll(m) * 1000000;
+}
+
 // Every device allocation of this file goes through here.  Fault-injection
 // hook for tests: with ANALISI_GB300_FAIL_ALLOC=1 in the environment every
 // allocation fails as if the device were out of memory, with
 // ANALISI_GB300_FAIL_ALLOC=<tag> only the allocations made with that tag
 // (e.g. "cells": the cell-sorted frames), so that the error paths and the
 // fallbacks can be run without a real shortage; they must leave the context
-// usable.  With ANALISI_GB300_FILL_ALLOC=<byte> every allocation is filled with
+// usable.  With ANALISI_GB300_MAX_ALLOC=<MB> those fail that would leave more than
+// that less of the device's memory free than the first one found.  With
+// ANALISI_GB300_FILL_ALLOC=<byte> every allocation is filled with
 // that byte, so that a test does not depend on what the memory held before.
 template <class T>
 cudaError_t dev_malloc(T **p, size_t bytes, const char *tag = nullptr)
 {
     const char *e = std::getenv("ANALISI_GB300_FAIL_ALLOC");
     if (e && (std::strcmp(e, "1") == 0 || (tag && std::strcmp(e, tag) == 0))) {
+        *p = nullptr;
+        return cudaErrorMemoryAllocation;
+    }
+    if (beyond_max_alloc(bytes)) {
         *p = nullptr;
         return cudaErrorMemoryAllocation;
     }
@@ -1293,6 +1313,7 @@ std::vector<CellwCand> cellw_candidates(const TrajDev &t, const gofr_params &p)
         CellwGeom g;
         if (!cell_grid(t, p, m, nc) || !cellw_geometry(t, p, nc, g)) continue;
         const double ncell = (double)nc[0] * nc[1] * nc[2];
+        if (m > 1 && ncell > t.reach_cells * (double)t.N + 64.0) continue;
         const double per_cell = (double)t.N / ncell;
         for (int wx = 1; wx <= 4; ++wx)
             for (int wy = 1; wy <= 4; ++wy)
@@ -1350,13 +1371,13 @@ bool cellw_choice(const TrajDev &t, const gofr_params &p, CellwCand &out)
 }
 
 // Cells per planner's cell in x: an eighth of the reach where the sorted frames
-// keep at most two cells per atom (a row's ends then follow the sphere to an
-// eighth of rmax: 8 % fewer pairs than whole cells at reach 2).
+// keep at most t.refine_cells, two cells per atom (a row's ends then follow the
+// sphere to an eighth of rmax: 8 % fewer pairs than whole cells at reach 2).
 int cellw_refine(const TrajDev &t, const CellwCand &c)
 {
     int fx = 1;
     while (c.reach * fx * 2 <= 8 && c.nc[0] * fx * 2 <= 1024 &&
-           (double)c.nc[0] * c.nc[1] * c.nc[2] * fx * 2 <= 2.0 * (double)t.N)
+           (double)c.nc[0] * c.nc[1] * c.nc[2] * fx * 2 <= t.refine_cells * (double)t.N)
         fx *= 2;
     return fx;
 }
@@ -2949,10 +2970,15 @@ int gofr_run_normalized(gofr_ctx *ctx, const gofr_params *p, unsigned nwin,
 }
 
 // Device bytes one frame of natoms takes in a run: FP64 positions, FP32
-// frames, the cell-sorted records and starts, with room for the boxes.
+// frames, the cell-sorted records, each atom's cell and rank while they are built,
+// starts and counts of half a cell per atom (which a grid of one cell to the reach
+// stays below from an rmax of 1.3 interatomic distances on), with room for the
+// boxes.
+constexpr double kStreamedCells = 0.5;
 static size_t frame_device_bytes(size_t natoms)
 {
-    return padded_natoms(natoms) * (3 * 8 + 3 * 4 + 16 + 4 + 8) + 512;
+    return padded_natoms(natoms) * (3 * 8 + 3 * 4 + 16 + 2 * 4 + (size_t)(kStreamedCells * 8)) +
+           512;
 }
 
 int gofr_run_streamed(gofr_ctx *ctx, const double *positions, const double *boxes, int box_kind,
@@ -3002,6 +3028,7 @@ int gofr_run_streamed(gofr_ctx *ctx, const double *positions, const double *boxe
             rc = upload_traj(ctx, ctx->trajs[0], positions + f0 * natoms * 3, boxes + f0 * stride,
                              box_kind, type_ids, ntypes, natoms, f1 - f0);
             if (rc) return rc;
+            ctx->trajs[0].refine_cells = ctx->trajs[0].reach_cells = kStreamedCells;
             const TrajDev &t = ctx->trajs[0];
             // this chunk: origins 0, skip, ... of the uploaded frames, every lag
             gofr_params q = *p;
