@@ -147,8 +147,10 @@ struct WarpState {
 
 // One unit: first atoms [i0, i1) (at most FA) of frame fo against part jp of
 // the atoms of frame fl (jc chunks), into the histogram at whist (rows of
-// nbin + 1 cells).  All lanes of the warp call it.
-template <bool TRI, bool WCHK, int MODE>
+// nbin + 1 cells).  All lanes of the warp call it.  FAR: 64 pairs of a first
+// atom that all lie beyond P.far2 are not binned (they end in the unread cell), for
+// jobs in which few pairs are within rmax (gofr_capi.cu, far_limit).
+template <bool TRI, bool WCHK, int MODE, bool FAR = false>
 __device__ __forceinline__ void unit(const PairLaunch &P, WarpArea &A, unsigned *whist,
                                      const unsigned short *chtab, long long fo, long long fl,
                                      int i0, int i1, int jp, WarpState &ws)
@@ -313,6 +315,17 @@ __device__ __forceinline__ void unit(const PairLaunch &P, WarpArea &A, unsigned 
                                                       f2sub(uz, za), bx, P.wlim, wa0, wa1);
                     const f2 db = image_d2<TRI, WCHK>(f2sub(u0.x, xb), f2sub(u0.y, yb),
                                                       f2sub(uz, zb), bx, P.wlim, wb0, wb1);
+                    if (FAR) {
+                        float d0, d1, d2, d3;
+                        f2up(da, d0, d1);
+                        f2up(db, d2, d3);
+                        if (__any_sync(0xffffffffu, fminf(d0, d1) <= P.far2))
+                            bin_pair2<MODE>(da, inv, off, P.rm, row[0], row[1], bit, mk[0], mk[1]);
+                        if (__any_sync(0xffffffffu, fminf(d2, d3) <= P.far2))
+                            bin_pair2<MODE>(db, inv, off, P.rm, row[2], row[3], bit, mk[2], mk[3]);
+                        bit <<= 1;
+                        continue;
+                    }
                     bin_pair2<MODE>(da, inv, off, P.rm, row[0], row[1], bit, mk[0], mk[1]);
                     bin_pair2<MODE>(db, inv, off, P.rm, row[2], row[3], bit, mk[2], mk[3]);
                     if (WCHK) {
@@ -393,7 +406,7 @@ __device__ __forceinline__ void add_stats(unsigned long long *stats, unsigned lo
 // atoms, part of the second atoms), the part fastest, dealt in chunks of
 // decreasing size (chunk_range); the histogram is flushed when the window,
 // partition or lag changes.
-template <bool TRI, bool WCHK, int MODE>
+template <bool TRI, bool WCHK, int MODE, bool FAR>
 __global__ void __launch_bounds__(NT, 4) k_allpairs(const PairLaunch P)
 {
     extern __shared__ __align__(128) unsigned char smem[];
@@ -473,8 +486,8 @@ __global__ void __launch_bounds__(NT, 4) k_allpairs(const PairLaunch P)
                     atomicAdd(&s_pairs, (unsigned long long)(i1 - i0) *
                                             (unsigned long long)min(P.N, P.jc * CH));
                 const long long fo = first + (long long)k * P.skip;
-                unit<TRI, WCHK, MODE>(P, A, hist + 1, chtab, fo,
-                                      fo + (long long)lag_idx * P.every, i0, i1, jp, ws);
+                unit<TRI, WCHK, MODE, FAR>(P, A, hist + 1, chtab, fo,
+                                           fo + (long long)lag_idx * P.every, i0, i1, jp, ws);
                 __syncwarp();  // every lane done with the first atoms
             }
             g0 = g1;
@@ -592,26 +605,26 @@ int grid_of(K kernel, size_t smem, int num_sms, long long blocks, int *grid)
     return 0;
 }
 
-template <bool TRI, bool WCHK, int MODE>
+template <bool TRI, bool WCHK, int MODE, bool FAR>
 int launch(const PairLaunch &P, int num_sms, cudaStream_t s)
 {
     const size_t smem = smem_bytes(P.nch * (P.nbin + 1) + 1, P.ntypes);
     const long long units = (long long)P.nwin * P.nparts * P.n_lags * P.n_orig * P.ng * P.nj;
     int grid = 0;
-    const int rc = grid_of(k_allpairs<TRI, WCHK, MODE>, smem, num_sms, (units + NWARP - 1) / NWARP,
-                           &grid);
+    const int rc = grid_of(k_allpairs<TRI, WCHK, MODE, FAR>, smem, num_sms,
+                           (units + NWARP - 1) / NWARP, &grid);
     if (rc) return rc;
-    k_allpairs<TRI, WCHK, MODE><<<(unsigned)grid, NT, smem, s>>>(P);
+    k_allpairs<TRI, WCHK, MODE, FAR><<<(unsigned)grid, NT, smem, s>>>(P);
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
-template <bool TRI, bool WCHK>
+template <bool TRI, bool WCHK, bool FAR>
 int launch_mode(const PairLaunch &P, int num_sms, cudaStream_t s)
 {
     switch (P.rm.mode) {
-    case 0: return launch<TRI, WCHK, 0>(P, num_sms, s);
-    case 1: return launch<TRI, WCHK, 1>(P, num_sms, s);
-    default: return launch<TRI, WCHK, 2>(P, num_sms, s);
+    case 0: return launch<TRI, WCHK, 0, FAR>(P, num_sms, s);
+    case 1: return launch<TRI, WCHK, 1, FAR>(P, num_sms, s);
+    default: return launch<TRI, WCHK, 2, FAR>(P, num_sms, s);
     }
 }
 
@@ -626,11 +639,14 @@ int launch_allpairs(const PairLaunch &P, bool wrapcheck, int num_sms, cudaStream
 {
     using namespace allpairs;
     if (P.n_lags <= 0 || P.n_orig <= 0 || P.ng <= 0) return 0;
-    if (P.tric)
-        return wrapcheck ? launch_mode<true, true>(P, num_sms, s)
-                         : launch_mode<true, false>(P, num_sms, s);
-    return wrapcheck ? launch_mode<false, true>(P, num_sms, s)
-                     : launch_mode<false, false>(P, num_sms, s);
+    if (wrapcheck)
+        return P.tric ? launch_mode<true, true, false>(P, num_sms, s)
+                      : launch_mode<false, true, false>(P, num_sms, s);
+    if (P.far2 < INFINITY)
+        return P.tric ? launch_mode<true, false, true>(P, num_sms, s)
+                      : launch_mode<false, false, true>(P, num_sms, s);
+    return P.tric ? launch_mode<true, false, false>(P, num_sms, s)
+                  : launch_mode<false, false, false>(P, num_sms, s);
 }
 
 // The batch's bin map is mode 0's when every member's is, else the general one.

@@ -88,6 +88,8 @@ struct PairLaunch {
     int gs, ng;               // first atoms per unit, groups of them per partition
     int jc, nj;               // chunks of second atoms per unit, parts of the frame they make
     long long most;           // units of a CTA's chunk at most
+    float far2;               // FP32 d2 from which a pair is certainly beyond the bins (infinite:
+                              // not looked for)
     unsigned *queue;          // {next chunk, CTAs done}, zero before and after a launch
     int n_lags, every;        // lags t = l*every, l < n_lags
     int n_orig, skip;         // origins primo + k*skip, k < n_orig
