@@ -78,6 +78,7 @@ struct TrajDev {
     double *d_cm = nullptr;          // [T][ntypes][3], then the extent per type [ntypes]
     double cm_max = 0.0;             // largest |component| of them
     unsigned *d_ext = nullptr;       // [256] largest extent per type over every frame (FP32 bits)
+    bool ext_ready = false;
 };
 
 }  // namespace
@@ -260,6 +261,7 @@ void free_traj(TrajDev &t)
     cudaFree(t.d_cm);
     cudaFree(t.d_ext);
     t.d_perm = nullptr; t.d_tbegin = nullptr; t.d_cm = nullptr; t.d_ext = nullptr;
+    t.ext_ready = false;
     t.pos64 = nullptr; t.pos32 = nullptr; t.box64 = nullptr; t.box32 = nullptr; t.types = nullptr;
     t.types8 = nullptr;
     t.d_cstart = nullptr; t.d_sidt = nullptr; t.d_spos = nullptr;
@@ -983,6 +985,7 @@ int upload_traj(gofr_ctx *ctx, TrajDev &t, const double *positions, const double
     CK(dev_malloc(&t.box64, nframes * 9 * sizeof(double)));
     CK(dev_malloc(&t.box32, nframes * sizeof(Box32)));
     CK(dev_malloc(&t.types, natoms * sizeof(int)));
+    CK(dev_malloc(&t.d_ext, 256 * sizeof(unsigned)));
     CK(cudaMemcpyAsync(t.pos64, positions, n3 * sizeof(double), cudaMemcpyHostToDevice,
                        ctx->stream));
     ctx->h2d_bytes += n3 * sizeof(double) + nframes * (9 * sizeof(double) + sizeof(Box32)) +
@@ -1038,13 +1041,21 @@ int upload_traj(gofr_ctx *ctx, TrajDev &t, const double *positions, const double
                        t.pos32, t.types8, ctx->stream))
         return fail(ctx, GOFR_ERR_CUDA, "convert kernel launch failed: %s",
                     cudaGetErrorString(cudaGetLastError()));
-    CK(dev_malloc(&t.d_ext, 256 * sizeof(unsigned)));
+    CK(cudaStreamSynchronize(ctx->stream));
+    return GOFR_OK;
+}
+
+// The largest extents per type over every frame, taken by the first calculation
+// that asks for them after an upload.
+int ensure_extent(gofr_ctx *ctx, const TrajDev &t)
+{
+    if (t.ext_ready) return GOFR_OK;
     CK(cudaMemsetAsync(t.d_ext, 0, 256 * sizeof(unsigned), ctx->stream));
     ++ctx->launches;
-    if (launch_extent(t.pos32, t.types8, natoms, 0, 1, (int)nframes, 0, t.d_ext, ctx->stream))
+    if (launch_extent(t.pos32, t.types8, t.N, 0, 1, (int)t.T, 0, t.d_ext, ctx->stream))
         return fail(ctx, GOFR_ERR_CUDA, "extent kernel launch failed: %s",
                     cudaGetErrorString(cudaGetLastError()));
-    CK(cudaStreamSynchronize(ctx->stream));
+    const_cast<TrajDev &>(t).ext_ready = true;
     return GOFR_OK;
 }
 
@@ -3477,6 +3488,14 @@ int gofr_msd_run(gofr_ctx *ctx, const gofr_msd_params *p, double *out_host)
     MsdFixed X{};
     bool fixed = bound < std::ldexp(1.0, 100) &&
                  msd_fixed_plan(M, t.h_tbegin.data(), ctx->num_sms, X);
+    // An atom's extent grows with the frames it is taken over (a random walk's with
+    // their root: over 2000 frames no lag loses bits that show).  Of a longer
+    // trajectory, the extents of this window where it is a small part, or within
+    // each origin's lags where these lie apart.
+    constexpr long long few = 2048;
+    const long long span = (long long)(n_orig - 1) * skip + leff;
+    const bool apart = skip >= 2ll * leff || (skip > leff && span > few);
+    const bool window = (long long)t.T > few && (apart || 4 * span < (long long)t.T);
     int rc = GOFR_OK;
     if (fixed) {
         rc = ensure(ctx, ctx->d_msd_partial, ctx->cap_msd_partial, msd_fixed_partial(M, X),
@@ -3497,20 +3516,19 @@ int gofr_msd_run(gofr_ctx *ctx, const gofr_msd_params *p, double *out_host)
     rc = ensure(ctx, ctx->d_msd_out, ctx->cap_msd_out, nout + 128 + (nout + 1) / 2);
     if (rc) return rc;
     M.partial = ctx->d_msd_partial;
+    CK(cudaEventRecord(ctx->ev[0], ctx->stream));
+    CK(clear_stats(ctx));
+    CK(cudaEventRecord(ctx->ev[1], ctx->stream));
     if (fixed) {
         // the FP32 frames: (|x - c| + 2^-150) 2^-24 and the rounding of x - c, at both ends
         X.pad = 2.0 * (eps * std::ldexp(1.0, -24) * (1.0 + std::ldexp(1.0, -20)) +
                        eps * std::ldexp(1.0, -52)) + std::ldexp(1.0, -148);
         X.cm_ext = t.d_cm ? t.d_cm + t.T * t.ntypes * 3 : nullptr;
         X.ext = t.d_ext;
-        const long long span = (long long)(n_orig - 1) * skip + leff;
-        // An atom's extent grows with the frames it is taken over (a random walk's with
-        // their root: over 2000 frames no lag loses bits that show).  Of a longer
-        // trajectory, the extents of this window where it is a small part, or within
-        // each origin's lags where these lie apart.
-        constexpr long long few = 2048;
-        const bool apart = skip >= 2ll * leff || (skip > leff && span > few);
-        if ((long long)t.T > few && (apart || 4 * span < (long long)t.T)) {
+        if (!window) {
+            rc = ensure_extent(ctx, t);
+            if (rc) return rc;
+        } else {
             unsigned *const ext = reinterpret_cast<unsigned *>(ctx->d_msd_out + nout);
             CK(cudaMemsetAsync(ext, 0, 256 * sizeof(unsigned), ctx->stream));
             ++ctx->launches;
@@ -3526,9 +3544,6 @@ int gofr_msd_run(gofr_ctx *ctx, const gofr_msd_params *p, double *out_host)
         X.n_entries = ctx->d_stats + ST_CANDIDATES;  // unused by this calculation
         X.n_terms = ctx->d_stats + ST_RECHECKS;
     }
-    CK(cudaEventRecord(ctx->ev[0], ctx->stream));
-    CK(clear_stats(ctx));
-    CK(cudaEventRecord(ctx->ev[1], ctx->stream));
     ctx->launches += 2;
     if (fixed ? launch_msd_fixed(M, X, ctx->d_msd_out, ctx->stream)
               : launch_msd(M, ctx->d_msd_out, ctx->num_sms, ctx->stream))
