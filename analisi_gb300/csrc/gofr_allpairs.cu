@@ -24,15 +24,17 @@
 //
 // Bound by instruction issue (77 % of the slots used, the FMA pipe 56 %, the
 // ALU 50 %, the shared-memory pipe 46 %): 80 instructions for a first atom
-// against a chunk, 94 with the loads and the pairs near an edge.  2187 atoms to
+// against a chunk, 94 with the loads and the pairs near an edge (fewer where FAR
+// leaves most pairs out).  2187 atoms to
 // 13.5 A in a box of 28 A (47 % of the pairs counted), 40 origins x 50 lags: 7.6
 // ms = 1260 Gpairs/s, where the form with tiles of 1024 atoms staged by bulk
 // copies and per-thread candidate slots binned by the warp took 26.1; with the
 // rounded quotient of the triclinic form 8.2.  5488 atoms to 9 A in four
 // partitions, 20 x 40: 18.3 ms against 32.7; 1000 atoms to 3.5 A (1.7 %
 // counted), 18 x 20: 0.32 against 0.44; 300 atoms, 6 x 6: 23 us against 78.  64
-// registers (spilling 60 bytes outside the loops): with 80 and three CTAs per
-// SM within 2 %.
+// registers, spilling outside the loops (bytes stored / loaded: 90 / 104, triclinic
+// 130 / 140, FAR 102 / 116 and 158 / 176, batch 220 / 424 and 276 / 640): with 80 and
+// three CTAs per SM within 2 %.
 #include <cstdint>
 #include <cuda_runtime.h>
 

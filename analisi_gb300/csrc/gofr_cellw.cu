@@ -77,10 +77,11 @@
 // Bound by instruction issue: 71 instructions per 128 pairs (46 of them the
 // pairs' own), 77 % of the issue slots used, the shared-memory pipe 57 %
 // busy, the FP32 pipe 59 %, no DRAM traffic to speak of.  16384 atoms, 25
-// origins x 100 lags (16 % of N^2 evaluated, 28 % of those within rmax): 59.7
+// origins x 100 lags (16 % of N^2 evaluated, 28 % of those within rmax): 59.5
 // ms, where the form that queued its candidates and binned the queue took
-// 178.9; 131072 atoms, 5 x 10: 7.6 ms against 21.7; 32768 atoms, triclinic,
-// 10 x 20: 17.3 ms against 59.8.  64 registers, 32 warps per SM (two CTAs of
+// 178.9; 131072 atoms, 5 x 10: 7.7 ms against 21.7; 32768 atoms, triclinic,
+// 10 x 20: 17.5 ms against 59.8.  64 registers (spilling 290 to 298 bytes stored, 472
+// to 508 loaded, outside the loop over first atoms), 32 warps per SM (two CTAs of
 // 16, one of 32 for a large histogram): with 128 registers and 16 warps 74.9 ms.
 #include <cstdint>
 #include <cuda_runtime.h>

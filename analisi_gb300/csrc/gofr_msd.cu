@@ -25,7 +25,7 @@
 // shared memory: thread = (lag, phase of the origins), consecutive lags reading
 // consecutive frames.
 //   Bound by the 32-bit integer multiplier.  16384 atoms in
-// three types, 100 origins x 100 lags: 0.46 ms against 2.79 for the FP64 form;
+// three types, 100 origins x 100 lags: 0.45 ms against 2.79 for the FP64 form;
 // 5003 atoms with both centre-of-mass options, 60 x 80: 0.12 against 0.48.
 //
 // k_msd_partial: the FP64 form, for windows of lags whose frames of one atom

@@ -399,7 +399,7 @@ def bench_msd(eng, w, p, reps=3):
     return {"workload": "c2 frames: reset(1800), tmax=200, skip=4, both centre-of-mass options",
             "displacements": disp, "ms": round(sum(ms) / len(ms), 3),
             "value": round(rate, 2), "unit": "G squared displacements/s",
-            "fp64_ops_per_displacement": 9,
+            "integer_multiply_adds_per_displacement": 9,
             "max_rel_diff_vs_oracle_sample": rel,
             "cpu_oracle_1thread": {"value": round(cpu_rate, 4), "unit": "G squared displacements/s",
                                    "sample": "20 lags x 10 origins", "seconds": round(dt, 3)}}

@@ -113,7 +113,8 @@ typedef struct gofr_stats {
     unsigned long long pairs;        /* ordered pairs of the reference loop (N^2 per lag/origin) */
     unsigned long long evaluated;    /* pairs whose distance was computed on the GPU */
     unsigned long long candidates;   /* FP32 pairs inside the accept window (+ its error bound;
-                                        warp-streamed kernel: pairs counted) */
+                                        warp-streamed and all-pairs kernels, batch:
+                                        pairs counted) */
     unsigned long long rechecks;     /* pairs recomputed in FP64 (MSD: displacements taken in
                                         FP64 sums) */
     double kernel_ms;                /* device time of the pair kernel(s), CUDA events */
